@@ -15,6 +15,7 @@
 // B is the weight tensor packed as [Cout][tap][Cin] (K-major), one 2-D TMA tile per k-block.
 #pragma once
 #include <cuda.h>
+#include <type_traits>
 #include "common.cuh"
 
 namespace msnh {
@@ -38,6 +39,14 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// True in exactly one lane of a converged warp. The single-thread roles of the kernel run under this predicate and not under
+// `lane == 0`: a TMA or tcgen05 instruction takes its operands from the warp's uniform registers, and only elect.sync tells
+// the compiler that a single lane is active.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one != 0;
 }
 // One poll of a barrier phase.
 __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity) {
@@ -338,8 +347,13 @@ __device__ __forceinline__ void activate_pairs(F2 (&y)[8], int act, float param)
 // Dynamic shared memory: [stages x A tile][stages x B tile][2 output staging slabs] (1024-byte
 // aligned), then barriers.
 // The accumulators form a ring of 2-8 TMEM stages, so the MMA warp runs several tiles ahead of the
-// drain. The two epilogue groups (4 warps each) either split the store slabs of every tile between
-// them (kSplit: a tile has at least two slabs, so its drain latency halves) or take alternate tiles.
+// drain.
+// What bounds the main loop: each of its three single-thread roles (loads of A, loads of B, MMA) takes some 300 cycles of
+// dependent instructions per k-block, an MMA of 128 pixels 66 cycles up to 128 channels and 130 at 256 (the tensor pipe's
+// own rate there), the loads about 80 bytes per cycle. With one thread loading both operands under `lane == 0` a k-block took
+// 616 cycles whatever the tile up to 256 channels; with elect.sync 470; with a role per operand and straight-line MMA
+// issue 330 (128 channels) and 520 (256). 3x3 512->512 at 19x19, 8 images: 37 -> 24.6 us; a step of YOLOv4-608 at 8 images
+// 2.06 -> 1.92 ms, at one image 1.12 -> 0.84 ms.
 // ---------------------------------------------------------------------------------------------
 // kPair: the kernel runs as clusters of two CTAs that share tiles of 256 pixels x bn channels through
 // cta_group::2 MMAs: each CTA stages its own 128 pixels of A and its half of the weight tile (so the
@@ -353,7 +367,7 @@ __device__ __forceinline__ void activate_pairs(F2 (&y)[8], int act, float param)
 // kAct: MSNH_ACT_MISH / MSNH_ACT_LEAKY (slope in [0, 1]) compile the first activation into the epilogue loops, kActGeneric
 // switches at run time. kTrace: the instantiation that records clock stamps (plans made with MSNH_PLAN_TRACE); the
 // production instantiations carry none of that code.
-template <typename T, int kMult, bool kSplit, bool kPair, bool kStreamK, int kAct = kActGeneric, bool kTrace = false>   // kMult: 128-pixel sub-tiles per tile (1, 2, 3, 4)
+template <typename T, int kMult, bool kPair, bool kStreamK, int kAct = kActGeneric, bool kTrace = false>   // kMult: 128-pixel sub-tiles per tile (1, 2, 3, 4)
 __global__ void __launch_bounds__(kUmmaThreads, 1)
 conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_c2, const ConvUmmaParams p) {
@@ -393,7 +407,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     long long *trace = nullptr;
     if constexpr (kTrace) {
         trace = p.trace ? p.trace + static_cast<size_t>(blockIdx.x) * kTraceSlots : nullptr;
-        if (trace && threadIdx.x == 0) { trace[0] = clock64(); long long g; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g)); trace[3] = g; }
+        if (trace && threadIdx.x == 0) { trace[0] = clock64(); long long g; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g)); trace[3] = g; uint32_t sm; asm volatile("mov.u32 %0, %%smid;" : "=r"(sm)); trace[5] = sm; }
     }
     const int num_tiles   = p.tiles_m * p.tiles_n;
     const int num_k_iters = p.taps * p.chunks_per_tap;
@@ -428,16 +442,16 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c) : "memory");
         if (p.split_n != 0x7fffffff) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c2) : "memory");
         cta_abort_slot = 0;
-        for (int s = 0; s < p.num_stages; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
+        for (int s = 0; s < p.num_stages; ++s) { mbar_init(full_bar(s), 2); mbar_init(empty_bar(s), 1); }
         // arrivals that free an accumulator: the team epilogue's warps (pair / stream-K kernels), or one per warp and
         // store unit of a tile (plain kernels: four warps x sub-tiles x slabs)
         const int units = kMult * ((p.bn * static_cast<int>(sizeof(T)) + p.out_chunk_bytes - 1) / p.out_chunk_bytes);
-        const uint32_t acc_arrivals = (kPair || kStreamK) ? (kSplit ? 16u : 8u) * (kPair ? 2u : 1u) : 4u * static_cast<uint32_t>(units);
+        const uint32_t acc_arrivals = (kPair || kStreamK) ? 16u * (kPair ? 2u : 1u) : 4u * static_cast<uint32_t>(units);
         for (int s = 0; s <= acc_mask; ++s) { mbar_init(acc_full_bar(s), 1); mbar_init(acc_empty_bar(s), acc_arrivals); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (sb_staged && threadIdx.x >= 64) {   // constants: no need to wait for the previous kernel
+    if (sb_staged && threadIdx.x >= 64 && threadIdx.x < 576) {   // constants: no need to wait for the previous kernel
         const int t = threadIdx.x - 64;      // 256 float4 of scale, then 256 of bias
         const float *src = (t < 256 ? p.scale : p.bias) + 4 * (t & 255);
         if (4 * (t & 255) < p.sb_channels) {
@@ -466,88 +480,95 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // starts from data the producer's loads deliver, so it is ordered behind that wait.
 
     if (warp == 0) {
-        // ------------------------------ TMA producer ------------------------------
-        if (lane == 0) {
+        // ------------------------------ TMA producer of the activations ------------------------------
+        // One k-block costs this thread a wait, an expect and a load (or two): the loop keeps running coordinates and
+        // nothing else, because a single thread's dependent instructions take several cycles each and the ring moves no
+        // faster than its slowest role. The weights have a producer of their own for the same reason.
+        if (elect_one()) {
             int stage = 0; uint32_t phase = 0;
             bool ok = true;
-            // Weights do not depend on the previous kernel: the weight tiles of the first k-blocks are
-            // requested before waiting for it, which also takes the tensor-map fetches off the critical path.
             // pair: both CTAs' loads complete on the even CTA's full barrier, which expects the bytes of both
             const uint32_t full0 = kPair ? map_to_cta(full_bar(0), 0) : full_bar(0);
-            const uint32_t stage_tx = (a_bytes + b_bytes) * (kPair ? 2u : 1u);
-            int pre_b = 0;
-            if (nseg > 0) {
-                int tile, k0, k1; segment(0, tile, k0, k1);
-                pre_b = min(p.num_stages, k1 - k0);
-                const int n0 = (tile % p.tiles_n) * p.bn + static_cast<int>(rank) * b_rows;
-                int tap = k0 / p.chunks_per_tap, chunk = k0 - tap * p.chunks_per_tap;
-                for (int kt = 0; kt < pre_b; ++kt) {
-                    if (lead) mbar_expect_tx(full_bar(kt), stage_tx);
-                    if constexpr (kPair) tma_load_2d_pair(b_base + kt * b_bytes, &map_b, full0 + 8u * kt, tap * p.cin_pad + chunk * p.bk_elems, n0);
-                    else                 tma_load_2d(b_base + kt * b_bytes, &map_b, full_bar(kt), tap * p.cin_pad + chunk * p.bk_elems, n0);
-                    if (++chunk == p.chunks_per_tap) { chunk = 0; ++tap; }
-                }
-            }
-            bool waited = false;
+            const uint32_t tx = a_bytes * (kPair ? 2u : 1u);
+            const bool im2col = p.a_mode == A_MODE_IM2COL;
+            pdl_wait();                     // the activations are the previous kernel's output
+            if constexpr (kTrace) { if (trace) trace[1] = clock64(); }
             for (int i = 0; i < nseg && ok; ++i) {
                 int tile, k0, k1; segment(i, tile, k0, k1);
-                const int tm = tile / p.tiles_n, tn = tile % p.tiles_n;
-                const int m0 = tm * tile_rows + static_cast<int>(rank) * kUmmaM, n0 = tn * p.bn + static_cast<int>(rank) * b_rows;
+                const int tm = tile / p.tiles_n;
+                const int m0 = tm * tile_rows + static_cast<int>(rank) * kUmmaM;
                 int img = 0, y0 = 0, x0 = 0;
-                if (p.a_mode == A_MODE_IM2COL) {
+                if (im2col) {
                     img = m0 / (p.oh * p.ow);
                     const int rem = m0 - img * p.oh * p.ow;
                     y0 = rem / p.ow; x0 = rem - y0 * p.ow;
                 }
                 const int cx = x0 * p.stride_w - p.pad_w, cy = y0 * p.stride_h - p.pad_h;
-                // k-blocks in tap-major order; plain counters instead of divisions keep this
-                // single-thread issue loop short
-                int chunk = 0, r = 0, s = 0;
+                int chunk = 0, s = 0, off_h = 0;
                 if (k0 > 0) {
-                    const int tap = k0 / p.chunks_per_tap;
-                    chunk = k0 - tap * p.chunks_per_tap; r = tap / p.kw; s = tap - r * p.kw;
+                    const int tap = k0 / p.chunks_per_tap, r = tap / p.kw;
+                    chunk = k0 - tap * p.chunks_per_tap; s = tap - r * p.kw; off_h = r * p.dil_h;
                 }
+                int c0 = chunk * p.bk_elems, off_w = s * p.dil_w;
                 for (int kt = k0; kt < k1; ++kt) {
-                    const int kb = (r * p.kw + s) * p.cin_pad;
-                    const int c0 = chunk * p.bk_elems;
-                    if (pre_b > 0) {
-                        --pre_b;                       // stage is fresh, its weight tile is already on the way
-                        if (!waited) {
-                            waited = true;
-                            pdl_wait();
-                            if constexpr (kTrace) { if (trace) trace[1] = clock64(); }
-                        }
-                    } else {
-                        ok = mbar_wait(empty_bar(stage), phase ^ 1u, cta_abort, p.err_flag, DEV_ERR_WAIT_EMPTY);
-                        if (!ok) break;
-                        if (lead) mbar_expect_tx(full_bar(stage), stage_tx);
-                        if constexpr (kPair) tma_load_2d_pair(b_base + stage * b_bytes, &map_b, full0 + 8u * stage, kb + c0, n0);
-                        else                 tma_load_2d(b_base + stage * b_bytes, &map_b, full_bar(stage), kb + c0, n0);
-                    }
+                    ok = mbar_wait(empty_bar(stage), phase ^ 1u, cta_abort, p.err_flag, DEV_ERR_WAIT_EMPTY);
+                    if (!ok) break;
+                    const uint32_t dst = a_base + stage * a_bytes, bar = full0 + 8u * stage;
+                    if (lead) mbar_expect_tx(full_bar(stage), tx);
                     if constexpr (kPair) {
-                        if (p.a_mode == A_MODE_IM2COL)
-                            tma_load_im2col_4d_pair(a_base + stage * a_bytes, &map_a, full0 + 8u * stage, c0, cx, cy, img,
-                                                    static_cast<uint16_t>(s * p.dil_w), static_cast<uint16_t>(r * p.dil_h));
-                        else
-                            tma_load_2d_pair(a_base + stage * a_bytes, &map_a, full0 + 8u * stage, c0, m0);
-                    } else if (p.a_mode == A_MODE_IM2COL)
-                        tma_load_im2col_4d(a_base + stage * a_bytes, &map_a, full_bar(stage), c0, cx, cy, img,
-                                           static_cast<uint16_t>(s * p.dil_w), static_cast<uint16_t>(r * p.dil_h));
-                    else
-                        for (int j = 0; j < m_mult; ++j)
-                            tma_load_2d(a_base + stage * a_bytes + j * sub_bytes, &map_a, full_bar(stage), c0, m0 + j * kUmmaM);
+                        if (im2col) tma_load_im2col_4d_pair(dst, &map_a, bar, c0, cx, cy, img, static_cast<uint16_t>(off_w), static_cast<uint16_t>(off_h));
+                        else        tma_load_2d_pair(dst, &map_a, bar, c0, m0);
+                    } else if (im2col) {
+                        tma_load_im2col_4d(dst, &map_a, bar, c0, cx, cy, img, static_cast<uint16_t>(off_w), static_cast<uint16_t>(off_h));
+                    } else {
+                        // a box holds up to 256 rows: tiles of three and four sub-tiles take two loads
+                        tma_load_2d(dst, &map_a, bar, c0, m0);
+                        if constexpr (kMult > 2) tma_load_2d(dst + a_bytes / 2, &map_a, bar, c0, m0 + kUmmaM * kMult / 2);
+                    }
                     if constexpr (kTrace) { if (trace && i == p.trace_tile && kt - k0 < 16) trace[8 + kt - k0] = clock64(); }
                     if (++stage == p.num_stages) { stage = 0; phase ^= 1u; }
-                    if (++chunk == p.chunks_per_tap) { chunk = 0; if (++s == p.kw) { s = 0; ++r; } }
+                    c0 += p.bk_elems;
+                    if (++chunk == p.chunks_per_tap) {
+                        chunk = 0; c0 = 0; off_w += p.dil_w;
+                        if (++s == p.kw) { s = 0; off_w = 0; off_h += p.dil_h; }
+                    }
+                }
+            }
+        }
+    } else if (warp == kUmmaWeightWarp) {
+        // ------------------------------ TMA producer of the weights ------------------------------
+        // Weights do not depend on the previous kernel: the first stages are requested while it still runs.
+        if (elect_one()) {
+            int stage = 0; uint32_t phase = 0;
+            bool ok = true;
+            const uint32_t full0 = kPair ? map_to_cta(full_bar(0), 0) : full_bar(0);
+            const uint32_t tx = b_bytes * (kPair ? 2u : 1u);
+            for (int i = 0; i < nseg && ok; ++i) {
+                int tile, k0, k1; segment(i, tile, k0, k1);
+                const int n0 = (tile % p.tiles_n) * p.bn + static_cast<int>(rank) * b_rows;
+                const int tap0 = k0 / p.chunks_per_tap;
+                int chunk = k0 - tap0 * p.chunks_per_tap, tap_c = tap0 * p.cin_pad, c0 = tap_c + chunk * p.bk_elems;
+                for (int kt = k0; kt < k1; ++kt) {
+                    ok = mbar_wait(empty_bar(stage), phase ^ 1u, cta_abort, p.err_flag, DEV_ERR_WAIT_EMPTY);
+                    if (!ok) break;
+                    if (lead) mbar_expect_tx(full_bar(stage), tx);
+                    if constexpr (kPair) tma_load_2d_pair(b_base + stage * b_bytes, &map_b, full0 + 8u * stage, c0, n0);
+                    else                 tma_load_2d(b_base + stage * b_bytes, &map_b, full_bar(stage), c0, n0);
+                    if (++stage == p.num_stages) { stage = 0; phase ^= 1u; }
+                    c0 += p.bk_elems;
+                    if (++chunk == p.chunks_per_tap) { chunk = 0; tap_c += p.cin_pad; c0 = tap_c; }
                 }
             }
         }
     } else if (warp == 1) {
         // ------------------------------ MMA issuer --------------------------------
-        if (lane == 0 && lead) {   // pair: the even CTA issues for both
+        if (lead && elect_one()) {   // pair: the even CTA issues for both
             int stage = 0; uint32_t phase = 0;
             bool ok = true;
-            const int mmas_per_block = p.bk_bytes / 32;   // each MMA consumes 32 bytes of K per row
+            const uint64_t desc_a0 = make_smem_desc(a_base, p.bk_bytes), desc_b0 = make_smem_desc(b_base, p.bk_bytes);
+            const uint64_t a_step = a_bytes >> 4, b_step = b_bytes >> 4;   // one stage, in descriptor units
+            const uint64_t sub_step = sub_bytes >> 4;                      // next sub-tile of A
+            uint64_t da = desc_a0, db = desc_b0;
             for (int tl = 0; tl < nseg && ok; ++tl) {     // tl: segments this CTA has started
                 int tile, k0, k1; segment(tl, tile, k0, k1);
                 const int seg_k = k1 - k0;
@@ -557,31 +578,35 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 if (!ok) break;
                 tcgen05_fence_after();
                 const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * m_mult * p.bn);
-                for (int kt = 0; kt < seg_k; ++kt) {
-                    ok = mbar_wait(full_bar(stage), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
-                    if (!ok) break;
-                    if constexpr (kTrace) { if (trace && tl == p.trace_tile && kt < 16) trace[24 + kt] = clock64(); }
-                    tcgen05_fence_after();
-                    const uint64_t db = make_smem_desc(b_base + stage * b_bytes, p.bk_bytes);
-                    const uint64_t da0 = make_smem_desc(a_base + stage * a_bytes, p.bk_bytes);
-                    const uint64_t da_step = static_cast<uint64_t>(sub_bytes >> 4);   // next sub-tile of A, in descriptor units
-                    // consecutive MMAs go to different accumulators (the sub-tiles share the weight tile), so an
-                    // MMA never waits for the one before it to write the accumulator back
-                    for (int k = 0; k < mmas_per_block; ++k) {
-                        for (int j = 0; j < m_mult; ++j) {
-                            // advancing K inside the swizzle span = advancing the start address
-                            if constexpr (kPair)
-                                tcgen05_mma_pair<kTf32>(tmem_d, da0 + static_cast<uint64_t>(2 * k), db + static_cast<uint64_t>(2 * k),
-                                                        p.idesc, (kt | k) != 0 ? 1u : 0u);
-                            else
-                                tcgen05_mma<kTf32>(tmem_d + static_cast<uint32_t>(j * p.bn), da0 + j * da_step + static_cast<uint64_t>(2 * k),
-                                                   db + static_cast<uint64_t>(2 * k), p.idesc, (kt | k) != 0 ? 1u : 0u);
+                uint32_t accumulate = 0;
+                // straight-line code per k-block (4, 2 or 1 MMAs per sub-tile, each 32 bytes of K per row)
+                auto k_blocks = [&](auto mmas) {
+                    for (int kt = 0; kt < seg_k; ++kt) {
+                        ok = mbar_wait(full_bar(stage), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
+                        if (!ok) break;
+                        if constexpr (kTrace) { if (trace && tl == p.trace_tile && kt < 16) trace[24 + kt] = clock64(); }
+                        tcgen05_fence_after();
+                        // consecutive MMAs go to different accumulators (the sub-tiles share the weight tile), so an
+                        // MMA never waits for the one before it to write the accumulator back
+#pragma unroll
+                        for (int k = 0; k < decltype(mmas)::value; ++k) {
+#pragma unroll
+                            for (int j = 0; j < m_mult; ++j) {
+                                // advancing K inside the swizzle span = advancing the start address
+                                if constexpr (kPair) tcgen05_mma_pair<kTf32>(tmem_d, da + 2 * k, db + 2 * k, p.idesc, k > 0 ? 1u : accumulate);
+                                else tcgen05_mma<kTf32>(tmem_d + static_cast<uint32_t>(j * p.bn), da + j * sub_step + 2 * k, db + 2 * k, p.idesc, k > 0 ? 1u : accumulate);
+                            }
                         }
+                        accumulate = 1;
+                        if constexpr (kPair) tcgen05_commit_pair(empty_bar(stage));   // frees the stage in both CTAs
+                        else                 tcgen05_commit(empty_bar(stage));        // frees the stage when these MMAs retire
+                        da += a_step; db += b_step;
+                        if (++stage == p.num_stages) { stage = 0; phase ^= 1u; da = desc_a0; db = desc_b0; }
                     }
-                    if constexpr (kPair) tcgen05_commit_pair(empty_bar(stage));   // frees the stage in both CTAs
-                    else                 tcgen05_commit(empty_bar(stage));        // frees the stage when these MMAs retire
-                    if (++stage == p.num_stages) { stage = 0; phase ^= 1u; }
-                }
+                };
+                if (p.bk_bytes == 128) k_blocks(std::integral_constant<int, 4>{});
+                else if (p.bk_bytes == 64) k_blocks(std::integral_constant<int, 2>{});
+                else k_blocks(std::integral_constant<int, 1>{});
                 if (!ok) break;
                 if constexpr (kPair) tcgen05_commit_pair(acc_full_bar(acc));   // accumulator complete, in both CTAs
                 else                 tcgen05_commit(acc_full_bar(acc));
@@ -750,9 +775,8 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const uint32_t row_swz = static_cast<uint32_t>((row >> swz_shift) & swz_mask);
         uint32_t store_count = 0;
         if constexpr (kTrace) { if (team == 1) trace = nullptr; }
-        // kSplit: every tile, items (sub-tile, slab) team, team+2, ...; otherwise tiles team, team+2, ... whole
-        const int tl_step = kSplit ? 1 : 2;
-        for (int tl = kSplit ? 0 : team; ok && tl < nseg; tl += tl_step) {
+        // every tile: items (sub-tile, slab) team, team+2, ...
+        for (int tl = 0; ok && tl < nseg; ++tl) {
             int tile, seg_k0, seg_k1; segment(tl, tile, seg_k0, seg_k1);
             // stream-K: a segment that stops short of the tile's last k-block hands its partial sums over
             // (sk_export); one that starts after the first k-block completes its predecessors' (CTAs
@@ -802,7 +826,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             if constexpr (kTrace) { if (trace && tl == 0 && leader) trace[40] = clock64(); }
             tcgen05_fence_after();
             const int slabs = (min(p.bn, p.cout - n0) + cols_per_store - 1) >> cols_shift;   // store slabs per sub-tile
-            for (int item = kSplit ? team : 0; item < kMult * slabs; item += kSplit ? 2 : 1) {
+            for (int item = team; item < kMult * slabs; item += 2) {
                 int sub = 0;
                 if (kMult > 1) { while (item >= (sub + 1) * slabs) ++sub; }
                 const int c0 = (item - sub * slabs) << cols_shift;

@@ -32,7 +32,8 @@ enum { DEV_ERR_NONE = 0, DEV_ERR_WAIT_FULL = 1, DEV_ERR_WAIT_EMPTY = 2, DEV_ERR_
 
 // ---- tensor-core convolution (conv_umma.cuh) --------------------------------------------------------------------------
 constexpr int kUmmaM          = 128;  // output pixels per tile (TMEM lanes)
-constexpr int kUmmaThreads    = 576;  // warp 0: TMA producer, warp 1: MMA issuer, warps 2-17: epilogue (two teams of 8)
+constexpr int kUmmaThreads    = 608;  // warp 0: TMA producer of A, warp 1: MMA issuer, warps 2-17: epilogue, warp 18: TMA producer of B
+constexpr int kUmmaWeightWarp = 18;
 constexpr int kUmmaMaxStages  = 8;
 constexpr int kUmmaMaxAccStages = 8; // accumulator ring in TMEM: 2, 4 or 8 stages, as many as fit in 512 columns
 constexpr uint32_t kStageCBytes = 128 * 128;   // one output staging slab: 128 rows x up to 128 bytes

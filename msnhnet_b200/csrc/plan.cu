@@ -46,7 +46,6 @@ PlanDebugOptions PlanDebugOptions::from_env() {
     o.forced_bn = num("MSNH_B200_BN", 0);
     o.stream_k = num("MSNH_B200_STREAM_K", 0);
     o.pair = num("MSNH_B200_PAIR", 0);
-    o.no_split = num("MSNH_B200_NO_SPLIT", -1);
     return o;
 }
 int check_device_flag(MsnhB200Plan *pl) {

@@ -82,10 +82,9 @@ struct PlanDebugOptions {
     int forced_mm = 0, forced_bn = 0;   // MSNH_B200_M_MULT, MSNH_B200_BN: force the conv tile shape
     int stream_k = 0;           // MSNH_B200_STREAM_K: -1 by cost, 0 never, 1 wherever possible
     int pair = 0;               // MSNH_B200_PAIR: 1 = CTA pairs wherever possible
-    int no_split = -1;          // MSNH_B200_NO_SPLIT: -1 unset, else the epilogue teams alternate over whole tiles (1) or not (0)
     static PlanDebugOptions from_env();
     // any switch that forces tile shapes: such plans neither take shapes from a pack file nor write one
-    bool forces_tiles() const { return forced_mm || forced_bn || pair == 1 || stream_k != 0 || no_split >= 0; }
+    bool forces_tiles() const { return forced_mm || forced_bn || pair == 1 || stream_k != 0; }
 };
 
 // ------------------------------------------------------------------------------------------------
@@ -147,7 +146,6 @@ struct Launch {
     TView out2{};              // second output of two 1x1 convs over the same input merged into this launch (ptr == nullptr: none)
     int split_n = 0;           // its first channel in the merged channel range
     ConvUmmaParams up{};
-    int no_split = 0;          // 128-pixel tiles with several store slabs: the epilogue teams take whole tiles in turn instead of sharing each
     int grid = 0; size_t smem = 0;
     // depthwise 3x3 on shared-memory tiles (map_a = the input's 4-D tensor map; grid / smem above)
     bool dw_tile = false; DwTileParams dwp{};

@@ -13,37 +13,33 @@ using namespace msnh;
 namespace msnh {
 namespace {
 
-// The instantiation of the tensor-core conv kernel a launch runs: tile form (sub-tiles per tile, epilogue teams sharing
-// or alternating tiles, CTA pair, stream-K), the activation compiled into the epilogue (mish and leaky with a slope in
+// The instantiation of the tensor-core conv kernel a launch runs: tile form (sub-tiles per tile, CTA pair, stream-K), the activation compiled into the epilogue (mish and leaky with a slope in
 // [0, 1] have their own fp16 instantiations; everything else switches at run time) and, for plans made with
 // MSNH_PLAN_TRACE, the form that records clock stamps.
 template <typename T> const void *umma_kernel(const Launch &L) {
     const ConvUmmaParams &u = L.up;
-    if (u.stream_k) return u.m_mult == 2 ? reinterpret_cast<const void *>(conv_umma_kernel<T, 2, true, false, true>)
-                                         : reinterpret_cast<const void *>(conv_umma_kernel<T, 1, true, false, true>);
-    if (u.pair) return reinterpret_cast<const void *>(conv_umma_kernel<T, 1, true, true, false>);
-    // both epilogue teams share every tile once a tile has at least two store slabs
-    const bool split = u.m_mult > 1 || (u.bn * static_cast<int>(sizeof(T)) > u.out_chunk_bytes && !L.no_split);
+    if (u.stream_k) return u.m_mult == 2 ? reinterpret_cast<const void *>(conv_umma_kernel<T, 2, false, true>)
+                                         : reinterpret_cast<const void *>(conv_umma_kernel<T, 1, false, true>);
+    if (u.pair) return reinterpret_cast<const void *>(conv_umma_kernel<T, 1, true, false>);
     const bool trace = u.trace != nullptr;
     int act = kActGeneric;
     if (sizeof(T) == 2 && !trace) {
         if (u.act1 == MSNH_ACT_MISH) act = MSNH_ACT_MISH;
         else if (u.act1 == MSNH_ACT_LEAKY && u.act1_param >= 0.f && u.act1_param <= 1.f) act = MSNH_ACT_LEAKY;
     }
-#define MSNH_UMMA_FORM(MM, SP)                                                                                                   \
+#define MSNH_UMMA_FORM(MM)                                                                                                   \
     do {                                                                                                                         \
-        if (trace) return reinterpret_cast<const void *>(conv_umma_kernel<T, MM, SP, false, false, kActGeneric, true>);          \
+        if (trace) return reinterpret_cast<const void *>(conv_umma_kernel<T, MM, false, false, kActGeneric, true>);          \
         if constexpr (sizeof(T) == 2) {                                                                                          \
-            if (act == MSNH_ACT_MISH) return reinterpret_cast<const void *>(conv_umma_kernel<T, MM, SP, false, false, MSNH_ACT_MISH>);   \
-            if (act == MSNH_ACT_LEAKY) return reinterpret_cast<const void *>(conv_umma_kernel<T, MM, SP, false, false, MSNH_ACT_LEAKY>); \
+            if (act == MSNH_ACT_MISH) return reinterpret_cast<const void *>(conv_umma_kernel<T, MM, false, false, MSNH_ACT_MISH>);   \
+            if (act == MSNH_ACT_LEAKY) return reinterpret_cast<const void *>(conv_umma_kernel<T, MM, false, false, MSNH_ACT_LEAKY>); \
         }                                                                                                                        \
-        return reinterpret_cast<const void *>(conv_umma_kernel<T, MM, SP, false, false>);                                        \
+        return reinterpret_cast<const void *>(conv_umma_kernel<T, MM, false, false>);                                        \
     } while (0)
-    if (u.m_mult == 4) MSNH_UMMA_FORM(4, true);
-    if (u.m_mult == 3) MSNH_UMMA_FORM(3, true);
-    if (u.m_mult == 2) MSNH_UMMA_FORM(2, true);
-    if (split) MSNH_UMMA_FORM(1, true);
-    MSNH_UMMA_FORM(1, false);
+    if (u.m_mult == 4) MSNH_UMMA_FORM(4);
+    if (u.m_mult == 3) MSNH_UMMA_FORM(3);
+    if (u.m_mult == 2) MSNH_UMMA_FORM(2);
+    MSNH_UMMA_FORM(1);
 #undef MSNH_UMMA_FORM
 }
 const void *umma_kernel_of(const Launch &L) { return L.dtype == MSNH_B200_F16 ? umma_kernel<__half>(L) : umma_kernel<float>(L); }

@@ -172,12 +172,10 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
     u.a_mode = linear ? A_MODE_LINEAR : A_MODE_IM2COL;
     const size_t fixed = 4 * kStageCBytes + 2 * 1024 + 512 + 2 * 4 * kSbMaxChannels;   // output staging slabs (2 per epilogue team), alignment slack, barriers, scale/bias tables
     const size_t budget = 227 * 1024 - fixed;
-    // Tile shape: 128 * m_mult pixels x bn channels (m_mult MMAs of 128 x bn per 32 bytes of K, sharing
-    // the weight tile). Measured on B200 (SM cycles): an MMA issues about every 156 cycles whatever its
-    // width up to 224 columns (165 at 256) when its neighbours use other weight slices; consecutive MMAs
-    // that share the weight slice (the sub-tiles of one k-step) issue every 48 + 108 / sub-tiles cycles
-    // (102 for two, 75 for four); an im2col load costs about 600 cycles whatever its pixel count. So the main loop of a k-block takes
-    // max(load issue, MMAs x issue interval, bytes / TMA rate), wide tiles are cheapest per FLOP, and
+    // Tile shape: 128 * m_mult pixels x bn channels (m_mult MMAs of 128 x bn per 32 bytes of K, sharing the weight tile).
+    // Measured on B200 (SM cycles per k-block of four MMAs per sub-tile): an MMA of 128 pixels takes 66 cycles up to 128
+    // channels and 0.51 per channel beyond (130 at 256); the producers issue a k-block in about 330; loads arrive at about
+    // 80 bytes per cycle. So the main loop of a k-block takes the largest of the three, wide tiles are cheapest per FLOP, and
     // the choice below trades that against the number of tiles left to spread over the SMs.
     // Modelled cost: waves x k-blocks x k-block time + drain of the last tile + start-up.
     {
@@ -200,12 +198,8 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
         // loop; kept selectable (MSNH_B200_PAIR=1) and covered by the GPU tests.
         const int pair_mode = dbg.pair;
         const int n_mma = u.bk_bytes / 32;
-        auto kblock_cycles = [&](int mm, int bn, size_t stage_bytes, bool pair) {
-            // measured per-MMA interval: 48 + 108 / (sub-tiles sharing the weight tile) cycles, 165 for one sub-tile of 256 channels
-            const double interval = std::max(mm >= 2 ? 48.0 + 108.0 / mm : (bn > 224 ? 165.0 : 156.0), bn * 0.5);
-            const double issue = linear ? 150.0 * mm : 600.0;
-            (void)pair;
-            return std::max(std::max(issue, mm * n_mma * interval), static_cast<double>(stage_bytes) / 75.0);
+        auto kblock_cycles = [&](int mm, int bn, size_t stage_bytes) {
+            return std::max(std::max(330.0, mm * n_mma * std::max(66.0, bn * 0.51)), static_cast<double>(stage_bytes) / 80.0);
         };
         for (int bn : bns) {
             if (pair_mode != 1 || bn * es <= 128 || (forced_bn && bn != std::min(forced_bn, bns.back()))) continue;
@@ -214,7 +208,7 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
             const int pairs = ((u.m_total + 2 * kUmmaM - 1) / (2 * kUmmaM)) * tiles_n;
             const double waves = std::ceil(static_cast<double>(pairs) / (ctx->sm_count / 2));
             const double drain = 900.0 * ((((bn + slab_cols - 1) / slab_cols) + 1) / 2);
-            const double cost = (waves * k_iters * kblock_cycles(1, bn, stage, true) + drain + 3000.0) * 1e-3;
+            const double cost = (waves * k_iters * kblock_cycles(1, bn, stage) + drain + 3000.0) * 1e-3;
             if (cost < best * 0.97) { best = cost; best_mm = 1; best_bn = bn; best_pair = 1; }
         }
         for (int bn : bns) {
@@ -230,15 +224,13 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
                 if (forced_mm && mm != forced_mm && !(mm == 1 && forced_mm * bn > 256)) continue;
                 const size_t stage = static_cast<size_t>(kUmmaM * mm + bn) * u.bk_bytes;
                 // stages to keep the loads ahead: two suffice when a k-block's MMAs outlast a load's latency
-                const size_t min_stages = (k_iters <= 2 || kblock_cycles(mm, bn, stage, false) >= 1000.0) ? 2 : 3;
+                const size_t min_stages = (k_iters <= 2 || kblock_cycles(mm, bn, stage) >= 1000.0) ? 2 : 3;
                 if (budget / stage < min_stages && !(mm == 1 && bn == bns[0])) continue;
                 const int tiles = ((u.m_total + kUmmaM * mm - 1) / (kUmmaM * mm)) * tiles_n;
                 const double waves = std::ceil(static_cast<double>(tiles) / ctx->sm_count);
                 const double drain = 900.0 * ((mm * ((bn + slab_cols - 1) / slab_cols) + 1) / 2);
-                const double cost = waves * k_iters * kblock_cycles(mm, bn, stage, false) + drain + 2500.0;
+                const double cost = waves * k_iters * kblock_cycles(mm, bn, stage) + drain + 2500.0;
                 cands.push_back({cost, mm, bn, 0});
-                // (sk = 2: the same 128-pixel tiles with the epilogue teams alternating over whole tiles)
-                if (mm == 1 && bn * es > 128 && tiles > ctx->sm_count) cands.push_back({cost * 1.02, mm, bn, 2});
                 if (measured_only && !(forced_mm && forced_bn)) continue;    // (forcing both picks such a shape: parity tests)
                 if (cost < best * 0.97 && sk_mode != 1) { best = cost; best_mm = mm; best_bn = bn; best_pair = 0; best_sk = 0; }
                 // stream-K: every SM takes units / SMs k-blocks; hand-over and completion of split tiles
@@ -251,7 +243,7 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
                     // measured: handing a 128 KB partial tile over costs ~6k cycles on the writer and ~3k per
                     // slot on the reader, one after the other on the critical path
                     const double parts = std::ceil(static_cast<double>(k_iters) / share);
-                    double cost_sk = share * kblock_cycles(mm, bn, stage, false) + drain + 2500.0 +
+                    double cost_sk = share * kblock_cycles(mm, bn, stage) + drain + 2500.0 +
                                      (6000.0 + 4000.0 * parts) * (mm * bn / 256.0);
                     if (sk_mode == 1) cost_sk *= 1e-3;
                     if (cost_sk < best * 0.95) { best = cost_sk; best_mm = mm; best_bn = bn; best_pair = 0; best_sk = 1; }
@@ -259,16 +251,14 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
             }
         }
         u.m_mult = best_mm; u.bn = best_bn; u.pair = best_pair; u.stream_k = best_sk;
-        if (dbg.no_split >= 0) L.no_split = dbg.no_split != 0;   // parity tests of that epilogue form
         tune_cands.clear();
         // a pack file carries the shapes its plan ended up with: no need to time them again
-        const bool stored = pl->pack_loaded && tt.umma_seen < pl->pack_picks.size() && !forced_mm && !forced_bn && pair_mode != 1 && sk_mode == 0 &&
-                            dbg.no_split < 0;
+        const bool stored = pl->pack_loaded && tt.umma_seen < pl->pack_picks.size() && !forced_mm && !forced_bn && pair_mode != 1 && sk_mode == 0;
         if (stored) {
             const std::array<int32_t, 3> &pk = pl->pack_picks[tt.umma_seen];
             bool valid = false;
             for (const Cand &c : cands) valid = valid || (c.mm == pk[0] && c.bn == pk[1]);
-            if (valid) { u.m_mult = pk[0]; u.bn = pk[1]; u.pair = 0; u.stream_k = 0; L.no_split = (pk[2] & 0xff) == 2; if (pk[2] >= 0x100) L.note += L.note.empty() ? "measured shape" : ", measured shape"; }
+            if (valid) { u.m_mult = pk[0]; u.bn = pk[1]; u.pair = 0; u.stream_k = 0; if (pk[2] >= 0x100) L.note += L.note.empty() ? "measured shape" : ", measured shape"; }
         }
         if (!stored && tt.autotune && !best_pair && !best_sk && !forced_mm && !forced_bn) {
             std::sort(cands.begin(), cands.end(), [](const Cand &x, const Cand &y) { return x.cost < y.cost; });
@@ -315,7 +305,7 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
     int rc;
     if (linear)
         rc = make_map_2d(ctx, &L.map_a, pl->dtype, L.in.ptr, static_cast<uint64_t>(cin), static_cast<uint64_t>(L.in.N) * L.in.H * L.in.W,
-                         static_cast<uint64_t>(L.in.ldc) * es, static_cast<uint32_t>(u.bk_elems), kUmmaM, u.bk_bytes);
+                         static_cast<uint64_t>(L.in.ldc) * es, static_cast<uint32_t>(u.bk_elems), static_cast<uint32_t>(u.m_mult > 2 ? kUmmaM * u.m_mult / 2 : kUmmaM * u.m_mult), u.bk_bytes);
     else
         rc = make_map_im2col(ctx, &L.map_a, pl->dtype, L.in, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, L.dh, L.dw, u.bk_elems, u.bk_bytes, kUmmaM * u.m_mult);
     if (rc) return rc;
@@ -349,7 +339,7 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
         { std::lock_guard<std::mutex> g(tune_mutex()); auto it = tune_cache().find(key); if (it != tune_cache().end()) { pick = it->second; known = true; } }
         if (!known) {
             auto time_shape = [&](int mm, int bn, int sk, float *ms) -> int {
-                Launch t = L; t.up.m_mult = mm; t.up.bn = bn; t.up.pair = 0; t.up.stream_k = sk == 1; t.no_split = sk == 2;
+                Launch t = L; t.up.m_mult = mm; t.up.bn = bn; t.up.pair = 0; t.up.stream_k = sk == 1;
                 const int rc = configure(t);
                 if (rc) return rc;
                 launch_one(ctx, t, ctx->stream);
@@ -383,11 +373,11 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
             std::lock_guard<std::mutex> g(tune_mutex());
             tune_cache()[key] = pick;
         }
-        if (pick[0] != u.m_mult || pick[1] != u.bn || pick[2] != 0) { u.m_mult = pick[0]; u.bn = pick[1]; u.stream_k = pick[2] == 1; L.no_split = pick[2] == 2; L.note += L.note.empty() ? "measured shape" : ", measured shape"; }
+        if (pick[0] != u.m_mult || pick[1] != u.bn || pick[2] != 0) { u.m_mult = pick[0]; u.bn = pick[1]; u.stream_k = pick[2] == 1; L.note += L.note.empty() ? "measured shape" : ", measured shape"; }
     }
     { const int rc = configure(L); if (rc) return rc; }
-    // form: 0 plain, 1 stream-K, 2 whole-tile epilogue teams, 4 CTA pair; + 0x100 when the shape was a measured choice
-    if (!pl->pack_loaded) pl->pack_picks.push_back({u.m_mult, u.bn, (u.stream_k ? 1 : (u.pair ? 4 : (L.no_split ? 2 : 0))) | (L.note.find("measured shape") != std::string::npos ? 0x100 : 0)});
+    // form: 0 plain, 1 stream-K, 4 CTA pair; + 0x100 when the shape was a measured choice
+    if (!pl->pack_loaded) pl->pack_picks.push_back({u.m_mult, u.bn, (u.stream_k ? 1 : (u.pair ? 4 : 0)) | (L.note.find("measured shape") != std::string::npos ? 0x100 : 0)});
     ++tt.umma_seen;
     return MSNH_B200_OK;
 }
