@@ -1,4 +1,7 @@
-// Dense convolution on the CUDA cores in fp32 arithmetic: an implicit GEMM with shared-memory tiles, for the plans that must
+// Dense convolutions on the CUDA cores in fp32 arithmetic.
+//
+// conv_tiled_kernel: an implicit GEMM with shared-memory tiles for 16-bit plans built without tensor cores (the cross-check of
+// the tensor-core kernel); fp32 views take conv_fp32_kernel below. Both serve the plans that must
 // reproduce the reference's fp32 results (its GPU path is fp32 Sgemm throughout, src/layers/MsnhConvolutionalLayer.cpp:1026-1160):
 // fp32 detection nets, whose exp()-decoded boxes do not survive tf32's 10-bit mantissa, and plans built without tensor cores.
 // D[m][n] = sum_k A[m][k] * B[n][k]: m = output pixel (linear over image, row, column), n = output channel, k = (filter
@@ -9,6 +12,7 @@
 #pragma once
 #include "common.cuh"
 #include "layer_kernels.cuh"
+#include "conv_umma.cuh"   // packed fp32 pairs, cluster barrier
 
 namespace msnh {
 
@@ -135,6 +139,195 @@ conv_tiled_kernel(TView in, TView out, const T *__restrict__ w, const ConvTiledP
             for (int e = 0; e < 4; ++e) if (c0 + e < cout) Elem<T>::st(dst + e, y[e]);
         }
     }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------------
+// conv_fp32_kernel: the fp32 form. Same GEMM view; A and B are streams of 16-byte vectors (k = four input channels of one filter
+// tap, taps in order), so a k-step of four vectors may straddle taps and a 3-channel stem wastes nothing but its pad channel.
+// What bounds it is the FMA pipe (128 lanes per SM and cycle) and, close behind, the register fill from shared memory; the rest
+// of its design serves the layers that do not fill the chip - a plane of 11 x 11 pixels under 768 channels is six tiles of
+// pixels and one chain of 3456 products:
+//  * a CTA of four warps computes tiles of 64 pixels x 64 channels, a thread 8 x 4 of them. Neighbouring lanes share the pixel
+//    rows they read: a 16-byte load whose lane pairs agree takes 2.3 SM cycles, one whose lane pairs differ 4.1 (measured), so
+//    per k the eight pixel values cost as much as the four channel values. Scalar FMAs: the packed form reads six registers at
+//    a time and reaches 54 TFLOP/s from registers alone, the scalar one 72.
+//  * a cluster of 1..8 CTAs splits the k of one tile. Every CTA sums its share, leaves it in its own shared memory, and reduces
+//    every size-th row of the tile from all of them through distributed shared memory, in rank order: deterministic, no
+//    workspace, no second launch. configure_conv_fp32 picks the split.
+//  * operands stay k-contiguous in shared memory as cp.async wrote them (row pitch 20 floats: the eight rows of a load
+//    fall in different banks); a ring of four k-steps, cp.async also zero-fills the padding, pad channels and ragged edges. A
+//    loader thread keeps its source addresses and moves them along while its vectors stay inside one filter tap.
+// ---------------------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+__global__ void __launch_bounds__(kFpThreads, 4)
+conv_fp32_kernel(TView in, TView out, const float *__restrict__ w, const ConvTiledParams p) {
+    constexpr int BM = kFpBM, BN = kFpBN, T = kFpThreads, PITCH = kFpPitch, LROWS = T / 4, LA = BM / LROWS, LB = BN / LROWS;
+    constexpr int kStageFloats = (BM + BN) * PITCH, kCPitch = BN + 4;
+    extern __shared__ __align__(16) float fp_smem[];
+    const uint32_t smem = smem_u32(fp_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m_total = out.N * out.H * out.W, cout = out.C;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int splits = gridDim.z, rank = blockIdx.z;
+    const int cvecs = p.cin_pad >> 2, kvecs = p.kh * p.kw * cvecs, steps = (kvecs + 3) >> 2;
+    const int step0 = static_cast<int>(static_cast<long long>(steps) * rank / splits), step1 = static_cast<int>(static_cast<long long>(steps) * (rank + 1) / splits);
+
+    // loader: vector kq of a k-step for pixels and channels lrow, lrow + LROWS, ...
+    const int kq = tid & 3, lrow = tid >> 2;
+    int a_pix[LA], ay[LA], ax[LA];                                // pixel index of the filter's first tap, its row and column
+#pragma unroll
+    for (int j = 0; j < LA; ++j) {
+        const int m = m0 + lrow + LROWS * j;
+        const int mm = m < m_total ? m : 0;
+        const int n = mm / (out.H * out.W), rem = mm - n * out.H * out.W;
+        const int oy = rem / out.W, ox = rem - oy * out.W;
+        ay[j] = oy * p.sh - p.ph; ax[j] = ox * p.sw - p.pw;
+        a_pix[j] = (n * in.H + ay[j]) * in.W + ax[j];
+        if (m >= m_total) ay[j] = -(1 << 28);                     // a row past the last pixel is never inside the plane
+    }
+    int v = step0 * 4 + kq, r, s, c4;                             // next vector of this thread's column: tap (r, s), vector c4
+    { const int tap = v / cvecs; c4 = v - tap * cvecs; r = tap / p.kw; s = tap - r * p.kw; }
+    const float *a_src[LA], *b_src[LB]; uint32_t a_take[LA], b_take[LB];   // sources of the next step; 16 or 0 bytes of them
+    auto aim = [&]() {                                            // a new filter tap: where this thread's pixels are under it
+        const int dy = r * p.dh, dx = s * p.dw, dpix = dy * in.W + dx;
+#pragma unroll
+        for (int j = 0; j < LA; ++j) {
+            const bool inside = v < kvecs && static_cast<unsigned>(ay[j] + dy) < static_cast<unsigned>(in.H) && static_cast<unsigned>(ax[j] + dx) < static_cast<unsigned>(in.W);
+            a_take[j] = inside ? 16u : 0u;
+            a_src[j] = static_cast<const float *>(in.ptr) + (inside ? static_cast<size_t>(a_pix[j] + dpix) * in.ldc + 4 * c4 : 0);
+        }
+    };
+    aim();
+#pragma unroll
+    for (int j = 0; j < LB; ++j) {
+        b_take[j] = n0 + lrow + LROWS * j < cout ? 16u : 0u;
+        b_src[j] = w + (b_take[j] ? (static_cast<size_t>(n0 + lrow + LROWS * j) * kvecs + v) * 4 : 0);
+    }
+    const uint32_t a_dst = smem + static_cast<uint32_t>(lrow * PITCH + kq * 4) * 4u;
+    const uint32_t b_dst = a_dst + static_cast<uint32_t>(BM * PITCH) * 4u;
+    auto load_step = [&](int slot) {
+        const uint32_t off = static_cast<uint32_t>(slot * kStageFloats) * 4u;
+        const uint32_t bytes = static_cast<uint32_t>(min(16, (in.C - 4 * c4) * 4));       // pad channels of the pitch hold no data
+        const bool live = v < kvecs;
+#pragma unroll
+        for (int j = 0; j < LA; ++j) { cp_async16(a_dst + off + static_cast<uint32_t>(LROWS * j * PITCH) * 4u, a_src[j], min(a_take[j], bytes)); a_src[j] += a_take[j]; }
+#pragma unroll
+        for (int j = 0; j < LB; ++j) {
+            cp_async16(b_dst + off + static_cast<uint32_t>(LROWS * j * PITCH) * 4u, live ? b_src[j] : w, live ? b_take[j] : 0u);
+            b_src[j] += b_take[j];
+        }
+        v += 4; c4 += 4;
+        if (c4 >= cvecs) {
+            do { c4 -= cvecs; if (++s == p.kw) { s = 0; ++r; } } while (c4 >= cvecs);
+            aim();
+        }
+    };
+
+    // arithmetic: a warp covers 64 pixels x 16 channels, a thread pixels tm + 8 i and channels tn + 4 j
+    const int tm = (lane >> 1) & 7, tn = (lane & 1) + 2 * (lane >> 4) + 16 * warp;
+    float acc[8][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+
+    pdl_wait();
+#pragma unroll
+    for (int q = 0; q < kFpStages - 1; ++q) {
+        if (step0 + q < step1) load_step(q);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int slot = 0;
+    for (int step = step0; step < step1; ++step) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kFpStages - 2) : "memory");
+        __syncthreads();                            // this k-step has landed, and everybody is done with the slot loaded next
+        if (step + kFpStages - 1 < step1) load_step((slot + kFpStages - 1) & (kFpStages - 1));
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float *As = fp_smem + slot * kStageFloats + tm * PITCH, *Bs = fp_smem + slot * kStageFloats + (BM + tn) * PITCH;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            float4 a[8], b[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = *reinterpret_cast<const float4 *>(Bs + 4 * j * PITCH + 4 * q);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const float4 *>(As + 8 * i * PITCH + 4 * q);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
+            }
+        }
+        slot = (slot + 1) & (kFpStages - 1);
+    }
+    // Only now may the next kernel's CTAs come in: launched at the start of this one they would pile up on the SMs that have
+    // room, that is on those that this layer leaves idle, and stay there.
+    pdl_launch_dependents();
+    // this CTA's sums -> shared memory (over the ring: everybody has to be done reading it)
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) fp_smem[(tm + 8 * i) * kCPitch + tn + 4 * j] = acc[i][j];
+    if (splits > 1) cluster_sync_all(); else __syncthreads();
+
+    // this CTA's rows of the tile: sum over the cluster, scale / bias, activation, residual (+ second activation), store
+    const float *res = static_cast<const float *>(p.res);
+    const bool out_vec = (out.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(out.ptr) & 15) == 0;
+    const bool res_vec = res && (p.ldc_res & 3) == 0 && (reinterpret_cast<uintptr_t>(res) & 15) == 0;
+    const int col = 4 * (tid & 15), c0 = n0 + col;
+    if (c0 < cout) {
+        float sc[4], bi[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            sc[e] = (p.scale && c0 + e < cout) ? p.scale[c0 + e] : 1.f;
+            bi[e] = (p.bias && c0 + e < cout) ? p.bias[c0 + e] : 0.f;
+        }
+        for (int row = rank + splits * (tid >> 4); row < BM && m0 + row < m_total; row += splits * (T / 16)) {
+            const int m = m0 + row;
+            float y[4] = {0.f, 0.f, 0.f, 0.f};
+            if (splits == 1) ld_vec(fp_smem + row * kCPitch + col, y);
+            else {
+                const uint32_t at = smem + static_cast<uint32_t>(row * kCPitch + col) * 4u;
+                for (int q = 0; q < splits; ++q) {
+                    float4 t;
+                    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "r"(map_to_cta(at, q)) : "memory");
+                    y[0] += t.x; y[1] += t.y; y[2] += t.z; y[3] += t.w;
+                }
+            }
+            float rr[4] = {0.f, 0.f, 0.f, 0.f};
+            if (res) {
+                const float *rp = res + static_cast<size_t>(m) * p.ldc_res + c0;
+                if (res_vec && c0 + 4 <= cout) ld_vec(rp, rr);
+                else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) if (c0 + e < cout) rr[e] = rp[e];
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                y[e] = activate(fmaf(y[e], sc[e], bi[e]), p.act1, p.act1_param);
+                if (res) y[e] = activate(y[e] + rr[e], p.act2, p.act2_param);
+                if (out.tf32) y[e] = round_tf32(y[e]);
+            }
+            float *dst = static_cast<float *>(out.ptr) + static_cast<size_t>(m) * out.ldc + c0;
+            if (out_vec && c0 + 4 <= cout) st_vec(dst, y);
+            else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) if (c0 + e < cout) dst[e] = y[e];
+            }
+        }
+    }
+    if (splits > 1) cluster_sync_all();              // nobody leaves while a peer still reads its shared memory
 }
 
 }  // namespace msnh

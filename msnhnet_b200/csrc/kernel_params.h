@@ -125,6 +125,10 @@ constexpr int kNmsThreads = 256;
 // ---- CUDA-core tiled convolution (conv_tiled.cuh) ---------------------------------------------------------------------
 constexpr int kCtBM = 128, kCtBN = 64, kCtThreads = 256;
 
+// fp32 form (conv_fp32_kernel)
+constexpr int kFpBM = 64, kFpBN = 64, kFpThreads = 128, kFpPitch = 20, kFpStages = 4, kFpMaxSplit = 8;
+constexpr size_t kFpSmemBytes = sizeof(float) * kFpStages * (kFpBM + kFpBN) * kFpPitch;   // >= the 64 x 68 tile of sums
+
 struct ConvTiledParams {
     int kh, kw, sh, sw, ph, pw, dh, dw;
     int cin_pad;                 // k extent of one tap in the packed weights

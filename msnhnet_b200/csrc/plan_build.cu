@@ -878,6 +878,7 @@ int build_launches(MsnhB200Plan *pl) {
         if (L.kind == L_CONV_DIRECT)
             L.tiled = L.groups == 1 && aligned(L.in) && (L.out.N * static_cast<long long>(L.out.H) * L.out.W + kCtBM - 1) / kCtBM < 2147483647LL &&
                       (L.out.C + kCtBN - 1) / kCtBN <= 65535 && !dbg.conv_simple;
+        if (L.kind == L_CONV_DIRECT && L.tiled && pl->dtype == MSNH_B200_F32) configure_conv_fp32(pl, L);
         if (L.kind == L_CONV_DIRECT && L.tiled) L.note += L.note.empty() ? "fp32 arithmetic, shared-memory tiles" : ", fp32 arithmetic, shared-memory tiles";
         pl->launches.push_back(L);
     }

@@ -80,6 +80,7 @@ struct PlanDebugOptions {
     int autotune = -1;          // MSNH_B200_AUTOTUNE: -1 unset (time six runners-up), 0 off, n runners-up
     int trace_tile = 0;         // MSNH_B200_TRACE_TILE: which tile of a CTA the producer / MMA stamps describe
     int forced_mm = 0, forced_bn = 0;   // MSNH_B200_M_MULT, MSNH_B200_BN: force the conv tile shape
+    int fp32_split = 0;         // MSNH_B200_FP32_SPLIT: force the k split of the fp32 conv (1..8)
     int stream_k = 0;           // MSNH_B200_STREAM_K: -1 by cost, 0 never, 1 wherever possible
     int pair = 0;               // MSNH_B200_PAIR: 1 = CTA pairs wherever possible
     static PlanDebugOptions from_env();
@@ -149,7 +150,8 @@ struct Launch {
     int grid = 0; size_t smem = 0;
     // depthwise 3x3 on shared-memory tiles (map_a = the input's 4-D tensor map; grid / smem above)
     bool dw_tile = false; DwTileParams dwp{};
-    bool tiled = false;        // L_CONV_DIRECT: dense conv on aligned views -> the shared-memory-tiled CUDA-core kernel
+    bool tiled = false;        // L_CONV_DIRECT: dense conv on aligned views -> the shared-memory-tiled CUDA-core kernels
+    int fp_split = 1;          // ... fp32: CTAs of a cluster that share a tile's k (1..8)
     // accounting
     double flops = 0, bytes = 0;
     std::string note;
@@ -262,6 +264,8 @@ int tile_tuning_begin(MsnhB200Plan *pl, TileTuning &tt);
 int tile_tuning_end(MsnhB200Plan *pl, TileTuning &tt);
 // tile shape, ring sizes, grid, shared memory and tensor maps of a tensor-core conv launch whose views are resolved
 int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L);
+// k split of a CUDA-core fp32 conv launch
+void configure_conv_fp32(MsnhB200Plan *pl, Launch &L);
 // the shared-memory tile form of a 3x3 depthwise launch, where it applies (sets L.dw_tile)
 void configure_dw_tile(MsnhB200Plan *pl, Launch &L);
 
@@ -301,6 +305,7 @@ int prepare_yolo_nms(MsnhB200Ctx *ctx);           // shared memory opt-in of the
 void launch_yolo_nms(const float *rows, const int *counts, int max_rows, float nms_thresh, int use_soft_nms, float sigma,
                      float *boxes, int box_pitch, int *box_counts, int n_images, cudaStream_t st);
 void prepare_dw_tile_launch(int dtype);
+void prepare_conv_fp32_launch();                  // shared memory opt-in of the fp32 conv kernels
 void launch_fill(MsnhB200Ctx *ctx, float *dst, size_t n, float value, cudaStream_t st);
 
 // ---- plan.cu ----

@@ -109,6 +109,17 @@ void launch_typed(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st) {
             if (L.tiled) {
                 const ConvTiledParams cp{L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, L.dh, L.dw, L.cin_pad, L.scale, L.bias, L.res, L.ldc_res, L.act1, L.act1_p, L.act2, L.act2_p};
                 const int m_total = L.out.N * L.out.H * L.out.W;
+                if constexpr (sizeof(T) == 4) {
+                    cudaLaunchConfig_t cfg = {};
+                    cfg.gridDim = dim3((m_total + kFpBM - 1) / kFpBM, (L.out.C + kFpBN - 1) / kFpBN, L.fp_split);
+                    cfg.blockDim = dim3(kFpThreads); cfg.dynamicSmemBytes = kFpSmemBytes; cfg.stream = st;
+                    cudaLaunchAttribute attr[2];
+                    int na = 0;
+                    if (L.fp_split > 1) { attr[na].id = cudaLaunchAttributeClusterDimension; attr[na].val.clusterDim.x = 1; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = L.fp_split; ++na; }
+                    if (ctx->pdl) { attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[na].val.programmaticStreamSerializationAllowed = 1; ++na; }
+                    cfg.attrs = attr; cfg.numAttrs = na;
+                    cudaLaunchKernelEx(&cfg, conv_fp32_kernel, L.in, L.out, static_cast<const float *>(L.weights), cp);
+                } else
                 launch_k(ctx->pdl, conv_tiled_kernel<T>, dim3((m_total + kCtBM - 1) / kCtBM, (L.out.C + kCtBN - 1) / kCtBN), kCtThreads, 0, st, L.in, L.out, static_cast<const T *>(L.weights), cp);
                 break;
             }
@@ -280,6 +291,9 @@ void launch_yolo_nms(const float *rows, const int *counts, int max_rows, float n
 }
 void launch_fill(MsnhB200Ctx *ctx, float *dst, size_t n, float value, cudaStream_t st) {
     fill_kernel<<<ctx->sm_count * 8, 256, 0, st>>>(dst, n, value);
+}
+void prepare_conv_fp32_launch() {
+    cudaFuncSetAttribute(conv_fp32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kFpSmemBytes));
 }
 // dynamic shared memory opt-in of the depthwise tile kernels of one dtype
 void prepare_dw_tile_launch(int dtype) {

@@ -117,6 +117,28 @@ void configure_dw_tile(MsnhB200Plan *pl, Launch &L) {
     }
 }
 
+void configure_conv_fp32(MsnhB200Plan *pl, Launch &L) {
+    const int m_total = L.out.N * L.out.H * L.out.W, steps = (L.kh * L.kw * (L.cin_pad / 4) + 3) / 4;
+    const long tiles = static_cast<long>((m_total + kFpBM - 1) / kFpBM) * ((L.out.C + kFpBN - 1) / kFpBN);
+    // Measured: a k-step of 1 / 2 / 3 / 4 CTAs that share an SM takes 0.65 / 1.15 / 1.5 / 1.86 us for all of them (a CTA alone
+    // cannot hide its own latencies), and clusters of three and more do not spread over all SMs: the second CTA of some SM
+    // arrives at about 128.
+    double best = 0;
+    for (int split = 1; split <= kFpMaxSplit; ++split) {
+        if (split > 1 && steps < 4 * split) break;                        // a share no longer than the ring is all start-up
+        const double spread = split <= 2 ? pl->ctx->sm_count : pl->ctx->sm_count * 0.88;
+        const double per_sm = std::ceil(tiles * split / spread);          // CTAs of the busiest SM
+        const double step_us = per_sm <= 4 ? 0.25 + 0.4 * per_sm : 0.46 * per_sm;
+        const double cost = ((steps + split - 1) / split) * step_us + (split > 1 ? 1.0 + 0.3 * split : 0.0);
+        if (split == 1 || cost < best) { best = cost; L.fp_split = split; }
+    }
+    if (pl->dbg.fp32_split >= 1 && pl->dbg.fp32_split <= kFpMaxSplit) L.fp_split = pl->dbg.fp32_split;
+    prepare_conv_fp32_launch();
+    char note[64];
+    snprintf(note, sizeof(note), "%ld tiles of %d k-steps, k over %d CTAs", tiles, steps, L.fp_split);
+    L.note += (L.note.empty() ? "" : ", ") + std::string(note);
+}
+
 int tile_tuning_begin(MsnhB200Plan *pl, TileTuning &tt) {
     // MSNH_B200_AUTOTUNE=0 keeps the modelled tile shapes; plans made for debugging (no graph, no fusion, every output
     // kept, traced) keep them too
