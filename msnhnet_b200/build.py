@@ -54,7 +54,7 @@ def build_kernels(force=False, verbose=False):
 
 
 def build_host(force=False):
-    deps = _sources(HOST, (".cpp", ".h")) + [os.path.join(ROOT, "include", "msnh_b200.h"),
+    deps = _sources(HOST, (".cpp", ".h")) + [os.path.join(CSRC, "host_pool.h"), os.path.join(ROOT, "include", "msnh_b200.h"),
                                              os.path.join(ROOT, "include", "msnhnet_capi.h")]
     deps = [d for d in deps if os.path.exists(d)]
     if not force and not _newer(HOST_LIB, deps):

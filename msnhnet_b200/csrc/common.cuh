@@ -17,6 +17,12 @@ __device__ __forceinline__ float round_tf32(float x) {
     return __uint_as_float(r);
 }
 
+// An error code for the host (the flag is pinned host memory; any one of several codes will do).
+__device__ __forceinline__ void report_error(int *flag, int code) {
+    *reinterpret_cast<volatile int *>(flag) = code;
+    __threadfence_system();
+}
+
 // Programmatic dependent launch: let the next grid in the stream be scheduled early, then wait until
 // every grid this one depends on has completed and its writes are visible. Both are no-ops for a
 // grid launched without the attribute. Called first thing by every kernel that reads tensors.

@@ -92,7 +92,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         if (*cta_abort) return false;
         if (clock64() - t0 > kWaitCycles) {
             *cta_abort = 1;
-            atomicCAS(err_flag, 0, code);
+            report_error(err_flag, code);
             return false;
         }
     }
@@ -796,7 +796,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         for (int j = sk_first; j < static_cast<int>(blockIdx.x) && ok; ++j) {
                             const long long t0 = clock64();
                             while (*reinterpret_cast<volatile int *>(p.sk_flags + j) == 0) {
-                                if (*cta_abort || clock64() - t0 > kWaitCycles) { *cta_abort = 1; atomicCAS(p.err_flag, 0, DEV_ERR_WAIT_ACC_FULL); ok = false; break; }
+                                if (*cta_abort || clock64() - t0 > kWaitCycles) { *cta_abort = 1; report_error(p.err_flag, DEV_ERR_WAIT_ACC_FULL); ok = false; break; }
                             }
                         }
                         __threadfence();

@@ -1,0 +1,90 @@
+// A few host threads for the work the entry points do beside the device: copies between the caller's pageable memory and
+// pinned staging (one thread copies at about 10 GB/s, PCIe takes 55), score sort + NMS of several images. A pool belongs to
+// one context or net, is started when that first has enough work for it, sleeps between jobs and ends with its owner. Driven by
+// one thread at a time, like its owner.
+#pragma once
+#include <sched.h>
+#include <atomic>
+#include <condition_variable>
+#include <functional>
+#include <memory>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace msnh {
+
+class HostPool {
+public:
+    // threads besides the caller: half of the cpus this process may use, seven at most (eight copying threads fill PCIe)
+    static int default_workers() {
+        cpu_set_t set;
+        int cpus = static_cast<int>(std::thread::hardware_concurrency());
+        if (sched_getaffinity(0, sizeof(set), &set) == 0) cpus = CPU_COUNT(&set);
+        return std::max(0, std::min(7, cpus / 2 - 1));
+    }
+    explicit HostPool(int workers) {
+        for (int t = 0; t < workers; ++t) threads_.emplace_back([this]() { work(); });
+    }
+    ~HostPool() {
+        { std::lock_guard<std::mutex> g(m_); stop_ = true; }
+        wake_.notify_all();
+        for (auto &t : threads_) t.join();
+    }
+    HostPool(const HostPool &) = delete;
+    HostPool &operator=(const HostPool &) = delete;
+
+    // Starts fn(0) .. fn(n - 1) (fn must not throw). The caller takes part through help() / finish() and has to call finish().
+    void begin(int n, std::function<void(int)> fn) {
+        std::unique_lock<std::mutex> g(m_);
+        idle_.wait(g, [&]() { return active_ == 0; });       // a worker that woke late for the job before
+        fn_ = std::move(fn); n_ = n;
+        if (static_cast<int>(done_size_) < n) { done_.reset(new std::atomic<bool>[n]); done_size_ = n; }
+        for (int i = 0; i < n; ++i) done_[i].store(false, std::memory_order_relaxed);
+        next_.store(0, std::memory_order_relaxed);
+        ++job_;
+        g.unlock();
+        wake_.notify_all();
+    }
+    bool help() {                                             // one item on the calling thread; false: none left to start
+        const int i = next_.fetch_add(1, std::memory_order_acq_rel);
+        if (i >= n_) return false;
+        fn_(i);
+        done_[i].store(true, std::memory_order_release);
+        return true;
+    }
+    bool done(int i) const { return done_[i].load(std::memory_order_acquire); }
+    void finish() {
+        while (help()) {}
+        for (int i = 0; i < n_; ++i) while (!done(i)) std::this_thread::yield();
+    }
+    void run(int n, std::function<void(int)> fn) { begin(n, std::move(fn)); finish(); }
+
+private:
+    void work() {
+        unsigned long seen = 0;
+        std::unique_lock<std::mutex> g(m_);
+        while (true) {
+            wake_.wait(g, [&]() { return stop_ || job_ != seen; });
+            if (stop_) return;
+            seen = job_;
+            ++active_;
+            g.unlock();
+            while (help()) {}
+            g.lock();
+            if (--active_ == 0) idle_.notify_all();
+        }
+    }
+    std::mutex m_;
+    std::condition_variable wake_, idle_;
+    std::vector<std::thread> threads_;
+    std::function<void(int)> fn_;
+    std::unique_ptr<std::atomic<bool>[]> done_;
+    size_t done_size_ = 0;
+    int n_ = 0, active_ = 0;
+    std::atomic<int> next_{0};
+    unsigned long job_ = 0;
+    bool stop_ = false;
+};
+
+}  // namespace msnh

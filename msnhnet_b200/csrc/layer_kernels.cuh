@@ -895,6 +895,14 @@ __global__ void yolo_decode_collect_kernel(const __grid_constant__ YoloHeadSet h
     }
 }
 
+// The candidates of a batch to pinned host memory, a CTA per image: the count and the first `cap` rows of those there are. A few
+// KB of posted writes in one launch, in place of a copy of every row a slot could hold.
+__global__ void candidates_to_host_kernel(const float4 *__restrict__ rows, int max_rows, const int *__restrict__ counts, float4 *host_rows, int cap, int *host_counts) {
+    const int n = blockIdx.x, count = counts[n], take = 2 * min(min(count, max_rows), cap);
+    if (threadIdx.x == 0) host_counts[n] = count;
+    for (int i = threadIdx.x; i < take; i += blockDim.x) host_rows[static_cast<size_t>(n) * cap * 2 + i] = rows[static_cast<size_t>(n) * max_rows * 2 + i];
+}
+
 // ---- raw 8-bit image -> the net's fp32 planar input ----
 // What the reference's C API does on the host before the forward (src/c_api/MsnhnetLib.cpp:540-600, :754-778 with
 // src/utils/MsnhCVUtil.cpp:91-373 and the bilinear MatOp::resize, src/cv/MsnhCVMatOp.cpp:142-160, :399-434):

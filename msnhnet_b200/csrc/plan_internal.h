@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "../../include/msnh_b200.h"
+#include "host_pool.h"
 #include "kernel_params.h"
 
 // ------------------------------------------------------------------------------------------------
@@ -48,7 +49,9 @@ struct MsnhB200Ctx {
     cudaStream_t stream = nullptr;
     EncodeTiledFn encode_tiled = nullptr;
     EncodeIm2colFn encode_im2col = nullptr;
-    int *dev_err_flag = nullptr;
+    int *dev_err_flag = nullptr;    // device address of *err_flag
+    volatile int *err_flag = nullptr;   // pinned host memory the kernels write an error code to: looking at it costs no copy
+    std::unique_ptr<msnh::HostPool> pool;   // copies of pageable memory (started by the first large one)
     bool pdl = true;                // programmatic dependent launch between consecutive kernels (MSNH_B200_NO_PDL=1 turns it off)
     float *flush_buf = nullptr;     // > L2 size, for per-launch profiling
     size_t flush_elems = 0;
@@ -209,19 +212,23 @@ struct MsnhB200Plan {
     std::vector<std::array<int32_t, 3>> pack_picks; // conv tile shapes (sub-tiles, channels, form) in launch order: stored in / taken from the pack
     uint8_t *d_pack = nullptr;
     std::vector<uint8_t> pack_blob; uint64_t pack_blob_bytes = 0, pack_blob_key = 0, pack_blob_tag = 0;   // a probed pack file: its arena bytes until they are copied
-    float *h_pinned = nullptr; size_t h_pinned_bytes = 0;   // staging for pageable callers
+    uint8_t *h_pinned = nullptr; size_t h_pinned_bytes = 0; bool staging_busy = false;   // pinned staging for callers whose memory is pageable; a copy out of it may be under way (ev_copy)
     int *h_counts = nullptr;                        // pinned
+    // Results of the last synchronous run, written to pinned memory behind its kernels so that the read call finds them there:
+    // candidate counts and the first kEarlyRows rows per image, or the one small output of a classifier.
+    int early_op = -1;                              // the op they belong to (-1: the plan has none that qualifies)
+    bool early_valid = false; int early_images = 0;
+    float *h_early = nullptr; int *h_early_counts = nullptr;
     cudaGraph_t graph = nullptr; cudaGraphExec_t graph_exec = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    float last_ms = 0.f;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_copy = nullptr;
+    float last_ms = 0.f; int timed_steps = 0;       // last_ms is brought up to date from the events when it is asked for (0 steps: it is)
     std::string description;
     // pipelined streaming (plan_stream_push / pop): two slots, a copy stream next to the compute stream
     struct StreamSlot {
         float *d_stage = nullptr;        // this slot's fp32 NCHW input staging on the device
         float *h_result = nullptr;       // pinned: candidate rows or output floats of the batch
         int   *h_counts = nullptr;       // pinned: candidate counts per image
-        float *d_result = nullptr;       // device: this slot's copy of the result (candidate rows or output floats)
-        int   *d_counts = nullptr;       // device: this slot's copy of the candidate counts + the error flag
+        float *d_result = nullptr;       // device: this slot's copy of an output (candidates go straight to h_result)
         cudaEvent_t h2d_done = nullptr, consumed = nullptr, fwd_done = nullptr, done = nullptr;
         int n_images = 0; bool busy = false;
         cudaGraphExec_t graph_exec = nullptr;   // the plan's graph with this slot's staging buffer as the image (float pushes: no device copy)
@@ -308,7 +315,17 @@ void prepare_dw_tile_launch(int dtype);
 void prepare_conv_fp32_launch();                  // shared memory opt-in of the fp32 conv kernels
 void launch_fill(MsnhB200Ctx *ctx, float *dst, size_t n, float value, cudaStream_t st);
 
+void launch_candidates_to_host(const float *rows, int max_rows, const int *counts, float *host_rows, int cap, int *host_counts, int n_images, cudaStream_t st);
+
 // ---- plan.cu ----
 int check_device_flag(MsnhB200Plan *pl);
+constexpr int kEarlyRows = 512;                     // candidate rows per image that come back with a synchronous run
+constexpr size_t kEarlyOutputBytes = 1 << 20;       // largest output that does
+// Copy to / from the caller's memory that ends or begins on ctx->stream: pageable memory of half a megabyte or more goes through
+// pinned staging, chunk by chunk, copied by the pool's threads.
+bool is_pageable(const void *p);
+int copy_in(MsnhB200Plan *pl, void *dev, const void *host, size_t bytes);
+int copy_out(MsnhB200Plan *pl, void *host, const void *dev, size_t bytes);   // the data is there when it returns
+void parallel_memcpy(MsnhB200Ctx *ctx, void *dst, const void *src, size_t bytes);
 
 }  // namespace msnh

@@ -276,6 +276,10 @@ void launch_readback(MsnhB200Ctx *ctx, int dtype, const TView &v, float *dst_nch
     if (dtype == MSNH_B200_F16) nhwc_to_nchw_f32_kernel<__half><<<grid, 256, 0, st>>>(v, dst_nchw);
     else                        nhwc_to_nchw_f32_kernel<float><<<grid, 256, 0, st>>>(v, dst_nchw);
 }
+// host_rows / host_counts: pinned memory the device writes to directly, only the rows that exist
+void launch_candidates_to_host(const float *rows, int max_rows, const int *counts, float *host_rows, int cap, int *host_counts, int n_images, cudaStream_t st) {
+    candidates_to_host_kernel<<<n_images, 256, 0, st>>>(reinterpret_cast<const float4 *>(rows), max_rows, counts, reinterpret_cast<float4 *>(host_rows), cap, host_counts);
+}
 void launch_preprocess_u8(const unsigned char *src, float *dst, const PrepParams &p, int n_images, cudaStream_t st) {
     // n_images raw images of p.w x p.h back to back -> n_images planar float images back to back, one launch
     const dim3 grid((p.out_w + 127) / 128, p.out_h, n_images);

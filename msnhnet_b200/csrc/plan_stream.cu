@@ -24,11 +24,12 @@ int msnh_b200_plan_preprocess_u8(MsnhB200Plan *pl, const unsigned char *host_hwc
         CUDA_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&pl->d_u8), bytes));
         pl->d_u8_bytes = bytes;
     }
-    CUDA_TRY(ctx, cudaMemcpyAsync(pl->d_u8, host_hwc, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    { const int rc = copy_in(pl, pl->d_u8, host_hwc, bytes); if (rc) return rc; }
     launch_preprocess_u8(pl->d_u8, pl->d_input + static_cast<size_t>(image) * 3 * pl->in_h * pl->in_w, p, 1, ctx->stream);
     CUDA_TRY(ctx, cudaGetLastError());
-    // the staging image may be overwritten by the next call: finish this one first
-    CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
+    // The caller may overwrite its image when this returns: a pageable one has been copied on by then, a pinned one is read by
+    // the device itself. Everything after that is in stream order.
+    if (!is_pageable(host_hwc)) CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     return MSNH_B200_OK;
 }
 
@@ -99,9 +100,8 @@ static int stream_setup(MsnhB200Plan *pl, int op) {
     for (auto &s : pl->slots) {
         CUDA_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&s.d_stage), in_elems * sizeof(float)));
         CUDA_TRY(ctx, cudaMallocHost(reinterpret_cast<void **>(&s.h_result), pl->stream_result_floats * sizeof(float)));
-        CUDA_TRY(ctx, cudaMallocHost(reinterpret_cast<void **>(&s.h_counts), sizeof(int) * (pl->batch + 1)));   // + the device error flag
-        CUDA_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&s.d_result), pl->stream_result_floats * sizeof(float)));
-        CUDA_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&s.d_counts), sizeof(int) * (pl->batch + 1)));
+        CUDA_TRY(ctx, cudaMallocHost(reinterpret_cast<void **>(&s.h_counts), sizeof(int) * pl->batch));
+        if (!pl->stream_cap) CUDA_TRY(ctx, cudaMalloc(reinterpret_cast<void **>(&s.d_result), pl->stream_result_floats * sizeof(float)));
         CUDA_TRY(ctx, cudaEventCreateWithFlags(&s.fwd_done, cudaEventDisableTiming));
         CUDA_TRY(ctx, cudaEventCreateWithFlags(&s.h2d_done, cudaEventDisableTiming));
         CUDA_TRY(ctx, cudaEventCreateWithFlags(&s.consumed, cudaEventDisableTiming));
@@ -168,42 +168,34 @@ static int stream_push_common(MsnhB200Plan *pl, int op, const void *host_images,
         else for (const Launch &L : pl->launches) launch_one(ctx, L, ctx->stream);
     }
     const OpState &o = pl->ops[op];
-    // The result goes to the slot's own device buffer on the compute stream (a short device copy), and
-    // from there to pinned host memory on a third stream, so the next forward does not wait for PCIe.
-    // The conv kernels' error flag rides along.
-    size_t result_bytes;
+    pl->early_valid = false;
+    // A short result (candidates, boxes, logits) is written to the slot's pinned memory by a kernel behind the forward. A long one
+    // goes to the slot's own device buffer on the compute stream and from there to pinned memory on a third stream, so that the
+    // next forward does not wait for PCIe.
+    const Launch *zl = nullptr;
     if (pl->stream_cap) {
-        const Launch *zl = nullptr;
         for (const Launch &L : pl->launches) if (L.kind == L_COLLECT_ZERO && L.op == op) zl = &L;
         if (!zl) return fail(ctx, MSNH_B200_ERR_STATE, "collect launch missing");
-        if (pl->stream_nms) {
-            // sort + NMS on the device, straight into the slot: only the kept boxes cross PCIe
-            const int cap = std::min(pl->stream_cap, kNmsMaxCandidates);
-            launch_yolo_nms(zl->rows, zl->counts, zl->max_rows, pl->nms_thresh, pl->nms_soft, pl->nms_sigma, s.d_result, pl->stream_cap, s.d_counts, n_images, ctx->stream);
-            (void)cap; result_bytes = 0;   // copied as a 2-D block below
-        } else {
-            CUDA_TRY(ctx, cudaMemcpyAsync(s.d_counts, zl->counts, sizeof(int) * n_images, cudaMemcpyDeviceToDevice, ctx->stream));
-            CUDA_TRY(ctx, cudaMemcpy2DAsync(s.d_result, static_cast<size_t>(pl->stream_cap) * 32, zl->rows, static_cast<size_t>(zl->max_rows) * 32,
-                                            static_cast<size_t>(pl->stream_cap) * 32, n_images, cudaMemcpyDeviceToDevice, ctx->stream));
-            result_bytes = static_cast<size_t>(pl->stream_cap) * 32 * n_images;
-        }
-    } else {
-        const size_t per = static_cast<size_t>(o.out.C) * o.out.H * o.out.W;
+    }
+    const size_t per = static_cast<size_t>(o.out.C) * o.out.H * o.out.W;
+    const bool direct = pl->stream_cap || per * n_images * sizeof(float) <= kEarlyOutputBytes;
+    if (pl->stream_cap && pl->stream_nms)
+        launch_yolo_nms(zl->rows, zl->counts, zl->max_rows, pl->nms_thresh, pl->nms_soft, pl->nms_sigma, s.h_result, pl->stream_cap, s.h_counts, n_images, ctx->stream);
+    else if (pl->stream_cap)
+        launch_candidates_to_host(zl->rows, zl->max_rows, zl->counts, s.h_result, pl->stream_cap, s.h_counts, n_images, ctx->stream);
+    else {
         TView v = view_of(pl, o.tensor);
         v.N = n_images;
-        launch_readback(ctx, pl->tensors[o.tensor].dtype, v, s.d_result, per * n_images, ctx->stream);
-        result_bytes = per * n_images * sizeof(float);
+        launch_readback(ctx, pl->tensors[o.tensor].dtype, v, direct ? s.h_result : s.d_result, per * n_images, ctx->stream);
     }
-    CUDA_TRY(ctx, cudaMemcpyAsync(s.d_counts + pl->batch, ctx->dev_err_flag, sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
-    CUDA_TRY(ctx, cudaEventRecord(s.fwd_done, ctx->stream));
-    CUDA_TRY(ctx, cudaStreamWaitEvent(pl->d2h_stream, s.fwd_done, 0));
-    CUDA_TRY(ctx, cudaMemcpyAsync(s.h_counts, s.d_counts, sizeof(int) * (pl->batch + 1), cudaMemcpyDeviceToHost, pl->d2h_stream));
-    if (pl->stream_cap && pl->stream_nms)
-        CUDA_TRY(ctx, cudaMemcpy2DAsync(s.h_result, static_cast<size_t>(pl->stream_cap) * 32, s.d_result, static_cast<size_t>(pl->stream_cap) * 32,
-                                        static_cast<size_t>(std::min(pl->stream_cap, kNmsMaxCandidates)) * 32, n_images, cudaMemcpyDeviceToHost, pl->d2h_stream));
-    else
-        CUDA_TRY(ctx, cudaMemcpyAsync(s.h_result, s.d_result, result_bytes, cudaMemcpyDeviceToHost, pl->d2h_stream));
-    CUDA_TRY(ctx, cudaEventRecord(s.done, pl->d2h_stream));
+    CUDA_TRY(ctx, cudaGetLastError());
+    if (direct) CUDA_TRY(ctx, cudaEventRecord(s.done, ctx->stream));
+    else {
+        CUDA_TRY(ctx, cudaEventRecord(s.fwd_done, ctx->stream));
+        CUDA_TRY(ctx, cudaStreamWaitEvent(pl->d2h_stream, s.fwd_done, 0));
+        CUDA_TRY(ctx, cudaMemcpyAsync(s.h_result, s.d_result, per * n_images * sizeof(float), cudaMemcpyDeviceToHost, pl->d2h_stream));
+        CUDA_TRY(ctx, cudaEventRecord(s.done, pl->d2h_stream));
+    }
     s.n_images = n_images; s.busy = true;
     ++pl->push_count;
     return MSNH_B200_OK;
@@ -265,12 +257,11 @@ int msnh_b200_plan_stream_pop(MsnhB200Plan *pl, float *result, size_t capacity_f
         const OpState &o = pl->ops[pl->stream_op];
         const size_t n = static_cast<size_t>(s.n_images) * o.out.C * o.out.H * o.out.W;
         if (capacity_floats < n) return fail(ctx, MSNH_B200_ERR_ARG, "stream_pop: output buffer too small (%zu floats needed)", n);
-        std::memcpy(result, s.h_result, n * sizeof(float));
+        parallel_memcpy(ctx, result, s.h_result, n * sizeof(float));
     }
     s.busy = false;
     ++pl->pop_count;
-    if (s.h_counts[pl->batch] != 0) return check_device_flag(pl);
-    return MSNH_B200_OK;
+    return check_device_flag(pl);
 }
 
 int msnh_b200_plan_stream_reset(MsnhB200Plan *pl) {

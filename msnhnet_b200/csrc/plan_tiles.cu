@@ -376,9 +376,7 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
                     *ms = std::min(*ms, burst);
                 }
                 // a shape whose bounded waits ran out is no candidate (and must not leave the flag set)
-                int flag = 0;
-                CUDA_TRY(ctx, cudaMemcpy(&flag, ctx->dev_err_flag, sizeof(int), cudaMemcpyDeviceToHost));
-                if (flag != 0) { CUDA_TRY(ctx, cudaMemset(ctx->dev_err_flag, 0, sizeof(int))); *ms = 1e30f; }
+                if (*ctx->err_flag != 0) { *ctx->err_flag = 0; *ms = 1e30f; }
                 return MSNH_B200_OK;
             };
             float best_ms = 0.f;

@@ -10,6 +10,7 @@
 #include "msnh_format.h"
 
 #include "msnh_b200.h"      // MsnhB200Op (the context and plan types stay opaque)
+#include "../csrc/host_pool.h"
 
 namespace Msnhnet {
 
@@ -168,6 +169,11 @@ private:
     bool _packCache = false, _usedPack = false;
     std::string _detail;
     std::vector<float> _candRows; std::vector<int> _candCounts; int _maxRows = 0;
+    std::vector<float> _streamRows; std::vector<int> _streamCounts;      // what a streaming call pops into, kept from call to call
+    std::unique_ptr<msnh::HostPool> _pool;                               // NMS of several images (started by the first call with enough of it)
+    void readCandidates(int nImages, std::vector<int> &counts);         // into _candRows
+    // boxes of several images at once: rows of image i (count counts[i]; negative: none) start at rows + i * pitch
+    void postProcessImages(const float *rows, size_t pitch, const int *counts, int nImages, std::vector<YoloBox> *out);
 };
 
 }  // namespace Msnhnet
