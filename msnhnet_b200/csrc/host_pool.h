@@ -4,6 +4,7 @@
 // one thread at a time, like its owner.
 #pragma once
 #include <sched.h>
+#include <algorithm>
 #include <atomic>
 #include <condition_variable>
 #include <functional>
@@ -18,10 +19,13 @@ class HostPool {
 public:
     // threads besides the caller: half of the cpus this process may use, seven at most (eight copying threads fill PCIe)
     static int default_workers() {
-        cpu_set_t set;
-        int cpus = static_cast<int>(std::thread::hardware_concurrency());
-        if (sched_getaffinity(0, sizeof(set), &set) == 0) cpus = CPU_COUNT(&set);
-        return std::max(0, std::min(7, cpus / 2 - 1));
+        static const int workers = []() {
+            cpu_set_t set;
+            int cpus = static_cast<int>(std::thread::hardware_concurrency());
+            if (sched_getaffinity(0, sizeof(set), &set) == 0) cpus = CPU_COUNT(&set);
+            return std::max(0, std::min(7, cpus / 2 - 1));
+        }();
+        return workers;
     }
     explicit HostPool(int workers) {
         for (int t = 0; t < workers; ++t) threads_.emplace_back([this]() { work(); });
