@@ -299,6 +299,11 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
     u.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(u.bn >> 3) << 17) |
               (static_cast<uint32_t>((u.pair ? 2 * kUmmaM : kUmmaM) >> 4) << 24);
     u.tiles_m = (u.m_total + tile_rows - 1) / tile_rows;
+    // Where no CTA has a second tile the drain of its only one is on the critical path: with fewer than four store units per
+    // lane quarter some of the sixteen epilogue warps would watch, so the units get narrower (16 columns at least). A forward of
+    // YOLOv4-608 with one image 0.831 -> 0.792 ms, of MobileNetV2 0.227 -> 0.210.
+    if (!u.pair && !u.stream_k && u.tiles_m * u.tiles_n <= ctx->sm_count)
+        while (u.out_chunk_bytes / 2 >= 16 * es && u.m_mult * ((u.bn * es + u.out_chunk_bytes - 1) / u.out_chunk_bytes) < 4) u.out_chunk_bytes /= 2;
     const int acc_cols = u.m_mult * u.bn;
     // accumulator ring: as many stages (2, 4, 8) as fit in the 512 TMEM columns; the epilogue reads 32
     // columns at a time, so the last accumulator needs up to 32 columns of room
