@@ -377,7 +377,8 @@ __device__ __forceinline__ void activate_pairs(F2 (&y)[8], int act, float param)
 template <typename T, int kMult, bool kPair, bool kStreamK, int kAct = kActGeneric, bool kTrace = false>   // kMult: 128-pixel sub-tiles per tile (1, 2, 3, 4)
 __global__ void __launch_bounds__(kUmmaThreads, 1)
 conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                 const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_c2, const ConvUmmaParams p) {
+                 const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_c2,
+                 const __grid_constant__ CUtensorMap map_res, const ConvUmmaParams p) {
     constexpr bool kTf32 = sizeof(T) == 4;
     extern __shared__ uint8_t smem_raw[];
     // 1024-byte alignment of the operand stages (required by the 128-byte swizzle atoms).
@@ -401,6 +402,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     auto empty_bar     = [&](int s) { return bar_base + 8u * (kUmmaMaxStages + s); };
     auto acc_full_bar  = [&](int s) { return bar_base + 8u * (2 * kUmmaMaxStages + s); };
     auto acc_empty_bar = [&](int s) { return bar_base + 8u * (2 * kUmmaMaxStages + kUmmaMaxAccStages + s); };
+    auto res_bar       = [&](int e) { return bar_base + 8u * (2 * kUmmaMaxStages + 2 * kUmmaMaxAccStages + e); };
     const int acc_mask = (1 << p.acc_shift) - 1;
     // per-channel scale and bias of the whole layer, staged once (layers of up to kSbMaxChannels channels)
     const uint32_t sb_base = bar_base + 512;                 // [2][kSbMaxChannels] floats
@@ -448,6 +450,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c) : "memory");
         if (p.split_n != 0x7fffffff) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c2) : "memory");
+        if (!kPair && !kStreamK && p.res) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_res) : "memory");
         cta_abort_slot = 0;
         for (int s = 0; s < p.num_stages; ++s) { mbar_init(full_bar(s), 2); mbar_init(empty_bar(s), 1); }
         // arrivals that free an accumulator: the team epilogue's warps (pair / stream-K kernels), or one per warp and
@@ -455,6 +458,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int units = kMult * ((p.bn * static_cast<int>(sizeof(T)) + p.out_chunk_bytes - 1) / p.out_chunk_bytes);
         const uint32_t acc_arrivals = (kPair || kStreamK) ? 16u * (kPair ? 2u : 1u) : 4u * static_cast<uint32_t>(units);
         for (int s = 0; s <= acc_mask; ++s) { mbar_init(acc_full_bar(s), 1); mbar_init(acc_empty_bar(s), acc_arrivals); }
+        for (int e = 0; e < 16; ++e) mbar_init(res_bar(e), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -630,7 +634,12 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int e = warp - 2;
         const int grp = e >> 2;
         const int lane_base = (warp & 3) * 32;
-        const T *res = static_cast<const T *>(p.res);
+        // The residual of a unit comes by TMA into the staging tile its result will leave from (same box, same swizzle), asked for
+        // before the accumulator is waited for. Read row by row behind the accumulator it cost 1700 cycles per 16 columns: a
+        // forward of ResNet-18 fp32 with one image 0.262 -> 0.258 ms, of YOLOv4-608 0.779 -> 0.768.
+        const bool has_res = p.res != nullptr;
+        const bool one = elect_one();                // issues this warp's loads and stores and waits for the latter
+        uint32_t res_phase = 0;
         constexpr int kVec = Elem<T>::kVec;
         const int cols_per_store = p.out_chunk_bytes / static_cast<int>(sizeof(T));
         const int cols_shift = 31 - __clz(cols_per_store);                 // a power of two
@@ -652,6 +661,24 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             if (p.tiles_n > 1) { tm = tile / p.tiles_n; tn = tile - tm * p.tiles_n; }
             const int n0 = tn * p.bn;
             const int acc = tl & acc_mask;
+            int sub = 0, slab = item;
+            if (kMult > 1) { while (slab >= slabs_max) { slab -= slabs_max; ++sub; } }
+            const int slabs = (min(p.bn, p.cout - n0) + cols_per_store - 1) >> cols_shift;   // slabs this tile really has
+            const int c0 = slab << cols_shift;
+            const int mw = tm * tile_rows + sub * kUmmaM + lane_base;      // this warp's first pixel of the unit
+            const bool work = slab < slabs && mw < p.m_total;              // (otherwise nothing to compute, only the release below)
+            if (work) {
+                // the staging tile is free once the previous store of this warp has read it
+                if (store_pending) {
+                    if (one) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    __syncwarp();
+                }
+                if (has_res && one) {
+                    if (!store_pending) pdl_wait();          // (the first of them: the residual is an earlier kernel's output)
+                    mbar_expect_tx(res_bar(e), 32u * static_cast<uint32_t>(p.out_chunk_bytes));
+                    tma_load_2d(buf, &map_res, res_bar(e), n0 + c0, mw);
+                }
+            }
             if (tl != tl_ready) {                    // first unit of this tile for this warp: its accumulator has to be complete
                 const uint32_t acc_phase = static_cast<uint32_t>(tl >> p.acc_shift) & 1u;
                 ok = mbar_wait<true>(acc_full_bar(acc), acc_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_ACC_FULL);
@@ -660,19 +687,13 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 tl_ready = tl;
                 if constexpr (kTrace) { if (trace && e == 0 && lane == 0 && tl == 0) trace[40] = clock64(); }
             }
-            int sub = 0, slab = item;
-            if (kMult > 1) { while (slab >= slabs_max) { slab -= slabs_max; ++sub; } }
-            const int slabs = (min(p.bn, p.cout - n0) + cols_per_store - 1) >> cols_shift;   // slabs this tile really has
-            const int c0 = slab << cols_shift;
-            const int mw = tm * tile_rows + sub * kUmmaM + lane_base;      // this warp's first pixel of the unit
-            if (slab < slabs && mw < p.m_total) {                          // (otherwise nothing to compute, only the release below)
-                const int m = mw + lane;
-                const bool row_ok = m < p.m_total;
+            if (work) {
                 const uint32_t acc_col = static_cast<uint32_t>((acc * kMult + sub) * p.bn);
-                // the staging tile is free once the previous store of this warp has read it
-                if (store_pending) {
-                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                    __syncwarp();
+                if (has_res) {
+                    ok = mbar_wait(res_bar(e), res_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    res_phase ^= 1u;
                 }
                 for (int l0 = 0; l0 < cols_per_store; l0 += 16) {
                     uint32_t v[16];
@@ -700,16 +721,21 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         }
                     }
                     activate_pairs<kAct>(y, p.act1, p.act1_param);
-                    if (res && row_ok) {
-                        const T *rrow = res + static_cast<size_t>(m) * p.ldc_res + cbase;
+                    const uint32_t piece0 = static_cast<uint32_t>(l0 / kVec);
+                    if (has_res) {
 #pragma unroll
-                        for (int j = 0; j < 16; j += kVec) {
-                            if (cbase + j < p.cout) {
-                                float rr[kVec];
-                                ld_vec(rrow + j, rr);
+                        for (int q = 0; q < 16 / kVec; ++q) {
+                            uint32_t h[4];
+                            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(h[0]), "=r"(h[1]), "=r"(h[2]), "=r"(h[3]) : "r"(row_addr + (((piece0 + q) ^ row_swz) << 4)) : "memory");
+                            if constexpr (sizeof(T) == 2) {
 #pragma unroll
-                                for (int q = 0; q < kVec; q += 2)
-                                    y[(j + q) / 2] = f2_add(y[(j + q) / 2], f2_pack(rr[q], rr[q + 1]));
+                                for (int k = 0; k < 4; ++k) {
+                                    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&h[k]));
+                                    y[4 * q + k] = f2_add(y[4 * q + k], f2_pack(f.x, f.y));
+                                }
+                            } else {
+                                y[2 * q]     = f2_add(y[2 * q], f2_pack(__uint_as_float(h[0]), __uint_as_float(h[1])));
+                                y[2 * q + 1] = f2_add(y[2 * q + 1], f2_pack(__uint_as_float(h[2]), __uint_as_float(h[3])));
                             }
                         }
                         activate_pairs<kActGeneric>(y, p.act2, p.act2_param);
@@ -719,7 +745,6 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         for (int q = 0; q < 8; ++q) { float a, b; f2_unpack(y[q], a, b); y[q] = f2_pack(round_tf32(a), round_tf32(b)); }
                     }
                     // this thread's 16 columns of the slab, 16 bytes at a time, XOR-swizzled like the TMA map
-                    const uint32_t piece0 = static_cast<uint32_t>(l0 / kVec);
 #pragma unroll
                     for (int q = 0; q < 16 / kVec; ++q) {
                         const uint32_t addr = row_addr + (((piece0 + q) ^ row_swz) << 4);
@@ -738,7 +763,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // staging writes -> visible to the TMA engine
                 __syncwarp();
-                if (lane == 0) {
+                if (one) {
                     const bool second = n0 + c0 >= p.split_n;          // slab of the second of two merged convs
                     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
                                  ::"l"(second ? &map_c2 : &map_c), "r"(buf), "r"(second ? n0 + c0 - p.split_n : n0 + c0), "r"(mw) : "memory");
@@ -749,13 +774,13 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             // this warp's TMEM reads of the unit are done: one of the arrivals that hand the accumulator back to the MMA warp
             tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty_bar(acc));
+            if (one) mbar_arrive(acc_empty_bar(acc));
             if constexpr (kTrace) { if (trace && e == 0 && lane == 0) { if (u == 0) trace[41] = clock64(); trace[42] += 1; } }
             item += 4;
             while (item >= units_per_tile) { item -= units_per_tile; ++tl; }
         }
         // the staging tile must outlive the store's reads of it; the writes themselves are complete when the grid is
-        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        if (one) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     } else {
         // ------------------------------ epilogue (16 warps), CTA-pair and stream-K kernels ------------------------
         // Warp w may read TMEM lanes [32*(w%4), 32*(w%4)+32): one output pixel (row) per thread.

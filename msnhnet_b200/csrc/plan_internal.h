@@ -146,7 +146,7 @@ struct Launch {
     // yolo collect
     float *rows = nullptr; int *counts = nullptr; int max_rows = 0;
     // umma
-    CUtensorMap map_a, map_b, map_c, map_c2;
+    CUtensorMap map_a, map_b, map_c, map_c2, map_res;
     TView out2{};              // second output of two 1x1 convs over the same input merged into this launch (ptr == nullptr: none)
     int split_n = 0;           // its first channel in the merged channel range
     ConvUmmaParams up{};

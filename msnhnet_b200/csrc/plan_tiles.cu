@@ -345,6 +345,11 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
     rc = make_map_2d(ctx, &L.map_c, pl->dtype, L.out.ptr, static_cast<uint64_t>(L.out.C), static_cast<uint64_t>(u.m_total),
                      static_cast<uint64_t>(L.out.ldc) * es, static_cast<uint32_t>(u.out_chunk_bytes / es), store_rows, u.out_chunk_bytes);
     if (rc) return rc;
+    if (L.res) {      // the residual, read in the boxes the result is stored in
+        rc = make_map_2d(ctx, &L.map_res, pl->dtype, L.res, static_cast<uint64_t>(L.out.C), static_cast<uint64_t>(u.m_total),
+                         static_cast<uint64_t>(L.ldc_res) * es, static_cast<uint32_t>(u.out_chunk_bytes / es), store_rows, u.out_chunk_bytes);
+        if (rc) return rc;
+    }
     if (L.out2.ptr) {
         rc = make_map_2d(ctx, &L.map_c2, pl->dtype, L.out2.ptr, static_cast<uint64_t>(L.out2.C), static_cast<uint64_t>(u.m_total),
                          static_cast<uint64_t>(L.out2.ldc) * es, static_cast<uint32_t>(u.out_chunk_bytes / es), store_rows, u.out_chunk_bytes);
