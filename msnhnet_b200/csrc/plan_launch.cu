@@ -85,6 +85,15 @@ void launch_typed(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st) {
                 static_cast<const float *>(L.in.ptr), L.out);
             break;
         case L_INPUT_PATCH:
+            if constexpr (sizeof(T) == 2) {
+                // (a staged row holds kPatchTx pixels at a stride of 1 or 2, a tile's rows a vertical stride of as much)
+                if (L.ival == 3 && L.kh == 3 && L.kw == 3 && L.out.ldc == 32 && L.dh == 1 && L.dw == 1 && L.sh <= 2 && L.sw <= 2 && L.out.N <= 65535 && (L.out.H + kPatchTy - 1) / kPatchTy <= 65535) {
+                    const dim3 tiles((L.out.W + kPatchTx - 1) / kPatchTx, (L.out.H + kPatchTy - 1) / kPatchTy, L.out.N);
+                    launch_k(ctx->pdl, L.sw == 1 ? nchw_f32_to_patches3_kernel<1> : nchw_f32_to_patches3_kernel<2>, tiles, kPatchTx, 0, st,
+                             static_cast<const float *>(L.in.ptr), L.out, L.ival2, L.max_rows, L.sh, L.ph, L.pw);
+                    break;
+                }
+            }
             if (L.ival == 3 && L.kh == 3 && L.kw == 3 && L.out.ldc == 32)
                 launch_k(ctx->pdl, nchw_f32_to_patches_fixed_kernel<T, 3, 3, 3>, grid_for(ctx, static_cast<size_t>(L.out.N) * L.out.H * L.out.W, 128), 128, 0, st, 
                     static_cast<const float *>(L.in.ptr), L.out, L.ival2, L.max_rows, L.sh, L.sw, L.ph, L.pw, L.dh, L.dw);
@@ -176,6 +185,13 @@ void launch_typed(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st) {
                 break;
             }
             if (L.pools.n > 1) break;    // (cannot happen: pools are merged only where the plane form applies; plan_finalize checks)
+            if (L.vec && L.kh == 2 && L.kw == 2) {
+                const int cvn = L.out.C / V;
+                int lc = 0; while (lc < 8 && (2 << lc) <= cvn) ++lc;              // threads along channels: largest power of two <= channel vectors (<= 256)
+                launch_k(ctx->pdl, maxpool2_rows_kernel<T>, std::min(L.out.N * L.out.H, 16 * ctx->sm_count), 256, 0, st,
+                         L.in, L.out, L.sh, L.sw, L.ph, L.pw, lc);
+                break;
+            }
             if (L.vec) launch_k(ctx->pdl, maxpool_kernel<T, V>, grid, block, 0, st, L.in, L.out, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw);
             else       launch_k(ctx->pdl, maxpool_kernel<T, 1>, grid, block, 0, st, L.in, L.out, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw);
             break;
