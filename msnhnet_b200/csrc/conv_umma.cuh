@@ -330,12 +330,13 @@ template <int kAct>
 __device__ __forceinline__ void activate_pairs(F2 (&y)[8], int act, float param) {
     if constexpr (kAct == MSNH_ACT_MISH) mish_pairs(y);
     else if constexpr (kAct == MSNH_ACT_LEAKY) leaky_pairs(y, param);
-    else {
-        if (act == MSNH_ACT_NONE) return;
+    else if constexpr (kAct != MSNH_ACT_NONE) {
+        const int a = kAct == kActGeneric ? act : kAct;        // (a compile-time activation leaves no switch)
+        if (a == MSNH_ACT_NONE) return;
         float f[16];
 #pragma unroll
         for (int q = 0; q < 8; ++q) f2_unpack(y[q], f[2 * q], f[2 * q + 1]);
-        activate16(f, act, param);
+        activate16(f, a, param);
 #pragma unroll
         for (int q = 0; q < 8; ++q) y[q] = f2_pack(f[2 * q], f[2 * q + 1]);
     }
@@ -364,8 +365,8 @@ __device__ __forceinline__ void activate_pairs(F2 (&y)[8], int act, float param)
 // fp32 accumulators) to its slot in global memory and raises its flag; the CTA that owns the tile's last
 // k-block adds the slots of its predecessors before the usual epilogue. Each CTA handles the segment it
 // hands over first and the segment it has to complete last, so nobody waits on a CTA that is itself waiting.
-// kAct: MSNH_ACT_MISH / MSNH_ACT_LEAKY (slope in [0, 1]) compile the first activation into the epilogue loops, kActGeneric
-// switches at run time. kTrace: the instantiation that records clock stamps (plans made with MSNH_PLAN_TRACE); the
+// kAct: a compile-time first activation leaves no switch in the epilogue loops (MSNH_ACT_LEAKY: slope in [0, 1]);
+// kActGeneric switches at run time. kTrace: the instantiation that records clock stamps (plans made with MSNH_PLAN_TRACE); the
 // production instantiations carry none of that code.
 template <typename T, int kMult, bool kPair, bool kStreamK, int kAct = kActGeneric, bool kTrace = false>   // kMult: 128-pixel sub-tiles per tile (1, 2, 3, 4)
 __global__ void __launch_bounds__(kUmmaThreads, 1)

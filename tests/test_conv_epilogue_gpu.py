@@ -1,5 +1,6 @@
 """The tensor-core conv's epilogue where it can go wrong: residuals fetched in boxes that hang over the last pixel and
-channel, store units of every width, several tiles per CTA."""
+channel, store units of every width, several tiles per CTA, each
+activation in layers of one wave and of several."""
 import numpy as np
 import pytest
 
@@ -41,3 +42,20 @@ def test_residual_boxes(dtype, cout, h, w, batch):
             a = a.astype(np.float16).astype(np.float32)
         b = mo.activate(mo.conv2d(a, w2, 3, 3, 1, 1, 1, 1, 1, 1, 1), "leaky", [0.1])
         assert H.rel_err(got[i], np.maximum(a + b, 0)) < (2e-3 if dtype == ffi.F16 else H.TOL_F32)
+
+
+@pytest.mark.parametrize("dtype", [ffi.F32, ffi.F16])
+@pytest.mark.parametrize("h,w,batch", [(13, 13, 1), (151, 149, 2)])
+@pytest.mark.parametrize("act,name", [(ffi.ACT_NONE, "none"), (ffi.ACT_RELU, "relu"), (ffi.ACT_RELU6, "relu6"),
+                                      (ffi.ACT_HARD_SWISH, "hardswish"), (ffi.ACT_MISH, "mish")])
+def test_activations_by_waves(dtype, h, w, batch, act, name):
+    rng = np.random.default_rng(4)
+    x = ((rng.random((batch, 32, h, w), dtype=np.float32) - 0.5) * 4).astype(np.float16).astype(np.float32)
+    wt = (rng.standard_normal((72, 32, 1, 1)) * 0.5).astype(np.float16).astype(np.float32)
+    ops = [ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=72, act=act, is_output=1)]
+    got = run(ops, [(0, ffi.W_WEIGHTS, wt)], (32, h, w), x, dtype)
+    for i in {0, batch - 1}:
+        want = mo.conv2d(x[i], wt, 1, 1, 1, 1, 0, 0, 1, 1, 1)
+        if name != "none":
+            want = mo.activate(want, name, [])
+        assert H.rel_err(got[i], want) < (2e-3 if dtype == ffi.F16 else H.TOL_F32)
