@@ -623,6 +623,7 @@ int msnh_b200_plan_destroy(MsnhB200Plan *pl) {
         if (sl.h2d_done) cudaEventDestroy(sl.h2d_done);
         if (sl.consumed) cudaEventDestroy(sl.consumed);
         if (sl.done) cudaEventDestroy(sl.done);
+        for (cudaEvent_t e : sl.piece) if (e) cudaEventDestroy(e);
         if (sl.fwd_done) cudaEventDestroy(sl.fwd_done);
     }
     if (pl->copy_stream) cudaStreamDestroy(pl->copy_stream);

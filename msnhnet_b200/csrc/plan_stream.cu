@@ -106,6 +106,7 @@ static int stream_setup(MsnhB200Plan *pl, int op) {
         CUDA_TRY(ctx, cudaEventCreateWithFlags(&s.h2d_done, cudaEventDisableTiming));
         CUDA_TRY(ctx, cudaEventCreateWithFlags(&s.consumed, cudaEventDisableTiming));
         CUDA_TRY(ctx, cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
+        for (cudaEvent_t &e : s.piece) CUDA_TRY(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         // Float images go from the slot's staging buffer straight into the forward: a copy of the plan's graph whose
         // input kernel reads this slot's buffer instead of the plan's own input buffer.
         if (pl->graph_exec) {
@@ -193,9 +194,15 @@ static int stream_push_common(MsnhB200Plan *pl, int op, const void *host_images,
     else {
         CUDA_TRY(ctx, cudaEventRecord(s.fwd_done, ctx->stream));
         CUDA_TRY(ctx, cudaStreamWaitEvent(pl->d2h_stream, s.fwd_done, 0));
-        CUDA_TRY(ctx, cudaMemcpyAsync(s.h_result, s.d_result, per * n_images * sizeof(float), cudaMemcpyDeviceToHost, pl->d2h_stream));
-        CUDA_TRY(ctx, cudaEventRecord(s.done, pl->d2h_stream));
+        // in pieces, so that pop copies one on while the next crosses PCIe
+        const size_t total = per * n_images;
+        for (int k = 0; k < kResultPieces; ++k) {
+            const size_t at = total * k / kResultPieces, end = total * (k + 1) / kResultPieces;
+            if (end > at) CUDA_TRY(ctx, cudaMemcpyAsync(s.h_result + at, s.d_result + at, (end - at) * sizeof(float), cudaMemcpyDeviceToHost, pl->d2h_stream));
+            CUDA_TRY(ctx, cudaEventRecord(k + 1 < kResultPieces ? s.piece[k] : s.done, pl->d2h_stream));
+        }
     }
+    s.in_pieces = !direct;
     s.n_images = n_images; s.busy = true;
     ++pl->push_count;
     return MSNH_B200_OK;
@@ -234,7 +241,7 @@ int msnh_b200_plan_stream_pop(MsnhB200Plan *pl, float *result, size_t capacity_f
     if (pl->pop_count >= pl->push_count) return fail(ctx, MSNH_B200_ERR_STATE, "stream_pop: nothing in flight");
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     auto &s = pl->slots[pl->pop_count & 1];
-    CUDA_TRY(ctx, cudaEventSynchronize(s.done));
+    if (!s.in_pieces) CUDA_TRY(ctx, cudaEventSynchronize(s.done));
     if (n_images) *n_images = s.n_images;
     if (pl->stream_cap) {
         if (!counts || max_rows < 1 || capacity_floats < static_cast<size_t>(s.n_images) * max_rows * 8)
@@ -257,7 +264,12 @@ int msnh_b200_plan_stream_pop(MsnhB200Plan *pl, float *result, size_t capacity_f
         const OpState &o = pl->ops[pl->stream_op];
         const size_t n = static_cast<size_t>(s.n_images) * o.out.C * o.out.H * o.out.W;
         if (capacity_floats < n) return fail(ctx, MSNH_B200_ERR_ARG, "stream_pop: output buffer too small (%zu floats needed)", n);
-        parallel_memcpy(ctx, result, s.h_result, n * sizeof(float));
+        for (int k = 0; s.in_pieces && k < kResultPieces; ++k) {
+            const size_t at = n * k / kResultPieces, end = n * (k + 1) / kResultPieces;
+            CUDA_TRY(ctx, cudaEventSynchronize(k + 1 < kResultPieces ? s.piece[k] : s.done));
+            parallel_memcpy(ctx, result + at, s.h_result + at, (end - at) * sizeof(float));
+        }
+        if (!s.in_pieces) std::memcpy(result, s.h_result, n * sizeof(float));
     }
     s.busy = false;
     ++pl->pop_count;

@@ -27,3 +27,30 @@ def test_pageable_images_and_results(c, h, w, batch, offset):
     finally:
         plan.close()
         ctx.close()
+
+
+@pytest.mark.parametrize("c,h,w,batch", [(3, 11, 13, 2), (1, 512, 512, 1), (1, 512, 513, 1), (5, 300, 177, 3)])
+def test_streamed_results(c, h, w, batch):
+    rng = np.random.default_rng(3)
+    ctx = ffi.Context(0)
+    plan = ffi.Plan(ctx, [ffi.make_op(ffi.OP_CLIP, [ffi.INPUT], const_val=-10.0, scale=10.0, is_output=1)], (c, h, w), batch, ffi.F32)
+    try:
+        plan.finalize()
+        sent = []
+        for k in (batch, 1, batch, batch):
+            if len(sent) == 2:
+                pop(plan, sent.pop(0))
+            x = rng.standard_normal((k, c, h, w), dtype=np.float32)
+            ctx.check(plan.lib.msnh_b200_plan_stream_push(plan.h, 0, x.ctypes.data, k))
+            sent.append(x)
+        for x in sent:
+            pop(plan, x)
+    finally:
+        plan.close()
+        ctx.close()
+
+
+def pop(plan, want):
+    out, n = np.empty_like(want), ffi.C.c_int()
+    plan.ctx.check(plan.lib.msnh_b200_plan_stream_pop(plan.h, out.ctypes.data_as(ffi.C.POINTER(ffi.C.c_float)), out.size, 0, None, ffi.C.byref(n)))
+    assert n.value == len(want) and np.array_equal(out, want)
