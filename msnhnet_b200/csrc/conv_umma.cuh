@@ -365,15 +365,20 @@ __device__ __forceinline__ void activate_pairs(F2 (&y)[8], int act, float param)
 // fp32 accumulators) to its slot in global memory and raises its flag; the CTA that owns the tile's last
 // k-block adds the slots of its predecessors before the usual epilogue. Each CTA handles the segment it
 // hands over first and the segment it has to complete last, so nobody waits on a CTA that is itself waiting.
+// kSplit: a cluster of p.k_split CTAs shares the k-blocks of one tile (128 pixels x bn channels), one tile per cluster. Each CTA runs
+// the main loop over its share and leaves the raw accumulators in its own shared memory; behind a cluster barrier each finishes every
+// k_split-th row of the tile, adding the shares through distributed shared memory in rank order (deterministic). fp32 only, for layers
+// whose k is long and whose tiles are few: a 3x3 512->512 layer at 7x7 is one tile of pixels and 144 tf32 k-blocks of 330 cycles.
 // kAct: a compile-time first activation leaves no switch in the epilogue loops (MSNH_ACT_LEAKY: slope in [0, 1]);
 // kActGeneric switches at run time. kTrace: the instantiation that records clock stamps (plans made with MSNH_PLAN_TRACE); the
 // production instantiations carry none of that code.
-template <typename T, int kMult, bool kPair, bool kStreamK, int kAct = kActGeneric, bool kTrace = false>   // kMult: 128-pixel sub-tiles per tile (1, 2, 3, 4)
+template <typename T, int kMult, bool kPair, bool kStreamK, int kAct = kActGeneric, bool kTrace = false, bool kSplit = false>   // kMult: 128-pixel sub-tiles per tile (1, 2, 3, 4)
 __global__ void __launch_bounds__(kUmmaThreads, 1)
 conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_c2,
                  const __grid_constant__ CUtensorMap map_res, const ConvUmmaParams p) {
     constexpr bool kTf32 = sizeof(T) == 4;
+    static_assert(!kSplit || kTf32, "the k of a tile is shared in fp32 plans only");
     extern __shared__ uint8_t smem_raw[];
     // 1024-byte alignment of the operand stages (required by the 128-byte swizzle atoms).
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -383,10 +388,12 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     uint32_t rank = 0;                                     // CTA rank in the pair
     if constexpr (kPair) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const bool lead = rank == 0;
+    int split_rank = 0;                                    // kSplit: which share of k this CTA sums
+    if constexpr (kSplit) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(split_rank));
     const int b_rows = kPair ? p.bn / 2 : p.bn;            // weight rows this CTA stages
     const uint32_t b_bytes = b_rows * p.bk_bytes;
-    const int first_tile  = kPair ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
-    const int tile_stride = kPair ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
+    const int first_tile  = kPair ? static_cast<int>(blockIdx.x >> 1) : kSplit ? static_cast<int>(blockIdx.x) / p.k_split : static_cast<int>(blockIdx.x);
+    const int tile_stride = kPair ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);   // (kSplit: past the last tile)
     const int tile_rows   = kPair ? 2 * kUmmaM : kUmmaM * kMult;
     const uint32_t a_base = smem_base;
     const uint32_t b_base = a_base + p.num_stages * a_bytes;
@@ -435,6 +442,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             k1 = static_cast<int>(min(sk_u1, base + num_k_iters) - base);
         } else {
             tile = first_tile + i * tile_stride; k0 = 0; k1 = num_k_iters;
+            if constexpr (kSplit) { k0 = num_k_iters * split_rank / p.k_split; k1 = num_k_iters * (split_rank + 1) / p.k_split; }
         }
     };
 
@@ -444,7 +452,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c) : "memory");
         if (p.split_n != 0x7fffffff) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c2) : "memory");
-        if (!kPair && !kStreamK && p.res) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_res) : "memory");
+        if (!kPair && !kStreamK && !kSplit && p.res) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_res) : "memory");
         cta_abort_slot = 0;
         for (int s = 0; s < p.num_stages; ++s) { mbar_init(full_bar(s), 2); mbar_init(empty_bar(s), 1); }
         // arrivals that free an accumulator: the team epilogue's warps (pair / stream-K kernels), or one per warp and
@@ -615,6 +623,24 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 if (!ok) break;
                 if constexpr (kPair) tcgen05_commit_pair(acc_full_bar(acc));   // accumulator complete, in both CTAs
                 else                 tcgen05_commit(acc_full_bar(acc));
+            }
+        }
+    } else if constexpr (kSplit) {
+        // ------------------------------ partial sums of a k-split tile ------------------------------
+        // raw accumulators -> this CTA's shared memory, [row][bn + 4] floats over the operand stages (the accumulator is complete,
+        // so every load has arrived and every MMA has read its operands)
+        const int lane_base = (warp & 3) * 32;
+        if (mbar_wait<true>(acc_full_bar(0), 0u, cta_abort, p.err_flag, DEV_ERR_WAIT_ACC_FULL)) {
+            tcgen05_fence_after();
+            for (int l0 = ((warp - 2) >> 2) * 16; l0 < p.bn; l0 += 64) {
+                uint32_t v[16];
+                __syncwarp();
+                tmem_ld_32x32b_x16(tmem_base + (static_cast<uint32_t>(lane_base) << 16) + static_cast<uint32_t>(l0), v);
+                tmem_ld_wait();
+                const uint32_t at = a_base + 4u * static_cast<uint32_t>((lane_base + lane) * (p.bn + 4) + l0);
+#pragma unroll
+                for (int j = 0; j < 16; j += 4)
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at + 4u * j), "r"(v[j]), "r"(v[j + 1]), "r"(v[j + 2]), "r"(v[j + 3]) : "memory");
             }
         }
     } else if constexpr (!kPair && !kStreamK) {
@@ -1010,6 +1036,48 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // teardown: everybody is past its last TMEM access (or gave up) before the columns are freed
     tcgen05_fence_before();
     __syncthreads();
+    if constexpr (kSplit) {
+        // Every share of the tile is in some CTA's shared memory: this CTA finishes the rows split_rank, split_rank + k_split, ...
+        // of the tile, the shares added in rank order.
+        cluster_sync_all();
+        const int t = static_cast<int>(threadIdx.x) - 64;
+        const int m0 = first_tile / p.tiles_n * kUmmaM, n0 = first_tile % p.tiles_n * p.bn;
+        const int rows = (min(kUmmaM, p.m_total - m0) - split_rank + p.k_split - 1) / p.k_split, quads = (min(p.bn, p.cout - n0) + 3) / 4;
+        if (t >= 0 && t < 512 && *cta_abort == 0) {
+            if (p.res) pdl_wait();                               // the residual is an earlier kernel's output
+            for (int item = t; item < rows * quads; item += 512) {
+                const int j = item / quads, row = split_rank + j * p.k_split, m = m0 + row;
+                const int col = 4 * (item - j * quads), c = n0 + col;
+                const uint32_t at = a_base + 4u * static_cast<uint32_t>(row * (p.bn + 4) + col);
+                float4 part[kUmmaMaxKSplit];
+#pragma unroll
+                for (int q = 0; q < kUmmaMaxKSplit; ++q)
+                    if (q < p.k_split)
+                        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(part[q].x), "=f"(part[q].y), "=f"(part[q].z), "=f"(part[q].w) : "r"(map_to_cta(at, q)) : "memory");
+                float y[4] = {part[0].x, part[0].y, part[0].z, part[0].w};
+#pragma unroll
+                for (int q = 1; q < kUmmaMaxKSplit; ++q)
+                    if (q < p.k_split) { y[0] += part[q].x; y[1] += part[q].y; y[2] += part[q].z; y[3] += part[q].w; }
+                const float4 sc = __ldg(reinterpret_cast<const float4 *>(p.scale + c)), bi = __ldg(reinterpret_cast<const float4 *>(p.bias + c));
+                y[0] = fmaf(y[0], sc.x, bi.x); y[1] = fmaf(y[1], sc.y, bi.y); y[2] = fmaf(y[2], sc.z, bi.z); y[3] = fmaf(y[3], sc.w, bi.w);
+                const float *res = p.res ? static_cast<const float *>(p.res) + static_cast<size_t>(m) * p.ldc_res + c : nullptr;
+                float *dst = static_cast<float *>(p.out) + static_cast<size_t>(m) * p.ldc_out + c;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    y[e] = activate(y[e], p.act1, p.act1_param);
+                    if (res && c + e < p.cout) y[e] = activate(y[e] + res[e], p.act2, p.act2_param);
+                    if (p.round_tf32) y[e] = round_tf32(y[e]);
+                }
+                if (c + 4 <= p.cout) *reinterpret_cast<float4 *>(dst) = make_float4(y[0], y[1], y[2], y[3]);   // (tensors of tensor-core layers start on 16 bytes, rows too)
+                else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) if (c + e < p.cout) dst[e] = y[e];
+                }
+            }
+        }
+        __syncwarp();
+        cluster_sync_all();          // nobody leaves while a peer still reads its shared memory
+    }
     if constexpr (kPair) cluster_sync_all();   // nothing of the peer targets this CTA's barriers or TMEM any more
     if constexpr (kTrace) { if (trace && threadIdx.x == 0) { trace[2] = clock64(); long long g; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(g)); trace[4] = g; } }
     if (warp == 1) {

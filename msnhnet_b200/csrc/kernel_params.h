@@ -35,6 +35,7 @@ constexpr int kUmmaM          = 128;  // output pixels per tile (TMEM lanes)
 constexpr int kUmmaThreads    = 608;  // warp 0: TMA producer of A, warp 1: MMA issuer, warps 2-17: epilogue, warp 18: TMA producer of B
 constexpr int kUmmaWeightWarp = 18;
 constexpr int kUmmaMaxStages  = 8;
+constexpr int kUmmaMaxKSplit  = 8;    // CTAs that may share the k of a tile (the largest portable cluster)
 constexpr int kUmmaMaxAccStages = 8; // accumulator ring in TMEM: 2, 4 or 8 stages, as many as fit in 512 columns
 constexpr uint32_t kStageCBytes = 128 * 128;   // one output staging slab: 128 rows x up to 128 bytes
 
@@ -48,6 +49,8 @@ struct ConvUmmaParams {
     int tiles_m, tiles_n;
     int m_mult;           // a tile covers m_mult (1, 2 or 4) sub-tiles of 128 pixels: one A load, m_mult MMAs sharing B
     int pair;             // 1: CTA-pair kernel, tiles of 256 pixels (tiles_m counts those), m_mult = 1
+    int k_split;          // > 1: clusters of that many CTAs share the k of one tile (grid = tiles x k_split, m_mult = 1)
+    void *out; int ldc_out;   // output tensor (kSplit kernels; the others store through map_c)
     int stream_k;         // 1: stream-K kernel (grid = number of SMs, equal shares of tiles x k-blocks)
     int bn;               // output channels per sub-tile (16..128, multiple of 16); m_mult * bn <= 256
     int bk_bytes;         // bytes of one A/B row per k-block: 128, 64 or 32 (= the swizzle span)

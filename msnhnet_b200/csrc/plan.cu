@@ -48,6 +48,7 @@ PlanDebugOptions PlanDebugOptions::from_env() {
     o.forced_mm = num("MSNH_B200_M_MULT", 0);
     o.forced_bn = num("MSNH_B200_BN", 0);
     o.fp32_split = num("MSNH_B200_FP32_SPLIT", 0);
+    o.k_split = num("MSNH_B200_K_SPLIT", 0);
     o.stream_k = num("MSNH_B200_STREAM_K", 0);
     o.pair = num("MSNH_B200_PAIR", 0);
     return o;

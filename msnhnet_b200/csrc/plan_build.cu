@@ -990,6 +990,7 @@ int build_launches(MsnhB200Plan *pl) {
                 snprintf(line, sizeof(line), " tiles=%dx%d mm=%d%s%s bn=%d bk=%dB stages=%d mode=%s grid=%d smem=%zu", L.up.tiles_m, L.up.tiles_n, L.up.m_mult, L.up.pair ? " pair" : "", L.up.stream_k ? " streamk" : "", L.up.bn,
                          L.up.bk_bytes, L.up.num_stages, L.up.a_mode == A_MODE_LINEAR ? "linear" : "im2col", L.grid, L.smem);
                 s += line;
+                if (L.up.k_split > 1) s += " k over " + std::to_string(L.up.k_split) + " CTAs";
             }
             if (!L.note.empty()) { s += " ["; s += L.note; s += "]"; }
             s += "\n";

@@ -84,11 +84,12 @@ struct PlanDebugOptions {
     int trace_tile = 0;         // MSNH_B200_TRACE_TILE: which tile of a CTA the producer / MMA stamps describe
     int forced_mm = 0, forced_bn = 0;   // MSNH_B200_M_MULT, MSNH_B200_BN: force the conv tile shape
     int fp32_split = 0;         // MSNH_B200_FP32_SPLIT: force the k split of the fp32 conv (1..8)
+    int k_split = 0;            // MSNH_B200_K_SPLIT: force the k split of the tensor-core conv where one is possible (1: never, 2, 4, 8)
     int stream_k = 0;           // MSNH_B200_STREAM_K: -1 by cost, 0 never, 1 wherever possible
     int pair = 0;               // MSNH_B200_PAIR: 1 = CTA pairs wherever possible
     static PlanDebugOptions from_env();
     // any switch that forces tile shapes: such plans neither take shapes from a pack file nor write one
-    bool forces_tiles() const { return forced_mm || forced_bn || pair == 1 || stream_k != 0; }
+    bool forces_tiles() const { return forced_mm || forced_bn || pair == 1 || stream_k != 0 || k_split != 0; }
 };
 
 // ------------------------------------------------------------------------------------------------
@@ -311,6 +312,7 @@ void pack_write(MsnhB200Plan *pl);            // best effort: temporary file uni
 // ---- plan_launch.cu ----
 void launch_one(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st);
 void prepare_conv_umma_launch(const Launch &L);   // dynamic shared memory opt-in of the kernel instantiation L runs
+int conv_umma_max_clusters(int split);   // k-split convs: clusters of `split` CTAs that run at once
 void launch_readback(MsnhB200Ctx *ctx, int dtype, const TView &v, float *dst_nchw, size_t count, cudaStream_t st);
 void launch_preprocess_u8(const unsigned char *src, float *dst, const PrepParams &p, int n_images, cudaStream_t st);
 int prepare_yolo_nms(MsnhB200Ctx *ctx);           // shared memory opt-in of the NMS kernel

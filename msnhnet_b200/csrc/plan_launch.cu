@@ -22,6 +22,9 @@ template <typename T> const void *umma_kernel(const Launch &L) {
     if (u.stream_k) return u.m_mult == 2 ? reinterpret_cast<const void *>(conv_umma_kernel<T, 2, false, true>)
                                          : reinterpret_cast<const void *>(conv_umma_kernel<T, 1, false, true>);
     if (u.pair) return reinterpret_cast<const void *>(conv_umma_kernel<T, 1, true, false>);
+    if constexpr (sizeof(T) == 4) {
+        if (u.k_split > 1) return reinterpret_cast<const void *>(conv_umma_kernel<T, 1, false, false, kActGeneric, false, true>);
+    }
     const bool trace = u.trace != nullptr;
     int act = kActGeneric;
     if (!trace) {
@@ -72,6 +75,29 @@ void set_smem_attr(const Launch &L) {
 
 void prepare_conv_umma_launch(const Launch &L) { set_smem_attr(L); }
 
+// Clusters of `split` CTAs of the k-split conv that run at the same time on the current device (a CTA takes most of an SM's
+// shared memory, a cluster's CTAs sit in one GPC).
+int conv_umma_max_clusters(int split) {
+    static std::mutex m;
+    static std::map<std::array<int, 2>, int> known;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return 0; }
+    std::lock_guard<std::mutex> g(m);
+    const auto it = known.find({dev, split});
+    if (it != known.end()) return it->second;
+    Launch L;
+    L.kind = L_CONV_UMMA; L.dtype = MSNH_B200_F32; L.up.k_split = split; L.smem = 224 * 1024;
+    set_smem_attr(L);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(split); cfg.blockDim = dim3(kUmmaThreads); cfg.dynamicSmemBytes = L.smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, umma_kernel_of(L), &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+    return known[{dev, split}] = n;
+}
+
 namespace {
 
 // Launch with the programmatic-dependent-launch attribute: the grid may be scheduled while its
@@ -120,7 +146,8 @@ void launch_typed(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st) {
             cfg.gridDim = dim3(L.grid); cfg.blockDim = dim3(kUmmaThreads); cfg.dynamicSmemBytes = L.smem; cfg.stream = st;
             cudaLaunchAttribute attr[2];
             int na = 0;
-            if (L.up.pair) { attr[na].id = cudaLaunchAttributeClusterDimension; attr[na].val.clusterDim.x = 2; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1; ++na; }
+            const int cluster = L.up.pair ? 2 : L.up.k_split;
+            if (cluster > 1) { attr[na].id = cudaLaunchAttributeClusterDimension; attr[na].val.clusterDim.x = cluster; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1; ++na; }
             if (ctx->pdl) { attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[na].val.programmaticStreamSerializationAllowed = 1; ++na; }
             cfg.attrs = attr; cfg.numAttrs = na;
             void *args[6] = {const_cast<CUtensorMap *>(&L.map_a), const_cast<CUtensorMap *>(&L.map_b), const_cast<CUtensorMap *>(&L.map_c),

@@ -272,17 +272,41 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
                 }
             }
         }
-        u.m_mult = best_mm; u.bn = best_bn; u.pair = best_pair; u.stream_k = best_sk;
+        // A long k over few tiles: the k-blocks of a tile shared by a cluster of 2, 4 or 8 CTAs, where all clusters run at once (74,
+        // 33 and 15 of them on B200: those of 8 do not use every SM, and a second wave of them costs more than the split saves, 192
+        // -> 242 us for the net below). Modelled, not measured: the sums of a layer are added in another order than without a split,
+        // so which form runs must not depend on timing. fp32 plans only: an fp16 plan gives an image the same bits whatever the batch
+        // size. Never in nets with a YOLO head, whose boxes flip at the confidence and IoU thresholds with the last bits of their scores.
+        // Putting the shares together takes some 5000 cycles more than the epilogue of a whole tile; shares of fewer than three
+        // k-blocks are all start-up. ResNet-18 fp32, one image: a forward 258 -> 168 us (3x3 512->512 at 7x7: 33.8 -> 14.4 us launch
+        // by launch, of which 6.5 are the events'); 32 images 622 -> 616.
+        int best_split = 1;
+        bool detects = false;
+        for (const OpState &o : pl->ops) detects = detects || o.d.kind == MSNH_OP_YOLO;
+        if (pl->dtype == MSNH_B200_F32 && !detects && !best_pair && !best_sk && !forced_mm && !forced_bn && !L.out2.ptr && !u.trace && dbg.k_split != 1)
+            for (int split = 2; split <= kUmmaMaxKSplit; split *= 2) {
+                if (dbg.k_split > 1 && split != dbg.k_split) continue;
+                const int clusters = conv_umma_max_clusters(split);
+                for (int bn : bns) {
+                    const size_t stage = static_cast<size_t>(kUmmaM + bn) * u.bk_bytes, stages = std::min<size_t>(kUmmaMaxStages, budget / stage);
+                    const int tiles = ((u.m_total + kUmmaM - 1) / kUmmaM) * ((cout + bn - 1) / bn);
+                    if (tiles > clusters || k_iters < (dbg.k_split > 1 ? split : 3 * split) || stages < 3 || stages * stage < static_cast<size_t>(kUmmaM) * (bn + 4) * 4) continue;
+                    const double drain = 900.0 * ((((bn + slab_cols - 1) / slab_cols) + 1) / 2);
+                    const double cost = ((k_iters + split - 1) / split) * kblock_cycles(1, bn, stage) + drain + 2500.0 + 5500.0;
+                    if (cost < best || (dbg.k_split > 1 && best_split == 1)) { best = cost; best_mm = 1; best_bn = bn; best_split = split; }
+                }
+            }
+        u.m_mult = best_mm; u.bn = best_bn; u.pair = best_pair; u.stream_k = best_sk; u.k_split = best_split;
         tune_cands.clear();
         // a pack file carries the shapes its plan ended up with: no need to time them again
-        const bool stored = pl->pack_loaded && tt.umma_seen < pl->pack_picks.size() && !forced_mm && !forced_bn && pair_mode != 1 && sk_mode == 0;
+        const bool stored = best_split == 1 && pl->pack_loaded && tt.umma_seen < pl->pack_picks.size() && !forced_mm && !forced_bn && pair_mode != 1 && sk_mode == 0;
         if (stored) {
             const std::array<int32_t, 3> &pk = pl->pack_picks[tt.umma_seen];
             bool valid = false;
             for (const Cand &c : cands) valid = valid || (c.mm == pk[0] && c.bn == pk[1]);
             if (valid) { u.m_mult = pk[0]; u.bn = pk[1]; u.pair = 0; u.stream_k = 0; if (pk[2] >= 0x100) L.note += L.note.empty() ? "measured shape" : ", measured shape"; }
         }
-        if (!stored && tt.autotune && !best_pair && !best_sk && !forced_mm && !forced_bn) {
+        if (!stored && tt.autotune && !best_pair && !best_sk && best_split == 1 && !forced_mm && !forced_bn) {
             std::sort(cands.begin(), cands.end(), [](const Cand &x, const Cand &y) { return x.cost < y.cost; });
             // (stream-K forms were measured too and never won a layer; more than six runners-up changed nothing)
             const int tune_max = dbg.autotune > 0 ? dbg.autotune : 6;
@@ -315,7 +339,8 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
     const size_t stage = static_cast<size_t>(kUmmaM * u.m_mult + b_rows) * u.bk_bytes;
     u.num_stages = static_cast<int>(std::min<size_t>(kUmmaMaxStages, budget / stage));
     L.smem = u.num_stages * stage + fixed;
-    L.grid = u.pair ? 2 * std::min(u.tiles_m * u.tiles_n, ctx->sm_count / 2) : std::min(u.tiles_m * u.tiles_n, ctx->sm_count);
+    L.grid = u.pair ? 2 * std::min(u.tiles_m * u.tiles_n, ctx->sm_count / 2) : u.k_split > 1 ? u.tiles_m * u.tiles_n * u.k_split : std::min(u.tiles_m * u.tiles_n, ctx->sm_count);
+    u.out = L.out.ptr; u.ldc_out = L.out.ldc;
     u.sk_ws = nullptr; u.sk_flags = nullptr;
     if (u.stream_k) {
         // one hand-over slot (largest tile: 256 x 128 or 128 x 256 fp32) and one flag per CTA, shared by
