@@ -238,8 +238,11 @@ void launch_typed(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st) {
             break;
         }
         case L_AVGPOOL:
-            if (L.vec) launch_k(ctx->pdl, avgpool_kernel<T, V>, grid, block, 0, st, L.in, L.out, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw);
-            else       launch_k(ctx->pdl, avgpool_kernel<T, 1>, grid, block, 0, st, L.in, L.out, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw);
+            {   // one-warp blocks while those fit the grid's cap
+                const int b = out_items <= static_cast<size_t>(ctx->sm_count) * 8 * 32 ? 32 : block;
+                if (L.vec) launch_k(ctx->pdl, avgpool_kernel<T, V>, grid_for(ctx, out_items, b), b, 0, st, L.in, L.out, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw);
+                else       launch_k(ctx->pdl, avgpool_kernel<T, 1>, grid_for(ctx, out_items, b), b, 0, st, L.in, L.out, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw);
+            }
             break;
         case L_UPSAMPLE:
             if (L.vec) launch_k(ctx->pdl, upsample_kernel<T, V>, grid, block, 0, st, L.in, L.out, L.sh, L.sw, L.fval);

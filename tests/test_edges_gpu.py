@@ -61,3 +61,14 @@ def test_patch_stem(h, w, stride, pad):
     for i in range(2):
         ref = mo.conv2d(half(x[i]), wt, 3, 3, stride, stride, pad, pad, 1, 1, 1)
         assert H.rel_err(got[i], ref) < 1e-3
+
+
+@pytest.mark.parametrize("dtype", [ffi.F32, ffi.F16])
+@pytest.mark.parametrize("c,h,w,k,s,p", [(1280, 7, 7, 7, 1, 0), (3, 4, 2, 2, 2, 0), (40, 9, 11, 3, 1, 1), (5, 8, 8, 8, 1, 0), (64, 61, 67, 3, 2, 1)])
+def test_average_pool(dtype, c, h, w, k, s, p):
+    rng = np.random.default_rng(3)
+    x = half(rng.standard_normal((4, c, h, w)).astype(np.float32))
+    got, _ = run([ffi.make_op(ffi.OP_AVGPOOL, [ffi.INPUT], k_h=k, k_w=k, stride_h=s, stride_w=s, pad_h=p, pad_w=p)], [], (c, h, w), x, dtype)
+    for i in range(4):
+        want = mo.avgpool(x[i], k, k, s, s, p, p, False)[:, :got.shape[2], :got.shape[3]]
+        assert got[i].shape == want.shape and H.rel_err(got[i], want) < (1e-3 if dtype == ffi.F16 else 1e-6)
