@@ -150,9 +150,10 @@ conv_tiled_kernel(TView in, TView out, const T *__restrict__ w, const ConvTiledP
 //    rows they read: a 16-byte load whose lane pairs agree takes 2.3 SM cycles, one whose lane pairs differ 4.1 (measured), so
 //    per k the eight pixel values cost as much as the four channel values. Scalar FMAs: the packed form reads six registers at
 //    a time and reaches 54 TFLOP/s from registers alone, the scalar one 72.
-//  * a cluster of 1..8 CTAs splits the k of one tile. Every CTA sums its share, leaves it in its own shared memory, and reduces
-//    every size-th row of the tile from all of them through distributed shared memory, in rank order: deterministic, no
-//    workspace, no second launch. configure_conv_fp32 picks the split.
+//  * the k of a tile is summed in 1..8 shares that are added in their order; how many is fixed by the layer and one image, never
+//    by the batch (configure_conv_fp32). Where tiles are few a cluster takes them, a CTA each: every CTA leaves its sum in its
+//    own shared memory and reduces every size-th row of the tile from all of them through distributed shared memory, in rank order:
+//    deterministic, no workspace, no second launch. Where the tiles fill the chip one CTA sums them one after the other (kShares).
 //  * operands stay k-contiguous in shared memory as cp.async wrote them (row pitch 20 floats: the eight rows of a load
 //    fall in different banks); a ring of four k-steps, cp.async also zero-fills the padding, pad channels and ragged edges. A
 //    loader thread keeps its source addresses and moves them along while its vectors stay inside one filter tap.
@@ -164,6 +165,7 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
+template <bool kShares>        // one CTA sums all shares of a tile's k, one after the other (no cluster)
 __global__ void __launch_bounds__(kFpThreads, 4)
 conv_fp32_kernel(TView in, TView out, const float *__restrict__ w, const ConvTiledParams p) {
     constexpr int BM = kFpBM, BN = kFpBN, T = kFpThreads, PITCH = kFpPitch, LROWS = T / 4, LA = BM / LROWS, LB = BN / LROWS;
@@ -236,6 +238,22 @@ conv_fp32_kernel(TView in, TView out, const float *__restrict__ w, const ConvTil
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 
+    // kShares: the sum of the shares behind this one. Touched once a share, so it stays on the stack (its address is shown to an empty
+    // asm): in registers it would push the addresses of the main loop out of theirs.
+    float sum[kShares ? 8 : 1][4];
+    int share = 0, share_end = step1;
+    bool first = true;
+    if constexpr (kShares) {
+        asm volatile("" ::"l"(&sum[0][0]) : "memory");
+        share_end = steps / p.shares;
+        while (share_end == 0) share_end = static_cast<int>(static_cast<long long>(steps) * (++share + 1) / p.shares);   // (more shares than k-steps)
+    }
+    auto fold = [&](bool first) {                                 // this share to the sum of those before it, in their order
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[i][j] = (first ? 0.f : sum[i][j]) + acc[i][j];
+    };
     pdl_wait();
 #pragma unroll
     for (int q = 0; q < kFpStages - 1; ++q) {
@@ -269,6 +287,19 @@ conv_fp32_kernel(TView in, TView out, const float *__restrict__ w, const ConvTil
             }
         }
         slot = (slot + 1) & (kFpStages - 1);
+        if constexpr (kShares) {
+            if (step + 1 == share_end) {
+                fold(first);
+                first = false;
+                if (step + 1 < steps) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) { sum[i][j] = acc[i][j]; acc[i][j] = 0.f; }
+                    do share_end = static_cast<int>(static_cast<long long>(steps) * (++share + 1) / p.shares); while (share_end == step + 1);
+                }
+            }
+        }
     }
     // Only now may the next kernel's CTAs come in: launched at the start of this one they would pile up on the SMs that have
     // room, that is on those that this layer leaves idle, and stay there.

@@ -201,7 +201,7 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, int bk_bytes)
     return d;
 }
 
-// Activation of 16 accumulator values held in registers. The switch sits outside the loop so each
+// Activation of N (even) accumulator values held in registers. The switch sits outside the loop so each
 // case is a short unrolled loop; the rarely used activations share one out-of-line call.
 // single SFU instructions (flush-to-zero forms: no range fix-up code around them)
 __device__ __forceinline__ float fast_ex2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
@@ -214,29 +214,30 @@ __device__ __forceinline__ void f2_unpack(F2 x, float &a, float &b) { asm("mov.b
 __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
 __device__ __forceinline__ F2 f2_mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
 __device__ __forceinline__ F2 f2_add(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ void activate16(float (&y)[16], int act, float param) {
+template <int N>
+__device__ __forceinline__ void activate_n(float (&y)[N], int act, float param) {
     switch (act) {
         case MSNH_ACT_NONE: break;
         case MSNH_ACT_LEAKY:
             if (param >= 0.f && param <= 1.f) {      // max(x, a*x) equals the select for slopes in [0, 1]
                 const F2 a2 = f2_pack(param, param);
 #pragma unroll
-                for (int j = 0; j < 16; j += 2) {
+                for (int j = 0; j < N; j += 2) {
                     float m0, m1; f2_unpack(f2_mul(f2_pack(y[j], y[j + 1]), a2), m0, m1);
                     y[j] = fmaxf(y[j], m0); y[j + 1] = fmaxf(y[j + 1], m1);
                 }
             } else {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) y[j] = y[j] > 0.f ? y[j] : param * y[j];
+                for (int j = 0; j < N; ++j) y[j] = y[j] > 0.f ? y[j] : param * y[j];
             }
             break;
         case MSNH_ACT_RELU:
 #pragma unroll
-            for (int j = 0; j < 16; ++j) y[j] = fmaxf(y[j], 0.f);
+            for (int j = 0; j < N; ++j) y[j] = fmaxf(y[j], 0.f);
             break;
         case MSNH_ACT_RELU6:
 #pragma unroll
-            for (int j = 0; j < 16; ++j) y[j] = fminf(fmaxf(y[j], 0.f), 6.f);
+            for (int j = 0; j < N; ++j) y[j] = fminf(fmaxf(y[j], 0.f), 6.f);
             break;
         case MSNH_ACT_MISH: {
             // x * tanh(log(1 + e^x)) = x * n / (n + 2), n = e^x (e^x + 2). Only e^x uses the SFU pipe; 1 / (n + 2)
@@ -245,7 +246,7 @@ __device__ __forceinline__ void activate16(float (&y)[16], int act, float param)
             // exponent is clamped at 20, where n / (n + 2) rounds to 1.
             const F2 two = f2_pack(2.f, 2.f), one = f2_pack(1.f, 1.f), l2e = f2_pack(1.4426950408889634f, 1.4426950408889634f);
 #pragma unroll
-            for (int j = 0; j < 16; j += 2) {
+            for (int j = 0; j < N; j += 2) {
                 const F2 t = f2_mul(f2_pack(fminf(y[j], 20.f), fminf(y[j + 1], 20.f)), l2e);
                 float t0, t1; f2_unpack(t, t0, t1);
                 const F2 e = f2_pack(fast_ex2(t0), fast_ex2(t1));
@@ -265,7 +266,7 @@ __device__ __forceinline__ void activate16(float (&y)[16], int act, float param)
         case MSNH_ACT_HARD_SWISH: {
             const F2 three = f2_pack(3.f, 3.f), sixth = f2_pack(0.16666667f, 0.16666667f);
 #pragma unroll
-            for (int j = 0; j < 16; j += 2) {
+            for (int j = 0; j < N; j += 2) {
                 const F2 x = f2_pack(y[j], y[j + 1]);
                 float c0, c1; f2_unpack(f2_add(x, three), c0, c1);
                 const F2 c = f2_pack(fminf(fmaxf(c0, 0.f), 6.f), fminf(fmaxf(c1, 0.f), 6.f));
@@ -274,26 +275,26 @@ __device__ __forceinline__ void activate16(float (&y)[16], int act, float param)
             break;
         }
         case MSNH_ACT_SWISH: {
-            float d[16];
+            float d[N];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) d[j] = 1.f + fast_ex2(-y[j] * 1.4426950408889634f);
+            for (int j = 0; j < N; ++j) d[j] = 1.f + fast_ex2(-y[j] * 1.4426950408889634f);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) d[j] = fast_rcp(d[j]);
+            for (int j = 0; j < N; ++j) d[j] = fast_rcp(d[j]);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) y[j] *= d[j];
+            for (int j = 0; j < N; ++j) y[j] *= d[j];
             break;
         }
         case MSNH_ACT_LOGISTIC: {
-            float d[16];
+            float d[N];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) d[j] = 1.f + fast_ex2(-y[j] * 1.4426950408889634f);
+            for (int j = 0; j < N; ++j) d[j] = 1.f + fast_ex2(-y[j] * 1.4426950408889634f);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) y[j] = fast_rcp(d[j]);
+            for (int j = 0; j < N; ++j) y[j] = fast_rcp(d[j]);
             break;
         }
         default:
 #pragma unroll
-            for (int j = 0; j < 16; ++j) y[j] = activate_slow(y[j], act, param);
+            for (int j = 0; j < N; ++j) y[j] = activate_slow(y[j], act, param);
             break;
     }
 }
@@ -336,7 +337,7 @@ __device__ __forceinline__ void activate_pairs(F2 (&y)[8], int act, float param)
         float f[16];
 #pragma unroll
         for (int q = 0; q < 8; ++q) f2_unpack(y[q], f[2 * q], f[2 * q + 1]);
-        activate16(f, a, param);
+        activate_n(f, a, param);
 #pragma unroll
         for (int q = 0; q < 8; ++q) y[q] = f2_pack(f[2 * q], f[2 * q + 1]);
     }
@@ -365,20 +366,24 @@ __device__ __forceinline__ void activate_pairs(F2 (&y)[8], int act, float param)
 // fp32 accumulators) to its slot in global memory and raises its flag; the CTA that owns the tile's last
 // k-block adds the slots of its predecessors before the usual epilogue. Each CTA handles the segment it
 // hands over first and the segment it has to complete last, so nobody waits on a CTA that is itself waiting.
-// kSplit: a cluster of p.k_split CTAs shares the k-blocks of one tile (128 pixels x bn channels), one tile per cluster. Each CTA runs
-// the main loop over its share and leaves the raw accumulators in its own shared memory; behind a cluster barrier each finishes every
-// k_split-th row of the tile, adding the shares through distributed shared memory in rank order (deterministic). fp32 only, for layers
-// whose k is long and whose tiles are few: a 3x3 512->512 layer at 7x7 is one tile of pixels and 144 tf32 k-blocks of 330 cycles.
+// k in shares (fp32 plans): a layer may sum its k-blocks in p.k_shares shares of (nearly) equal length that are added in their order.
+// How many is fixed by the layer and one image (configure_conv_umma), never by the batch, and it decides the bits; who sums
+// them does not. kShares: one CTA sums them all, each in an accumulator of its own, and the epilogue adds those.
+// kSplit: a cluster of p.k_split = p.k_shares CTAs sums a share each of one tile (128 pixels x bn channels), one tile per cluster. Each
+// CTA leaves its raw accumulators in its own shared memory; behind a cluster barrier each finishes every k_split-th row of the tile,
+// adding the shares through distributed shared memory. For layers whose k is long and whose tiles are few: a 3x3 512->512 layer at 7x7
+// is one tile of pixels and 144 tf32 k-blocks of 330 cycles.
 // kAct: a compile-time first activation leaves no switch in the epilogue loops (MSNH_ACT_LEAKY: slope in [0, 1]);
 // kActGeneric switches at run time. kTrace: the instantiation that records clock stamps (plans made with MSNH_PLAN_TRACE); the
 // production instantiations carry none of that code.
-template <typename T, int kMult, bool kPair, bool kStreamK, int kAct = kActGeneric, bool kTrace = false, bool kSplit = false>   // kMult: 128-pixel sub-tiles per tile (1, 2, 3, 4)
+template <typename T, int kMult, bool kPair, bool kStreamK, int kAct = kActGeneric, bool kTrace = false, bool kSplit = false, bool kShares = false>   // kMult: 128-pixel sub-tiles per tile (1, 2, 3, 4)
 __global__ void __launch_bounds__(kUmmaThreads, 1)
 conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_c2,
                  const __grid_constant__ CUtensorMap map_res, const ConvUmmaParams p) {
     constexpr bool kTf32 = sizeof(T) == 4;
-    static_assert(!kSplit || kTf32, "the k of a tile is shared in fp32 plans only");
+    static_assert(!(kSplit || kShares) || (kTf32 && !kPair && !kStreamK && kSplit != kShares), "the k of a tile is summed in shares in fp32 plans only");
+    const int shares = kShares ? p.k_shares : 1;
     extern __shared__ uint8_t smem_raw[];
     // 1024-byte alignment of the operand stages (required by the 128-byte swizzle atoms).
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -590,11 +595,16 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 ok = mbar_wait<true>(acc_empty_bar(acc), acc_phase ^ 1u, cta_abort, p.err_flag, DEV_ERR_WAIT_ACC_EMPTY);
                 if (!ok) break;
                 tcgen05_fence_after();
-                const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * m_mult * p.bn);
+                uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * shares * m_mult * p.bn);
                 uint32_t accumulate = 0;
                 // straight-line code per k-block (4, 2 or 1 MMAs per sub-tile, each 32 bytes of K per row)
                 auto k_blocks = [&](auto mmas) {
+                    int share = 1, share_end = seg_k / shares;
                     for (int kt = 0; kt < seg_k; ++kt) {
+                        if (kShares && kt == share_end) {            // the next share of k has an accumulator of its own
+                            tmem_d += static_cast<uint32_t>(m_mult * p.bn); accumulate = 0;
+                            share_end = seg_k * ++share / shares;
+                        }
                         ok = mbar_wait(full_bar(stage), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
                         if (!ok) break;
                         if constexpr (kTrace) { if (trace && tl == p.trace_tile && kt < 16) trace[24 + kt] = clock64(); }
@@ -708,7 +718,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 if constexpr (kTrace) { if (trace && e == 0 && lane == 0 && tl == 0) trace[40] = clock64(); }
             }
             if (work) {
-                const uint32_t acc_col = static_cast<uint32_t>((acc * kMult + sub) * p.bn);
+                const uint32_t acc_col = static_cast<uint32_t>((acc * shares * kMult + sub) * p.bn);
                 if (has_res) {
                     ok = mbar_wait(res_bar(e), res_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
                     ok = __all_sync(0xffffffffu, ok);
@@ -717,8 +727,18 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 }
                 for (int l0 = 0; l0 < cols_per_store; l0 += 16) {
                     uint32_t v[16];
-                    tmem_ld_32x32b_x16(tmem_base + (static_cast<uint32_t>(lane_base) << 16) + acc_col + static_cast<uint32_t>(c0 + l0), v);
+                    const uint32_t at = tmem_base + (static_cast<uint32_t>(lane_base) << 16) + acc_col + static_cast<uint32_t>(c0 + l0);
+                    tmem_ld_32x32b_x16(at, v);
                     tmem_ld_wait();
+                    if constexpr (kShares) {
+                        for (int q = 1; q < shares; ++q) {       // the shares of k in their order, as the kSplit kernel adds them
+                            uint32_t w[16];
+                            tmem_ld_32x32b_x16(at + static_cast<uint32_t>(q * kMult * p.bn), w);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+                        }
+                    }
                     const int cbase = n0 + c0 + l0;          // the scale / bias arrays are padded past the last channel tile
                     F2 y[8];
                     if (sb_staged) {
@@ -1062,11 +1082,16 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 y[0] = fmaf(y[0], sc.x, bi.x); y[1] = fmaf(y[1], sc.y, bi.y); y[2] = fmaf(y[2], sc.z, bi.z); y[3] = fmaf(y[3], sc.w, bi.w);
                 const float *res = p.res ? static_cast<const float *>(p.res) + static_cast<size_t>(m) * p.ldc_res + c : nullptr;
                 float *dst = static_cast<float *>(p.out) + static_cast<size_t>(m) * p.ldc_out + c;
+                // the operations of the plain kernels' epilogue, one by one: which of the two a layer runs may not show in its bits
+                activate_n(y, p.act1, p.act1_param);
+                if (res) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    y[e] = activate(y[e], p.act1, p.act1_param);
-                    if (res && c + e < p.cout) y[e] = activate(y[e] + res[e], p.act2, p.act2_param);
-                    if (p.round_tf32) y[e] = round_tf32(y[e]);
+                    for (int e = 0; e < 4; ++e) if (c + e < p.cout) y[e] = __fadd_rn(y[e], res[e]);
+                    activate_n(y, p.act2, p.act2_param);
+                }
+                if (p.round_tf32) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) y[e] = round_tf32(y[e]);
                 }
                 if (c + 4 <= p.cout) *reinterpret_cast<float4 *>(dst) = make_float4(y[0], y[1], y[2], y[3]);   // (tensors of tensor-core layers start on 16 bytes, rows too)
                 else {

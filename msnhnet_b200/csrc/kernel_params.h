@@ -35,7 +35,7 @@ constexpr int kUmmaM          = 128;  // output pixels per tile (TMEM lanes)
 constexpr int kUmmaThreads    = 608;  // warp 0: TMA producer of A, warp 1: MMA issuer, warps 2-17: epilogue, warp 18: TMA producer of B
 constexpr int kUmmaWeightWarp = 18;
 constexpr int kUmmaMaxStages  = 8;
-constexpr int kUmmaMaxKSplit  = 8;    // CTAs that may share the k of a tile (the largest portable cluster)
+constexpr int kUmmaMaxKSplit  = 8;    // shares of a tile's k (a CTA each: the largest portable cluster)
 constexpr int kUmmaMaxAccStages = 8; // accumulator ring in TMEM: 2, 4 or 8 stages, as many as fit in 512 columns
 constexpr uint32_t kStageCBytes = 128 * 128;   // one output staging slab: 128 rows x up to 128 bytes
 
@@ -49,7 +49,8 @@ struct ConvUmmaParams {
     int tiles_m, tiles_n;
     int m_mult;           // a tile covers m_mult (1, 2 or 4) sub-tiles of 128 pixels: one A load, m_mult MMAs sharing B
     int pair;             // 1: CTA-pair kernel, tiles of 256 pixels (tiles_m counts those), m_mult = 1
-    int k_split;          // > 1: clusters of that many CTAs share the k of one tile (grid = tiles x k_split, m_mult = 1)
+    int k_shares;         // the k of a tile is summed in this many shares, added in their order (fp32; 1: one sum)
+    int k_split;          // CTAs those shares are spread over: 1, or k_shares (clusters; grid = tiles x k_split, m_mult = 1)
     void *out; int ldc_out;   // output tensor (kSplit kernels; the others store through map_c)
     int stream_k;         // 1: stream-K kernel (grid = number of SMs, equal shares of tiles x k-blocks)
     int bn;               // output channels per sub-tile (16..128, multiple of 16); m_mult * bn <= 256
@@ -77,7 +78,7 @@ struct ConvUmmaParams {
     int *sk_flags;        // one flag per CTA: its slot is filled (reset by the reader)
     uint32_t idesc;       // tcgen05 instruction descriptor
     int acc_shift;        // log2 of the number of accumulator stages (1..3)
-    uint32_t tmem_cols;   // power of two >= acc stages * m_mult * bn
+    uint32_t tmem_cols;   // power of two >= acc stages * shares summed here * m_mult * bn
     int round_tf32;       // fp32 output feeds another tensor-core conv: store tf32-rounded values
     int sb_channels;      // channels of scale / bias staged in shared memory at kernel start (0: read through L1 instead)
     int split_n;          // two convs over the same input run as one launch: output channels from split_n on (a multiple
@@ -135,6 +136,7 @@ constexpr size_t kFpSmemBytes = sizeof(float) * kFpStages * (kFpBM + kFpBN) * kF
 struct ConvTiledParams {
     int kh, kw, sh, sw, ph, pw, dh, dw;
     int cin_pad;                 // k extent of one tap in the packed weights
+    int shares;                  // conv_fp32_kernel: shares the k of a tile is summed in (1, or the cluster's CTAs, without a cluster any number)
     const float *scale, *bias;   // folded BatchNorm / bias per output channel (nullptr: 1 / 0)
     const void *res; int ldc_res;
     int act1; float act1_param; int act2; float act2_param;

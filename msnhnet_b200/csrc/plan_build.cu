@@ -991,6 +991,7 @@ int build_launches(MsnhB200Plan *pl) {
                          L.up.bk_bytes, L.up.num_stages, L.up.a_mode == A_MODE_LINEAR ? "linear" : "im2col", L.grid, L.smem);
                 s += line;
                 if (L.up.k_split > 1) s += " k over " + std::to_string(L.up.k_split) + " CTAs";
+                else if (L.up.k_shares > 1) s += " k in " + std::to_string(L.up.k_shares) + " shares";
             }
             if (!L.note.empty()) { s += " ["; s += L.note; s += "]"; }
             s += "\n";

@@ -71,7 +71,7 @@ int fail(MsnhB200Ctx *ctx, int code, const char *fmt, ...);
     } while (0)
 
 // Debug switches, read from the environment once per plan_finalize (and context creation). They change how a plan is
-// built, never what it computes.
+// built, never what it computes (the two that force the shares of a k: in the order of its sums, that is in the last bits).
 struct PlanDebugOptions {
     bool no_pdl = false;        // MSNH_B200_NO_PDL=1: plain stream order between kernels
     bool no_merge = false;      // MSNH_B200_NO_MERGE: no sibling 1x1 / SPP pool merging
@@ -83,8 +83,9 @@ struct PlanDebugOptions {
     int autotune = -1;          // MSNH_B200_AUTOTUNE: -1 unset (time six runners-up), 0 off, n runners-up
     int trace_tile = 0;         // MSNH_B200_TRACE_TILE: which tile of a CTA the producer / MMA stamps describe
     int forced_mm = 0, forced_bn = 0;   // MSNH_B200_M_MULT, MSNH_B200_BN: force the conv tile shape
-    int fp32_split = 0;         // MSNH_B200_FP32_SPLIT: force the k split of the fp32 conv (1..8)
-    int k_split = 0;            // MSNH_B200_K_SPLIT: force the k split of the tensor-core conv where one is possible (1: never, 2, 4, 8)
+    int fp32_split = 0;         // MSNH_B200_FP32_SPLIT: shares of the fp32 conv's k (1..8), a CTA each; negative: all of them in one CTA
+    int k_split = 0;            // MSNH_B200_K_SPLIT: shares of the tensor-core conv's k in fp32 plans (1: one; 2, 4, 8: a CTA each where
+                                // the clusters fit; negative: all of them in one CTA)
     int stream_k = 0;           // MSNH_B200_STREAM_K: -1 by cost, 0 never, 1 wherever possible
     int pair = 0;               // MSNH_B200_PAIR: 1 = CTA pairs wherever possible
     static PlanDebugOptions from_env();
@@ -155,7 +156,8 @@ struct Launch {
     // depthwise 3x3 on shared-memory tiles (map_a = the input's 4-D tensor map; grid / smem above)
     bool dw_tile = false; DwTileParams dwp{};
     bool tiled = false;        // L_CONV_DIRECT: dense conv on aligned views -> the shared-memory-tiled CUDA-core kernels
-    int fp_split = 1;          // ... fp32: CTAs of a cluster that share a tile's k (1..8)
+    int fp_shares = 1;         // ... fp32: shares the k of a tile is summed in (1..8)
+    int fp_split = 1;          // ... and the CTAs of a cluster they are spread over: 1, or fp_shares
     // accounting
     double flops = 0, bytes = 0;
     std::string note;
@@ -277,7 +279,7 @@ int tile_tuning_begin(MsnhB200Plan *pl, TileTuning &tt);
 int tile_tuning_end(MsnhB200Plan *pl, TileTuning &tt);
 // tile shape, ring sizes, grid, shared memory and tensor maps of a tensor-core conv launch whose views are resolved
 int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L);
-// k split of a CUDA-core fp32 conv launch
+// shares of the k of a CUDA-core fp32 conv launch, and the CTAs they are spread over
 void configure_conv_fp32(MsnhB200Plan *pl, Launch &L);
 // the shared-memory tile form of a 3x3 depthwise launch, where it applies (sets L.dw_tile)
 void configure_dw_tile(MsnhB200Plan *pl, Launch &L);

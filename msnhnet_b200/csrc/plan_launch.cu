@@ -24,6 +24,12 @@ template <typename T> const void *umma_kernel(const Launch &L) {
     if (u.pair) return reinterpret_cast<const void *>(conv_umma_kernel<T, 1, true, false>);
     if constexpr (sizeof(T) == 4) {
         if (u.k_split > 1) return reinterpret_cast<const void *>(conv_umma_kernel<T, 1, false, false, kActGeneric, false, true>);
+        if (u.k_shares > 1) {
+            if (u.m_mult == 4) return reinterpret_cast<const void *>(conv_umma_kernel<T, 4, false, false, kActGeneric, false, false, true>);
+            if (u.m_mult == 3) return reinterpret_cast<const void *>(conv_umma_kernel<T, 3, false, false, kActGeneric, false, false, true>);
+            if (u.m_mult == 2) return reinterpret_cast<const void *>(conv_umma_kernel<T, 2, false, false, kActGeneric, false, false, true>);
+            return reinterpret_cast<const void *>(conv_umma_kernel<T, 1, false, false, kActGeneric, false, false, true>);
+        }
     }
     const bool trace = u.trace != nullptr;
     int act = kActGeneric;
@@ -157,7 +163,7 @@ void launch_typed(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st) {
         }
         case L_CONV_DIRECT:
             if (L.tiled) {
-                const ConvTiledParams cp{L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, L.dh, L.dw, L.cin_pad, L.scale, L.bias, L.res, L.ldc_res, L.act1, L.act1_p, L.act2, L.act2_p};
+                const ConvTiledParams cp{L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, L.dh, L.dw, L.cin_pad, L.fp_shares, L.scale, L.bias, L.res, L.ldc_res, L.act1, L.act1_p, L.act2, L.act2_p};
                 const int m_total = L.out.N * L.out.H * L.out.W;
                 if constexpr (sizeof(T) == 4) {
                     cudaLaunchConfig_t cfg = {};
@@ -168,7 +174,7 @@ void launch_typed(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st) {
                     if (L.fp_split > 1) { attr[na].id = cudaLaunchAttributeClusterDimension; attr[na].val.clusterDim.x = 1; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = L.fp_split; ++na; }
                     if (ctx->pdl) { attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[na].val.programmaticStreamSerializationAllowed = 1; ++na; }
                     cfg.attrs = attr; cfg.numAttrs = na;
-                    cudaLaunchKernelEx(&cfg, conv_fp32_kernel, L.in, L.out, static_cast<const float *>(L.weights), cp);
+                    cudaLaunchKernelEx(&cfg, L.fp_shares > L.fp_split ? conv_fp32_kernel<true> : conv_fp32_kernel<false>, L.in, L.out, static_cast<const float *>(L.weights), cp);
                 } else
                 launch_k(ctx->pdl, conv_tiled_kernel<T>, dim3((m_total + kCtBM - 1) / kCtBM, (L.out.C + kCtBN - 1) / kCtBN), kCtThreads, 0, st, L.in, L.out, static_cast<const T *>(L.weights), cp);
                 break;
@@ -357,7 +363,8 @@ void launch_fill(MsnhB200Ctx *ctx, float *dst, size_t n, float value, cudaStream
     fill_kernel<<<ctx->sm_count * 8, 256, 0, st>>>(dst, n, value);
 }
 void prepare_conv_fp32_launch() {
-    cudaFuncSetAttribute(conv_fp32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kFpSmemBytes));
+    cudaFuncSetAttribute(conv_fp32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kFpSmemBytes));
+    cudaFuncSetAttribute(conv_fp32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kFpSmemBytes));
 }
 // dynamic shared memory opt-in of the depthwise tile kernels of one dtype
 void prepare_dw_tile_launch(int dtype) {

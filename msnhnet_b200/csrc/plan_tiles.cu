@@ -63,7 +63,7 @@ int pick_bk_bytes(int cin, int es) {
 }
 
 // measured tile shapes, one entry per distinct conv layer signature (process-wide)
-using TuneKey = std::array<int, 22>;
+using TuneKey = std::array<int, 23>;
 static std::mutex &tune_mutex() { static std::mutex m; return m; }
 static std::map<TuneKey, std::array<int, 3>> &tune_cache() { static std::map<TuneKey, std::array<int, 3>> c; return c; }
 
@@ -118,24 +118,36 @@ void configure_dw_tile(MsnhB200Plan *pl, Launch &L) {
 }
 
 void configure_conv_fp32(MsnhB200Plan *pl, Launch &L) {
-    const int m_total = L.out.N * L.out.H * L.out.W, steps = (L.kh * L.kw * (L.cin_pad / 4) + 3) / 4;
-    const long tiles = static_cast<long>((m_total + kFpBM - 1) / kFpBM) * ((L.out.C + kFpBN - 1) / kFpBN);
+    const int m_image = L.out.H * L.out.W, m_total = L.out.N * m_image, steps = (L.kh * L.kw * (L.cin_pad / 4) + 3) / 4;
+    auto tiles_of = [&](int m) { return static_cast<long>((m + kFpBM - 1) / kFpBM) * ((L.out.C + kFpBN - 1) / kFpBN); };
     // Measured: a k-step of 1 / 2 / 3 / 4 CTAs that share an SM takes 0.65 / 1.15 / 1.5 / 1.86 us for all of them (a CTA alone
     // cannot hide its own latencies), and clusters of three and more do not spread over all SMs: the second CTA of some SM
     // arrives at about 128.
-    double best = 0;
-    for (int split = 1; split <= kFpMaxSplit; ++split) {
-        if (split > 1 && steps < 4 * split) break;                        // a share no longer than the ring is all start-up
+    auto cost_of = [&](long tiles, int split) {
         const double spread = split <= 2 ? pl->ctx->sm_count : pl->ctx->sm_count * 0.88;
         const double per_sm = std::ceil(tiles * split / spread);          // CTAs of the busiest SM
         const double step_us = per_sm <= 4 ? 0.25 + 0.4 * per_sm : 0.46 * per_sm;
-        const double cost = ((steps + split - 1) / split) * step_us + (split > 1 ? 1.0 + 0.3 * split : 0.0);
-        if (split == 1 || cost < best) { best = cost; L.fp_split = split; }
+        return ((steps + split - 1) / split) * step_us + (split > 1 ? 1.0 + 0.3 * split : 0.0);
+    };
+    // The number of shares decides the order of a layer's sums, so it comes from the layer and ONE image: an image has the same
+    // bits in a plan of any batch size. Who sums the shares - a cluster, or one CTA one after the other where the tiles fill the
+    // chip by themselves - is free. Free to choose the shares by the batch, a forward of YOLOv5m-352 with three images takes 2.83 ms
+    // (2.93 so), of YOLOv3-tiny-416 with four 1.120 (1.124) and with sixteen 3.96 (3.99); one image is the same.
+    double best = 0;
+    for (int split = 1; split <= kFpMaxSplit; ++split) {
+        if (split > 1 && steps < 4 * split) break;                        // a share no longer than the ring is all start-up
+        const double cost = cost_of(tiles_of(m_image), split);
+        if (split == 1 || cost < best) { best = cost; L.fp_shares = split; }
     }
-    if (pl->dbg.fp32_split >= 1 && pl->dbg.fp32_split <= kFpMaxSplit) L.fp_split = pl->dbg.fp32_split;
+    const int forced = std::abs(pl->dbg.fp32_split);
+    if (forced >= 1 && forced <= kFpMaxSplit) L.fp_shares = forced;
+    const long tiles = tiles_of(m_total);
+    L.fp_split = L.fp_shares;
+    if (forced ? pl->dbg.fp32_split < 0 : cost_of(tiles, 1) <= cost_of(tiles, L.fp_shares)) L.fp_split = 1;
     prepare_conv_fp32_launch();
-    char note[64];
+    char note[96];
     snprintf(note, sizeof(note), "%ld tiles of %d k-steps, k over %d CTAs", tiles, steps, L.fp_split);
+    if (L.fp_shares > L.fp_split) snprintf(note + strlen(note), sizeof(note) - strlen(note), " in %d shares", L.fp_shares);
     L.note += (L.note.empty() ? "" : ", ") + std::string(note);
 }
 
@@ -151,6 +163,16 @@ int tile_tuning_begin(MsnhB200Plan *pl, TileTuning &tt) {
 int tile_tuning_end(MsnhB200Plan *pl, TileTuning &tt) {
     if (tt.ev0) { cudaEventDestroy(tt.ev0); cudaEventDestroy(tt.ev1); tt.ev0 = tt.ev1 = nullptr; CUDA_TRY(pl->ctx, cudaStreamSynchronize(pl->ctx->stream)); }
     return MSNH_B200_OK;
+}
+
+// Columns an epilogue read may touch past the last accumulator: a store unit is up to 32 columns wide. (Plans that sum k in shares are
+// fp32 ones, whose tiles are 16 channels or a multiple of 32 wide: whole units.)
+static int acc_room(int bn, int shares) { return shares > 1 ? 0 : round_up(bn, 32) - bn; }
+// Accumulator ring of `cols` columns a stage: log2 of the stages (1, 2, 4 or 8) that fit in the 512 TMEM columns; negative: not one.
+static int acc_ring_shift(int cols, int bn, int shares) {
+    int shift = cols + acc_room(bn, shares) <= 512 ? 0 : -1;
+    while (shift >= 0 && shift < 3 && (2 << shift) * cols + acc_room(bn, shares) <= 512) ++shift;
+    return shift;
 }
 
 int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
@@ -233,30 +255,88 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
             const double cost = (waves * k_iters * kblock_cycles(1, bn, stage) + drain + 3000.0) * 1e-3;
             if (cost < best * 0.97) { best = cost; best_mm = 1; best_bn = bn; best_pair = 1; }
         }
+        // Cost of a plain shape over m pixels, the k of a tile summed in `shares` accumulators; negative: no shape of this layer.
+        // 384 columns (3 x 128): one accumulator stage. 256 x 256 tiles (512 columns) were tried and lost
+        // to 128 x 192 on the layers they fit (46 vs 42 us on 3x3 256->512 at 38x38).
+        auto drain_cycles = [&](int mm, int bn) { return 900.0 * ((mm * ((bn + slab_cols - 1) / slab_cols) + 1) / 2); };
+        auto plain_cost = [&](int m, int mm, int bn, int shares) -> double {
+            const int shift = acc_ring_shift(shares * mm * bn, bn, shares);
+            if (shift < 0 || (mm * ((bn + 15) / 16)) << shift < 4) return -1.0;          // (four store units in the ring, see below)
+            if (forced_mm && mm != forced_mm && !(mm == 1 && forced_mm * bn > 256)) return -1.0;
+            const size_t stage = static_cast<size_t>(kUmmaM * mm + bn) * u.bk_bytes;
+            // stages to keep the loads ahead: two suffice when a k-block's MMAs outlast a load's latency
+            const size_t min_stages = (k_iters <= 2 || kblock_cycles(mm, bn, stage) >= 1000.0) ? 2 : 3;
+            if (budget / stage < min_stages && !(mm == 1 && bn == bns[0])) return -1.0;
+            const int tiles = ((m + kUmmaM * mm - 1) / (kUmmaM * mm)) * ((cout + bn - 1) / bn);
+            const double waves = std::ceil(static_cast<double>(tiles) / ctx->sm_count);
+            // (where the shares take more than half of TMEM, no drain but the last runs under a main loop)
+            const double drains = shares > 1 && shift == 0 ? waves : 1.0;
+            return waves * k_iters * kblock_cycles(mm, bn, stage) + drains * drain_cycles(mm, bn) + 2500.0;
+        };
+        // Shapes that fill more than half of TMEM (a single accumulator stage, so the epilogue of a tile does
+        // not run under the next tile's main loop) are only offered to the measured choice, except 384 x 128.
+        auto measured_only = [&](int mm, int bn) { return mm * bn > 256 && !(mm == 3 && bn == 128); };
+        // A cluster of `split` CTAs per tile of 128 x bn: the shares are put together in some 5000 cycles more than the epilogue of a
+        // whole tile takes; shares of fewer than three k-blocks are all start-up. Negative: not all clusters run at once (those of 8
+        // do not use every SM, and a second wave of them costs more than they save: 192 -> 242 us for the net below), or no room.
+        auto cluster_cost = [&](int m, int split, int bn) -> double {
+            const size_t stage = static_cast<size_t>(kUmmaM + bn) * u.bk_bytes, stages = std::min<size_t>(kUmmaMaxStages, budget / stage);
+            const int tiles = ((m + kUmmaM - 1) / kUmmaM) * ((cout + bn - 1) / bn);
+            if (tiles > conv_umma_max_clusters(split) || k_iters < (dbg.k_split > 1 ? split : 3 * split) || stages < 3 ||
+                stages * stage < static_cast<size_t>(kUmmaM) * (bn + 4) * 4) return -1.0;
+            return ((k_iters + split - 1) / split) * kblock_cycles(1, bn, stage) + drain_cycles(1, bn) + 2500.0 + 5500.0;
+        };
+        // The cheapest way to sum k in `shares` shares over m pixels, on one CTA a tile or on a cluster.
+        auto shared_cost = [&](int m, int shares) {
+            double least = 1e30;
+            for (int bn : bns) {
+                for (int mm = 1; mm <= 4; ++mm) {
+                    const double cost = plain_cost(m, mm, bn, shares);
+                    if (cost >= 0 && !(shares == 1 && measured_only(mm, bn))) least = std::min(least, cost);
+                }
+                const double cost = shares > 1 ? cluster_cost(m, shares, bn) : -1.0;
+                if (cost >= 0) least = std::min(least, cost);
+            }
+            return least;
+        };
+        // How many shares the k of a tile is summed in. A long k over few tiles is a serial chain of k-blocks on a few SMs; a cluster
+        // of 2, 4 or 8 CTAs sums it side by side. The sums of a layer are then added in another order than without, so the number of
+        // shares may depend on the layer only, never on the plan's batch - an image has the same bits in a plan of any size - and is
+        // modelled, not measured: the least product of the costs of 1, 4, 16 and 64 images (shares that a cluster does not take need
+        // an accumulator each, and eight of those leave tiles of 64 channels: 3x3 256->256 at 14x14, 32 images 25 us in one sum or
+        // in four, 38 in eight). fp32 plans only, and never in nets with a YOLO head, whose boxes flip at the confidence and IoU
+        // thresholds with the last bits of their scores.
+        // ResNet-18 fp32, a forward in one sum / in shares: one image 258 / 162 us (3x3 512->512 at 7x7: 33.8 / 14.4 us launch by
+        // launch, of which 6.5 are the events'), four 200, 16 387, 32 622 / 647. Free to choose the shares by the batch, four images
+        // took 209 us, 16 396 and 32 616.
+        int shares = 1;
+        bool detects = false;
+        for (const OpState &o : pl->ops) detects = detects || o.d.kind == MSNH_OP_YOLO;
+        if (pl->dtype == MSNH_B200_F32 && !detects && pair_mode != 1 && sk_mode == 0 && !forced_mm && !forced_bn && !L.out2.ptr && !u.trace && dbg.k_split != 1) {
+            const int forced = std::abs(dbg.k_split);
+            if (forced == 2 || forced == 4 || forced == kUmmaMaxKSplit) shares = k_iters >= forced ? forced : 1;
+            else {
+                double least = 0;
+                for (int s = 1; s <= kUmmaMaxKSplit && k_iters >= 3 * s; s *= 2) {
+                    double product = 1;
+                    for (int images = 1; images <= 64; images *= 4) product *= shared_cost(static_cast<int>(std::min(1LL << 30, static_cast<long long>(images) * L.out.H * L.out.W)), s);
+                    if (s == 1 || product < least) { least = product; shares = s; }
+                }
+            }
+        }
+        int best_split = 1;      // CTAs the shares are spread over
         for (int bn : bns) {
             if (forced_bn && bn != std::min(forced_bn, bns.back())) continue;
-            const int tiles_n = (cout + bn - 1) / bn;
             for (int mm = 1; mm <= 4; ++mm) {
-                // 384 columns (3 x 128): one accumulator stage. 256 x 256 tiles (512 columns) were tried and lost
-                // to 128 x 192 on the layers they fit (46 vs 42 us on 3x3 256->512 at 38x38).
-                // Shapes that fill more than half of TMEM (a single accumulator stage, so the epilogue of a tile does
-                // not run under the next tile's main loop) are only offered to the measured choice, except 384 x 128.
-                if (mm * bn > 512) continue;
-                const bool measured_only = mm * bn > 256 && !(mm == 3 && bn == 128);
-                if (forced_mm && mm != forced_mm && !(mm == 1 && forced_mm * bn > 256)) continue;
-                const size_t stage = static_cast<size_t>(kUmmaM * mm + bn) * u.bk_bytes;
-                // stages to keep the loads ahead: two suffice when a k-block's MMAs outlast a load's latency
-                const size_t min_stages = (k_iters <= 2 || kblock_cycles(mm, bn, stage) >= 1000.0) ? 2 : 3;
-                if (budget / stage < min_stages && !(mm == 1 && bn == bns[0])) continue;
-                const int tiles = ((u.m_total + kUmmaM * mm - 1) / (kUmmaM * mm)) * tiles_n;
-                const double waves = std::ceil(static_cast<double>(tiles) / ctx->sm_count);
-                const double drain = 900.0 * ((mm * ((bn + slab_cols - 1) / slab_cols) + 1) / 2);
-                const double cost = waves * k_iters * kblock_cycles(mm, bn, stage) + drain + 2500.0;
+                const double cost = plain_cost(u.m_total, mm, bn, shares);
+                if (cost < 0) continue;
                 cands.push_back({cost, mm, bn, 0});
-                if (measured_only && !(forced_mm && forced_bn)) continue;    // (forcing both picks such a shape: parity tests)
+                if (shares == 1 && measured_only(mm, bn) && !(forced_mm && forced_bn)) continue;    // (forcing both picks such a shape: parity tests)
                 if (cost < best * 0.97 && sk_mode != 1) { best = cost; best_mm = mm; best_bn = bn; best_pair = 0; best_sk = 0; }
                 // stream-K: every SM takes units / SMs k-blocks; hand-over and completion of split tiles
                 // cost about one extra drain. Needs two store slabs per tile (both epilogue teams meet).
+                const size_t stage = static_cast<size_t>(kUmmaM * mm + bn) * u.bk_bytes;
+                const int tiles = ((u.m_total + kUmmaM * mm - 1) / (kUmmaM * mm)) * ((cout + bn - 1) / bn);
                 const long long units = static_cast<long long>(tiles) * k_iters;
                 const bool sk_fits = mm <= 2 && mm * ((bn + slab_cols - 1) / slab_cols) >= 2 && bn * es > 128 / (mm > 1 ? 2 : 1) &&
                                      units >= 2LL * ctx->sm_count && tiles % ctx->sm_count != 0;
@@ -265,38 +345,19 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
                     // measured: handing a 128 KB partial tile over costs ~6k cycles on the writer and ~3k per
                     // slot on the reader, one after the other on the critical path
                     const double parts = std::ceil(static_cast<double>(k_iters) / share);
-                    double cost_sk = share * kblock_cycles(mm, bn, stage) + drain + 2500.0 +
+                    double cost_sk = share * kblock_cycles(mm, bn, stage) + drain_cycles(mm, bn) + 2500.0 +
                                      (6000.0 + 4000.0 * parts) * (mm * bn / 256.0);
                     if (sk_mode == 1) cost_sk *= 1e-3;
                     if (cost_sk < best * 0.95) { best = cost_sk; best_mm = mm; best_bn = bn; best_pair = 0; best_sk = 1; }
                 }
             }
         }
-        // A long k over few tiles: the k-blocks of a tile shared by a cluster of 2, 4 or 8 CTAs, where all clusters run at once (74,
-        // 33 and 15 of them on B200: those of 8 do not use every SM, and a second wave of them costs more than the split saves, 192
-        // -> 242 us for the net below). Modelled, not measured: the sums of a layer are added in another order than without a split,
-        // so which form runs must not depend on timing. fp32 plans only: an fp16 plan gives an image the same bits whatever the batch
-        // size. Never in nets with a YOLO head, whose boxes flip at the confidence and IoU thresholds with the last bits of their scores.
-        // Putting the shares together takes some 5000 cycles more than the epilogue of a whole tile; shares of fewer than three
-        // k-blocks are all start-up. ResNet-18 fp32, one image: a forward 258 -> 168 us (3x3 512->512 at 7x7: 33.8 -> 14.4 us launch
-        // by launch, of which 6.5 are the events'); 32 images 622 -> 616.
-        int best_split = 1;
-        bool detects = false;
-        for (const OpState &o : pl->ops) detects = detects || o.d.kind == MSNH_OP_YOLO;
-        if (pl->dtype == MSNH_B200_F32 && !detects && !best_pair && !best_sk && !forced_mm && !forced_bn && !L.out2.ptr && !u.trace && dbg.k_split != 1)
-            for (int split = 2; split <= kUmmaMaxKSplit; split *= 2) {
-                if (dbg.k_split > 1 && split != dbg.k_split) continue;
-                const int clusters = conv_umma_max_clusters(split);
-                for (int bn : bns) {
-                    const size_t stage = static_cast<size_t>(kUmmaM + bn) * u.bk_bytes, stages = std::min<size_t>(kUmmaMaxStages, budget / stage);
-                    const int tiles = ((u.m_total + kUmmaM - 1) / kUmmaM) * ((cout + bn - 1) / bn);
-                    if (tiles > clusters || k_iters < (dbg.k_split > 1 ? split : 3 * split) || stages < 3 || stages * stage < static_cast<size_t>(kUmmaM) * (bn + 4) * 4) continue;
-                    const double drain = 900.0 * ((((bn + slab_cols - 1) / slab_cols) + 1) / 2);
-                    const double cost = ((k_iters + split - 1) / split) * kblock_cycles(1, bn, stage) + drain + 2500.0 + 5500.0;
-                    if (cost < best || (dbg.k_split > 1 && best_split == 1)) { best = cost; best_mm = 1; best_bn = bn; best_split = split; }
-                }
+        if (shares > 1 && dbg.k_split >= 0)      // (a negative MSNH_B200_K_SPLIT keeps every tile's shares in one CTA)
+            for (int bn : bns) {
+                const double cost = cluster_cost(u.m_total, shares, bn);
+                if (cost >= 0 && (cost < best || (dbg.k_split > 1 && best_split == 1))) { best = cost; best_mm = 1; best_bn = bn; best_split = shares; }
             }
-        u.m_mult = best_mm; u.bn = best_bn; u.pair = best_pair; u.stream_k = best_sk; u.k_split = best_split;
+        u.m_mult = best_mm; u.bn = best_bn; u.pair = best_pair; u.stream_k = best_sk; u.k_shares = shares; u.k_split = best_split;
         tune_cands.clear();
         // a pack file carries the shapes its plan ended up with: no need to time them again
         const bool stored = best_split == 1 && pl->pack_loaded && tt.umma_seen < pl->pack_picks.size() && !forced_mm && !forced_bn && pair_mode != 1 && sk_mode == 0;
@@ -323,17 +384,20 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
     u.idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (static_cast<uint32_t>(u.bn >> 3) << 17) |
               (static_cast<uint32_t>((u.pair ? 2 * kUmmaM : kUmmaM) >> 4) << 24);
     u.tiles_m = (u.m_total + tile_rows - 1) / tile_rows;
+    const int shares_here = u.k_split > 1 ? 1 : u.k_shares, acc_cols = shares_here * u.m_mult * u.bn;
+    u.acc_shift = acc_ring_shift(acc_cols, u.bn, shares_here);
     // Where no CTA has a second tile the drain of its only one is on the critical path: with fewer than four store units per
     // lane quarter some of the sixteen epilogue warps would watch, so the units get narrower (16 columns at least). A forward of
     // YOLOv4-608 with one image 0.831 -> 0.792 ms, of MobileNetV2 0.227 -> 0.210.
-    if (!u.pair && !u.stream_k && u.tiles_m * u.tiles_n <= ctx->sm_count)
-        while (u.out_chunk_bytes / 2 >= 16 * es && u.m_mult * ((u.bn * es + u.out_chunk_bytes - 1) / u.out_chunk_bytes) < 4) u.out_chunk_bytes /= 2;
-    const int acc_cols = u.m_mult * u.bn;
-    // accumulator ring: as many stages (2, 4, 8) as fit in the 512 TMEM columns; the epilogue reads 32
-    // columns at a time, so the last accumulator needs up to 32 columns of room
-    u.acc_shift = 2 * acc_cols - u.bn + round_up(u.bn, 32) <= 512 ? 1 : 0;   // (384-column tiles: a single stage)
-    while (u.acc_shift >= 1 && u.acc_shift < 3 && (2 << u.acc_shift) * acc_cols - u.bn + round_up(u.bn, 32) <= 512) ++u.acc_shift;
-    uint32_t cols = 32; while (cols < static_cast<uint32_t>((1 << u.acc_shift) * acc_cols - u.bn + round_up(u.bn, 32))) cols <<= 1;
+    // They also get narrower where shares of k leave fewer than four units in the whole accumulator ring: the units go round four
+    // groups of warps, and a group whose next tile lies further on than the ring is long would take a phase of its barrier
+    // for one that has not begun.
+    auto units = [&]() { return u.m_mult * ((u.bn * es + u.out_chunk_bytes - 1) / u.out_chunk_bytes); };
+    if (!u.pair && !u.stream_k)
+        while (u.out_chunk_bytes / 2 >= 16 * es && (u.tiles_m * u.tiles_n <= ctx->sm_count ? units() : units() << u.acc_shift) < 4) u.out_chunk_bytes /= 2;
+    if (u.acc_shift < 0 || (u.tiles_m * u.tiles_n > ctx->sm_count && units() << u.acc_shift < 4 && !u.pair && !u.stream_k))
+        return fail(ctx, MSNH_B200_ERR_STATE, "conv of op %d: no room in TMEM for %d shares of %d x %d channels", L.op, shares_here, u.m_mult, u.bn);
+    uint32_t cols = 32; while (cols < static_cast<uint32_t>(((1 << u.acc_shift) * acc_cols) + acc_room(u.bn, shares_here))) cols <<= 1;
     u.tmem_cols = cols;
     const int b_rows = u.pair ? u.bn / 2 : u.bn;                     // weight rows one CTA stages
     const size_t stage = static_cast<size_t>(kUmmaM * u.m_mult + b_rows) * u.bk_bytes;
@@ -390,7 +454,7 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
     // signature and process; a shape has to beat the model's choice by 3 % to replace it.
     if (!tune_cands.empty()) {
         const TuneKey key{pl->dtype, pl->batch, cin, cout, L.in.H, L.in.W, L.out.H, L.out.W, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, L.dh, L.dw,
-                          L.act1, L.act2, L.res ? 1 : 0, L.in.ldc, L.out.ldc, ctx->sm_count};
+                          L.act1, L.act2, L.res ? 1 : 0, L.in.ldc, L.out.ldc, u.k_shares, ctx->sm_count};
         std::array<int, 3> pick{u.m_mult, u.bn, 0};
         bool known = false;
         { std::lock_guard<std::mutex> g(tune_mutex()); auto it = tune_cache().find(key); if (it != tune_cache().end()) { pick = it->second; known = true; } }
