@@ -215,6 +215,10 @@ int  msnh_b200_plan_stream_push(MsnhB200Plan *plan, int op, const float *host_nc
 int  msnh_b200_plan_stream_pop(MsnhB200Plan *plan, float *result, size_t capacity_floats, int max_rows_per_image,
                                int *counts, int *n_images);
 int  msnh_b200_plan_stream_reset(MsnhB200Plan *plan);
+/* For tests of failure handling: leaves `code` where the kernels of the batch pushed last report a bounded wait that ran
+ * out. Done by the host; no kernel is involved. The pop of that batch, and of no other, returns
+ * MSNH_B200_ERR_DEVICE_TIMEOUT (its result is handed out and the slot freed all the same). */
+int  msnh_b200_plan_stream_set_error(MsnhB200Plan *plan, int code);
 /* stream_push for 8-bit images: n_images raw HWC RGB images of width x height pixels back to back (a quarter of the
  * bytes of the float images over PCIe); the preprocessing of plan_preprocess_u8 (same mode / swap_rgb / mean / std)
  * runs on the device between the copy and the forward. The images of one batch must fit the staging buffer of a

@@ -53,12 +53,21 @@ PlanDebugOptions PlanDebugOptions::from_env() {
     o.pair = num("MSNH_B200_PAIR", 0);
     return o;
 }
-int check_device_flag(MsnhB200Plan *pl) {
-    const int flag = *pl->ctx->err_flag;
-    if (flag != 0) {
-        *pl->ctx->err_flag = 0;
-        return fail(pl->ctx, MSNH_B200_ERR_DEVICE_TIMEOUT, "a bounded wait inside the conv kernel ran out (code %d)", flag);
+int check_device_flag(MsnhB200Ctx *ctx, volatile int *flag) {
+    const int code = *flag;
+    if (code != 0) {
+        *flag = 0;
+        return fail(ctx, MSNH_B200_ERR_DEVICE_TIMEOUT, "a bounded wait inside the conv kernel ran out (code %d)", code);
     }
+    return MSNH_B200_OK;
+}
+int alloc_device_flag(MsnhB200Ctx *ctx, volatile int **flag, int **dev_flag) {
+    void *host = nullptr, *dev = nullptr;
+    CUDA_TRY(ctx, cudaHostAlloc(&host, sizeof(int), cudaHostAllocMapped));
+    *flag = static_cast<volatile int *>(host);
+    **flag = 0;
+    CUDA_TRY(ctx, cudaHostGetDevicePointer(&dev, host, 0));
+    *dev_flag = static_cast<int *>(dev);
     return MSNH_B200_OK;
 }
 
@@ -210,11 +219,12 @@ int msnh_b200_ctx_create(int device, MsnhB200Ctx **out) {
     fn = nullptr;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &fn, cudaEnableDefault, &q) != cudaSuccess || !fn) { delete ctx; return MSNH_B200_ERR_CUDA; }
     ctx->encode_im2col = reinterpret_cast<EncodeIm2colFn>(fn);
-    void *flag = nullptr, *dev_flag = nullptr;
-    if (cudaHostAlloc(&flag, sizeof(int), cudaHostAllocMapped) != cudaSuccess) { delete ctx; return MSNH_B200_ERR_NOMEM; }
-    if (cudaHostGetDevicePointer(&dev_flag, flag, 0) != cudaSuccess) { cudaFreeHost(flag); delete ctx; return MSNH_B200_ERR_CUDA; }
-    ctx->err_flag = static_cast<volatile int *>(flag); ctx->dev_err_flag = static_cast<int *>(dev_flag);
-    *ctx->err_flag = 0;
+    if (alloc_device_flag(ctx, &ctx->err_flag, &ctx->dev_err_flag) != MSNH_B200_OK) {
+        const bool got = ctx->err_flag != nullptr;
+        if (got) cudaFreeHost(const_cast<int *>(ctx->err_flag));
+        delete ctx;
+        return got ? MSNH_B200_ERR_CUDA : MSNH_B200_ERR_NOMEM;
+    }
     *out = ctx;
     return MSNH_B200_OK;
 }
@@ -619,7 +629,8 @@ int msnh_b200_plan_destroy(MsnhB200Plan *pl) {
     if (pl->d_u8) cudaFree(pl->d_u8);
     if (pl->h_counts) cudaFreeHost(pl->h_counts);
     for (auto &sl : pl->slots) {
-        if (sl.graph_exec) cudaGraphExecDestroy(sl.graph_exec);
+        for (cudaGraphExec_t g : sl.graph_exec) if (g) cudaGraphExecDestroy(g);
+        if (sl.err_flag) cudaFreeHost(const_cast<int *>(sl.err_flag));
         if (sl.d_stage) cudaFree(sl.d_stage);
         if (sl.d_result) cudaFree(sl.d_result);
         if (sl.h_result) cudaFreeHost(sl.h_result);

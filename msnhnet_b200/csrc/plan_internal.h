@@ -239,7 +239,12 @@ struct MsnhB200Plan {
         cudaEvent_t h2d_done = nullptr, consumed = nullptr, fwd_done = nullptr, done = nullptr;
         int n_images = 0; bool busy = false;
         bool in_pieces = false; cudaEvent_t piece[msnh::kResultPieces - 1] = {};   // a long result comes in pieces; the last one is `done`
-        cudaGraphExec_t graph_exec = nullptr;   // the plan's graph with this slot's staging buffer as the image (float pushes: no device copy)
+        // A batch's kernels report a wait that ran out here and not on the context, so that the pop of this batch says so: the next
+        // batch already runs when this one is popped. (pinned and mapped, like the context's)
+        volatile int *err_flag = nullptr; int *dev_err_flag = nullptr;
+        // The plan's launches as this slot runs them, put together by the first push of their kind: [0] with the plan's input buffer
+        // as the image, [1] with the slot's staging buffer (float pushes: no device copy).
+        std::vector<msnh::Launch> launches[2]; cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
     } slots[2];
     cudaStream_t copy_stream = nullptr, d2h_stream = nullptr;   // host->device of the next batch / device->host of the last
     int stream_op = -1, stream_cap = 0; size_t stream_result_floats = 0;
@@ -327,7 +332,9 @@ void launch_fill(MsnhB200Ctx *ctx, float *dst, size_t n, float value, cudaStream
 void launch_candidates_to_host(const float *rows, int max_rows, const int *counts, float *host_rows, int cap, int *host_counts, int n_images, cudaStream_t st);
 
 // ---- plan.cu ----
-int check_device_flag(MsnhB200Plan *pl);
+int check_device_flag(MsnhB200Ctx *ctx, volatile int *flag);      // reads and clears an error word
+inline int check_device_flag(MsnhB200Plan *pl) { return check_device_flag(pl->ctx, pl->ctx->err_flag); }
+int alloc_device_flag(MsnhB200Ctx *ctx, volatile int **flag, int **dev_flag);   // a pinned, mapped word that kernels write error codes to
 constexpr int kEarlyRows = 512;                     // candidate rows per image that come back with a synchronous run
 constexpr size_t kEarlyOutputBytes = 1 << 20;       // largest output that does
 // Copy to / from the caller's memory that ends or begins on ctx->stream: pageable memory of half a megabyte or more goes through

@@ -107,25 +107,37 @@ static int stream_setup(MsnhB200Plan *pl, int op) {
         CUDA_TRY(ctx, cudaEventCreateWithFlags(&s.consumed, cudaEventDisableTiming));
         CUDA_TRY(ctx, cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
         for (cudaEvent_t &e : s.piece) CUDA_TRY(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        // Float images go from the slot's staging buffer straight into the forward: a copy of the plan's graph whose
-        // input kernel reads this slot's buffer instead of the plan's own input buffer.
-        if (pl->graph_exec) {
-            std::vector<Launch> mine = pl->launches;
-            bool found = false;
-            for (Launch &L : mine) if (L.in.ptr == pl->d_input) { L.in.ptr = s.d_stage; found = true; }
-            if (found) {
-                cudaGraph_t g = nullptr;
-                CUDA_TRY(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-                for (const Launch &L : mine) launch_one(ctx, L, ctx->stream);
-                const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
-                if (e != cudaSuccess) return fail(ctx, MSNH_B200_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
-                const cudaError_t ei = cudaGraphInstantiate(&s.graph_exec, g, 0);
-                cudaGraphDestroy(g);
-                if (ei != cudaSuccess) return fail(ctx, MSNH_B200_ERR_CUDA, "graph instantiation failed: %s", cudaGetErrorString(ei));
-            }
-        }
+        { const int rc = alloc_device_flag(ctx, &s.err_flag, &s.dev_err_flag); if (rc) return rc; }
     }
     pl->stream_op = op;
+    return MSNH_B200_OK;
+}
+
+// The forward as a slot runs it: the plan's launches with the slot's error word and, for a float push, with the slot's staging
+// buffer as the image where some kernel reads the image itself (`staged`; otherwise the images are copied to the plan's input buffer).
+static int slot_forward(MsnhB200Plan *pl, MsnhB200Plan::StreamSlot &s, bool staged) {
+    MsnhB200Ctx *ctx = pl->ctx;
+    std::vector<Launch> &mine = s.launches[staged];
+    if (mine.empty()) {
+        std::vector<Launch> copy = pl->launches;
+        for (Launch &L : copy) {
+            L.up.err_flag = L.dwp.err_flag = s.dev_err_flag;
+            if (staged && L.in.ptr == pl->d_input) L.in.ptr = s.d_stage;
+        }
+        if (pl->graph_exec) {
+            cudaGraph_t g = nullptr;
+            CUDA_TRY(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+            for (const Launch &L : copy) launch_one(ctx, L, ctx->stream);
+            const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
+            if (e != cudaSuccess) return fail(ctx, MSNH_B200_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
+            const cudaError_t ei = cudaGraphInstantiate(&s.graph_exec[staged], g, 0);
+            cudaGraphDestroy(g);
+            if (ei != cudaSuccess) return fail(ctx, MSNH_B200_ERR_CUDA, "graph instantiation failed: %s", cudaGetErrorString(ei));
+        }
+        mine.swap(copy);
+    }
+    if (s.graph_exec[staged]) CUDA_TRY(ctx, cudaGraphLaunch(s.graph_exec[staged], ctx->stream));
+    else for (const Launch &L : mine) launch_one(ctx, L, ctx->stream);
     return MSNH_B200_OK;
 }
 
@@ -148,6 +160,8 @@ static int stream_push_common(MsnhB200Plan *pl, int op, const void *host_images,
     const size_t bytes = prep ? static_cast<size_t>(n_images) * u8_per_image : static_cast<size_t>(n_images) * image_floats * sizeof(float);
     if (prep && bytes > static_cast<size_t>(pl->batch) * image_floats * sizeof(float))
         return fail(ctx, MSNH_B200_ERR_ARG, "stream_push_u8: %d images of %dx%d do not fit the staging buffer of a batch", n_images, prep->w, prep->h);
+    bool staged = false;
+    for (const Launch &L : pl->launches) staged = staged || (!prep && pl->graph_exec && L.in.ptr == pl->d_input);
     // the slot's staging buffer was last read by the device copy of the batch two pushes ago
     if (pl->push_count >= 2) CUDA_TRY(ctx, cudaStreamWaitEvent(pl->copy_stream, s.consumed, 0));
     CUDA_TRY(ctx, cudaMemcpyAsync(s.d_stage, host_images, bytes, cudaMemcpyHostToDevice, pl->copy_stream));
@@ -156,18 +170,14 @@ static int stream_push_common(MsnhB200Plan *pl, int op, const void *host_images,
     if (prep) {
         launch_preprocess_u8(reinterpret_cast<const unsigned char *>(s.d_stage), pl->d_input, *prep, n_images, ctx->stream);
         CUDA_TRY(ctx, cudaGetLastError());
-    } else if (!s.graph_exec) {
+    } else if (!staged) {
         CUDA_TRY(ctx, cudaMemcpyAsync(pl->d_input, s.d_stage, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     }
-    if (!prep && s.graph_exec) {
-        // the forward reads the staging buffer itself: it is free for the next copy-in when the forward is done
-        CUDA_TRY(ctx, cudaGraphLaunch(s.graph_exec, ctx->stream));
-        CUDA_TRY(ctx, cudaEventRecord(s.consumed, ctx->stream));
-    } else {
-        CUDA_TRY(ctx, cudaEventRecord(s.consumed, ctx->stream));
-        if (pl->graph_exec) CUDA_TRY(ctx, cudaGraphLaunch(pl->graph_exec, ctx->stream));
-        else for (const Launch &L : pl->launches) launch_one(ctx, L, ctx->stream);
-    }
+    // staged: the forward reads the staging buffer itself, which is free for the next copy-in when the forward is done
+    if (!staged) CUDA_TRY(ctx, cudaEventRecord(s.consumed, ctx->stream));
+    rc = slot_forward(pl, s, staged);
+    if (rc) return rc;
+    if (staged) CUDA_TRY(ctx, cudaEventRecord(s.consumed, ctx->stream));
     const OpState &o = pl->ops[op];
     pl->early_valid = false;
     // A short result (candidates, boxes, logits) is written to the slot's pinned memory by a kernel behind the forward. A long one
@@ -273,7 +283,7 @@ int msnh_b200_plan_stream_pop(MsnhB200Plan *pl, float *result, size_t capacity_f
     }
     s.busy = false;
     ++pl->pop_count;
-    return check_device_flag(pl);
+    return check_device_flag(ctx, s.err_flag);
 }
 
 int msnh_b200_plan_stream_reset(MsnhB200Plan *pl) {
@@ -283,8 +293,15 @@ int msnh_b200_plan_stream_reset(MsnhB200Plan *pl) {
     if (pl->copy_stream) CUDA_TRY(ctx, cudaStreamSynchronize(pl->copy_stream));
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     if (pl->d2h_stream) CUDA_TRY(ctx, cudaStreamSynchronize(pl->d2h_stream));
-    for (auto &s : pl->slots) s.busy = false;
+    for (auto &s : pl->slots) { s.busy = false; if (s.err_flag) *s.err_flag = 0; }
     pl->pop_count = pl->push_count;
+    return MSNH_B200_OK;
+}
+
+int msnh_b200_plan_stream_set_error(MsnhB200Plan *pl, int code) {
+    if (!pl) return MSNH_B200_ERR_ARG;
+    if (pl->pop_count >= pl->push_count) return fail(pl->ctx, MSNH_B200_ERR_STATE, "stream_set_error: nothing in flight");
+    *pl->slots[(pl->push_count - 1) & 1].err_flag = code;
     return MSNH_B200_OK;
 }
 
