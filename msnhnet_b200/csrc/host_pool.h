@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
+#include <exception>
 #include <functional>
 #include <memory>
 #include <mutex>
@@ -14,6 +15,24 @@
 #include <vector>
 
 namespace msnh {
+
+// Starts fn(0) .. fn(n - 1) on a thread each, as far as the process may start threads; returns how many did.
+template <typename F> int start_threads(std::vector<std::thread> &threads, int n, F fn) {
+    int started = 0;
+    try {
+        threads.reserve(threads.size() + static_cast<size_t>(std::max(0, n)));
+        for (; started < n; ++started) threads.emplace_back(fn, started);
+    } catch (const std::exception &) {}                       // std::system_error: no more threads; std::bad_alloc
+    return started;
+}
+// fn(0) .. fn(n - 1) shared out over `threads` threads (the caller is one of them); fn must not throw.
+template <typename F> void strided_rows(int n, int threads, F &&fn) {
+    auto share = [&](int t) { for (int i = t; i < n; i += threads) fn(i); };
+    std::vector<std::thread> others;
+    const int started = start_threads(others, threads - 1, share);
+    for (int t = started; t < threads; ++t) share(t);         // the caller's own, and those that no thread took
+    for (auto &th : others) th.join();
+}
 
 class HostPool {
 public:
@@ -27,9 +46,12 @@ public:
         }();
         return workers;
     }
+    // Where the process may start no more threads the pool makes do with those that started, none of them if need be: the caller
+    // takes part in every job.
     explicit HostPool(int workers) {
-        for (int t = 0; t < workers; ++t) threads_.emplace_back([this]() { work(); });
+        start_threads(threads_, workers, [this](int) { work(); });
     }
+    int workers() const { return static_cast<int>(threads_.size()); }
     ~HostPool() {
         { std::lock_guard<std::mutex> g(m_); stop_ = true; }
         wake_.notify_all();
@@ -42,8 +64,8 @@ public:
     void begin(int n, std::function<void(int)> fn) {
         std::unique_lock<std::mutex> g(m_);
         idle_.wait(g, [&]() { return active_ == 0; });       // a worker that woke late for the job before
-        fn_ = std::move(fn); n_ = n;
         if (static_cast<int>(done_size_) < n) { done_.reset(new std::atomic<bool>[n]); done_size_ = n; }
+        fn_ = std::move(fn); n_ = n;
         for (int i = 0; i < n; ++i) done_[i].store(false, std::memory_order_relaxed);
         next_.store(0, std::memory_order_relaxed);
         ++job_;

@@ -134,7 +134,7 @@ void parallel_memcpy(MsnhB200Ctx *ctx, void *dst, const void *src, size_t bytes)
 }
 int copy_in(MsnhB200Plan *pl, void *dev, const void *host, size_t bytes) {
     MsnhB200Ctx *ctx = pl->ctx;
-    if (bytes < kPoolBytes || HostPool::default_workers() < kMinWorkers || !is_pageable(host)) {
+    if (bytes < kPoolBytes || !is_pageable(host) || HostPool::default_workers() < kMinWorkers || pool_of(ctx).workers() < kMinWorkers) {
         CUDA_TRY(ctx, cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, ctx->stream));
         return MSNH_B200_OK;
     }
@@ -165,7 +165,7 @@ int copy_in(MsnhB200Plan *pl, void *dev, const void *host, size_t bytes) {
 }
 int copy_out(MsnhB200Plan *pl, void *host, const void *dev, size_t bytes) {
     MsnhB200Ctx *ctx = pl->ctx;
-    if (bytes < kPoolBytes || HostPool::default_workers() < kMinWorkers || !is_pageable(host)) {
+    if (bytes < kPoolBytes || !is_pageable(host) || HostPool::default_workers() < kMinWorkers || pool_of(ctx).workers() < kMinWorkers) {
         CUDA_TRY(ctx, cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream));
         CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
         return MSNH_B200_OK;

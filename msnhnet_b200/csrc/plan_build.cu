@@ -67,11 +67,7 @@ bool sole_consumer(MsnhB200Plan *pl, int op, int *consumer) {
 template <typename F> void parallel_rows(int n, size_t work_per_row, F &&fn) {
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     const int threads = static_cast<int>(std::min<size_t>(std::min<unsigned>(hw, 16), static_cast<size_t>(n) * work_per_row / 262144 + 1));
-    if (threads <= 1) { for (int i = 0; i < n; ++i) fn(i); return; }
-    std::vector<std::thread> pool;
-    for (int t = 0; t < threads; ++t)
-        pool.emplace_back([&, t]() { for (int i = t; i < n; i += threads) fn(i); });
-    for (auto &th : pool) th.join();
+    strided_rows(n, threads, fn);
 }
 
 // fp32 -> nearest tf32 (10-bit mantissa, ties away from zero like cvt.rna), still stored as fp32
