@@ -85,17 +85,19 @@ int msnh_b200_clock_probe_stop(void *handle, double *mhz_median, double *mhz_min
     *p->h_stop = 1;
     int rc = cudaStreamSynchronize(p->stream) == cudaSuccess ? MSNH_B200_OK : MSNH_B200_ERR_CUDA;
     int n = 0;
-    std::vector<long long> s;
-    if (rc == MSNH_B200_OK && cudaMemcpy(&n, p->d_count, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess && n > 1) {
-        s.resize(2 * static_cast<size_t>(n));
-        if (cudaMemcpy(s.data(), p->d_samples, sizeof(long long) * s.size(), cudaMemcpyDeviceToHost) != cudaSuccess) n = 0;
-    }
     std::vector<double> mhz;
-    for (int i = 1; i < n; ++i) {
-        const double ns = static_cast<double>(s[2 * i] - s[2 * i - 2]);
-        if (ns > 0) mhz.push_back(static_cast<double>(s[2 * i + 1] - s[2 * i - 1]) / ns * 1000.0);
-    }
-    std::sort(mhz.begin(), mhz.end());
+    try {
+        std::vector<long long> s;
+        if (rc == MSNH_B200_OK && cudaMemcpy(&n, p->d_count, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess && n > 1) {
+            s.resize(2 * static_cast<size_t>(n));
+            if (cudaMemcpy(s.data(), p->d_samples, sizeof(long long) * s.size(), cudaMemcpyDeviceToHost) != cudaSuccess) n = 0;
+        }
+        for (int i = 1; i < n; ++i) {
+            const double ns = static_cast<double>(s[2 * i] - s[2 * i - 2]);
+            if (ns > 0) mhz.push_back(static_cast<double>(s[2 * i + 1] - s[2 * i - 1]) / ns * 1000.0);
+        }
+        std::sort(mhz.begin(), mhz.end());
+    } catch (const std::bad_alloc &) { rc = MSNH_B200_ERR_NOMEM; mhz.clear(); }
     if (mhz_median) *mhz_median = mhz.empty() ? 0.0 : mhz[mhz.size() / 2];
     if (mhz_min) *mhz_min = mhz.empty() ? 0.0 : mhz.front();
     if (mhz_max) *mhz_max = mhz.empty() ? 0.0 : mhz.back();

@@ -31,6 +31,17 @@ int fail(MsnhB200Ctx *ctx, int code, const char *fmt, ...) {
     return code;
 }
 
+int caught(MsnhB200Ctx *ctx) noexcept {
+    int code = MSNH_B200_ERR_STATE;
+    try {
+        try { throw; }
+        catch (const std::bad_alloc &) { code = MSNH_B200_ERR_NOMEM; return fail(ctx, code, "out of host memory"); }
+        catch (const std::length_error &) { code = MSNH_B200_ERR_NOMEM; return fail(ctx, code, "out of host memory"); }
+        catch (const std::exception &e) { return fail(ctx, code, "%s", e.what()); }
+        catch (...) { return fail(ctx, code, "unknown exception"); }
+    } catch (...) { return code; }                            // (no room for the text)
+}
+
 PlanDebugOptions PlanDebugOptions::from_env() {
     auto flag = [](const char *name) { const char *e = std::getenv(name); return e != nullptr; };
     auto num = [](const char *name, int unset) { const char *e = std::getenv(name); return e ? atoi(e) : unset; };
@@ -198,7 +209,7 @@ int msnh_b200_device_count(int *count) {
     return MSNH_B200_OK;
 }
 
-int msnh_b200_ctx_create(int device, MsnhB200Ctx **out) {
+int msnh_b200_ctx_create(int device, MsnhB200Ctx **out) try {
     if (!out) return MSNH_B200_ERR_ARG;
     *out = nullptr;
     int n = 0;
@@ -227,7 +238,7 @@ int msnh_b200_ctx_create(int device, MsnhB200Ctx **out) {
     }
     *out = ctx;
     return MSNH_B200_OK;
-}
+} catch (...) { return caught(nullptr); }
 
 int msnh_b200_ctx_destroy(MsnhB200Ctx *ctx) {
     if (!ctx) return MSNH_B200_ERR_ARG;
@@ -241,40 +252,40 @@ int msnh_b200_ctx_destroy(MsnhB200Ctx *ctx) {
 
 const char *msnh_b200_last_error(MsnhB200Ctx *ctx) { return ctx ? ctx->last_error.c_str() : "null context"; }
 
-int msnh_b200_host_alloc(MsnhB200Ctx *ctx, size_t bytes, void **ptr) {
+int msnh_b200_host_alloc(MsnhB200Ctx *ctx, size_t bytes, void **ptr) try {
     if (!ctx || !ptr) return MSNH_B200_ERR_ARG;
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
     CUDA_TRY(ctx, cudaMallocHost(ptr, bytes));
     return MSNH_B200_OK;
-}
-int msnh_b200_host_free(MsnhB200Ctx *ctx, void *ptr) {
+} catch (...) { return caught(ctx); }
+int msnh_b200_host_free(MsnhB200Ctx *ctx, void *ptr) try {
     if (!ctx) return MSNH_B200_ERR_ARG;
     CUDA_TRY(ctx, cudaFreeHost(ptr));
     return MSNH_B200_OK;
-}
+} catch (...) { return caught(ctx); }
 
 int msnh_b200_plan_create(MsnhB200Ctx *ctx, const MsnhB200Op *ops, int n_ops, int in_c, int in_h, int in_w, int batch,
-                          int dtype, uint32_t flags, MsnhB200Plan **out) {
+                          int dtype, uint32_t flags, MsnhB200Plan **out) try {
     if (!ctx || !ops || !out || n_ops <= 0) return fail(ctx, MSNH_B200_ERR_ARG, "plan_create: null or empty argument");
     *out = nullptr;
     if (in_c <= 0 || in_h <= 0 || in_w <= 0 || batch <= 0) return fail(ctx, MSNH_B200_ERR_ARG, "plan_create: bad input shape %dx%dx%d batch %d", in_c, in_h, in_w, batch);
     if (dtype != MSNH_B200_F32 && dtype != MSNH_B200_F16) return fail(ctx, MSNH_B200_ERR_ARG, "plan_create: dtype %d", dtype);
-    MsnhB200Plan *pl = new MsnhB200Plan();
+    std::unique_ptr<MsnhB200Plan> pl(new MsnhB200Plan());
     pl->ctx = ctx; pl->in_c = in_c; pl->in_h = in_h; pl->in_w = in_w; pl->batch = batch; pl->dtype = dtype; pl->flags = flags;
     pl->ops.resize(n_ops);
     for (int i = 0; i < n_ops; ++i) {
         pl->ops[i].d = ops[i];
         std::string err;
-        int rc = infer_shape(pl, i, err);
-        if (rc) { int r = fail(ctx, rc, "op %d (kind %d): %s", i, ops[i].kind, err.c_str()); delete pl; return r; }
-        if (ops[i].act < 0 || ops[i].act >= MSNH_ACT_COUNT) { int r = fail(ctx, MSNH_B200_ERR_UNSUPPORTED, "op %d: activation %d not supported", i, ops[i].act); delete pl; return r; }
+        int rc = infer_shape(pl.get(), i, err);
+        if (rc) return fail(ctx, rc, "op %d (kind %d): %s", i, ops[i].kind, err.c_str());
+        if (ops[i].act < 0 || ops[i].act >= MSNH_ACT_COUNT) return fail(ctx, MSNH_B200_ERR_UNSUPPORTED, "op %d: activation %d not supported", i, ops[i].act);
     }
     // fp32 detection nets: fp32 arithmetic throughout unless tf32 is asked for (see MSNH_PLAN_TF32_DETECT)
     if (dtype == MSNH_B200_F32 && !(flags & MSNH_PLAN_TF32_DETECT))
         for (int i = 0; i < n_ops; ++i) if (ops[i].kind == MSNH_OP_YOLO) { pl->flags |= MSNH_PLAN_NO_TENSOR_CORE; break; }
-    *out = pl;
+    *out = pl.release();
     return MSNH_B200_OK;
-}
+} catch (...) { return caught(ctx); }
 
 int msnh_b200_plan_op_shape(MsnhB200Plan *pl, int op, int *c, int *h, int *w) {
     if (!pl || op < 0 || op >= static_cast<int>(pl->ops.size())) return MSNH_B200_ERR_ARG;
@@ -288,23 +299,23 @@ int msnh_b200_plan_weight_count(MsnhB200Plan *pl, int op, int slot, size_t *coun
     return MSNH_B200_OK;
 }
 
-int msnh_b200_plan_set_weights(MsnhB200Plan *pl, int op, int slot, const float *data, size_t count) {
+int msnh_b200_plan_set_weights(MsnhB200Plan *pl, int op, int slot, const float *data, size_t count) try {
     if (!pl) return MSNH_B200_ERR_ARG;
     if (pl->finalized) return fail(pl->ctx, MSNH_B200_ERR_STATE, "set_weights after finalize");
     if (!data || op < 0 || op >= static_cast<int>(pl->ops.size()) || slot < 0 || slot >= MSNH_W_SLOTS) return fail(pl->ctx, MSNH_B200_ERR_ARG, "set_weights: bad argument");
     if (count != pl->ops[op].wcount[slot]) return fail(pl->ctx, MSNH_B200_ERR_ARG, "set_weights: op %d slot %d expects %zu floats, got %zu", op, slot, pl->ops[op].wcount[slot], count);
     pl->ops[op].w[slot].assign(data, data + count);
     return MSNH_B200_OK;
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
-int msnh_b200_plan_use_pack(MsnhB200Plan *pl, const char *path, uint64_t weights_tag, int *usable) {
+int msnh_b200_plan_use_pack(MsnhB200Plan *pl, const char *path, uint64_t weights_tag, int *usable) try {
     if (!pl || !path || !*path) return MSNH_B200_ERR_ARG;
     if (pl->finalized) return fail(pl->ctx, MSNH_B200_ERR_STATE, "use_pack after finalize");
     pl->pack_path = path; pl->pack_tag = weights_tag;
     pl->dbg = PlanDebugOptions::from_env();
     if (usable) *usable = pack_probe(pl) ? 1 : 0;
     return MSNH_B200_OK;
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
 // The result a synchronous run brings back with it: that of the plan's only output op, when it is a candidate list or small.
 static int early_result_setup(MsnhB200Plan *pl) {
@@ -329,7 +340,7 @@ static int early_result_setup(MsnhB200Plan *pl) {
     return MSNH_B200_OK;
 }
 
-int msnh_b200_plan_finalize(MsnhB200Plan *pl) {
+int msnh_b200_plan_finalize(MsnhB200Plan *pl) try {
     if (!pl) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (pl->finalized) return fail(ctx, MSNH_B200_ERR_STATE, "finalize called twice");
@@ -359,14 +370,17 @@ int msnh_b200_plan_finalize(MsnhB200Plan *pl) {
     CUDA_TRY(ctx, cudaGetLastError());
     pl->finalized = true;
     return MSNH_B200_OK;
+} catch (...) {
+    if (pl && !pl->finalized) pl->finalize_failed = true;
+    return caught(pl ? pl->ctx : nullptr);
 }
 
-int msnh_b200_plan_input_buffer(MsnhB200Plan *pl, float **dev_ptr) {
+int msnh_b200_plan_input_buffer(MsnhB200Plan *pl, float **dev_ptr) try {
     if (!pl || !dev_ptr) return MSNH_B200_ERR_ARG;
     if (!pl->finalized) return fail(pl->ctx, MSNH_B200_ERR_STATE, "plan not finalized");
     *dev_ptr = pl->d_input;
     return MSNH_B200_OK;
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
 static const Launch *collect_launch(const MsnhB200Plan *pl, int op) {
     for (const Launch &L : pl->launches) if (L.kind == L_COLLECT_ZERO && L.op == op) return &L;
@@ -402,7 +416,7 @@ static int run_common(MsnhB200Plan *pl, int n_images, int sync) {
     return MSNH_B200_OK;
 }
 
-int msnh_b200_plan_run(MsnhB200Plan *pl, const float *host_nchw, int n_images) {
+int msnh_b200_plan_run(MsnhB200Plan *pl, const float *host_nchw, int n_images) try {
     if (!pl || !host_nchw) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (!pl->finalized) return fail(ctx, MSNH_B200_ERR_STATE, "plan not finalized");
@@ -411,9 +425,9 @@ int msnh_b200_plan_run(MsnhB200Plan *pl, const float *host_nchw, int n_images) {
     const size_t bytes = static_cast<size_t>(n_images) * pl->in_c * pl->in_h * pl->in_w * sizeof(float);
     { const int rc = copy_in(pl, pl->d_input, host_nchw, bytes); if (rc) return rc; }
     return run_common(pl, n_images, 1);
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
-int msnh_b200_plan_run_device(MsnhB200Plan *pl, const float *dev_nchw, int n_images, int sync) {
+int msnh_b200_plan_run_device(MsnhB200Plan *pl, const float *dev_nchw, int n_images, int sync) try {
     if (!pl) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (!pl->finalized) return fail(ctx, MSNH_B200_ERR_STATE, "plan not finalized");
@@ -424,9 +438,9 @@ int msnh_b200_plan_run_device(MsnhB200Plan *pl, const float *dev_nchw, int n_ima
         CUDA_TRY(ctx, cudaMemcpyAsync(pl->d_input, dev_nchw, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     }
     return run_common(pl, n_images, sync);
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
-int msnh_b200_plan_run_timed(MsnhB200Plan *pl, int n_images, int steps, float *total_ms) {
+int msnh_b200_plan_run_timed(MsnhB200Plan *pl, int n_images, int steps, float *total_ms) try {
     if (!pl || !total_ms || steps < 1) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (!pl->finalized) return fail(ctx, MSNH_B200_ERR_STATE, "plan not finalized");
@@ -444,9 +458,9 @@ int msnh_b200_plan_run_timed(MsnhB200Plan *pl, int n_images, int steps, float *t
     CUDA_TRY(ctx, cudaEventElapsedTime(total_ms, pl->ev0, pl->ev1));
     pl->timed_steps = steps;
     return check_device_flag(pl);
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
-int msnh_b200_plan_run_instrumented(MsnhB200Plan *pl, int n_images, int steps, float *ms, int capacity) {
+int msnh_b200_plan_run_instrumented(MsnhB200Plan *pl, int n_images, int steps, float *ms, int capacity) try {
     if (!pl || !ms || steps < 1) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (!pl->finalized) return fail(ctx, MSNH_B200_ERR_STATE, "plan not finalized");
@@ -474,9 +488,9 @@ int msnh_b200_plan_run_instrumented(MsnhB200Plan *pl, int n_images, int steps, f
     for (auto &e : ev) cudaEventDestroy(e);
     (void)n_images;
     return check_device_flag(pl);
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
-int msnh_b200_plan_read_output(MsnhB200Plan *pl, int op, float *host, size_t count) {
+int msnh_b200_plan_read_output(MsnhB200Plan *pl, int op, float *host, size_t count) try {
     if (!pl || !host) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (!pl->finalized) return fail(ctx, MSNH_B200_ERR_STATE, "plan not finalized");
@@ -502,9 +516,9 @@ int msnh_b200_plan_read_output(MsnhB200Plan *pl, int op, float *host, size_t cou
     const int dt = pl->tensors[o.tensor].dtype;
     launch_readback(ctx, dt, v, pl->d_readback, count, ctx->stream);
     return copy_out(pl, host, pl->d_readback, count * sizeof(float));
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
-int msnh_b200_plan_read_candidates(MsnhB200Plan *pl, int op, int n_images, float *rows, int max_rows, int *counts) {
+int msnh_b200_plan_read_candidates(MsnhB200Plan *pl, int op, int n_images, float *rows, int max_rows, int *counts) try {
     if (!pl || !rows || !counts) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (!pl->finalized) return fail(ctx, MSNH_B200_ERR_STATE, "plan not finalized");
@@ -540,7 +554,7 @@ int msnh_b200_plan_read_candidates(MsnhB200Plan *pl, int op, int n_images, float
         std::sort(r, r + counts[i], [](const Row &a, const Row &b) { return a.v[7] < b.v[7]; });
     }
     return MSNH_B200_OK;
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
 
 int msnh_b200_plan_last_ms(MsnhB200Plan *pl, float *ms) {
@@ -562,7 +576,7 @@ int msnh_b200_plan_stats(MsnhB200Plan *pl, int *launches, size_t *arena_bytes) {
 
 const char *msnh_b200_plan_describe(MsnhB200Plan *pl) { return pl ? pl->description.c_str() : ""; }
 
-int msnh_b200_plan_profile(MsnhB200Plan *pl, int iters, float *ms, int capacity) {
+int msnh_b200_plan_profile(MsnhB200Plan *pl, int iters, float *ms, int capacity) try {
     if (!pl || !ms || iters < 1) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (!pl->finalized) return fail(ctx, MSNH_B200_ERR_STATE, "plan not finalized");
@@ -593,9 +607,9 @@ int msnh_b200_plan_profile(MsnhB200Plan *pl, int iters, float *ms, int capacity)
         ms[k] = total / iters;
     }
     return check_device_flag(pl);
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
-int msnh_b200_plan_read_trace(MsnhB200Plan *pl, int launch, long long *stamps, int capacity, int *ctas) {
+int msnh_b200_plan_read_trace(MsnhB200Plan *pl, int launch, long long *stamps, int capacity, int *ctas) try {
     if (!pl || !stamps || !ctas) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (launch < 0 || launch >= static_cast<int>(pl->launches.size())) return fail(ctx, MSNH_B200_ERR_ARG, "read_trace: launch %d", launch);
@@ -609,7 +623,7 @@ int msnh_b200_plan_read_trace(MsnhB200Plan *pl, int launch, long long *stamps, i
     CUDA_TRY(ctx, cudaMemset(L.up.trace, 0, sizeof(long long) * n));
     *ctas = L.grid;
     return MSNH_B200_OK;
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
 int msnh_b200_plan_destroy(MsnhB200Plan *pl) {
     if (!pl) return MSNH_B200_ERR_ARG;

@@ -24,6 +24,7 @@
 #include <memory>
 #include <mutex>
 #include <new>
+#include <stdexcept>
 #include <string>
 #include <vector>
 
@@ -62,6 +63,8 @@ namespace msnh {
 
 // records the message on the context (when there is one) and returns `code`
 int fail(MsnhB200Ctx *ctx, int code, const char *fmt, ...);
+// the status of the exception being handled: what a C entry point that allocates or starts threads returns for it
+int caught(MsnhB200Ctx *ctx) noexcept;
 #define CUDA_TRY(ctx, expr)                                                                          \
     do {                                                                                             \
         cudaError_t e_ = (expr);                                                                     \

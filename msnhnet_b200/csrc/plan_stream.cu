@@ -8,7 +8,7 @@ extern "C" {
 static int prep_params(MsnhB200Plan *pl, int width, int height, int mode, int swap_rgb, const float *mean, const float *std, PrepParams *p);
 
 int msnh_b200_plan_preprocess_u8(MsnhB200Plan *pl, const unsigned char *host_hwc, int width, int height, int image, int mode,
-                                 int swap_rgb, const float *mean, const float *std) {
+                                 int swap_rgb, const float *mean, const float *std) try {
     if (!pl || !host_hwc) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (!pl->finalized) return fail(ctx, MSNH_B200_ERR_STATE, "plan not finalized");
@@ -31,7 +31,7 @@ int msnh_b200_plan_preprocess_u8(MsnhB200Plan *pl, const unsigned char *host_hwc
     // the device itself. Everything after that is in stream order.
     if (!is_pageable(host_hwc)) CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     return MSNH_B200_OK;
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
 static int nms_buffers(MsnhB200Plan *pl) {
     MsnhB200Ctx *ctx = pl->ctx;
@@ -43,7 +43,7 @@ static int nms_buffers(MsnhB200Plan *pl) {
     return MSNH_B200_OK;
 }
 
-int msnh_b200_plan_nms(MsnhB200Plan *pl, int op, int n_images, float nms_thresh, int use_soft_nms, float sigma, float *boxes, int max_boxes, int *counts) {
+int msnh_b200_plan_nms(MsnhB200Plan *pl, int op, int n_images, float nms_thresh, int use_soft_nms, float sigma, float *boxes, int max_boxes, int *counts) try {
     if (!pl || !boxes || !counts) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (!pl->finalized) return fail(ctx, MSNH_B200_ERR_STATE, "plan not finalized");
@@ -68,14 +68,14 @@ int msnh_b200_plan_nms(MsnhB200Plan *pl, int op, int n_images, float nms_thresh,
     }
     CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     return check_device_flag(pl);
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
-int msnh_b200_plan_stream_nms(MsnhB200Plan *pl, int enable, float nms_thresh, int use_soft_nms, float sigma) {
+int msnh_b200_plan_stream_nms(MsnhB200Plan *pl, int enable, float nms_thresh, int use_soft_nms, float sigma) try {
     if (!pl) return MSNH_B200_ERR_ARG;
     if (pl->push_count != pl->pop_count) return fail(pl->ctx, MSNH_B200_ERR_STATE, "stream_nms: batches in flight");
     pl->stream_nms = enable != 0; pl->nms_thresh = nms_thresh; pl->nms_soft = use_soft_nms; pl->nms_sigma = sigma;
     return enable ? nms_buffers(pl) : MSNH_B200_OK;
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
 // ---- pipelined streaming -------------------------------------------------------------------------
 // Batch i+1 is copied host->device on the copy stream while batch i computes; the (small) result of
@@ -218,9 +218,9 @@ static int stream_push_common(MsnhB200Plan *pl, int op, const void *host_images,
     return MSNH_B200_OK;
 }
 
-int msnh_b200_plan_stream_push(MsnhB200Plan *pl, int op, const float *host_nchw, int n_images) {
+int msnh_b200_plan_stream_push(MsnhB200Plan *pl, int op, const float *host_nchw, int n_images) try {
     return stream_push_common(pl, op, host_nchw, n_images, nullptr);
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
 static int prep_params(MsnhB200Plan *pl, int width, int height, int mode, int swap_rgb, const float *mean, const float *std, PrepParams *p) {
     MsnhB200Ctx *ctx = pl->ctx;
@@ -237,15 +237,15 @@ static int prep_params(MsnhB200Plan *pl, int width, int height, int mode, int sw
 }
 
 int msnh_b200_plan_stream_push_u8(MsnhB200Plan *pl, int op, const unsigned char *host_hwc, int width, int height, int n_images, int mode,
-                                  int swap_rgb, const float *mean, const float *std) {
+                                  int swap_rgb, const float *mean, const float *std) try {
     if (!pl || !host_hwc) return MSNH_B200_ERR_ARG;
     PrepParams p{};
     const int rc = prep_params(pl, width, height, mode, swap_rgb, mean, std, &p);
     if (rc) return rc;
     return stream_push_common(pl, op, host_hwc, n_images, &p);
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
-int msnh_b200_plan_stream_pop(MsnhB200Plan *pl, float *result, size_t capacity_floats, int max_rows, int *counts, int *n_images) {
+int msnh_b200_plan_stream_pop(MsnhB200Plan *pl, float *result, size_t capacity_floats, int max_rows, int *counts, int *n_images) try {
     if (!pl || !result) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     if (pl->pop_count >= pl->push_count) return fail(ctx, MSNH_B200_ERR_STATE, "stream_pop: nothing in flight");
@@ -284,9 +284,9 @@ int msnh_b200_plan_stream_pop(MsnhB200Plan *pl, float *result, size_t capacity_f
     s.busy = false;
     ++pl->pop_count;
     return check_device_flag(ctx, s.err_flag);
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
-int msnh_b200_plan_stream_reset(MsnhB200Plan *pl) {
+int msnh_b200_plan_stream_reset(MsnhB200Plan *pl) try {
     if (!pl) return MSNH_B200_ERR_ARG;
     MsnhB200Ctx *ctx = pl->ctx;
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
@@ -296,13 +296,13 @@ int msnh_b200_plan_stream_reset(MsnhB200Plan *pl) {
     for (auto &s : pl->slots) { s.busy = false; if (s.err_flag) *s.err_flag = 0; }
     pl->pop_count = pl->push_count;
     return MSNH_B200_OK;
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
-int msnh_b200_plan_stream_set_error(MsnhB200Plan *pl, int code) {
+int msnh_b200_plan_stream_set_error(MsnhB200Plan *pl, int code) try {
     if (!pl) return MSNH_B200_ERR_ARG;
     if (pl->pop_count >= pl->push_count) return fail(pl->ctx, MSNH_B200_ERR_STATE, "stream_set_error: nothing in flight");
     *pl->slots[(pl->push_count - 1) & 1].err_flag = code;
     return MSNH_B200_OK;
-}
+} catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
 }  // extern "C"
