@@ -6,11 +6,15 @@
 #include <sched.h>
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <condition_variable>
+#include <cstdlib>
 #include <exception>
+#include <fstream>
 #include <functional>
 #include <memory>
 #include <mutex>
+#include <string>
 #include <thread>
 #include <vector>
 
@@ -34,18 +38,52 @@ template <typename F> void strided_rows(int n, int threads, F &&fn) {
     for (auto &th : others) th.join();
 }
 
+// The cpus whose time the control groups of this process grant it (rounded up; 0: no limit): the least along the way from its
+// group to the root, in the unified hierarchy (cpu.max) and in the cpu controller's own (cpu.cfs_quota_us).
+inline int cpu_quota(const std::string &groups = "/proc/self/cgroup", const std::string &root = "/sys/fs/cgroup") {
+    double least = 0;
+    auto limit = [&](double quota, double period) {
+        if (quota > 0 && period > 0 && (least == 0 || quota / period < least)) least = quota / period;
+    };
+    std::ifstream in(groups);
+    std::string line;
+    while (std::getline(in, line)) {                          // hierarchy : controllers : path
+        const size_t a = line.find(':'), b = a == std::string::npos ? a : line.find(':', a + 1);
+        if (b == std::string::npos) continue;
+        const std::string controllers = line.substr(a + 1, b - a - 1);
+        if (!controllers.empty() && ("," + controllers + ",").find(",cpu,") == std::string::npos) continue;
+        const std::string mount = root + (controllers.empty() ? "" : "/" + controllers);
+        for (std::string path = line.substr(b + 1);; path.erase(path.find_last_of('/'))) {
+            const std::string dir = mount + (path == "/" ? "" : path);
+            std::string quota;
+            double period = 0, us = 0;
+            if (controllers.empty()) {
+                std::ifstream f(dir + "/cpu.max");
+                if (f >> quota >> period && quota != "max") limit(std::atof(quota.c_str()), period);
+            } else {
+                std::ifstream q(dir + "/cpu.cfs_quota_us"), p(dir + "/cpu.cfs_period_us");
+                if (q >> us && p >> period) limit(us, period);          // (-1: none)
+            }
+            if (path.find('/') == std::string::npos) break;
+        }
+    }
+    return static_cast<int>(std::ceil(least));
+}
+
 class HostPool {
 public:
-    // threads besides the caller: half of the cpus this process may use, seven at most (eight copying threads fill PCIe)
+    // threads besides the caller: half of the cpus this process may use (the other half are the same cores' second threads), no
+    // more than its control group grants the time of, seven at most (eight copying threads fill PCIe)
     static int default_workers() {
         static const int workers = []() {
             cpu_set_t set;
             int cpus = static_cast<int>(std::thread::hardware_concurrency());
             if (sched_getaffinity(0, sizeof(set), &set) == 0) cpus = CPU_COUNT(&set);
-            return std::max(0, std::min(7, cpus / 2 - 1));
+            return workers_for(cpus, cpu_quota());
         }();
         return workers;
     }
+    static int workers_for(int cpus, int quota) { return std::max(0, std::min({7, cpus / 2 - 1, quota > 0 ? quota - 1 : 7})); }
     // Where the process may start no more threads the pool makes do with those that started, none of them if need be: the caller
     // takes part in every job.
     explicit HostPool(int workers) {

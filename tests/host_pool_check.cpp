@@ -1,5 +1,7 @@
 // The thread pool (host_pool.h) where the process may start only argv[1] more threads: every job is done all the same. Stands
 // in front of pthread_create, so that no limit of the machine has to be touched. Exit code 0: everything was done.
+// With "quota" and the paths of a list of control groups and of their root: prints the cpus they grant; with "workers", a number of
+// cpus and a quota: the pool's threads.
 #include <dlfcn.h>
 #include <errno.h>
 #include <pthread.h>
@@ -16,6 +18,8 @@ extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*fn)
 }
 
 int main(int argc, char **argv) {
+    if (argc > 3 && argv[1][0] == 'w') { std::printf("%d\n", msnh::HostPool::workers_for(std::atoi(argv[2]), std::atoi(argv[3]))); return 0; }   // workers <cpus> <quota>
+    if (argc > 3) { std::printf("%d\n", msnh::cpu_quota(argv[2], argv[3])); return 0; }        // quota <groups> <root>
     const int may_start = argc > 1 ? std::atoi(argv[1]) : 0;
     g_left = may_start;
     std::vector<int> done(1000, 0);
