@@ -110,13 +110,14 @@ public:
         g.unlock();
         wake_.notify_all();
     }
-    bool help() {                                             // one item on the calling thread; false: none left to start
-        const int i = next_.fetch_add(1, std::memory_order_acq_rel);
-        if (i >= n_) return false;
+    bool help(int below = 0x7fffffff) {                       // one item (one before `below`) on the calling thread; false: none left to start
+        int i = next_.load(std::memory_order_relaxed);
+        do { if (i >= n_ || i >= below) return false; } while (!next_.compare_exchange_weak(i, i + 1, std::memory_order_acq_rel, std::memory_order_relaxed));
         fn_(i);
         done_[i].store(true, std::memory_order_release);
         return true;
     }
+    bool all_started(int below) const { return next_.load(std::memory_order_relaxed) >= std::min(below, n_); }   // (of the items before `below`)
     bool done(int i) const { return done_[i].load(std::memory_order_acquire); }
     void finish() {
         while (help()) {}

@@ -8,6 +8,7 @@
 // It stands in for NetBuilder's GPU loop and memory pools (src/net/MsnhNetBuilder.cpp:565-620,
 // :820-1007 in the reference) and for the per-layer forwardGPU bodies.
 #include "plan_internal.h"
+#include <atomic>
 #ifdef __SSE2__
 #include <emmintrin.h>
 #endif
@@ -149,25 +150,40 @@ int copy_in(MsnhB200Plan *pl, void *dev, const void *host, size_t bytes) {
         CUDA_TRY(ctx, cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, ctx->stream));
         return MSNH_B200_OK;
     }
-    { const int rc = pinned_staging(pl, bytes); if (rc) return rc; }
     const size_t chunk = std::min(kCopyChunk, std::max(kMinChunk, (bytes / 8 + 4095) / 4096 * 4096));
-    const int n = static_cast<int>((bytes + chunk - 1) / chunk);
+    const int n = static_cast<int>((bytes + chunk - 1) / chunk), part = static_cast<int>(kStagingBytes / kStagingParts / chunk), ring = kStagingParts * part;
+    { const int rc = pinned_staging(pl, std::min(n, ring) * chunk); if (rc) return rc; }
     HostPool &pool = pool_of(ctx);
     uint8_t *pinned = pl->h_pinned;
-    pool.begin(n, [=](int i) {
+    std::atomic<int> open{ring};                 // chunks before this one may be written: what lay in their place has been sent
+    pool.begin(n, [=, &open](int i) {
+        for (int spins = 0; open.load(std::memory_order_acquire) <= i; ++spins) {
+            if (spins < 200) std::this_thread::yield();
+            else std::this_thread::sleep_for(std::chrono::microseconds(20));           // (the stream is busy with something long)
+        }
         const size_t at = i * chunk;
-        copy_past_caches(pinned + at, static_cast<const uint8_t *>(host) + at, std::min(chunk, bytes - at));
+        copy_past_caches(pinned + static_cast<size_t>(i % ring) * chunk, static_cast<const uint8_t *>(host) + at, std::min(chunk, bytes - at));
     });
-    // send what is ready, in order; copy along while the next chunk is not
+    // send what is ready, in order and up to the ring's end; copy along while the next chunk is not
     cudaError_t e = cudaSuccess;
+    int parts_sent = 0, parts_left = 0;          // parts of the ring behind which an event is queued, and those whose event has come
     for (int sent = 0; sent < n && e == cudaSuccess;) {
+        const int writable = open.load(std::memory_order_relaxed);
+        if (parts_left < parts_sent && pool.all_started(writable)) {
+            const cudaEvent_t ev = pl->ev_part[parts_left % kStagingParts];
+            e = sent < writable ? cudaEventQuery(ev) : cudaEventSynchronize(ev);
+            if (e == cudaSuccess) open.store(ring + ++parts_left * part, std::memory_order_release);
+            else if (e == cudaErrorNotReady) e = cudaSuccess;
+        }
         int ready = sent;
-        while (ready < n && pool.done(ready)) ++ready;
-        if (ready == sent) { if (!pool.help()) std::this_thread::yield(); continue; }
+        while (ready < n && pool.done(ready) && (ready == sent || ready % ring)) ++ready;
+        if (ready == sent) { if (!pool.help(writable)) std::this_thread::yield(); continue; }
         const size_t at = sent * chunk, end = std::min(ready * chunk, bytes);
-        e = cudaMemcpyAsync(static_cast<uint8_t *>(dev) + at, pinned + at, end - at, cudaMemcpyHostToDevice, ctx->stream);
+        e = cudaMemcpyAsync(static_cast<uint8_t *>(dev) + at, pinned + static_cast<size_t>(sent % ring) * chunk, end - at, cudaMemcpyHostToDevice, ctx->stream);
         sent = ready;
+        for (; n > ring && e == cudaSuccess && (parts_sent + 1) * part <= sent; ++parts_sent) e = cudaEventRecord(pl->ev_part[parts_sent % kStagingParts], ctx->stream);
     }
+    open.store(n, std::memory_order_release);
     pool.finish();
     CUDA_TRY(ctx, e);
     CUDA_TRY(ctx, cudaEventRecord(pl->ev_copy, ctx->stream));
@@ -181,16 +197,22 @@ int copy_out(MsnhB200Plan *pl, void *host, const void *dev, size_t bytes) {
         CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
         return MSNH_B200_OK;
     }
-    { const int rc = pinned_staging(pl, bytes); if (rc) return rc; }
-    // two halves, so that the second crosses PCIe while the first is copied on
-    const size_t half = std::min(bytes, (bytes / 2 + kCopyChunk - 1) / kCopyChunk * kCopyChunk);
-    CUDA_TRY(ctx, cudaMemcpyAsync(pl->h_pinned, dev, half, cudaMemcpyDeviceToHost, ctx->stream));
-    CUDA_TRY(ctx, cudaEventRecord(pl->ev_copy, ctx->stream));
-    if (bytes > half) CUDA_TRY(ctx, cudaMemcpyAsync(pl->h_pinned + half, static_cast<const uint8_t *>(dev) + half, bytes - half, cudaMemcpyDeviceToHost, ctx->stream));
-    CUDA_TRY(ctx, cudaEventSynchronize(pl->ev_copy));
-    parallel_memcpy(ctx, host, pl->h_pinned, half);
-    CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-    parallel_memcpy(ctx, static_cast<uint8_t *>(host) + half, pl->h_pinned + half, bytes - half);
+    // in pieces of half the staging at most, so that one crosses PCIe while the one before it is copied on
+    const size_t piece = std::min(kStagingBytes / 2, (bytes / 2 + kCopyChunk - 1) / kCopyChunk * kCopyChunk);
+    const int n = static_cast<int>((bytes + piece - 1) / piece);
+    { const int rc = pinned_staging(pl, std::min(bytes, 2 * piece)); if (rc) return rc; }
+    auto fetch = [&](int k) -> cudaError_t {
+        const size_t at = k * piece;
+        const cudaError_t e = cudaMemcpyAsync(pl->h_pinned + (k & 1) * piece, static_cast<const uint8_t *>(dev) + at, std::min(piece, bytes - at), cudaMemcpyDeviceToHost, ctx->stream);
+        return e == cudaSuccess ? cudaEventRecord(pl->ev_part[k & 1], ctx->stream) : e;
+    };
+    for (int k = 0; k < n && k < 2; ++k) CUDA_TRY(ctx, fetch(k));
+    for (int k = 0; k < n; ++k) {
+        const size_t at = k * piece;
+        CUDA_TRY(ctx, cudaEventSynchronize(pl->ev_part[k & 1]));
+        parallel_memcpy(ctx, static_cast<uint8_t *>(host) + at, pl->h_pinned + (k & 1) * piece, std::min(piece, bytes - at));
+        if (k + 2 < n) CUDA_TRY(ctx, fetch(k + 2));
+    }
     return MSNH_B200_OK;
 }
 
@@ -358,6 +380,7 @@ int msnh_b200_plan_finalize(MsnhB200Plan *pl) try {
     CUDA_TRY(ctx, cudaEventCreate(&pl->ev0));
     CUDA_TRY(ctx, cudaEventCreate(&pl->ev1));
     CUDA_TRY(ctx, cudaEventCreateWithFlags(&pl->ev_copy, cudaEventDisableTiming));
+    for (cudaEvent_t &e : pl->ev_part) CUDA_TRY(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     { const int rc2 = early_result_setup(pl); if (rc2) return rc2; }
     for (OpState &o : pl->ops) for (int s = 0; s < MSNH_W_SLOTS; ++s) { std::vector<float>().swap(o.w[s]); }
     if (!(pl->flags & MSNH_PLAN_NO_GRAPH)) {
@@ -633,6 +656,7 @@ int msnh_b200_plan_destroy(MsnhB200Plan *pl) {
     if (pl->ev0) cudaEventDestroy(pl->ev0);
     if (pl->ev1) cudaEventDestroy(pl->ev1);
     if (pl->ev_copy) cudaEventDestroy(pl->ev_copy);
+    for (cudaEvent_t e : pl->ev_part) if (e) cudaEventDestroy(e);
     if (pl->h_pinned) cudaFreeHost(pl->h_pinned);
     if (pl->h_early) cudaFreeHost(pl->h_early);
     if (pl->h_early_counts) cudaFreeHost(pl->h_early_counts);

@@ -166,6 +166,10 @@ struct Launch {
     std::string note;
 };
 
+// Pinned staging of a plan: a ring that larger images and results go round, in parts the copy engine and the threads hand each
+// other. PCIe moves it in 0.3 ms: room for threads that are late.
+constexpr size_t kStagingBytes = 16 << 20;
+constexpr int kStagingParts = 4;
 // Pieces a long streaming result crosses PCIe in: pop copies one on to the caller's buffer while the next crosses. After the last
 // batch nothing else hides that copy (four batches of FCN-S-320, 16 images and 13 MB of results each: 6.34 -> 6.20 ms).
 constexpr int kResultPieces = 4;
@@ -222,7 +226,7 @@ struct MsnhB200Plan {
     std::vector<std::array<int32_t, 3>> pack_picks; // conv tile shapes (sub-tiles, channels, form) in launch order: stored in / taken from the pack
     uint8_t *d_pack = nullptr;
     std::vector<uint8_t> pack_blob; uint64_t pack_blob_bytes = 0, pack_blob_key = 0, pack_blob_tag = 0;   // a probed pack file: its arena bytes until they are copied
-    uint8_t *h_pinned = nullptr; size_t h_pinned_bytes = 0; bool staging_busy = false;   // pinned staging for callers whose memory is pageable; a copy out of it may be under way (ev_copy)
+    uint8_t *h_pinned = nullptr; size_t h_pinned_bytes = 0; bool staging_busy = false;   // pinned staging (kStagingBytes at most) for callers whose memory is pageable; a copy out of it may be under way (ev_copy)
     int *h_counts = nullptr;                        // pinned
     // Results of the last synchronous run, written to pinned memory behind its kernels so that the read call finds them there:
     // candidate counts and the first kEarlyRows rows per image, or the one small output of a classifier.
@@ -231,6 +235,7 @@ struct MsnhB200Plan {
     float *h_early = nullptr; int *h_early_counts = nullptr;
     cudaGraph_t graph = nullptr; cudaGraphExec_t graph_exec = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_copy = nullptr;
+    cudaEvent_t ev_part[msnh::kStagingParts] = {};  // the copies of a part of the staging have left or arrived
     float last_ms = 0.f; int timed_steps = 0;       // last_ms is brought up to date from the events when it is asked for (0 steps: it is)
     std::string description;
     // pipelined streaming (plan_stream_push / pop): two slots, a copy stream next to the compute stream

@@ -54,3 +54,47 @@ def pop(plan, want):
     out, n = np.empty_like(want), ffi.C.c_int()
     plan.ctx.check(plan.lib.msnh_b200_plan_stream_pop(plan.h, out.ctypes.data_as(ffi.C.POINTER(ffi.C.c_float)), out.size, 0, None, ffi.C.byref(n)))
     assert n.value == len(want) and np.array_equal(out, want)
+
+
+def clip_plan(ctx, c, h, w, batch):
+    plan = ffi.Plan(ctx, [ffi.make_op(ffi.OP_CLIP, [ffi.INPUT], const_val=-10.0, scale=10.0, is_output=1)], (c, h, w), batch, ffi.F32)
+    plan.finalize()
+    return plan
+
+
+# (the pinned staging is a ring of 16 MB: just below it, at it, just above, several times round)
+@pytest.mark.parametrize("floats", [4193792, 4194304, 4194305, 4200000, 8388608, 10000001, 33000003])
+def test_copies_that_go_round_the_staging(floats):
+    rng = np.random.default_rng(4)
+    ctx = ffi.Context(0)
+    plan = clip_plan(ctx, 1, 1, floats, 1)
+    try:
+        for _ in range(3):
+            x = rng.standard_normal(floats, dtype=np.float32)
+            plan.run(x.reshape(1, 1, 1, floats))
+            assert np.array_equal(plan.read_output(0, 1).ravel(), x)
+    finally:
+        plan.close()
+        ctx.close()
+
+
+def address_space_mb():
+    return [int(line.split()[1]) for line in open("/proc/self/status") if line.startswith("VmSize")][0] / 1024
+
+
+def test_staging_does_not_grow_with_the_images():
+    ctx = ffi.Context(0)
+    x = np.zeros((1, 1, 1, 64 << 20), np.float32)            # 256 MB
+    out = np.empty_like(x)
+    small, plan = clip_plan(ctx, 1, 1, 1 << 20, 1), clip_plan(ctx, 1, 1, x.size, 1)
+    try:
+        small.run(x[..., :1 << 20])                           # starts the threads
+        plan.run_device(None, 1)
+        before = address_space_mb()
+        plan.run(x)
+        ctx.check(plan.lib.msnh_b200_plan_read_output(plan.h, 0, out.ctypes.data_as(ffi.C.POINTER(ffi.C.c_float)), out.size))
+        assert address_space_mb() - before < 300              # (the read-back's device buffer of 256 MB may be counted; the staging was as much again)
+    finally:
+        small.close()
+        plan.close()
+        ctx.close()
