@@ -65,7 +65,7 @@ int pick_bk_bytes(int cin, int es) {
 // measured tile shapes, one entry per distinct conv layer signature (process-wide)
 using TuneKey = std::array<int, 23>;
 static std::mutex &tune_mutex() { static std::mutex m; return m; }
-static std::map<TuneKey, std::array<int, 3>> &tune_cache() { static std::map<TuneKey, std::array<int, 3>> c; return c; }
+static std::map<TuneKey, std::array<int, 2>> &tune_cache() { static std::map<TuneKey, std::array<int, 2>> c; return c; }
 
 // The shared-memory tile form of a 3x3 depthwise launch (dwconv_tile.cuh) where it applies: stride 1 or 2, no dilation,
 // whole 16-byte channel vectors. Fills L.dwp, L.map_a, L.grid, L.smem and sets L.dw_tile; leaves L untouched otherwise.
@@ -179,7 +179,7 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
     MsnhB200Ctx *ctx = pl->ctx;
     const int es = esize(pl->dtype);
     const PlanDebugOptions &dbg = pl->dbg;
-    std::vector<std::array<int, 3>> tune_cands;
+    std::vector<std::array<int, 2>> tune_cands;
     ConvUmmaParams &u = L.up;
     const int cin = L.in.C, cout = L.out.C + (L.out2.ptr ? L.out2.C : 0);   // (two merged convs: both channel ranges)
     u.split_n = L.out2.ptr ? L.split_n : 0x7fffffff;
@@ -229,7 +229,7 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
         if (cout <= slab_cols) bns.push_back(round_up(cout, 16));
         else for (int bn = slab_cols; bn <= 256; bn += slab_cols) { bns.push_back(bn); if (bn >= cout) break; }
         double best = 1e30; int best_mm = 1, best_bn = bns[0], best_pair = 0, best_sk = 0;
-        struct Cand { double cost; int mm, bn, sk; };
+        struct Cand { double cost; int mm, bn; };
         std::vector<Cand> cands;                         // every plain (no pair, no stream-K) shape the layer allows
         // Stream-K (equal shares of tiles x k-blocks per SM, partial tiles handed over through global
         // memory): built and parity-tested; on YOLOv4-608 the hand-over (~6k cycles to write a 128 KB
@@ -330,7 +330,7 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
             for (int mm = 1; mm <= 4; ++mm) {
                 const double cost = plain_cost(u.m_total, mm, bn, shares);
                 if (cost < 0) continue;
-                cands.push_back({cost, mm, bn, 0});
+                cands.push_back({cost, mm, bn});
                 if (shares == 1 && measured_only(mm, bn) && !(forced_mm && forced_bn)) continue;    // (forcing both picks such a shape: parity tests)
                 if (cost < best * 0.97 && sk_mode != 1) { best = cost; best_mm = mm; best_bn = bn; best_pair = 0; best_sk = 0; }
                 // stream-K: every SM takes units / SMs k-blocks; hand-over and completion of split tiles
@@ -372,7 +372,7 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
             // (stream-K forms were measured too and never won a layer; more than six runners-up changed nothing)
             const int tune_max = dbg.autotune > 0 ? dbg.autotune : 6;
             for (const Cand &c : cands)
-                if (static_cast<int>(tune_cands.size()) < tune_max && !(c.mm == best_mm && c.bn == best_bn && c.sk == 0)) tune_cands.push_back({c.mm, c.bn, c.sk});
+                if (static_cast<int>(tune_cands.size()) < tune_max && !(c.mm == best_mm && c.bn == best_bn)) tune_cands.push_back({c.mm, c.bn});
         }
     }
     // everything that follows from the tile shape in L.up: ring sizes, shared memory, grid, tensor maps
@@ -455,12 +455,12 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
     if (!tune_cands.empty()) {
         const TuneKey key{pl->dtype, pl->batch, cin, cout, L.in.H, L.in.W, L.out.H, L.out.W, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, L.dh, L.dw,
                           L.act1, L.act2, L.res ? 1 : 0, L.in.ldc, L.out.ldc, u.k_shares, ctx->sm_count};
-        std::array<int, 3> pick{u.m_mult, u.bn, 0};
+        std::array<int, 2> pick{u.m_mult, u.bn};
         bool known = false;
         { std::lock_guard<std::mutex> g(tune_mutex()); auto it = tune_cache().find(key); if (it != tune_cache().end()) { pick = it->second; known = true; } }
         if (!known) {
-            auto time_shape = [&](int mm, int bn, int sk, float *ms) -> int {
-                Launch t = L; t.up.m_mult = mm; t.up.bn = bn; t.up.pair = 0; t.up.stream_k = sk == 1;
+            auto time_shape = [&](int mm, int bn, float *ms) -> int {
+                Launch t = L; t.up.m_mult = mm; t.up.bn = bn;
                 const int rc = configure(t);
                 if (rc) return rc;
                 launch_one(ctx, t, ctx->stream);
@@ -479,20 +479,20 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
                 return MSNH_B200_OK;
             };
             float best_ms = 0.f;
-            int rc = time_shape(u.m_mult, u.bn, 0, &best_ms);
+            int rc = time_shape(u.m_mult, u.bn, &best_ms);
             if (rc) return rc;
             if (best_ms > 1e29f) return fail(ctx, MSNH_B200_ERR_DEVICE_TIMEOUT, "a bounded wait ran out while timing the conv of op %d", L.op);
             const float model_ms = best_ms;
             for (const auto &c : tune_cands) {
                 float ms = 0.f;
-                rc = time_shape(c[0], c[1], c[2], &ms);
+                rc = time_shape(c[0], c[1], &ms);
                 if (rc) return rc;
                 if (ms < best_ms && ms < model_ms * 0.97f) { best_ms = ms; pick = c; }
             }
             std::lock_guard<std::mutex> g(tune_mutex());
             tune_cache()[key] = pick;
         }
-        if (pick[0] != u.m_mult || pick[1] != u.bn || pick[2] != 0) { u.m_mult = pick[0]; u.bn = pick[1]; u.stream_k = pick[2] == 1; L.note += L.note.empty() ? "measured shape" : ", measured shape"; }
+        if (pick[0] != u.m_mult || pick[1] != u.bn) { u.m_mult = pick[0]; u.bn = pick[1]; L.note += L.note.empty() ? "measured shape" : ", measured shape"; }
     }
     { const int rc = configure(L); if (rc) return rc; }
     // form: 0 plain, 1 stream-K, 4 CTA pair; + 0x100 when the shape was a measured choice
