@@ -44,6 +44,7 @@ WORKLOADS = {
     "fcns-320": ("fcns", 320, 16, "fp16", 64.54),
 }
 HEADLINE = "yolov4-608"
+FP32_FMA_TFLOPS = 72.0       # scalar fp32 FMAs from registers, measured (128 lanes x 148 SMs at 1.965 GHz give 74.4)
 # the benchmark configs besides the headline, measured briefly by the default run
 OTHERS = ["yolov5m-640", "yolov3-tiny-416", "mobilenetv2-224", "resnet18-224"]
 # fixed-size jobs split over the GPUs: (workload, images of the whole job)
@@ -302,7 +303,8 @@ def layer_table(desc, per, pk, title):
            f"Per-launch device time: CUDA events between consecutive launches, mean of 5 steps, warm (each figure carries the few microseconds of a "
            f"launch boundary that the graph replay of the timed step overlaps). Roofs: {pk['tflops']:.1f} TFLOP/s sustained dense 16-bit tensor peak and "
            f"{pk['hbm_gbs']:.1f} GB/s copy bandwidth ({pk['source']}), ridge {ridge:.0f} FLOP/B. A launch is held to the tensor roof when its unfused "
-           f"arithmetic intensity (FLOPs over input + output + weight bytes) is above the ridge, to the HBM roof otherwise.", "",
+           f"arithmetic intensity (FLOPs over input + output + weight bytes) is above the ridge, to the HBM roof otherwise; a conv that runs in fp32 "
+           f"arithmetic on the CUDA cores is held to {FP32_FMA_TFLOPS} TFLOP/s in the tensor roof's place.", "",
            "| # | kernel | in -> out | k/s | us | FLOP/B | roof | achieved | fraction |", "|---|---|---|---|---|---|---|---|---|"]
     for line, t in zip(desc, per):
         f = line.split()
@@ -312,14 +314,17 @@ def layer_table(desc, per, pk, title):
         if t <= 0 or (fl == 0 and by == 0):
             continue
         ai = fl / by if by else 0.0
-        if fl > 0 and ai >= ridge:
+        if "fp32 arithmetic" in line and ai >= FP32_FMA_TFLOPS * 1e3 / pk["hbm_gbs"]:
+            ach = fl / (t * 1e-3) / 1e12
+            roof, frac, ach_s = "fp32 FMA", ach / FP32_FMA_TFLOPS, f"{ach:.1f} TFLOP/s"
+        elif fl > 0 and ai >= ridge:
             ach, roof, frac = fl / (t * 1e-3) / 1e12, "tensor", fl / (t * 1e-3) / 1e12 / pk["tflops"]
             ach_s = f"{ach:.0f} TFLOP/s"
         else:
             ach, roof, frac = by / (t * 1e-3) / 1e9, "hbm", by / (t * 1e-3) / 1e9 / pk["hbm_gbs"]
             ach_s = f"{ach:.0f} GB/s"
-        shape = re.search(r"(mm=\d+(?: \w+)* bn=\d+)", line)
-        out.append(f"| {f[0]} | {f[1]}{' ' + shape.group(1) if shape else ''} | {io.group(1)} -> {io.group(2)} | {io.group(3)}/{io.group(4)} | {t * 1000:.1f} | {ai:.0f} | {roof} | {ach_s} | {frac:.2f} |")
+        shape = " ".join(m.group(0) for m in (re.search(r"mm=\d+(?: \w+)* bn=\d+", line), re.search(r"k (?:over|in) \d+ \w+(?: in \d+ shares)?", line)) if m)
+        out.append(f"| {f[0]} | {f[1]}{' ' + shape if shape else ''} | {io.group(1)} -> {io.group(2)} | {io.group(3)}/{io.group(4)} | {t * 1000:.1f} | {ai:.0f} | {roof} | {ach_s} | {frac:.2f} |")
     return "\n".join(out) + "\n"
 
 
@@ -505,7 +510,7 @@ def measure(D, workload, B, fp16, steps, warmup, min_seconds, total_images=None,
             res["kernels"][name] = e
         if profile_out and D.rank == 0:
             with open(profile_out, "w") as f:
-                f.write(layer_table(desc, per, pk, f"Every launch of one step: {workload}, {B} images, {'fp16' if fp16 else 'fp32'} (python bench.py --workload {workload} --profile-out <file>)"))
+                f.write(layer_table(desc, per, pk, f"Every launch of one step: {workload}, {B} images, {'fp16' if fp16 else 'fp32'} (python bench.py --workload {workload} --dtype {'fp16' if fp16 else 'fp32'} --per-gpu-batch {B} --profile-out <file>)"))
                 f.write("\n## By kernel\n\n| kernel | launches | ms | share | TFLOP/s | GB/s |\n|---|---|---|---|---|---|\n")
                 for name, k in sorted(by_kernel.items(), key=lambda kv: -kv[1]["ms"]):
                     f.write(f"| {name} | {k['launches']} | {k['ms']:.4f} | {k['ms'] / step_ms_sum:.3f} | {k['flops'] / max(k['ms'], 1e-9) / 1e9:.1f} | {k['bytes'] / max(k['ms'], 1e-9) / 1e6:.1f} |\n")

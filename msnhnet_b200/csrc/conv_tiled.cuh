@@ -1,8 +1,10 @@
 // Dense convolutions on the CUDA cores in fp32 arithmetic.
 //
+// conv_fp32_kernel (below) serves the plans that must reproduce the reference's fp32 results (its GPU path is fp32 Sgemm
+// throughout, src/layers/MsnhConvolutionalLayer.cpp:1026-1160): fp32 detection nets, whose exp()-decoded boxes do not survive
+// tf32's 10-bit mantissa, and fp32 plans built without tensor cores.
 // conv_tiled_kernel: an implicit GEMM with shared-memory tiles for 16-bit plans built without tensor cores (the cross-check of
-// the tensor-core kernel); fp32 views take conv_fp32_kernel below. Both serve the plans that must reproduce the reference's fp32 results (its GPU path is fp32 Sgemm throughout, src/layers/MsnhConvolutionalLayer.cpp:1026-1160):
-// fp32 detection nets, whose exp()-decoded boxes do not survive tf32's 10-bit mantissa, and plans built without tensor cores.
+// the tensor-core kernel).
 // D[m][n] = sum_k A[m][k] * B[n][k]: m = output pixel (linear over image, row, column), n = output channel, k = (filter
 // tap, input channel) tap-major like the packed weights [Cout][tap][cin_pad]. A CTA of 256 threads computes 128 pixels x
 // 64 channels; a k-step stages 128 x BK input values (gathered with the conv's stride / padding / dilation, zero outside the
@@ -158,8 +160,9 @@ conv_tiled_kernel(TView in, TView out, const T *__restrict__ w, const ConvTiledP
 //    fall in different banks); a ring of four k-steps, cp.async also zero-fills the padding, pad channels and ragged edges. A
 //    loader thread keeps its source addresses and moves them along while its vectors stay inside one filter tap.
 // Measured against the 128 x 64 tile form above: 3x3 384->384 at 11x11, three images 514 -> 46 us; YOLOv5m-352, three images
-// 14.9 -> 2.8 ms a forward; YOLOv3-tiny-416, one image 3.0 -> 0.42 ms. Layers that fill the chip run at 41 TFLOP/s (3x3
-// 512->512 at 38x38, eight images), where loads from shared memory and FMAs take the SM equally long.
+// 14.9 -> 2.9 ms a forward; YOLOv3-tiny-416, one image 3.0 -> 0.43 ms. Layers that fill the chip run at 41 TFLOP/s (3x3
+// 512->512 at 38x38, eight images), where loads from shared memory and FMAs take the SM equally long; the k-step by CTAs an SM is in
+// the table at configure_conv_fp32.
 // ---------------------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, uint32_t bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");

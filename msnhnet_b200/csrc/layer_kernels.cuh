@@ -380,10 +380,7 @@ __global__ void maxpool_kernel(TView in, TView out, int kh, int kw, int sh, int 
     }
 }
 
-// Stride-1 max pool that keeps the plane size (the SPP pools: 5x5 / 9x9 / 13x13 over a 19x19 plane):
-// a block stages the whole plane of G 16-byte channel groups of one image in shared memory and takes
-// the window max as a row pass followed by a column pass (kh + kw reads per output instead of kh * kw).
-// Shared memory: 2 * H * W * G * 16 bytes.
+// maximum of two 16-byte vectors of elements
 template <typename T>
 __device__ __forceinline__ uint4 vec_max16(uint4 a, uint4 b) {
     uint4 r;
@@ -400,8 +397,6 @@ __device__ __forceinline__ uint4 vec_max16(uint4 a, uint4 b) {
     }
     return r;
 }
-// Up to three such pools over the same input (the SPP block: one tensor through a 5, a 9 and a 13 window) run as one
-// launch: the plane is staged once and every pool takes its own row pass and column pass over it.
 // 2 x 2 pools, vector channels: CTAs walk output rows with a power-of-two grid of (channel
 // vector, pixel) threads, so that no division is left per value, the window's loads are independent of one another, and the
 // maximum is taken on the stored type. 64 channels at 320 x 320, 16 images, fp16: 78 -> 54 us for 262 MB (3 x 3 windows gain
@@ -440,6 +435,12 @@ __global__ void maxpool2_rows_kernel(TView in, TView out, int sh, int sw, int ph
     }
 }
 
+// Stride-1 max pool that keeps the plane size (the SPP pools: 5x5 / 9x9 / 13x13 over a 19x19 plane):
+// a block stages the whole plane of G 16-byte channel groups of one image in shared memory and takes
+// the window max as a row pass followed by a column pass (kh + kw reads per output instead of kh * kw).
+// Shared memory: 2 * H * W * G * 16 bytes.
+// Up to three such pools over the same input (the SPP block: one tensor through a 5, a 9 and a 13 window) run as one
+// launch: the plane is staged once and every pool takes its own row pass and column pass over it.
 template <typename T>
 __global__ void maxpool_plane_kernel(TView in, const __grid_constant__ PoolSet ps, int G) {
     pdl_prologue();
@@ -486,10 +487,10 @@ __global__ void maxpool_plane_kernel(TView in, const __grid_constant__ PoolSet p
 }
 
 // ---- local / global average pool: mean over the valid taps ----
+// (localAvgPoolNormalKernel, src/layers/cuda/MsnhLocalAvgPoolLayerGPU.cu:5-79)
 // Latency bounds it: a classifier's global pool is some hundred vectors of outputs with a chain of 49 loads each. Eight loads are
 // in flight at a time and small pools run as one-warp blocks, so that the vectors spread over the SMs: a call of
 // MobileNetV2 with one image (1280 channels of 7x7) 290 -> 285 us, of ResNet-18 fp32 243 -> 239.
-// (localAvgPoolNormalKernel, src/layers/cuda/MsnhLocalAvgPoolLayerGPU.cu:5-79)
 template <typename T, int V>
 __global__ void avgpool_kernel(TView in, TView out, int kh, int kw, int sh, int sw, int ph, int pw) {
     pdl_prologue();

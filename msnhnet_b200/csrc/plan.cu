@@ -88,7 +88,13 @@ bool is_pageable(const void *p) {
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return true; }
     return a.type == cudaMemoryTypeUnregistered;
 }
-constexpr size_t kPoolBytes = 512 * 1024;   // below this waking the pool costs more than the driver's own single-threaded staging
+// Copies of pageable memory from here on are the pool's. A synchronous call with an image of so many KB, its copy through the
+// driver's own single-threaded staging / through the pool, in us:
+//     KB                                        300      432      588      768      972     2028     3072     17328
+//     image in the caller's cache            53 / 60  57 / 67  67 / 79  82 / 90  99 / 98  149 / 155  217 / 169  1275 / 485
+//     image elsewhere in memory              67 / 57  78 / 64  95 / 72  120 / 78 142 / 87 243 / 129  340 / 165  1630 / 493
+// The line lies between the two: what the pool loses to waking up in the one it more than wins in the other.
+constexpr size_t kPoolBytes = 512 * 1024;
 // What a thread copies and PCIe carries at a time: 5 us of PCIe, less where that would leave threads of the pool without a chunk
 // (an image of 602 KB: a call of ResNet-18 343 -> 336 us, of MobileNetV2 296 -> 290)
 constexpr size_t kCopyChunk = 256 * 1024, kMinChunk = 64 * 1024;

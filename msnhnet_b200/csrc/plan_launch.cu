@@ -34,10 +34,16 @@ template <typename T> const void *umma_kernel(const Launch &L) {
     const bool trace = u.trace != nullptr;
     int act = kActGeneric;
     if (!trace) {
-        // The cheap activations are worth a kernel of their own where a CTA has several tiles (with them YOLOv5m-640, 32
-        // images: 3.40 -> 3.34 ms a forward; MobileNetV2-224, 64 images: 0.641 -> 0.625). In a chain of single-wave
-        // launches, a different kernel in every other layer costs more than the switch, because its instructions are
-        // cold (MobileNetV2, one image: 0.211 -> 0.232 ms).
+        // The cheap activations have a kernel of their own where a CTA has several tiles. A forward in us with them never / there /
+        // always compiled in, by the number of images:
+        //                      1                4                 8                  16                 32                 64
+        //   MobileNetV2-224    207 / 209 / 228  227 / 227 / 241   252 / 251 / 265    318 / 320 / 323    417 / 417 / 419    636 / 617 / 620
+        //   YOLOv5m-640        572 / 570 / 553  792 / 784 / 750   1133 / 1103 / 1068 1798 / 1737 / 1726 3266 / 3181 / 3154
+        //   FCN-S-320          262 / 262 / 260  450 / 447 / 445                      1360 / 1352 / 1339
+        //   ResNet-18 fp32     160 / 160 / 160                    275 / 274 / 273                       643 / 642 / 641
+        // MobileNetV2's convs come with relu6 and without an activation in turn, so "always" makes neighbouring launches different
+        // kernels; YOLOv5m's are hard-swish nearly throughout and would gain another 1 to 4 % from it. Why the change of kernels
+        // costs some 0.5 us a launch has not been looked into.
         const bool long_run = u.tiles_m * u.tiles_n > L.grid;
         if (long_run && (u.act1 == MSNH_ACT_NONE || u.act1 == MSNH_ACT_RELU)) act = u.act1;
         else if (long_run && sizeof(T) == 2 && (u.act1 == MSNH_ACT_HARD_SWISH || u.act1 == MSNH_ACT_RELU6)) act = u.act1;

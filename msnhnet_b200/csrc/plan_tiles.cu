@@ -120,9 +120,16 @@ void configure_dw_tile(MsnhB200Plan *pl, Launch &L) {
 void configure_conv_fp32(MsnhB200Plan *pl, Launch &L) {
     const int m_image = L.out.H * L.out.W, m_total = L.out.N * m_image, steps = (L.kh * L.kw * (L.cin_pad / 4) + 3) / 4;
     auto tiles_of = [&](int m) { return static_cast<long>((m + kFpBM - 1) / kFpBM) * ((L.out.C + kFpBN - 1) / kFpBN); };
-    // Measured: a k-step of 1 / 2 / 3 / 4 CTAs that share an SM takes 0.65 / 1.15 / 1.5 / 1.86 us for all of them (a CTA alone
-    // cannot hide its own latencies), and clusters of three and more do not spread over all SMs: the second CTA of some SM
-    // arrives at about 128.
+    // A k-step (16 products a value) of all the CTAs that share an SM, measured as the slope between 144 and 288 steps of a 3x3 layer:
+    //     CTAs of the busiest SM    1     2     3     4     5     6     8
+    //     us                      0.58  1.04  1.44  1.80  2.10  2.73  3.55   (8: 42 TFLOP/s; from five on the CTAs come in rounds of four)
+    // A CTA alone cannot hide its own latencies. Clusters of three and more do not spread over all SMs; the most CTAs that still
+    // get an SM each:
+    //     cluster                   2    3    4    5    6    7    8
+    //     CTAs                    148  132  132  130  132  98+  120           (7: 98 do, 119 do not)
+    // The model takes 0.25 + 0.4 n and 0.46 n for the first table and 130 for the second (clusters of seven and eight fill up a
+    // little earlier than it thinks). Measured launches of clusters are no longer than the slope says; the last term is a margin,
+    // a microsecond or three, below which a split is not worth its CTAs.
     auto cost_of = [&](long tiles, int split) {
         const double spread = split <= 2 ? pl->ctx->sm_count : pl->ctx->sm_count * 0.88;
         const double per_sm = std::ceil(tiles * split / spread);          // CTAs of the busiest SM
