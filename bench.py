@@ -44,6 +44,7 @@ WORKLOADS = {
     "fcns-320": ("fcns", 320, 16, "fp16", 64.54),
 }
 HEADLINE = "yolov4-608"
+REF_DRIVER = os.path.join(ROOT, "oracle", "_ref", "ref_driver")     # the reference's CPU path compiled from its own sources
 FP32_FMA_TFLOPS = 72.0       # scalar fp32 FMAs from registers, measured (128 lanes x 148 SMs at 1.965 GHz give 74.4)
 # the benchmark configs besides the headline, measured briefly by the default run
 OTHERS = ["yolov5m-640", "yolov3-tiny-416", "mobilenetv2-224", "resnet18-224"]
@@ -204,7 +205,7 @@ def reference_cpu(net, size, warmup, iters, budget_s=60.0):
     text = topologies.NETS[net](size=size)
     blob = synth.make_blob(text, synth.load_factors(net))
     img = synth.make_images(1, 3, size, size)[0]
-    drv = os.path.join(ROOT, "oracle", "_ref", "ref_driver")
+    drv = REF_DRIVER
     affinity, quota, physical = host_cpu_counts()
     if os.path.exists(drv):
         with tempfile.TemporaryDirectory() as d:
@@ -252,9 +253,15 @@ def run_reference(args, net, size, config):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
+    if not os.path.exists(REF_DRIVER):
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's own binary is not built here (oracle/Makefile compiles it from the reference's sources, which this machine does not have)"}), flush=True)
+        return
     # each step is a bounded sample: `sample` images, one at a time, through the reference CPU path
     sample = {"yolov4": 2, "yolov5m": 3}.get(net, 8)
     ips, kind, threads, desc, details = reference_cpu(net, size, max(1, min(args.warmup, 2)), max(1, args.steps) * sample, budget_s=120.0)
+    if kind != "reference":
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's own binary did not run here"}), flush=True)
+        return
     config = dict(config, reference_arm=f"batch 1 looped, {sample} images per step (the reference's block layers are batch-1 only)")
     line = {"impl": "reference", "metric": "images/sec", "value": ips, "unit": "images/s", "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": 1000.0 * sample / ips, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
