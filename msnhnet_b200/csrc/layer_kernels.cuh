@@ -30,6 +30,9 @@ template <typename T, int V> struct VecIO {
         st(p, v);
     }
 };
+template <typename T> __device__ __forceinline__ void st_out(const TView &out, T *p, float v) {
+    Elem<T>::st(p, sizeof(T) == 4 && out.tf32 ? round_tf32(v) : v);
+}
 
 __device__ __forceinline__ size_t pix_off(const TView &t, int n, int h, int w) {
     return (static_cast<size_t>(n) * t.H + h) * t.W * static_cast<size_t>(t.ldc) + static_cast<size_t>(w) * t.ldc;
@@ -376,10 +379,20 @@ __global__ void maxpool_kernel(TView in, TView out, int kh, int kw, int sh, int 
 #pragma unroll
                 for (int e = 0; e < V; ++e) m[e] = fmaxf(m[e], v[e]);
             }
-        VecIO<T, V>::st(static_cast<T *>(out.ptr) + pix_off(out, n, oh, ow) + c, m);
+        VecIO<T, V>::st_out(out, static_cast<T *>(out.ptr) + pix_off(out, n, oh, ow) + c, m);
     }
 }
 
+// 16 bytes of elements rounded to tf32 when the view asks for it
+template <typename T> __device__ __forceinline__ uint4 round_out16(const TView &out, uint4 v) {
+    if constexpr (sizeof(T) == 4) {
+        if (out.tf32) {
+            v.x = __float_as_uint(round_tf32(__uint_as_float(v.x))); v.y = __float_as_uint(round_tf32(__uint_as_float(v.y)));
+            v.z = __float_as_uint(round_tf32(__uint_as_float(v.z))); v.w = __float_as_uint(round_tf32(__uint_as_float(v.w)));
+        }
+    }
+    return v;
+}
 // maximum of two 16-byte vectors of elements
 template <typename T>
 __device__ __forceinline__ uint4 vec_max16(uint4 a, uint4 b) {
@@ -429,7 +442,7 @@ __global__ void maxpool2_rows_kernel(TView in, TView out, int sh, int sw, int ph
                 uint4 m = lowest;
 #pragma unroll
                 for (int k = 0; k < K * K; ++k) m = vec_max16<T>(m, v[k]);
-                *reinterpret_cast<uint4 *>(dst + static_cast<size_t>(ow) * out.ldc + c * V) = m;
+                *reinterpret_cast<uint4 *>(dst + static_cast<size_t>(ow) * out.ldc + c * V) = round_out16<T>(out, m);
             }
         }
     }
@@ -479,7 +492,7 @@ __global__ void maxpool_plane_kernel(TView in, const __grid_constant__ PoolSet p
                 const int hb = max(h - ph, 0), he = min(h - ph + kh, in.H);
                 uint4 m = rowmax[(hb * in.W + w) * G + g];
                 for (int y = hb + 1; y < he; ++y) m = vec_max16<T>(m, rowmax[(y * in.W + w) * G + g]);
-                *reinterpret_cast<uint4 *>(obase + static_cast<size_t>(pix) * out.ldc + g * V) = m;
+                *reinterpret_cast<uint4 *>(obase + static_cast<size_t>(pix) * out.ldc + g * V) = round_out16<T>(out, m);
             }
             __syncthreads();
         }
@@ -554,7 +567,7 @@ __global__ void upsample_kernel(TView in, TView out, int sh, int sw, float scale
 #pragma unroll
             for (int e = 0; e < V; ++e) v[e] *= scale;
         }
-        VecIO<T, V>::st(static_cast<T *>(out.ptr) + pix_off(out, n, oh, ow) + c, v);
+        VecIO<T, V>::st_out(out, static_cast<T *>(out.ptr) + pix_off(out, n, oh, ow) + c, v);
     }
 }
 
@@ -571,7 +584,9 @@ __global__ void slice_kernel(TView in, TView out, int o0, int s0, int o1, int s1
         const int n  = pix / out.H;
         const T *src = static_cast<const T *>(in.ptr) + pix_off(in, n, oh * s1 + o1, ow * s2 + o2) + o0;
         T *dst = static_cast<T *>(out.ptr) + pix_off(out, n, oh, ow);
-        for (int c = 0; c < out.C; ++c) dst[c] = src[c * s0];
+        for (int c = 0; c < out.C; ++c) {
+            if constexpr (sizeof(T) == 4) dst[c] = out.tf32 ? round_tf32(src[c * s0]) : src[c * s0]; else dst[c] = src[c * s0];
+        }
     }
 }
 
@@ -671,7 +686,7 @@ __global__ void pad_kernel(TView in, TView out, int top, int left, float val) {
 #pragma unroll
             for (int e = 0; e < V; ++e) v[e] = val;
         }
-        VecIO<T, V>::st(static_cast<T *>(out.ptr) + pix_off(out, n, oh, ow) + c, v);
+        VecIO<T, V>::st_out(out, static_cast<T *>(out.ptr) + pix_off(out, n, oh, ow) + c, v);
     }
 }
 
@@ -706,7 +721,7 @@ __global__ void softmax_kernel(TView in, TView out, int groups, float temperatur
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         for (size_t j = lane; j < len; j += 32) {
             const float e = expf(Elem<T>::ld(static_cast<const T *>(in.ptr) + addr(in, j)) / temperature - mx / temperature);
-            Elem<T>::st(static_cast<T *>(out.ptr) + addr(out, j), e / sum);
+            st_out(out, static_cast<T *>(out.ptr) + addr(out, j), e / sum);
         }
     }
 }
@@ -1252,7 +1267,7 @@ __global__ void maxpool_depth_kernel(TView in, TView out) {
         const T *src = static_cast<const T *>(in.ptr) + pix * in.ldc;
         float m = -FLT_MAX;
         for (int k = g; k < in.C; k += out.C) m = fmaxf(m, Elem<T>::ld(src + k));
-        Elem<T>::st(static_cast<T *>(out.ptr) + pix * out.ldc + g, m);
+        st_out(out, static_cast<T *>(out.ptr) + pix * out.ldc + g, m);
     }
 }
 
@@ -1270,7 +1285,7 @@ __global__ void clip_kernel(TView in, TView out, float lo, float hi) {
         VecIO<T, V>::ld(static_cast<const T *>(in.ptr) + static_cast<size_t>(pix) * in.ldc + c, v);
 #pragma unroll
         for (int e = 0; e < V; ++e) v[e] = fminf(fmaxf(v[e], lo), hi);
-        VecIO<T, V>::st(static_cast<T *>(out.ptr) + static_cast<size_t>(pix) * out.ldc + c, v);
+        VecIO<T, V>::st_out(out, static_cast<T *>(out.ptr) + static_cast<size_t>(pix) * out.ldc + c, v);
     }
 }
 
@@ -1306,6 +1321,7 @@ __global__ void remap_kernel(TView in, TView out, int kind, int d0, int d1, int 
             ih = r / in.W; iw = r - ih * in.W;
         }
         T v = static_cast<const T *>(in.ptr)[pix_off(in, n, ih, iw) + ic];
+        if constexpr (sizeof(T) == 4) { if (out.tf32) v = round_tf32(v); }
         static_cast<T *>(out.ptr)[pix_off(out, n, oh, ow) + oc] = v;
     }
 }
@@ -1342,7 +1358,7 @@ __global__ void reduce_kernel(TView in, TView out, int axis, int mean) {
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
         if (mean) s = s / static_cast<float>(len);
-        if (lane == 0) Elem<T>::st(static_cast<T *>(out.ptr) + pix_off(out, n, oh, ow) + oc, s);
+        if (lane == 0) st_out(out, static_cast<T *>(out.ptr) + pix_off(out, n, oh, ow) + oc, s);
     }
 }
 

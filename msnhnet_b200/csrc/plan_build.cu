@@ -879,26 +879,21 @@ int build_launches(MsnhB200Plan *pl) {
         pl->launches.push_back(L);
     }
     { const int rc = tile_tuning_end(pl, tt); if (rc) return rc; }
-    // fp32 plans: every launch that writes a tensor some tensor-core conv reads rounds to tf32
+    // fp32 plans: every launch that writes into a buffer some tensor-core conv reads rounds to tf32. (By the buffer and not by its
+    // place in the arena, where dead and living buffers of other sizes overlap, other ones at another batch size.)
     if (pl->dtype == MSNH_B200_F32) {
-        std::vector<std::pair<const uint8_t *, const uint8_t *>> reads;   // [begin, end) of root buffers read by UMMA convs
-        for (size_t k = 0; k < pend.size(); ++k) {
-            if (pl->launches[k].kind != L_CONV_UMMA) continue;
-            const Buffer &b = pl->buffers[root_of(pl, pl->tensors[pend[k].in_t].buffer, nullptr)];
-            reads.push_back({pl->arena + b.offset, pl->arena + b.offset + b.bytes});
-        }
+        std::vector<bool> read(pl->buffers.size(), false);
+        auto root = [&](int t) { return static_cast<size_t>(root_of(pl, pl->tensors[t].buffer, nullptr)); };
+        for (size_t k = 0; k < pend.size(); ++k)
+            if (pl->launches[k].kind == L_CONV_UMMA) read[root(pend[k].in_t)] = true;
         for (size_t k = 0; k < pend.size(); ++k) {
             Launch &L = pl->launches[k];
             if (pend[k].out_t < 0) continue;
-            bool hit = false;
-            for (int t : {pend[k].out_t, pend[k].out2_t}) {
-                if (t < 0) continue;
-                const Buffer &b = pl->buffers[root_of(pl, pl->tensors[t].buffer, nullptr)];
-                const uint8_t *lo = pl->arena + b.offset;
-                for (auto &r : reads) if (lo >= r.first && lo < r.second) hit = true;
+            if (read[root(pend[k].out_t)] || (pend[k].out2_t >= 0 && read[root(pend[k].out2_t)])) { L.out.tf32 = 1; if (L.kind == L_CONV_UMMA) L.up.round_tf32 = 1; }
+            if (L.kind == L_MAXPOOL) {
+                L.pools.out[0].tf32 = L.out.tf32;
+                for (size_t q = 0; q < pend[k].more_out_t.size(); ++q) L.pools.out[q + 1].tf32 = read[root(pend[k].more_out_t[q])];
             }
-            // buffers are reused over time, so this may round a little more than needed, never less
-            if (hit) { L.out.tf32 = 1; if (L.kind == L_CONV_UMMA) L.up.round_tf32 = 1; }
         }
     }
     // candidate counters: one int per image per collect op

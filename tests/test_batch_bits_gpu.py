@@ -132,3 +132,68 @@ def test_shares_of_many_tiles(shares, cout, monkeypatch):
         assert H.rel_err(got, conv_plan(ctx, x, wt, 1, 0)[0]) < 2.0**-10   # (the result is rounded to tf32: 2^-11 apart where the sums' last bits differ)
     finally:
         ctx.close()
+
+
+def test_an_output_is_not_rounded_for_a_conv_that_reads_another_tensor():
+    """Outputs are stored as they are, tensors that a tensor-core conv reads rounded to tf32, whatever memory the two share over time:
+    with one image the last tensor of this chain lies behind every conv's input, with 64 where one of them was."""
+    ch = (252, 248, 4, 492, 300)
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((64, ch[0], 1, 1), dtype=np.float32)
+    weights = [(rng.standard_normal((ch[i + 1], ch[i], 1, 1)) / np.sqrt(ch[i])).astype(np.float32) for i in range(4)]
+    ctx = ffi.Context(0)
+    try:
+        out = {}
+        for batch in (1, 64):
+            plan = ffi.Plan(ctx, [ffi.make_op(ffi.OP_CONV, [ffi.INPUT if i == 0 else i - 1], filters=ch[i + 1], is_output=int(i == 3)) for i in range(4)], (ch[0], 1, 1), batch, ffi.F32)
+            for i, w in enumerate(weights):
+                plan.set_weights(i, ffi.W_WEIGHTS, w)
+            plan.finalize()
+            plan.run(x[:batch])
+            out[batch] = plan.read_output(3, batch)
+            plan.close()
+        assert np.array_equal(out[1][0], out[64][0])
+        assert (out[64].view(np.uint32) & 0x1FFF).any()                   # (more than tf32's ten bits of mantissa)
+    finally:
+        ctx.close()
+
+
+def to_tf32(a):
+    """Nearest tf32, ties away from zero (cvt.rna)."""
+    u = np.ascontiguousarray(a, np.float32).view(np.uint32)
+    return ((u + np.uint32(0x1000)) & np.uint32(0xFFFFE000)).view(np.float32)
+
+
+COPIES = {"pool 2x2": (dict(kind=ffi.OP_MAXPOOL, k_h=2, k_w=2, stride_h=2, stride_w=2), 8, lambda x: x.reshape(x.shape[0], 8, 6, 2, 6, 2).max((3, 5))),
+          "pool 3x3": (dict(kind=ffi.OP_MAXPOOL, k_h=3, k_w=3, stride_h=3, stride_w=3), 8, lambda x: x.reshape(x.shape[0], 8, 4, 3, 4, 3).max((3, 5))),
+          "pool 5x5": (dict(kind=ffi.OP_MAXPOOL, k_h=5, k_w=5, pad_h=2, pad_w=2), 8, None),
+          "upsample": (dict(kind=ffi.OP_UPSAMPLE, stride_h=2, stride_w=2), 8, lambda x: x.repeat(2, 2).repeat(2, 3)),
+          "clip": (dict(kind=ffi.OP_CLIP, const_val=-0.7371, scale=0.9173), 8, lambda x: np.clip(x, np.float32(-0.7371), np.float32(0.9173))),
+          "slice": (dict(kind=ffi.OP_SLICE, slice_start=(0, 1, 0), slice_step=(1, 2, 2)), 8, lambda x: x[:, :, 1::2, ::2])}
+
+
+@pytest.mark.parametrize("name", sorted(COPIES))
+def test_what_a_conv_reads_is_rounded_to_nearest_behind_layers_that_move_values(name):
+    """The image goes through a layer that stores values as it finds them into a 1x1 conv with unit weights, whose products and sums
+    are exact: out comes the layer's result, each value the tf32 nearest to it (the tensor cores by themselves would cut bits off)."""
+    kw, c, want = COPIES[name]
+    kw = dict(kw)
+    rng = np.random.default_rng(6)
+    x = rng.standard_normal((3, c, 12, 12), dtype=np.float32)
+    ctx = ffi.Context(0)
+    plan = ffi.Plan(ctx, [ffi.make_op(kw.pop("kind"), [ffi.INPUT], **kw), ffi.make_op(ffi.OP_CONV, [0], filters=c, is_output=1)], (c, 12, 12), 3, ffi.F32)
+    try:
+        plan.set_weights(1, ffi.W_WEIGHTS, np.eye(c, dtype=np.float32)[:, :, None, None])
+        plan.finalize()
+        assert "conv_umma" in plan.describe()
+        plan.run(x)
+        got = plan.read_output(1, 3)
+    finally:
+        plan.close()
+        ctx.close()
+    if want is None:
+        pad = np.pad(x, ((0, 0), (0, 0), (2, 2), (2, 2)), constant_values=-np.inf)
+        ref = np.max([pad[:, :, r:r + 12, s:s + 12] for r in range(5) for s in range(5)], axis=0)
+    else:
+        ref = want(x)
+    assert np.array_equal(got, to_tf32(ref))
