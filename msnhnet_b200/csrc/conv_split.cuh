@@ -1,0 +1,473 @@
+// fp32 convolution on the tensor cores: every fp32 operand is split into two tf32 numbers whose sum it is to 2^-24, and a
+// product into three tensor-core products. What the fp32 plans of detection nets run (boxes decoded through exp() do not hold
+// through tf32's 10 mantissa bits); the CUDA-core form of the same arithmetic is conv_fp32_kernel (conv_tiled.cuh). Replaces the
+// reference's im2col + cublasSgemm (src/layers/MsnhConvolutionalLayer.cpp:1026-1160).
+#pragma once
+#include "conv_umma.cuh"
+
+namespace msnh {
+
+// ---------------------------------------------------------------------------------------------------------------------------
+// x = x0 + x1, w = w0 + w1, each part the nearest tf32 of what is left. x w = x0 w0 + (x0 w1 + x1 w0) + x1 w1, the last term below
+// 2^-24 and left out where k is long enough for it to drown in the rounding of the sums. Weights are split on the host, activations here.
+//
+// The sums. The tensor core adds into its fp32 accumulator without rounding to nearest, an error of up to an ulp of the sum for
+// every eight products and always towards zero, which over a few hundred k-steps is worse than a chain of fp32 FMAs. So x0 w0
+// is accumulated over one k-block at a time (32 values of k, four tensor-core steps) and the k-blocks are added up in registers
+// with ordinary rounded additions; the two small products, 2^-11 of the large one, stay in an accumulator of their own
+// over the whole share of k.
+// (inf and NaN: x1 of an infinite x is NaN, so where the large sum is not finite it is the result and the small one is dropped.)
+//
+// Roles of the 28 warps, connected by rings of mbarriers. A wait costs a single thread some 170 cycles even where it passes, so the
+// MMA threads have one a k-block: ready(k-block) counts the four splitting warps, the weights' bytes and the sixteen adding warps
+// that have emptied the accumulator; the one commit, done(k-block), frees the slot and the weights and says that the sums are there.
+//   0      loads activations, fp32 as they are: 128 pixels x 32 values of k (one filter tap), im2col or 2-D TMA, 128-byte swizzle
+//   1      loads the weights' two parts: 2 x kBn channels x 32 values of k, one 3-D TMA
+//   4-11   split: shared memory -> registers -> TMEM, a pixel (TMEM lane) per thread, 32 columns of x0 and 32 of x1; two groups
+//          of four warps take k-blocks in turn. With both parts in TMEM the tensor core reads only the weights from shared memory and an
+//          MMA of N channels takes N / 2 cycles (17 at 32, 33 at 64); with A in shared memory it takes 41 and 49, bound by
+//          reading A.
+//   2, 3   issue the MMAs of k-blocks in turn (beside its 400 cycles of MMAs a k-block costs its thread some 300 of its own, which the
+//          other one's MMAs cover; each has an accumulator of small products): 12 of N = kBn for a k-block (four steps x three products), fewer where a tap's last channels end
+//   12-27  add up: the k-block's sums, TMEM -> registers, kBn / 4 channels of a pixel per thread; at the end of a share of k
+//          to shared memory; then scale / bias, activation, residual and the store, in rows of 16-byte vectors
+// TMEM: columns 0-319 a ring of accumulators of x0 w0 and those of the small products, then three slots of x0 | x1 (320 + 64 s).
+//
+// The k of a tile is summed in p.shares shares that are added in their order. How many comes from the layer and one image
+// (configure_conv_split), so an image has the same bits in a plan of any batch size. kSplit: a cluster of that many CTAs sums one
+// each, one tile per cluster, and every CTA finishes every shares-th row through distributed shared memory. Else a CTA walks tiles
+// and sums a tile's shares one after the other.
+//
+// Measured against fp32 FMAs on the CUDA cores (conv_fp32_kernel), a forward in us: YOLOv3-tiny-416, one image 431 -> 207 and sixteen
+// 3965 -> 1490; YOLOv5m-352, three images 2889 -> 1407; YOLOv5m-640, two 4604 -> 1925. Norm error against 64 bits, FMAs / here: 64 values
+// of k 1.44e-7 / 1.28e-7, 288 1.54e-7 / 1.46e-7, 2304 3.8e-7 / 2.0e-7, 4608 4.3e-7 / 2.5e-7 (one share; less in several). A k-block takes 550-650 cycles: its 12
+// MMAs 300 (48 channels) to 400 (64), the rest is the way of a slot round the roles (split, MMA, commit, sums read, some 1800 cycles
+// for three k-blocks). With one MMA thread it took 780, with eight adding warps the end of a tile 2600 cycles (now half), with
+// cvt.rna.tf32 in place of integer rounding (a quarter of the rate) 1000.
+// ---------------------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+// D (TMEM) += A (TMEM) x B (shared memory), tf32
+__device__ __forceinline__ void tcgen05_mma_ts_tf32(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t *r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 "
+        "[%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+        ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t *r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_32x32b_x4(uint32_t taddr, uint32_t *r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+template <int N>                       // N columns (a multiple of four) without waiting for them
+__device__ __forceinline__ void tmem_ld_columns(uint32_t taddr, uint32_t (&r)[N]) {
+#pragma unroll
+    for (int c = 0; c + 8 <= N; c += 8) tmem_ld_32x32b_x8(taddr + static_cast<uint32_t>(c), r + c);
+    if constexpr (N % 8 != 0) tmem_ld_32x32b_x4(taddr + static_cast<uint32_t>(N - 4), r + N - 4);
+}
+
+// The end of a tile: scale / bias, activation, residual (+ second activation), store. Of kThreads threads each has four channels of
+// every kRows-th row; rows row0, row0 + step, ... are these threads'. A thread's scale and bias are loaded long before its
+// sums are there, its rows kBatch at a time: row by row, with the tables read for each, the end of a tile of 128 x 64 took 9000
+// cycles, most of them latency. `sum` gives the sums at a byte offset into the tile.
+template <int kBn, int kThreads, int kBatch>
+struct SplitFinish {
+    static constexpr int kQuads = kBn / 4, kRows = kThreads / kQuads;
+    int row, col, c;
+    float4 sc, bi;
+    bool live;
+    __device__ __forceinline__ SplitFinish(const ConvSplitParams &p, int n0, int t) : row(t / kQuads), col(4 * (t % kQuads)), c(n0 + col), live(t < kRows * kQuads && c < p.cout) {
+        if (live) { sc = __ldg(reinterpret_cast<const float4 *>(p.scale + c)); bi = __ldg(reinterpret_cast<const float4 *>(p.bias + c)); }   // (padded past the last channel tile)
+    }
+    template <typename Sum>
+    __device__ __forceinline__ void operator()(const ConvSplitParams &p, const TView &out, int m0, int row0, int step, Sum &&sum) const {
+        if (!live) return;
+        const int rows = min(kUmmaM, p.m_total - m0);
+        const bool whole = c + 4 <= p.cout;
+        for (int j = row0 + row * step; j < rows; j += kBatch * kRows * step) {
+            float y[4 * kBatch], rr[4 * kBatch];
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) {
+                const int r = min(j + q * kRows * step, rows - 1);                    // (rows past the last are computed and not stored)
+                sum(4u * static_cast<uint32_t>(r * (kBn + 4) + col), y + 4 * q);
+                if (p.res) {
+                    const float *rp = static_cast<const float *>(p.res) + static_cast<size_t>(m0 + r) * p.ldc_res + c;
+                    if (whole) {
+                        const float4 t = *reinterpret_cast<const float4 *>(rp);
+                        rr[4 * q] = t.x; rr[4 * q + 1] = t.y; rr[4 * q + 2] = t.z; rr[4 * q + 3] = t.w;
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) rr[4 * q + e] = c + e < p.cout ? rp[e] : 0.f;
+                    }
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4 * kBatch; q += 4) { y[q] = fmaf(y[q], sc.x, bi.x); y[q + 1] = fmaf(y[q + 1], sc.y, bi.y); y[q + 2] = fmaf(y[q + 2], sc.z, bi.z); y[q + 3] = fmaf(y[q + 3], sc.w, bi.w); }
+            activate_all(y, p.act1, p.act1_param);
+            if (p.res) {
+#pragma unroll
+                for (int q = 0; q < 4 * kBatch; ++q) y[q] = __fadd_rn(y[q], rr[q]);
+                activate_all(y, p.act2, p.act2_param);
+            }
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q) {
+                const int r = j + q * kRows * step;
+                if (r >= rows) break;
+                float *dst = static_cast<float *>(out.ptr) + static_cast<size_t>(m0 + r) * out.ldc + c;
+                if (whole) *reinterpret_cast<float4 *>(dst) = make_float4(y[4 * q], y[4 * q + 1], y[4 * q + 2], y[4 * q + 3]);
+                else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) if (c + e < p.cout) dst[e] = y[4 * q + e];
+                }
+            }
+        }
+    }
+    static __device__ __forceinline__ void activate_all(float (&v)[4 * kBatch], int act, float param) {      // (one branch for all of them)
+        if (act == MSNH_ACT_NONE) return;
+        if (act == MSNH_ACT_LEAKY) {
+#pragma unroll
+            for (int e = 0; e < 4 * kBatch; ++e) v[e] = activate(v[e], MSNH_ACT_LEAKY, param);
+        } else if (act == MSNH_ACT_HARD_SWISH) {
+#pragma unroll
+            for (int e = 0; e < 4 * kBatch; ++e) v[e] = activate(v[e], MSNH_ACT_HARD_SWISH, param);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4 * kBatch; ++e) v[e] = activate_slow(v[e], act, param);
+        }
+    }
+};
+
+template <int kBn, bool kSplit>
+__global__ void __launch_bounds__(kSpThreads, 1)
+conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TView out, const ConvSplitParams p) {
+    constexpr int kCols = kBn / 4;                                   // channels of a pixel an adding thread holds
+    constexpr int kPitch = kBn + 4;                                  // floats of a row of the tile of sums
+    constexpr uint32_t kABytes = kUmmaM * 128, kBBytes = 2 * kBn * 128;
+    // TMEM columns 0-319: accumulators of x0 w0 (a ring) and of the small products (one per issuer, twice where there is room)
+    constexpr uint32_t kMain = kBn >= 48 ? 3 : 4, kSmall = kBn >= 48 ? 1 : 2, kSmallCol = kMain * kBn, kSlotCol = 320;
+    static_assert((kMain + 2 * kSmall) * kBn <= kSlotCol && kSlotCol + 64 * kSpSlots <= 512, "TMEM columns");
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t a_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t b_base = a_base + kSpAStages * kABytes;
+    const uint32_t sum_base = b_base + kSpBStages * kBBytes;         // [128][kPitch] floats
+    const uint32_t bar_base = sum_base + kUmmaM * kPitch * 4;
+    auto full_a  = [&](uint32_t s) { return bar_base + 8u * s; };
+    auto empty_a = [&](uint32_t s) { return bar_base + 8u * (8 + s); };
+    auto ready   = [&](uint32_t s) { return bar_base + 8u * (16 + s); };
+    auto done    = [&](uint32_t s) { return bar_base + 8u * (24 + s); };
+    auto s_full  = [&](uint32_t s) { return bar_base + 8u * (32 + s); };
+    auto s_empty = [&](uint32_t s) { return bar_base + 8u * (34 + s); };
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int cta_abort_slot;
+    volatile int *cta_abort = &cta_abort_slot;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int num_tiles = p.tiles_m * p.tiles_n, num_k = p.taps * p.chunks_per_tap;
+    int rank = 0;
+    if constexpr (kSplit) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const int first_tile = kSplit ? static_cast<int>(blockIdx.x) / p.shares : static_cast<int>(blockIdx.x);
+    const int tile_stride = kSplit ? num_tiles : static_cast<int>(gridDim.x);
+    const int share_first = kSplit ? rank : 0, share_end = kSplit ? rank + 1 : p.shares;
+
+    pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+        cta_abort_slot = 0;
+        for (uint32_t s = 0; s < kSpAStages; ++s) { mbar_init(full_a(s), 1); mbar_init(empty_a(s), 4); }
+        for (uint32_t s = 0; s < kSpRing; ++s) { mbar_init(ready(s), 4 + 1 + 16); mbar_init(done(s), 1); }
+        for (uint32_t s = 0; s < 2; ++s) { mbar_init(s_full(s), 2); mbar_init(s_empty(s), 16); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 2) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tcgen05_fence_before();
+    __syncthreads();
+    tcgen05_fence_after();
+    const uint32_t tmem = tmem_base_slot;
+
+    if (warp == 0) {
+        // ------------------------------ activations ------------------------------
+        if (elect_one()) {
+            uint32_t stage = 0, phase = 1;
+            bool ok = true;
+            const bool im2col = p.a_mode == A_MODE_IM2COL;
+            pdl_wait();                     // the activations are the previous kernel's output
+            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_stride) {
+                const int m0 = tile / p.tiles_n * kUmmaM;
+                const int img = m0 / (p.oh * p.ow), rem = m0 - img * p.oh * p.ow, y0 = rem / p.ow, x0 = rem - y0 * p.ow;
+                const int cx = x0 * p.stride_w - p.pad_w, cy = y0 * p.stride_h - p.pad_h;
+                const int k0 = kSplit ? num_k * rank / p.shares : 0, k1 = kSplit ? num_k * (rank + 1) / p.shares : num_k;
+                const int tap = k0 / p.chunks_per_tap, r = tap / p.kw;
+                int chunk = k0 - tap * p.chunks_per_tap, s = tap - r * p.kw, off_h = r * p.dil_h, off_w = s * p.dil_w;
+                for (int kt = k0; kt < k1; ++kt) {
+                    ok = mbar_wait(empty_a(stage), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_EMPTY);
+                    if (!ok) break;
+                    mbar_expect_tx(full_a(stage), kABytes);
+                    if (im2col) tma_load_im2col_4d(a_base + stage * kABytes, &map_a, full_a(stage), p.chunk_elems * chunk, cx, cy, img, static_cast<uint16_t>(off_w), static_cast<uint16_t>(off_h));
+                    else        tma_load_2d(a_base + stage * kABytes, &map_a, full_a(stage), p.chunk_elems * chunk, m0);
+                    if (++stage == kSpAStages) { stage = 0; phase ^= 1u; }
+                    if (++chunk == p.chunks_per_tap) {
+                        chunk = 0; off_w += p.dil_w;
+                        if (++s == p.kw) { s = 0; off_w = 0; off_h += p.dil_h; }
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------ weights (constants: asked for while the previous kernel still runs) ------------------------------
+        if (elect_one()) {
+            uint32_t stage = 0, at = 0, freed = 0, phase = 0, ahead = kSpBStages;     // (the first stages are free)
+            bool ok = true;
+            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_stride) {
+                const int n0 = tile % p.tiles_n * kBn;
+                const int k0 = kSplit ? num_k * rank / p.shares : 0, k1 = kSplit ? num_k * (rank + 1) / p.shares : num_k;
+                const int tap = k0 / p.chunks_per_tap;
+                int chunk = k0 - tap * p.chunks_per_tap, c_tap = tap * p.cin_pad;
+                for (int kt = k0; kt < k1; ++kt) {
+                    if (ahead) --ahead;
+                    else {
+                        ok = mbar_wait(done(freed), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_EMPTY);
+                        if (!ok) break;
+                        if (++freed == kSpRing) { freed = 0; phase ^= 1u; }
+                    }
+                    mbar_expect_tx(ready(at), kBBytes);
+                    tma_load_3d(b_base + stage * kBBytes, &map_b, ready(at), c_tap + p.chunk_elems * chunk, n0, 0);
+                    if (++stage == kSpBStages) stage = 0;
+                    if (++at == kSpRing) at = 0;
+                    if (++chunk == p.chunks_per_tap) { chunk = 0; c_tap += p.cin_pad; }
+                }
+            }
+        }
+    } else if (warp < 4) {
+        // ------------------------------ MMA issuers: k-blocks in turn ------------------------------
+        if (elect_one()) {
+            constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(kBn >> 3) << 17) | (static_cast<uint32_t>(kUmmaM >> 4) << 24);
+            const uint32_t turn = static_cast<uint32_t>(warp - 2);
+            const uint64_t desc_b0 = make_smem_desc(b_base, 128);
+            uint32_t at = 0, phase = 0, stage = 0, slot = 0, acc = 0;          // of the next k-block, whoever issues it
+            uint32_t small = 0, small_phase = 1;
+            bool ok = true;
+            for (int tile = first_tile; tile < num_tiles && ok; tile += tile_stride)
+                for (int share = share_first; share < share_end && ok; ++share) {
+                    const int k0 = num_k * share / p.shares, k1 = num_k * (share + 1) / p.shares;
+                    int chunk = k0 % p.chunks_per_tap;
+                    ok = mbar_wait(s_empty(small), small_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_ACC_EMPTY);
+                    if (!ok) break;
+                    const uint32_t d_small = tmem + kSmallCol + kBn * (2 * small + turn);
+                    uint32_t more = 0;                                          // the share's first MMA begins its small sums
+                    for (int kt = k0; kt < k1; ++kt) {
+                        const bool last = ++chunk == p.chunks_per_tap;
+                        if (last) chunk = 0;
+                        if ((at & 1u) == turn) {
+                            ok = mbar_wait(ready(at), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
+                            if (!ok) break;
+                            tcgen05_fence_after();
+                            const uint64_t w0 = desc_b0 + static_cast<uint64_t>(stage) * (kBBytes >> 4), w1 = w0 + (kBn * 128 >> 4);
+                            const uint32_t x0 = tmem + kSlotCol + 64u * slot, x1 = x0 + 32u, d_main = tmem + kBn * acc;
+                            const uint32_t steps = static_cast<uint32_t>(last ? p.tail_steps : p.chunk_steps);
+                            if (steps == 4) {
+#pragma unroll
+                                for (uint32_t k = 0; k < 4; ++k) {
+                                    tcgen05_mma_ts_tf32(d_small, x0 + 8 * k, w1 + 2 * k, idesc, k ? 1u : more);
+                                    tcgen05_mma_ts_tf32(d_small, x1 + 8 * k, w0 + 2 * k, idesc, 1u);
+                                    tcgen05_mma_ts_tf32(d_main, x0 + 8 * k, w0 + 2 * k, idesc, k ? 1u : 0u);
+                                }
+                            } else {
+                                for (uint32_t k = 0; k < steps; ++k) {
+                                    tcgen05_mma_ts_tf32(d_small, x0 + 8 * k, w1 + 2 * k, idesc, k ? 1u : more);
+                                    tcgen05_mma_ts_tf32(d_small, x1 + 8 * k, w0 + 2 * k, idesc, 1u);
+                                    tcgen05_mma_ts_tf32(d_main, x0 + 8 * k, w0 + 2 * k, idesc, k ? 1u : 0u);
+                                }
+                            }
+                            if (p.all_products) {
+                                for (uint32_t k = 0; k < steps; ++k) tcgen05_mma_ts_tf32(d_small, x1 + 8 * k, w1 + 2 * k, idesc, 1u);
+                            }
+                            more = 1;
+                            tcgen05_commit(done(at));
+                        }
+                        if (++at == kSpRing) { at = 0; phase ^= 1u; }
+                        if (++stage == kSpBStages) stage = 0;
+                        if (++slot == kSpSlots) slot = 0;
+                        if (++acc == kMain) acc = 0;
+                    }
+                    if (!ok) break;
+                    tcgen05_commit(s_full(small));
+                    if (++small == kSmall) { small = 0; small_phase ^= 1u; }
+                }
+        }
+    } else if (warp >= 4 && warp < 12) {
+        // ------------------------------ split: fp32 in shared memory -> two tf32 parts in TMEM ------------------------------
+        const int group = (warp - 4) >> 2;
+        const uint32_t row = static_cast<uint32_t>((warp & 3) * 32 + lane), swz = row & 7u;
+        const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
+        const int k_tile = kSplit ? num_k * (rank + 1) / p.shares - num_k * rank / p.shares : num_k;
+        const int tiles_here = first_tile < num_tiles ? (num_tiles - first_tile + tile_stride - 1) / tile_stride : 0;
+        const long long total = static_cast<long long>(tiles_here) * k_tile;
+        uint32_t stage = static_cast<uint32_t>(group), a_phase = 0, slot = static_cast<uint32_t>(group), at = slot, freed = at + kSpRing - kSpSlots, s_phase = 1;
+        for (long long q = group; q < total; q += 2) {
+            bool ok = mbar_wait(full_a(stage), a_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            const uint32_t src = a_base + stage * kABytes + row * 128u, dst = tmem + lanes + kSlotCol + 64u * slot;
+            uint32_t x[32];
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j)
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[4 * j]), "=r"(x[4 * j + 1]), "=r"(x[4 * j + 2]), "=r"(x[4 * j + 3]) : "r"(src + ((j ^ swz) << 4)) : "memory");
+            if (q >= kSpSlots) {                    // the slot's k-block before this one
+                ok = mbar_wait(done(freed), s_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_EMPTY);
+                if (!__all_sync(0xffffffffu, ok)) break;
+            }
+            tcgen05_fence_after();
+#pragma unroll
+            for (int h = 0; h < 32; h += 16) {
+                uint32_t x1[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    const float v = __uint_as_float(x[h + e]);
+                    x[h + e] = (x[h + e] + 0x1000u) & 0xffffe000u;
+                    x1[e] = __float_as_uint(__fsub_rn(v, __uint_as_float(x[h + e])));
+                }
+                tmem_st_32x32b_x16(dst + static_cast<uint32_t>(h), x + h);
+                tmem_st_32x32b_x16(dst + 32u + static_cast<uint32_t>(h), x1);
+            }
+            tmem_st_wait();
+            tcgen05_fence_before();
+            __syncwarp();
+            // (the stage is given back behind the last use of its values: an arrive overtakes loads that nothing has waited for)
+            if (lane == 0) { mbar_arrive(empty_a(stage)); mbar_arrive(ready(at)); }
+            stage += 2; if (stage >= kSpAStages) { stage -= kSpAStages; a_phase ^= 1u; }
+            slot += 2; if (slot >= kSpSlots) slot -= kSpSlots;
+            at += 2; if (at >= kSpRing) at -= kSpRing;
+            freed += 2; if (freed >= kSpRing) { freed -= kSpRing; s_phase ^= 1u; }
+        }
+    } else if (warp >= 12) {
+        // ------------------------------ sums in registers, epilogue ------------------------------
+        const int t = static_cast<int>(threadIdx.x) - 12 * 32;
+        const int part = (warp - 12) >> 2;
+        const uint32_t row = static_cast<uint32_t>((warp & 3) * 32 + lane);
+        const uint32_t from = tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + static_cast<uint32_t>(part * kCols);
+        const uint32_t mine = sum_base + 4u * (row * kPitch + static_cast<uint32_t>(part * kCols));
+        uint32_t at = 0, phase = 0, from_acc = 0, small = 0, small_phase = 0;
+        bool ok = true;
+        if (lane == 0)
+            for (uint32_t a = 0; a < kMain; ++a) mbar_arrive(ready(a));                 // all accumulators are free
+        auto load = [&](uint32_t at, uint32_t (&v)[kCols]) {
+            tmem_ld_columns(at, v);
+            tmem_ld_wait();
+#pragma unroll
+            for (int c = 0; c < kCols; ++c) asm volatile("" : "+r"(v[c]));      // (no use of them moves up past the wait)
+        };
+        for (int tile = first_tile; tile < num_tiles && ok; tile += tile_stride) {
+            const SplitFinish<kBn, 512, 4> finish(p, tile % p.tiles_n * kBn, t);
+            for (int share = share_first; share < share_end && ok; ++share) {
+                const int k0 = num_k * share / p.shares, k1 = num_k * (share + 1) / p.shares;
+                float acc[kCols];
+#pragma unroll
+                for (int c = 0; c < kCols; ++c) acc[c] = 0.f;
+                for (int kt = k0; kt < k1; ++kt) {
+                    ok = mbar_wait(done(at), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_ACC_FULL);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    tcgen05_fence_after();
+                    uint32_t v[kCols];
+                    load(from + kBn * from_acc, v);
+                    tcgen05_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(ready((at + kMain) % kSpRing));      // the accumulator is the k-block's that comes kMain later
+                    if (++at == kSpRing) { at = 0; phase ^= 1u; }
+                    if (++from_acc == kMain) from_acc = 0;
+#pragma unroll
+                    for (int c = 0; c < kCols; ++c) acc[c] = __fadd_rn(acc[c], __uint_as_float(v[c]));
+                }
+                if (!ok) break;
+                ok = mbar_wait(s_full(small), small_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_ACC_FULL);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tcgen05_fence_after();
+                // the small sums of both issuers (of the only one, where the share is a single k-block)
+                const uint32_t first = (at + kSpRing - 1u) & 1u;                  // issuer of the share's last k-block
+                uint32_t v[kCols], w[kCols];
+#pragma unroll
+                for (int c = 0; c < kCols; ++c) w[c] = 0u;
+                if (k1 - k0 > 1) tmem_ld_columns(from + kSmallCol + kBn * (2 * small + 1u - first), w);
+                load(from + kSmallCol + kBn * (2 * small + first), v);
+#pragma unroll
+                for (int c = 0; c < kCols; ++c) {
+                    asm volatile("" : "+r"(w[c]));
+                    if ((__float_as_uint(acc[c]) & 0x7f800000u) != 0x7f800000u) acc[c] = __fadd_rn(acc[c], __fadd_rn(__uint_as_float(v[c]), __uint_as_float(w[c])));
+                }
+                tcgen05_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_empty(small));
+                if (++small == kSmall) { small = 0; small_phase ^= 1u; }
+#pragma unroll
+                for (int c = 0; c < kCols; c += 4) {
+                    const uint32_t to = mine + 4u * static_cast<uint32_t>(c);
+                    if (!kSplit && share > 0) {      // the shares before this one, in their order
+                        float4 s;
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(s.x), "=f"(s.y), "=f"(s.z), "=f"(s.w) : "r"(to) : "memory");
+                        acc[c] = __fadd_rn(s.x, acc[c]); acc[c + 1] = __fadd_rn(s.y, acc[c + 1]); acc[c + 2] = __fadd_rn(s.z, acc[c + 2]); acc[c + 3] = __fadd_rn(s.w, acc[c + 3]);
+                    }
+                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(acc[c]), "f"(acc[c + 1]), "f"(acc[c + 2]), "f"(acc[c + 3]) : "memory");
+                }
+            }
+            if constexpr (!kSplit) {
+                // the sixteen warps decide together: they meet at the tile of sums
+                uint32_t all_ok;
+                asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, 1, 512, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                             : "=r"(all_ok) : "r"(static_cast<uint32_t>(ok)) : "memory");
+                ok = all_ok != 0;
+                if (!ok) break;
+                if (p.res) pdl_wait();                               // the residual is an earlier kernel's output
+                finish(p, out, tile / p.tiles_n * kUmmaM, 0, 1, [&](uint32_t at, float *y) {
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(y[0]), "=f"(y[1]), "=f"(y[2]), "=f"(y[3]) : "r"(sum_base + at) : "memory");
+                });
+                asm volatile("bar.sync 1, 512;" ::: "memory");        // the tile of sums is free for the next tile
+            }
+        }
+    }
+
+    tcgen05_fence_before();
+    __syncthreads();
+    if constexpr (kSplit) {
+        const SplitFinish<kBn, kSpThreads, 1> finish(p, first_tile % p.tiles_n * kBn, static_cast<int>(threadIdx.x));
+        cluster_sync_all();          // every share of the tile is in some CTA's shared memory
+        if (*cta_abort == 0) {
+            if (p.res) pdl_wait();
+            finish(p, out, first_tile / p.tiles_n * kUmmaM, rank, p.shares, [&](uint32_t at, float *y) {
+#pragma unroll
+                for (int q = 0; q < kUmmaMaxKSplit; ++q)
+                    if (q < p.shares) {
+                        float4 s;
+                        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(s.x), "=f"(s.y), "=f"(s.z), "=f"(s.w) : "r"(map_to_cta(sum_base + at, q)) : "memory");
+                        if (q == 0) { y[0] = s.x; y[1] = s.y; y[2] = s.z; y[3] = s.w; }
+                        else { y[0] = __fadd_rn(y[0], s.x); y[1] = __fadd_rn(y[1], s.y); y[2] = __fadd_rn(y[2], s.z); y[3] = __fadd_rn(y[3], s.w); }
+                    }
+            });
+        }
+        __syncwarp();
+        cluster_sync_all();          // nobody leaves while a peer still reads its shared memory
+    }
+    if (warp == 2) {
+        __syncwarp();
+        tcgen05_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
+}  // namespace msnh

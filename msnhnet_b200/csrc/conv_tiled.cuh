@@ -1,7 +1,7 @@
 // Dense convolutions on the CUDA cores in fp32 arithmetic.
 //
 // conv_fp32_kernel (below) serves the plans that must reproduce the reference's fp32 results (its GPU path is fp32 Sgemm
-// throughout, src/layers/MsnhConvolutionalLayer.cpp:1026-1160): fp32 detection nets, whose exp()-decoded boxes do not survive
+// throughout, src/layers/MsnhConvolutionalLayer.cpp:1026-1160): fp32 detection nets without tensor cores, whose exp()-decoded boxes do not survive
 // tf32's 10-bit mantissa, and fp32 plans built without tensor cores.
 // conv_tiled_kernel: an implicit GEMM with shared-memory tiles for 16-bit plans built without tensor cores (the cross-check of
 // the tensor-core kernel).
@@ -143,7 +143,8 @@ conv_tiled_kernel(TView in, TView out, const T *__restrict__ w, const ConvTiledP
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------
-// conv_fp32_kernel: the fp32 form. Same GEMM view; A and B are streams of 16-byte vectors (k = four input channels of one filter
+// conv_fp32_kernel: the fp32 form, for plans that ask for no tensor cores and for views TMA cannot read (fp32 detection nets run
+// conv_split.cuh). Same GEMM view; A and B are streams of 16-byte vectors (k = four input channels of one filter
 // tap, taps in order), so a k-step of four vectors may straddle taps and a 3-channel stem wastes nothing but its pad channel.
 // What bounds it is the FMA pipe (128 lanes per SM and cycle) and, close behind, the register fill from shared memory; the rest
 // of its design serves the layers that do not fill the chip - a plane of 11 x 11 pixels under 768 channels is six tiles of

@@ -86,6 +86,31 @@ struct ConvUmmaParams {
     long long *trace;     // per-CTA clock64 stamps (kTraceSlots per CTA), written by the kTrace instantiations only
     int trace_tile;       // which of the CTA's tiles (0 = its first) the producer / MMA stamps describe
 };
+
+// ---- fp32 convolution on the tensor cores (conv_split.cuh) -------------------------------------------------------------
+constexpr int kSpThreads = 896;      // warp 0: activations, 1: weights, 2 and 3: MMA, 4-11: split, 12-27: sums and epilogue
+// (an even ring of activations: the two groups of splitting warps take k-blocks in turn, and a stage has to be the same group's every
+// time, or a group could be a whole round of its barrier behind and take an old phase for the one it waits for)
+constexpr uint32_t kSpAStages = 6, kSpBStages = 5;     // rings of activations and weights in shared memory
+constexpr uint32_t kSpSlots = 3, kSpRing = 6;          // split activations in TMEM; barriers of the k-blocks under way
+static_assert(kSpAStages % 2 == 0 && kSpRing % 2 == 0, "a stage belongs to one group of splitting warps");
+struct ConvSplitParams {
+    int m_total, cout, tiles_m, tiles_n;
+    int shares;           // the k of a tile is summed in this many shares, added in their order
+    int a_mode;
+    int taps, kw, chunks_per_tap, cin_pad, dil_h, dil_w;
+    int chunk_elems, chunk_steps;   // channels of a k-block (32, fewer where the whole k is short) and the tensor-core steps they take (8 values of k each)
+    int tail_steps;       // steps of a tap's last k-block
+    int all_products;     // x1 w1 too
+    int oh, ow, stride_h, stride_w, pad_h, pad_w;
+    const void *res; int ldc_res;
+    const float *scale, *bias;
+    int act1; float act1_param; int act2; float act2_param;
+    int *err_flag;
+};
+constexpr size_t split_smem_bytes(int bn) {
+    return 1024 + kSpAStages * kUmmaM * 128 + kSpBStages * 2 * bn * 128 + static_cast<size_t>(kUmmaM) * (bn + 4) * 4 + 512;
+}
 constexpr int kSbMaxChannels = 1024;   // capacity of the staged scale / bias tables
 // Activation handled by a dedicated epilogue instantiation (no switch inside the loops); every other activation takes
 // the generic instantiation, which switches per 16 values.

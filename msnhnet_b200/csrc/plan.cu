@@ -20,7 +20,7 @@ namespace msnh {
 const char *const kLaunchNames[] = {"input_nchw_to_nhwc", "conv_umma", "conv_direct", "dwconv", "scale_bias_act",
                                     "add_n", "binary", "maxpool", "avgpool", "upsample", "slice", "pad", "softmax",
                                     "yolo_decode", "collect_zero", "yolo_collect", "input_nchw_to_patches",
-                                    "yolo_decode_collect", "focus_slices", "bilinear", "deconv_col2im", "clip", "remap", "reduce", "prelu", "maxpool_depth"};
+                                    "yolo_decode_collect", "focus_slices", "bilinear", "deconv_col2im", "clip", "remap", "reduce", "prelu", "maxpool_depth", "conv_direct_tf32x3"};
 
 int fail(MsnhB200Ctx *ctx, int code, const char *fmt, ...) {
     char buf[1024];
@@ -60,6 +60,7 @@ PlanDebugOptions PlanDebugOptions::from_env() {
     o.forced_mm = num("MSNH_B200_M_MULT", 0);
     o.forced_bn = num("MSNH_B200_BN", 0);
     o.fp32_split = num("MSNH_B200_FP32_SPLIT", 0);
+    o.conv_split = num("MSNH_B200_CONV_SPLIT", 0);
     o.k_split = num("MSNH_B200_K_SPLIT", 0);
     o.stream_k = num("MSNH_B200_STREAM_K", 0);
     o.pair = num("MSNH_B200_PAIR", 0);
@@ -308,9 +309,9 @@ int msnh_b200_plan_create(MsnhB200Ctx *ctx, const MsnhB200Op *ops, int n_ops, in
         if (rc) return fail(ctx, rc, "op %d (kind %d): %s", i, ops[i].kind, err.c_str());
         if (ops[i].act < 0 || ops[i].act >= MSNH_ACT_COUNT) return fail(ctx, MSNH_B200_ERR_UNSUPPORTED, "op %d: activation %d not supported", i, ops[i].act);
     }
-    // fp32 detection nets: fp32 arithmetic throughout unless tf32 is asked for (see MSNH_PLAN_TF32_DETECT)
+    // fp32 detection nets: fp32 arithmetic throughout unless tf32 is asked for (see MSNH_PLAN_TF32_DETECT), convs on split operands
     if (dtype == MSNH_B200_F32 && !(flags & MSNH_PLAN_TF32_DETECT))
-        for (int i = 0; i < n_ops; ++i) if (ops[i].kind == MSNH_OP_YOLO) { pl->flags |= MSNH_PLAN_NO_TENSOR_CORE; break; }
+        for (int i = 0; i < n_ops; ++i) if (ops[i].kind == MSNH_OP_YOLO) { pl->split_fp32 = !(flags & MSNH_PLAN_NO_TENSOR_CORE); pl->flags |= MSNH_PLAN_NO_TENSOR_CORE; break; }
     *out = pl.release();
     return MSNH_B200_OK;
 } catch (...) { return caught(ctx); }

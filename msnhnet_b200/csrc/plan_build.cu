@@ -227,7 +227,7 @@ int build_launches(MsnhB200Plan *pl) {
     // matrix [pixel][tap*Cin + c] directly and the conv runs as a 1x1 GEMM over it. An image has so
     // few channels that per-tap im2col loads would move 6 useful bytes per 32-byte row.
     int patch_op = -1, patch_k = 0;
-    if (!no_fusion && !(pl->flags & MSNH_PLAN_NO_TENSOR_CORE)) {
+    if (!no_fusion && (!(pl->flags & MSNH_PLAN_NO_TENSOR_CORE) || splits_fp32(pl))) {
         int users = 0, user = -1;
         for (int i = 0; i < n_ops; ++i) for (int k = 0; k < pl->ops[i].d.n_in; ++k) if (pl->ops[i].d.in[k] == MSNH_B200_INPUT) { ++users; user = i; }
         if (users == 1 && pl->ops[user].d.kind == MSNH_OP_CONV && pl->ops[user].d.groups == 1 && pl->ops[user].absorbed_into < 0 &&
@@ -324,6 +324,13 @@ int build_launches(MsnhB200Plan *pl) {
         push(p);
     }
     const int es = esize(pl->dtype), V = vec_of(pl->dtype);
+    // 16-byte alignment of a tensor's pixels, known before the arena is (buffers start on 1024 bytes)
+    auto aligned_view = [&](int tensor) {
+        const Tensor &t = pl->tensors[tensor];
+        int off = 0;
+        const int root = root_of(pl, t.buffer, &off);
+        return (t.c_off + off) % V == 0 && pl->buffers[root].ldc % V == 0;
+    };
     for (int i = 0; i < n_ops; ++i) {
         OpState &o = pl->ops[i];
         if (o.absorbed_into >= 0) continue;
@@ -410,6 +417,9 @@ int build_launches(MsnhB200Plan *pl) {
                     const size_t row_len = patched ? static_cast<size_t>(patch_k) : static_cast<size_t>(taps) * cin_pad;
                     p.L.cin_pad = cin_pad;
                     const size_t n = static_cast<size_t>(cout) * row_len;
+                    // what an im2col tensor map can walk
+                    const bool tma_walks = groups == 1 && p.L.sh <= 8 && p.L.sw <= 8 && p.L.ph < 128 && p.L.pw < 128 && kh * p.L.dh < 256 && kw * p.L.dw < 256;
+                    bool split = false;
                     // packed straight into the arena's staging bytes (zero-filled, so the pad channels stay zero)
                     if (pl->dtype == MSNH_B200_F16) {
                         PackSlot<__half> ps = reserve_pack<__half>(pl, n);
@@ -420,20 +430,23 @@ int build_launches(MsnhB200Plan *pl) {
                         });
                         p.L.weights = ps.dev;
                     } else {
-                        PackSlot<float> ps = reserve_pack<float>(pl, n);
+                        // split operands: the matrix of the nearest tf32 values and, behind it, that of what they leave
+                        split = splits_fp32(pl) && tma_walks && aligned_view(in0) && aligned_view(o.tensor) && (p.res_t < 0 || aligned_view(p.res_t));
+                        PackSlot<float> ps = reserve_pack<float>(pl, split ? 2 * n : n);
                         float *pk = ps.host;
                         const bool tc = groups == 1 && !(pl->flags & MSNH_PLAN_NO_TENSOR_CORE);
                         if (pk) parallel_rows(cout, static_cast<size_t>(cin_g) * taps, [&](int co) {
                             for (int ci = 0; ci < cin_g; ++ci) for (int t = 0; t < taps; ++t) {
                                 const float v = w[(static_cast<size_t>(co) * cin_g + ci) * taps + t];
-                                pk[static_cast<size_t>(co) * row_len + static_cast<size_t>(t) * tap_stride + ci] = tc ? host_round_tf32(v) : v;
+                                const size_t at = static_cast<size_t>(co) * row_len + static_cast<size_t>(t) * tap_stride + ci;
+                                pk[at] = tc || split ? host_round_tf32(v) : v;
+                                if (split) pk[n + at] = host_round_tf32(v - pk[at]);
                             }
                         });
                         p.L.weights = ps.dev;
                     }
-                    const bool tensor_core = groups == 1 && !(pl->flags & MSNH_PLAN_NO_TENSOR_CORE) && p.L.sh <= 8 && p.L.sw <= 8 &&
-                                             p.L.ph < 128 && p.L.pw < 128 && kh * p.L.dh < 256 && kw * p.L.dw < 256;
-                    p.L.kind = tensor_core ? L_CONV_UMMA : L_CONV_DIRECT;
+                    const bool tensor_core = !(pl->flags & MSNH_PLAN_NO_TENSOR_CORE) && tma_walks;
+                    p.L.kind = split ? L_CONV_SPLIT : tensor_core ? L_CONV_UMMA : L_CONV_DIRECT;
                     if (patched) { p.L.kh = p.L.kw = 1; p.L.sh = p.L.sw = 1; p.L.ph = p.L.pw = 0; p.L.dh = p.L.dw = 1; p.L.note = "patch-matrix input"; }
                 }
                 if (!p.L.weights || !p.L.bias) return fail(ctx, MSNH_B200_ERR_NOMEM, "weight upload failed for op %d", i);
@@ -871,6 +884,12 @@ int build_launches(MsnhB200Plan *pl) {
             if (!ok) { L.kind = L_CONV_DIRECT; L.note = "unaligned view: CUDA-core fallback"; }
         }
         if (L.kind == L_CONV_UMMA) { const int rc = configure_conv_umma(pl, tt, L); if (rc) return rc; }
+        if (L.kind == L_CONV_SPLIT) {
+            if (!aligned(L.in) || !aligned(L.out) || (L.res && (reinterpret_cast<uintptr_t>(L.res) % 16 || L.ldc_res % V)))
+                return fail(ctx, MSNH_B200_ERR_STATE, "fp32 conv of op %d landed on an unaligned view", L.op);
+            const int rc = configure_conv_split(pl, L);
+            if (rc) return rc;
+        }
         if (L.kind == L_CONV_DIRECT)
             L.tiled = L.groups == 1 && aligned(L.in) && (L.out.N * static_cast<long long>(L.out.H) * L.out.W + kCtBM - 1) / kCtBM < 2147483647LL &&
                       (L.out.C + kCtBN - 1) / kCtBN <= 65535 && !dbg.conv_simple;

@@ -87,6 +87,8 @@ struct PlanDebugOptions {
     int trace_tile = 0;         // MSNH_B200_TRACE_TILE: which tile of a CTA the producer / MMA stamps describe
     int forced_mm = 0, forced_bn = 0;   // MSNH_B200_M_MULT, MSNH_B200_BN: force the conv tile shape
     int fp32_split = 0;         // MSNH_B200_FP32_SPLIT: shares of the fp32 conv's k (1..8), a CTA each; negative: all of them in one CTA
+    int conv_split = 0;         // MSNH_B200_CONV_SPLIT: shares of the split-operand fp32 conv's k (1..8, a CTA each where the clusters fit; negative:
+                                // all of them in one CTA)
     int k_split = 0;            // MSNH_B200_K_SPLIT: shares of the tensor-core conv's k in fp32 plans (1: one; 2, 4, 8: a CTA each where
                                 // the clusters fit; negative: all of them in one CTA)
     int stream_k = 0;           // MSNH_B200_STREAM_K: -1 by cost, 0 never, 1 wherever possible
@@ -123,7 +125,7 @@ struct Buffer {
 
 enum LaunchKind { L_INPUT = 0, L_CONV_UMMA, L_CONV_DIRECT, L_DWCONV, L_SBA, L_ADD, L_BINARY, L_MAXPOOL, L_AVGPOOL,
                   L_UPSAMPLE, L_SLICE, L_PAD, L_SOFTMAX, L_YOLO, L_COLLECT_ZERO, L_COLLECT, L_INPUT_PATCH, L_COLLECT_RAW, L_FOCUS,
-                  L_BILINEAR, L_COL2IM, L_CLIP, L_REMAP, L_REDUCE, L_PRELU, L_MAXPOOL_DEPTH };
+                  L_BILINEAR, L_COL2IM, L_CLIP, L_REMAP, L_REDUCE, L_PRELU, L_MAXPOOL_DEPTH, L_CONV_SPLIT };
 extern const char *const kLaunchNames[];
 
 struct Launch {
@@ -155,6 +157,7 @@ struct Launch {
     TView out2{};              // second output of two 1x1 convs over the same input merged into this launch (ptr == nullptr: none)
     int split_n = 0;           // its first channel in the merged channel range
     ConvUmmaParams up{};
+    ConvSplitParams sp{}; int sp_bn = 0, sp_split = 1;   // L_CONV_SPLIT: channels of a tile; CTAs of a cluster its shares are spread over
     int grid = 0; size_t smem = 0;
     // depthwise 3x3 on shared-memory tiles (map_a = the input's 4-D tensor map; grid / smem above)
     bool dw_tile = false; DwTileParams dwp{};
@@ -198,6 +201,7 @@ struct MsnhB200Plan {
     MsnhB200Ctx *ctx = nullptr;
     int in_c = 0, in_h = 0, in_w = 0, batch = 0, dtype = 0;
     uint32_t flags = 0;
+    bool split_fp32 = false;                        // convs in fp32 arithmetic on the tensor cores (conv_split.cuh) where they can
     msnh::PlanDebugOptions dbg;                     // the debug switches as they stood when plan_finalize began
     std::vector<msnh::OpState> ops;
     std::vector<msnh::Tensor> tensors;
@@ -261,6 +265,8 @@ struct MsnhB200Plan {
 
 namespace msnh {
 
+// fp32 convs on split operands (conv_split.cuh): the default of detection nets
+inline bool splits_fp32(const MsnhB200Plan *pl) { return pl->dtype == MSNH_B200_F32 && (pl->flags & MSNH_PLAN_NO_TENSOR_CORE) && (pl->split_fp32 || pl->dbg.conv_split != 0); }
 inline int esize(int dtype) { return dtype == MSNH_B200_F16 ? 2 : 4; }
 inline int vec_of(int dtype) { return dtype == MSNH_B200_F16 ? 8 : 4; }
 inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
@@ -294,6 +300,8 @@ int tile_tuning_end(MsnhB200Plan *pl, TileTuning &tt);
 int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L);
 // shares of the k of a CUDA-core fp32 conv launch, and the CTAs they are spread over
 void configure_conv_fp32(MsnhB200Plan *pl, Launch &L);
+// shares, tiles, grid and tensor maps of a split-operand fp32 conv launch whose views are resolved
+int configure_conv_split(MsnhB200Plan *pl, Launch &L);
 // the shared-memory tile form of a 3x3 depthwise launch, where it applies (sets L.dw_tile)
 void configure_dw_tile(MsnhB200Plan *pl, Launch &L);
 
@@ -328,6 +336,8 @@ void pack_write(MsnhB200Plan *pl);            // best effort: temporary file uni
 void launch_one(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st);
 void prepare_conv_umma_launch(const Launch &L);   // dynamic shared memory opt-in of the kernel instantiation L runs
 int conv_umma_max_clusters(int split);   // k-split convs: clusters of `split` CTAs that run at once
+int conv_split_max_clusters(int split);  // the same of the split-operand fp32 conv
+void prepare_conv_split_launch();        // shared memory opt-in of its kernels
 void launch_readback(MsnhB200Ctx *ctx, int dtype, const TView &v, float *dst_nchw, size_t count, cudaStream_t st);
 void launch_preprocess_u8(const unsigned char *src, float *dst, const PrepParams &p, int n_images, cudaStream_t st);
 int prepare_yolo_nms(MsnhB200Ctx *ctx);           // shared memory opt-in of the NMS kernel

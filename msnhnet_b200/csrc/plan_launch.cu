@@ -9,6 +9,7 @@ using namespace msnh;
 #include "layer_kernels.cuh"
 #include "dwconv_tile.cuh"
 #include "conv_tiled.cuh"
+#include "conv_split.cuh"
 
 namespace msnh {
 namespace {
@@ -86,6 +87,46 @@ void set_smem_attr(const Launch &L) {
 }  // namespace
 
 void prepare_conv_umma_launch(const Launch &L) { set_smem_attr(L); }
+
+namespace {
+const void *split_kernel(int bn, bool cluster) {
+#define MSNH_SPLIT_FORM(BN) if (bn == BN) return cluster ? reinterpret_cast<const void *>(conv_split_kernel<BN, true>) : reinterpret_cast<const void *>(conv_split_kernel<BN, false>)
+    MSNH_SPLIT_FORM(16); MSNH_SPLIT_FORM(32); MSNH_SPLIT_FORM(48);
+    MSNH_SPLIT_FORM(64);
+#undef MSNH_SPLIT_FORM
+    return nullptr;
+}
+}  // namespace
+
+void prepare_conv_split_launch() {
+    static std::mutex m;
+    static std::map<int, bool> done;           // by device: the attribute belongs to a context's module
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return;
+    std::lock_guard<std::mutex> g(m);
+    if (done[dev]) return;
+    for (int bn = 16; bn <= 64; bn += 16) for (bool cluster : {false, true})
+        cudaFuncSetAttribute(split_kernel(bn, cluster), cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(split_smem_bytes(bn)));
+    done[dev] = true;
+}
+int conv_split_max_clusters(int split) {
+    static std::mutex m;
+    static std::map<std::array<int, 2>, int> known;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return 0; }
+    prepare_conv_split_launch();
+    std::lock_guard<std::mutex> g(m);
+    const auto it = known.find({dev, split});
+    if (it != known.end()) return it->second;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(split); cfg.blockDim = dim3(kSpThreads); cfg.dynamicSmemBytes = split_smem_bytes(64);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension; attr[0].val.clusterDim.x = split; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, split_kernel(64, true), &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+    return known[{dev, split}] = n;
+}
 
 // Clusters of `split` CTAs of the k-split conv that run at the same time on the current device (a CTA takes most of an SM's
 // shared memory, a cluster's CTAs sit in one GPC).
@@ -165,6 +206,18 @@ void launch_typed(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st) {
             void *args[6] = {const_cast<CUtensorMap *>(&L.map_a), const_cast<CUtensorMap *>(&L.map_b), const_cast<CUtensorMap *>(&L.map_c),
                              const_cast<CUtensorMap *>(L.out2.ptr ? &L.map_c2 : &L.map_c), const_cast<CUtensorMap *>(L.res ? &L.map_res : &L.map_c), const_cast<ConvUmmaParams *>(&L.up)};
             cudaLaunchKernelExC(&cfg, umma_kernel<T>(L), args);
+            break;
+        }
+        case L_CONV_SPLIT: {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(L.grid); cfg.blockDim = dim3(kSpThreads); cfg.dynamicSmemBytes = L.smem; cfg.stream = st;
+            cudaLaunchAttribute attr[2];
+            int na = 0;
+            if (L.sp_split > 1) { attr[na].id = cudaLaunchAttributeClusterDimension; attr[na].val.clusterDim.x = L.sp_split; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1; ++na; }
+            if (ctx->pdl) { attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[na].val.programmaticStreamSerializationAllowed = 1; ++na; }
+            cfg.attrs = attr; cfg.numAttrs = na;
+            void *args[4] = {const_cast<CUtensorMap *>(&L.map_a), const_cast<CUtensorMap *>(&L.map_b), const_cast<TView *>(&L.out), const_cast<ConvSplitParams *>(&L.sp)};
+            cudaLaunchKernelExC(&cfg, split_kernel(L.sp_bn, L.sp_split > 1), args);
             break;
         }
         case L_CONV_DIRECT:

@@ -121,7 +121,7 @@ static int slot_forward(MsnhB200Plan *pl, MsnhB200Plan::StreamSlot &s, bool stag
     if (mine.empty()) {
         std::vector<Launch> copy = pl->launches;
         for (Launch &L : copy) {
-            L.up.err_flag = L.dwp.err_flag = s.dev_err_flag;
+            L.up.err_flag = L.sp.err_flag = L.dwp.err_flag = s.dev_err_flag;
             if (staged && L.in.ptr == pl->d_input) L.in.ptr = s.d_stage;
         }
         if (pl->graph_exec) {

@@ -158,6 +158,70 @@ void configure_conv_fp32(MsnhB200Plan *pl, Launch &L) {
     L.note += (L.note.empty() ? "" : ", ") + std::string(note);
 }
 
+int configure_conv_split(MsnhB200Plan *pl, Launch &L) {
+    MsnhB200Ctx *ctx = pl->ctx;
+    ConvSplitParams &u = L.sp;
+    const int cin = L.in.C, cout = L.out.C;
+    u.m_total = L.out.N * L.out.H * L.out.W; u.cout = cout;
+    // tiles of up to 64 channels (what TMEM holds beside four slots of split activations), evenly wide
+    u.tiles_n = (cout + 63) / 64;
+    L.sp_bn = round_up((cout + u.tiles_n - 1) / u.tiles_n, 16);
+    u.tiles_m = (u.m_total + kUmmaM - 1) / kUmmaM;
+    u.taps = L.kh * L.kw; u.kw = L.kw;
+    // What an accumulator loses to truncation shows beside the FMA chain it replaces where k is very short (norm error against 64 bits,
+    // 27 values of k: FMAs 9.6e-8, k-blocks of 32 / 16 / 8 values 1.35e-7 / 1.00e-7 / 9.2e-8; 48 values: 1.27e-7 and 1.20e-7 in blocks of 32), and so
+    // does the smallest product (64 values: 1.46e-7, without it 1.33e-7, with it 1.28e-7).
+    u.chunk_elems = u.taps * cin < 48 ? 8 : 32; u.chunk_steps = u.chunk_elems / 8;
+    u.all_products = u.taps * cin <= 128;
+    u.chunks_per_tap = (cin + u.chunk_elems - 1) / u.chunk_elems; u.cin_pad = L.cin_pad;
+    u.tail_steps = (cin - u.chunk_elems * (u.chunks_per_tap - 1) + 7) / 8;
+    u.dil_h = L.dh; u.dil_w = L.dw;
+    u.oh = L.out.H; u.ow = L.out.W; u.stride_h = L.sh; u.stride_w = L.sw; u.pad_h = L.ph; u.pad_w = L.pw;
+    u.res = L.res; u.ldc_res = L.ldc_res; u.scale = L.scale; u.bias = L.bias;
+    u.act1 = L.act1; u.act1_param = L.act1_p; u.act2 = L.act2; u.act2_param = L.act2_p;
+    u.err_flag = ctx->dev_err_flag;
+    const int num_k = u.taps * u.chunks_per_tap;
+    // us over m pixels with the k of a tile in `shares` shares, on a cluster or (on_cluster = false) one after the other in a CTA
+    auto cost_of = [&](int m, int shares, bool on_cluster) {
+        const long tiles = static_cast<long>((m + kUmmaM - 1) / kUmmaM) * u.tiles_n;
+        if (!on_cluster || shares == 1) return std::ceil(static_cast<double>(tiles) / ctx->sm_count) * (num_k * 0.23 + 0.3 * shares + 0.8) + 1.5;
+        return std::ceil(static_cast<double>(tiles) / std::max(1, conv_split_max_clusters(shares))) * (std::ceil(static_cast<double>(num_k) / shares) * 0.23 + 3.8);
+    };
+    // The number of shares decides the order of a layer's sums, so it comes from the layer and one image; who sums them does not.
+    const int m_image = L.out.H * L.out.W;
+    u.shares = 1;
+    double best = cost_of(m_image, 1, false);
+    for (int s = 2; s <= kUmmaMaxKSplit && num_k >= 3 * s; ++s) {
+        const double cost = cost_of(m_image, s, true);
+        if (cost < best * 0.95) { best = cost; u.shares = s; }
+    }
+    const int forced = std::min(std::abs(pl->dbg.conv_split), kUmmaMaxKSplit);
+    if (forced) u.shares = std::min(forced, num_k);
+    const bool cluster = u.shares > 1 && (forced ? pl->dbg.conv_split > 0 : cost_of(u.m_total, u.shares, true) < cost_of(u.m_total, u.shares, false));
+    L.sp_split = cluster ? u.shares : 1;
+    const int tiles = u.tiles_m * u.tiles_n;
+    L.grid = cluster ? tiles * u.shares : std::min(tiles, ctx->sm_count);
+    L.smem = split_smem_bytes(L.sp_bn);
+    const bool linear = L.kh == 1 && L.kw == 1 && L.sh == 1 && L.sw == 1 && L.ph == 0 && L.pw == 0;
+    u.a_mode = linear ? A_MODE_LINEAR : A_MODE_IM2COL;
+    int rc;
+    if (linear) rc = make_map_2d(ctx, &L.map_a, MSNH_B200_F32, L.in.ptr, static_cast<uint64_t>(cin), static_cast<uint64_t>(L.in.N) * L.in.H * L.in.W, static_cast<uint64_t>(L.in.ldc) * 4, 32, kUmmaM, 128);
+    else        rc = make_map_im2col(ctx, &L.map_a, MSNH_B200_F32, L.in, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, L.dh, L.dw, 32, 128, kUmmaM);
+    if (rc) return rc;
+    const cuuint64_t ktot = static_cast<cuuint64_t>(u.taps) * u.cin_pad;
+    cuuint64_t dims[3] = {ktot, static_cast<cuuint64_t>(cout), 2}, strides[2] = {ktot * 4, ktot * 4 * cout};
+    cuuint32_t box[3] = {32, static_cast<cuuint32_t>(L.sp_bn), 2}, estr[3] = {1, 1, 1};
+    const CUresult r = ctx->encode_tiled(&L.map_b, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(L.weights), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(ctx, MSNH_B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d): split weights %llu x %d", (int)r, (unsigned long long)ktot, cout);
+    prepare_conv_split_launch();
+    char note[128];
+    snprintf(note, sizeof(note), "fp32 arithmetic, %d x %d tiles of 128 x %d, %d k-blocks, grid %d, k over %d CTAs", u.tiles_m, u.tiles_n, L.sp_bn, num_k, L.grid, L.sp_split);
+    if (u.shares > L.sp_split) snprintf(note + strlen(note), sizeof(note) - strlen(note), " in %d shares", u.shares);
+    L.note += (L.note.empty() ? "" : ", ") + std::string(note);
+    return MSNH_B200_OK;
+}
+
 int tile_tuning_begin(MsnhB200Plan *pl, TileTuning &tt) {
     // MSNH_B200_AUTOTUNE=0 keeps the modelled tile shapes; plans made for debugging (no graph, no fusion, every output
     // kept, traced) keep them too
