@@ -118,6 +118,11 @@ constexpr int kActGeneric = -1;
 constexpr int kTraceSlots = 64;
 
 // ---- other layers (layer_kernels.cuh) ---------------------------------------------------------------------------------
+// shared memory of nchw_f32_to_row_patches_kernel: the image rows under one output row of patches, with their padding
+constexpr size_t row_patch_smem(int c, int w, int kw, int pw, int sw, int ow) {
+    const int left = pw, need = (ow - 1) * sw + kw - left;          // columns from the image's first on
+    return static_cast<size_t>(c) * (left + (need > w ? need : w)) * sizeof(float);
+}
 // inputs of an n-ary sum
 struct AddInputs { const void *ptr[MSNH_B200_MAX_IN]; int ldc[MSNH_B200_MAX_IN]; int n; };
 // the pools of one maxpool_plane_kernel launch: up to three stride-1 windows over the same staged plane

@@ -143,6 +143,58 @@ __global__ void nchw_f32_to_patches_fixed_kernel(const float *__restrict__ src, 
     }
 }
 
+// Row patches: for every image row and output column the kw pixels under a filter row, [row][output column][pixel * C + c], padded with
+// zeros; a conv reads them as kh x 1. A CTA stages `rows` image rows in shared memory, their padding included, and writes the patches of a row as
+// one stream of 16-byte vectors; a vector's place inside a patch decides what it gathers, and the number of threads is a multiple of the
+// vectors of a patch, so that a thread's gather is the same throughout. Bound by the writes: 32 images of 224 x 224 under a 7-wide
+// filter at stride 2 are 77 MB.
+template <typename T>
+__global__ void __launch_bounds__(256)
+nchw_f32_to_row_patches_kernel(const float *__restrict__ src, TView dst, int C, int H, int W, int kw, int sw, int pw, int rows) {
+    constexpr int V = Elem<T>::kVec;
+    extern __shared__ float row_smem[];
+    const int pieces = dst.ldc / V, threads = blockDim.x / pieces * pieces, t = threadIdx.x;
+    const int width = pw + max(W, (dst.W - 1) * sw + kw - pw);
+    int at[V];                                     // offset of a vector's values in the staged row (output column 0); negative: pad channel
+    const int piece = t % pieces;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+        const int v = piece * V + e, s = v / C;
+        at[e] = s < kw ? (v - s * C) * width + s : -1;
+    }
+    const int warp = t >> 5, lane = t & 31, warps = blockDim.x >> 5;
+    pdl_prologue();
+    for (int row0 = blockIdx.x * rows; row0 < dst.N * H; row0 += gridDim.x * rows) {
+        const int here = min(rows, dst.N * H - row0);
+        for (int q = warp; q < here * C; q += warps) {                 // a warp per row and channel
+            const int r = q / C, c = q - r * C, n = (row0 + r) / H, y = row0 + r - n * H;
+            const float *s = src + (static_cast<size_t>(n * C + c) * H + y) * W;
+            float *to = row_smem + q * width;
+#pragma unroll 4
+            for (int i = lane; i < width; i += 32) {
+                const int x = i - pw;
+                const float v = x >= 0 && x < W ? __ldg(s + x) : 0.f;
+                to[i] = dst.tf32 ? round_tf32(v) : v;
+            }
+        }
+        __syncthreads();
+        if (t < threads)
+            for (int r = 0; r < here; ++r) {
+                T *d = static_cast<T *>(dst.ptr) + static_cast<size_t>(row0 + r) * dst.W * dst.ldc;
+                const float *from = row_smem + r * C * width;
+#pragma unroll 2
+                for (int i = t; i < dst.W * pieces; i += threads) {
+                    const int x = i / pieces * sw;
+                    float v[V];
+#pragma unroll
+                    for (int e = 0; e < V; ++e) v[e] = at[e] >= 0 ? from[at[e] + x] : 0.f;
+                    st_vec(d + static_cast<size_t>(i) * V, v);
+                }
+            }
+        __syncthreads();
+    }
+}
+
 // The same for fp16 and the 3x3x3 stem without dilation. The kernel above converts every image value nine times and reads it as
 // often through L1 (27 loads and conversions per pixel: 85 us for eight images of 608 x 608, 225 MB). Here a CTA of 128 threads
 // stages the input rows of 128 x 4 output pixels in shared memory as interleaved fp16 pixels, so that the nine values of a filter

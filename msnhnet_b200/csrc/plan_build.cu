@@ -227,6 +227,7 @@ int build_launches(MsnhB200Plan *pl) {
     // matrix [pixel][tap*Cin + c] directly and the conv runs as a 1x1 GEMM over it. An image has so
     // few channels that per-tap im2col loads would move 6 useful bytes per 32-byte row.
     int patch_op = -1, patch_k = 0;
+    bool row_patches = false;
     if (!no_fusion && (!(pl->flags & MSNH_PLAN_NO_TENSOR_CORE) || splits_fp32(pl))) {
         int users = 0, user = -1;
         for (int i = 0; i < n_ops; ++i) for (int k = 0; k < pl->ops[i].d.n_in; ++k) if (pl->ops[i].d.in[k] == MSNH_B200_INPUT) { ++users; user = i; }
@@ -235,6 +236,16 @@ int build_launches(MsnhB200Plan *pl) {
             patch_op = user;
             patch_k = round_up(pl->in_c * pl->ops[user].d.k_h * pl->ops[user].d.k_w, 16);
             in_s.C = patch_k; in_s.H = pl->ops[user].out.H; in_s.W = pl->ops[user].out.W;
+        }
+        // A receptive field too large for that (the 7x7 stem: 147 values) is taken row by row: the layout kernel writes, for every
+        // input row and output column, the kw pixels that the filter's rows cover there, and the conv runs as kh x 1 over those, one
+        // k-block a filter row. Tap by tap the stem of ResNet-18 fp32 was 49 k-blocks of three useful values: a forward with 32
+        // images 641 -> 524 us, with one 159 -> 153.
+        else if (users == 1 && pl->ops[user].d.kind == MSNH_OP_CONV && pl->ops[user].d.groups == 1 && pl->ops[user].absorbed_into < 0 && !splits_fp32(pl) &&
+                 pl->ops[user].d.k_w > 1 && pl->ops[user].d.dil_w == 1 && pl->in_c <= 4 && pl->in_c * pl->ops[user].d.k_w <= 64 &&
+                 row_patch_smem(pl->in_c, pl->in_w, pl->ops[user].d.k_w, pl->ops[user].d.pad_w, pl->ops[user].d.stride_w, pl->ops[user].out.W) <= 48 * 1024) {
+            patch_op = user; row_patches = true;
+            in_s.C = pl->in_c * pl->ops[user].d.k_w; in_s.W = pl->ops[user].out.W;
         }
     }
     pl->input_tensor = new_tensor(pl, in_s, pl->dtype);
@@ -318,6 +329,10 @@ int build_launches(MsnhB200Plan *pl) {
             p.L.kind = L_INPUT_PATCH; p.L.op = patch_op;
             p.L.kh = c.k_h; p.L.kw = c.k_w; p.L.sh = c.stride_h; p.L.sw = c.stride_w; p.L.ph = c.pad_h; p.L.pw = c.pad_w; p.L.dh = c.dil_h; p.L.dw = c.dil_w;
             p.L.ival = pl->in_c; p.L.ival2 = pl->in_h; p.L.max_rows = pl->in_w;
+            if (row_patches) {
+                p.L.kind = L_INPUT_ROWS;
+                p.L.bytes = (static_cast<double>(pl->in_c) * pl->in_h * pl->in_w * 4.0 + static_cast<double>(in_s.C) * in_s.H * in_s.W * esize(pl->dtype)) * pl->batch;
+            } else
             p.L.bytes = static_cast<double>(pl->in_c) * pl->in_h * pl->in_w * pl->batch * 4.0 +
                         static_cast<double>(patch_k) * pl->ops[patch_op].out.H * pl->ops[patch_op].out.W * pl->batch * esize(pl->dtype);
         }
@@ -345,8 +360,8 @@ int build_launches(MsnhB200Plan *pl) {
             case MSNH_OP_CONV: case MSNH_OP_CONNECTED: {
                 const Fused &f = fused[i];
                 const bool fc = d.kind == MSNH_OP_CONNECTED;
-                const bool patched = i == patch_op;
-                if (patched) { a.C = pl->in_c; a.H = pl->in_h; a.W = pl->in_w; }   // the conv's real input, not the patch matrix
+                const bool rows = i == patch_op && row_patches, patched = i == patch_op && !rows;
+                if (i == patch_op) { a.C = pl->in_c; a.H = pl->in_h; a.W = pl->in_w; }   // the conv's real input, not the patch matrix
                 const int kh = fc ? a.H : d.k_h, kw = fc ? a.W : d.k_w;
                 const int groups = fc ? 1 : d.groups;
                 const int cin_g = a.C / groups;
@@ -412,9 +427,10 @@ int build_launches(MsnhB200Plan *pl) {
                 } else {
                     // [Cout][Cin/g][kh][kw] -> [Cout][tap][cin_pad], zero in the pad channels
                     // (patch mode: one "tap" of patch_k values ordered tap-major, like the patch matrix)
-                    const int cin_pad = patched ? patch_k : round_up(cin_g, V);
-                    const int tap_stride = patched ? cin_g : cin_pad;        // distance between taps inside a row
-                    const size_t row_len = patched ? static_cast<size_t>(patch_k) : static_cast<size_t>(taps) * cin_pad;
+                    // (row patches: one "tap" per filter row, of kw x cin values)
+                    const int cin_pad = patched ? patch_k : round_up(rows ? kw * cin_g : cin_g, V);
+                    const size_t row_len = patched ? static_cast<size_t>(patch_k) : static_cast<size_t>(rows ? kh : taps) * cin_pad;
+                    auto tap_at = [&](int t) { return static_cast<size_t>(patched ? t * cin_g : rows ? t / kw * cin_pad + t % kw * cin_g : t * cin_pad); };   // where a tap starts inside a row
                     p.L.cin_pad = cin_pad;
                     const size_t n = static_cast<size_t>(cout) * row_len;
                     // what an im2col tensor map can walk
@@ -426,7 +442,7 @@ int build_launches(MsnhB200Plan *pl) {
                         __half *pk = ps.host;
                         if (pk) parallel_rows(cout, static_cast<size_t>(cin_g) * taps, [&](int co) {
                             for (int ci = 0; ci < cin_g; ++ci) for (int t = 0; t < taps; ++t)
-                                pk[static_cast<size_t>(co) * row_len + static_cast<size_t>(t) * tap_stride + ci] = __float2half_rn(w[(static_cast<size_t>(co) * cin_g + ci) * taps + t]);
+                                pk[static_cast<size_t>(co) * row_len + tap_at(t) + ci] = __float2half_rn(w[(static_cast<size_t>(co) * cin_g + ci) * taps + t]);
                         });
                         p.L.weights = ps.dev;
                     } else {
@@ -438,7 +454,7 @@ int build_launches(MsnhB200Plan *pl) {
                         if (pk) parallel_rows(cout, static_cast<size_t>(cin_g) * taps, [&](int co) {
                             for (int ci = 0; ci < cin_g; ++ci) for (int t = 0; t < taps; ++t) {
                                 const float v = w[(static_cast<size_t>(co) * cin_g + ci) * taps + t];
-                                const size_t at = static_cast<size_t>(co) * row_len + static_cast<size_t>(t) * tap_stride + ci;
+                                const size_t at = static_cast<size_t>(co) * row_len + tap_at(t) + ci;
                                 pk[at] = tc || split ? host_round_tf32(v) : v;
                                 if (split) pk[n + at] = host_round_tf32(v - pk[at]);
                             }
@@ -448,6 +464,7 @@ int build_launches(MsnhB200Plan *pl) {
                     const bool tensor_core = !(pl->flags & MSNH_PLAN_NO_TENSOR_CORE) && tma_walks;
                     p.L.kind = split ? L_CONV_SPLIT : tensor_core ? L_CONV_UMMA : L_CONV_DIRECT;
                     if (patched) { p.L.kh = p.L.kw = 1; p.L.sh = p.L.sw = 1; p.L.ph = p.L.pw = 0; p.L.dh = p.L.dw = 1; p.L.note = "patch-matrix input"; }
+                    if (rows) { p.L.kw = 1; p.L.sw = 1; p.L.pw = 0; p.L.note = "row patches"; }
                 }
                 if (!p.L.weights || !p.L.bias) return fail(ctx, MSNH_B200_ERR_NOMEM, "weight upload failed for op %d", i);
                 push(p);
@@ -834,7 +851,7 @@ int build_launches(MsnhB200Plan *pl) {
         if (p.in_t >= 0) L.in = view_of(pl, p.in_t);
         if (p.out_t >= 0) L.out = view_of(pl, p.out_t);
         if (p.out2_t >= 0) L.out2 = view_of(pl, p.out2_t);
-        if (L.kind == L_INPUT || L.kind == L_INPUT_PATCH) { L.in.ptr = pl->d_input; }
+        if (L.kind == L_INPUT || L.kind == L_INPUT_PATCH || L.kind == L_INPUT_ROWS) { L.in.ptr = pl->d_input; }
         if (p.c_sub >= 0) {   // concat copy: a channel window of the destination / source
             L.out.ptr = static_cast<uint8_t *>(L.out.ptr) + static_cast<size_t>(p.c_off_out) * es; L.out.C = p.c_sub;
             L.in.ptr = static_cast<uint8_t *>(L.in.ptr) + static_cast<size_t>(p.c_in_off) * es; L.in.C = p.c_in_sub;

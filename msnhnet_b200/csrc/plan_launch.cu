@@ -194,6 +194,15 @@ void launch_typed(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st) {
             launch_k(ctx->pdl, nchw_f32_to_patches_kernel<T>, grid_for(ctx, static_cast<size_t>(L.out.N) * L.out.H * L.out.W, block), block, 0, st, 
                 static_cast<const float *>(L.in.ptr), L.out, L.ival, L.ival2, L.max_rows, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, L.dh, L.dw);
             break;
+        case L_INPUT_ROWS: {
+            // several rows a turn where there are enough of them for every SM's eight CTAs
+            const long long total = static_cast<long long>(L.out.N) * L.out.H;
+            const size_t row = row_patch_smem(L.ival, L.max_rows, L.kw, L.pw, L.sw, L.out.W);
+            const int rows = total >= 32LL * ctx->sm_count && 4 * row <= 24 * 1024 ? 4 : 1;
+            launch_k(ctx->pdl, nchw_f32_to_row_patches_kernel<T>, static_cast<int>(std::min<long long>((total + rows - 1) / rows, 16LL * ctx->sm_count)), 256, rows * row, st,
+                     static_cast<const float *>(L.in.ptr), L.out, L.ival, L.ival2, L.max_rows, L.kw, L.sw, L.pw, rows);
+            break;
+        }
         case L_CONV_UMMA: {
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3(L.grid); cfg.blockDim = dim3(kUmmaThreads); cfg.dynamicSmemBytes = L.smem; cfg.stream = st;
