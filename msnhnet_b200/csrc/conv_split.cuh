@@ -182,15 +182,16 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const int share_first = kSplit ? rank : 0, share_end = kSplit ? rank + 1 : p.shares;
 
     pdl_launch_dependents();
-    if (threadIdx.x == 0) {
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
-        cta_abort_slot = 0;
-        for (uint32_t s = 0; s < kSpAStages; ++s) { mbar_init(full_a(s), 1); mbar_init(empty_a(s), 4); }
-        for (uint32_t s = 0; s < kSpRing; ++s) { mbar_init(ready(s), 4 + 1 + 16); mbar_init(done(s), 1); }
-        for (uint32_t s = 0; s < 2; ++s) { mbar_init(s_full(s), 2); mbar_init(s_empty(s), 16); }
+    if (threadIdx.x < 36) {             // a barrier per thread
+        const uint32_t t = threadIdx.x;
+        mbar_init(bar_base + 8u * t, t < 8 ? 1u : t < 16 ? 4u : t < 24 ? 4 + 1 + 16u : t < 32 ? 1u : t < 34 ? 2u : 16u);      // full_a, empty_a, ready, done, s_full, s_empty
+        if (t == 0) cta_abort_slot = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (threadIdx.x == 96) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
     }
     if (warp == 2) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_slot)), "r"(512u) : "memory");

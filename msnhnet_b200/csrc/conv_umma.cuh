@@ -452,22 +452,24 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     };
 
     pdl_launch_dependents();
-    if (threadIdx.x == 0) {
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c) : "memory");
-        if (p.split_n != 0x7fffffff) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c2) : "memory");
-        if (!kPair && !kStreamK && !kSplit && p.res) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_res) : "memory");
-        cta_abort_slot = 0;
-        for (int s = 0; s < p.num_stages; ++s) { mbar_init(full_bar(s), 2); mbar_init(empty_bar(s), 1); }
+    // a barrier per thread: one thread after the other they took some 300 cycles of every launch
+    if (threadIdx.x < 2 * kUmmaMaxStages + 2 * kUmmaMaxAccStages + 16) {
+        const int t = static_cast<int>(threadIdx.x);
         // arrivals that free an accumulator: the team epilogue's warps (pair / stream-K kernels), or one per warp and
         // store unit of a tile (plain kernels: four warps x sub-tiles x slabs)
         const int units = kMult * ((p.bn * static_cast<int>(sizeof(T)) + p.out_chunk_bytes - 1) / p.out_chunk_bytes);
         const uint32_t acc_arrivals = (kPair || kStreamK) ? 16u * (kPair ? 2u : 1u) : 4u * static_cast<uint32_t>(units);
-        for (int s = 0; s <= acc_mask; ++s) { mbar_init(acc_full_bar(s), 1); mbar_init(acc_empty_bar(s), acc_arrivals); }
-        for (int e = 0; e < 16; ++e) mbar_init(res_bar(e), 1);
+        mbar_init(bar_base + 8u * threadIdx.x, t < kUmmaMaxStages ? 2u : t >= 2 * kUmmaMaxStages + kUmmaMaxAccStages && t < 2 * kUmmaMaxStages + 2 * kUmmaMaxAccStages ? acc_arrivals : 1u);
+        if (t == 0) cta_abort_slot = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (threadIdx.x == 32 * kUmmaWeightWarp) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c) : "memory");
+        if (p.split_n != 0x7fffffff) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_c2) : "memory");
+        if (!kPair && !kStreamK && !kSplit && p.res) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_res) : "memory");
     }
     if (sb_staged && threadIdx.x >= 64 && threadIdx.x < 576) {   // constants: no need to wait for the previous kernel
         const int t = threadIdx.x - 64;      // 256 float4 of scale, then 256 of bias
