@@ -373,15 +373,19 @@ __device__ __forceinline__ void activate_pairs(F2 (&y)[8], int act, float param)
 // CTA leaves its raw accumulators in its own shared memory; behind a cluster barrier each finishes every k_split-th row of the tile,
 // adding the shares through distributed shared memory. For layers whose k is long and whose tiles are few: a 3x3 512->512 layer at 7x7
 // is one tile of pixels and 144 tf32 k-blocks of 330 cycles.
+// kBlocks: k-blocks a stage holds. Two share a wait, an expect and a commit, which the short k-loops of clusters gain by: ResNet-18 fp32 with one image
+// 154 -> 150.5 us a forward. The other forms stay at one: in nets whose layers would mix both the change of kernels costs what it gains (MobileNetV2, 64 images
+// 615 -> 623, YOLOv4-608, eight 1817 -> 1826), and a number that is not compiled in costs more than it gains (one image 767 -> 795).
 // kAct: a compile-time first activation leaves no switch in the epilogue loops (MSNH_ACT_LEAKY: slope in [0, 1]);
 // kActGeneric switches at run time. kTrace: the instantiation that records clock stamps (plans made with MSNH_PLAN_TRACE); the
 // production instantiations carry none of that code.
-template <typename T, int kMult, bool kPair, bool kStreamK, int kAct = kActGeneric, bool kTrace = false, bool kSplit = false, bool kShares = false>   // kMult: 128-pixel sub-tiles per tile (1, 2, 3, 4)
+template <typename T, int kMult, bool kPair, bool kStreamK, int kAct = kActGeneric, bool kTrace = false, bool kSplit = false, bool kShares = false, int kBlocks = 1>   // kMult: 128-pixel sub-tiles per tile (1, 2, 3, 4)
 __global__ void __launch_bounds__(kUmmaThreads, 1)
 conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                  const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_c2,
                  const __grid_constant__ CUtensorMap map_res, const ConvUmmaParams p) {
     constexpr bool kTf32 = sizeof(T) == 4;
+    static_assert(kBlocks == 1 || (kBlocks == 2 && !kPair && !kStreamK && !kShares), "stages of two k-blocks");
     static_assert(!(kSplit || kShares) || (kTf32 && !kPair && !kStreamK && kSplit != kShares), "the k of a tile is summed in shares in fp32 plans only");
     const int shares = kShares ? p.k_shares : 1;
     extern __shared__ uint8_t smem_raw[];
@@ -401,8 +405,8 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int tile_stride = kPair ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);   // (kSplit: past the last tile)
     const int tile_rows   = kPair ? 2 * kUmmaM : kUmmaM * kMult;
     const uint32_t a_base = smem_base;
-    const uint32_t b_base = a_base + p.num_stages * a_bytes;
-    const uint32_t stage_c_base = (b_base + p.num_stages * b_bytes + 1023u) & ~1023u;   // two output staging slabs
+    const uint32_t b_base = a_base + p.num_stages * kBlocks * a_bytes;
+    const uint32_t stage_c_base = (b_base + p.num_stages * kBlocks * b_bytes + 1023u) & ~1023u;   // two output staging slabs
     const uint32_t bar_base = stage_c_base + 4 * kStageCBytes;
     auto full_bar      = [&](int s) { return bar_base + 8u * s; };
     auto empty_bar     = [&](int s) { return bar_base + 8u * (kUmmaMaxStages + s); };
@@ -530,28 +534,36 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     chunk = k0 - tap * p.chunks_per_tap; s = tap - r * p.kw; off_h = r * p.dil_h;
                 }
                 int c0 = chunk * p.bk_elems, off_w = s * p.dil_w;
-                for (int kt = k0; kt < k1; ++kt) {
+                for (int kt = k0; kt < k1; kt += kBlocks) {
                     ok = mbar_wait(empty_bar(stage), phase ^ 1u, cta_abort, p.err_flag, DEV_ERR_WAIT_EMPTY);
                     if (!ok) break;
-                    const uint32_t dst = a_base + stage * a_bytes, bar = full0 + 8u * stage;
-                    if (lead) mbar_expect_tx(full_bar(stage), tx);
-                    if constexpr (kPair) {
-                        if (im2col) tma_load_im2col_4d_pair(dst, &map_a, bar, c0, cx, cy, img, static_cast<uint16_t>(off_w), static_cast<uint16_t>(off_h));
-                        else        tma_load_2d_pair(dst, &map_a, bar, c0, m0);
-                    } else if (im2col) {
-                        tma_load_im2col_4d(dst, &map_a, bar, c0, cx, cy, img, static_cast<uint16_t>(off_w), static_cast<uint16_t>(off_h));
-                    } else {
-                        // a box holds up to 256 rows: tiles of three and four sub-tiles take two loads
-                        tma_load_2d(dst, &map_a, bar, c0, m0);
-                        if constexpr (kMult > 2) tma_load_2d(dst + a_bytes / 2, &map_a, bar, c0, m0 + kUmmaM * kMult / 2);
-                    }
+                    const uint32_t dst = a_base + stage * kBlocks * a_bytes, bar = full0 + 8u * stage;
+                    const bool second = kBlocks == 2 && kt + 1 < k1;
+                    if (lead) mbar_expect_tx(full_bar(stage), second ? 2 * tx : tx);
+                    auto load = [&](uint32_t to) {
+                        if constexpr (kPair) {
+                            if (im2col) tma_load_im2col_4d_pair(to, &map_a, bar, c0, cx, cy, img, static_cast<uint16_t>(off_w), static_cast<uint16_t>(off_h));
+                            else        tma_load_2d_pair(to, &map_a, bar, c0, m0);
+                        } else if (im2col) {
+                            tma_load_im2col_4d(to, &map_a, bar, c0, cx, cy, img, static_cast<uint16_t>(off_w), static_cast<uint16_t>(off_h));
+                        } else {
+                            // a box holds up to 256 rows: tiles of three and four sub-tiles take two loads
+                            tma_load_2d(to, &map_a, bar, c0, m0);
+                            if constexpr (kMult > 2) tma_load_2d(to + a_bytes / 2, &map_a, bar, c0, m0 + kUmmaM * kMult / 2);
+                        }
+                    };
+                    auto advance = [&]() {
+                        c0 += p.bk_elems;
+                        if (++chunk == p.chunks_per_tap) {
+                            chunk = 0; c0 = 0; off_w += p.dil_w;
+                            if (++s == p.kw) { s = 0; off_w = 0; off_h += p.dil_h; }
+                        }
+                    };
+                    load(dst);
                     if constexpr (kTrace) { if (trace && i == p.trace_tile && kt - k0 < 16) trace[8 + kt - k0] = clock64(); }
                     if (++stage == p.num_stages) { stage = 0; phase ^= 1u; }
-                    c0 += p.bk_elems;
-                    if (++chunk == p.chunks_per_tap) {
-                        chunk = 0; c0 = 0; off_w += p.dil_w;
-                        if (++s == p.kw) { s = 0; off_w = 0; off_h += p.dil_h; }
-                    }
+                    advance();
+                    if constexpr (kBlocks == 2) { if (second) { load(dst + a_bytes); advance(); } }
                 }
             }
         }
@@ -568,15 +580,21 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 const int n0 = (tile % p.tiles_n) * p.bn + static_cast<int>(rank) * b_rows;
                 const int tap0 = k0 / p.chunks_per_tap;
                 int chunk = k0 - tap0 * p.chunks_per_tap, tap_c = tap0 * p.cin_pad, c0 = tap_c + chunk * p.bk_elems;
-                for (int kt = k0; kt < k1; ++kt) {
+                for (int kt = k0; kt < k1; kt += kBlocks) {
                     ok = mbar_wait(empty_bar(stage), phase ^ 1u, cta_abort, p.err_flag, DEV_ERR_WAIT_EMPTY);
                     if (!ok) break;
-                    if (lead) mbar_expect_tx(full_bar(stage), tx);
-                    if constexpr (kPair) tma_load_2d_pair(b_base + stage * b_bytes, &map_b, full0 + 8u * stage, c0, n0);
-                    else                 tma_load_2d(b_base + stage * b_bytes, &map_b, full_bar(stage), c0, n0);
+                    const uint32_t dst = b_base + stage * kBlocks * b_bytes, bar = full0 + 8u * stage;
+                    const bool second = kBlocks == 2 && kt + 1 < k1;
+                    if (lead) mbar_expect_tx(full_bar(stage), second ? 2 * tx : tx);
+                    if constexpr (kPair) tma_load_2d_pair(dst, &map_b, bar, c0, n0);
+                    else                 tma_load_2d(dst, &map_b, bar, c0, n0);
                     if (++stage == p.num_stages) { stage = 0; phase ^= 1u; }
-                    c0 += p.bk_elems;
-                    if (++chunk == p.chunks_per_tap) { chunk = 0; tap_c += p.cin_pad; c0 = tap_c; }
+                    auto advance = [&]() {
+                        c0 += p.bk_elems;
+                        if (++chunk == p.chunks_per_tap) { chunk = 0; tap_c += p.cin_pad; c0 = tap_c; }
+                    };
+                    advance();
+                    if constexpr (kBlocks == 2) { if (second) { tma_load_2d(dst + b_bytes, &map_b, bar, c0, n0); advance(); } }
                 }
             }
         }
@@ -586,7 +604,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             int stage = 0; uint32_t phase = 0;
             bool ok = true;
             const uint64_t desc_a0 = make_smem_desc(a_base, p.bk_bytes), desc_b0 = make_smem_desc(b_base, p.bk_bytes);
-            const uint64_t a_step = a_bytes >> 4, b_step = b_bytes >> 4;   // one stage, in descriptor units
+            const uint64_t a_step = a_bytes >> 4, b_step = b_bytes >> 4;   // one k-block, in descriptor units
             const uint64_t sub_step = sub_bytes >> 4;                      // next sub-tile of A
             uint64_t da = desc_a0, db = desc_b0;
             for (int tl = 0; tl < nseg && ok; ++tl) {     // tl: segments this CTA has started
@@ -602,7 +620,7 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                 // straight-line code per k-block (4, 2 or 1 MMAs per sub-tile, each 32 bytes of K per row)
                 auto k_blocks = [&](auto mmas) {
                     int share = 1, share_end = seg_k / shares;
-                    for (int kt = 0; kt < seg_k; ++kt) {
+                    for (int kt = 0; kt < seg_k; kt += kBlocks) {
                         if (kShares && kt == share_end) {            // the next share of k has an accumulator of its own
                             tmem_d += static_cast<uint32_t>(m_mult * p.bn); accumulate = 0;
                             share_end = seg_k * ++share / shares;
@@ -623,9 +641,18 @@ conv_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                             }
                         }
                         accumulate = 1;
+                        if constexpr (kBlocks == 2) {
+                            if (kt + 1 < seg_k) {                    // (an odd number of k-blocks ends in half a stage)
+#pragma unroll
+                                for (int k = 0; k < decltype(mmas)::value; ++k) {
+#pragma unroll
+                                    for (int j = 0; j < m_mult; ++j) tcgen05_mma<kTf32>(tmem_d + static_cast<uint32_t>(j * p.bn), da + a_step + j * sub_step + 2 * k, db + b_step + 2 * k, p.idesc, 1u);
+                                }
+                            }
+                        }
                         if constexpr (kPair) tcgen05_commit_pair(empty_bar(stage));   // frees the stage in both CTAs
                         else                 tcgen05_commit(empty_bar(stage));        // frees the stage when these MMAs retire
-                        da += a_step; db += b_step;
+                        da += kBlocks * a_step; db += kBlocks * b_step;
                         if (++stage == p.num_stages) { stage = 0; phase ^= 1u; da = desc_a0; db = desc_b0; }
                     }
                 };

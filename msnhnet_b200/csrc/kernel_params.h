@@ -57,6 +57,7 @@ struct ConvUmmaParams {
     int bk_bytes;         // bytes of one A/B row per k-block: 128, 64 or 32 (= the swizzle span)
     int bk_elems;         // bk_bytes / sizeof(element)
     int num_stages;
+    int stage_blocks;     // k-blocks a stage holds (2: k-split kernels with room for three such stages)
     int a_mode;
     // k loop
     int taps, kh, kw;     // taps = kh*kw

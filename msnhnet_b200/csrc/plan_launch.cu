@@ -24,7 +24,8 @@ template <typename T> const void *umma_kernel(const Launch &L) {
                                          : reinterpret_cast<const void *>(conv_umma_kernel<T, 1, false, true>);
     if (u.pair) return reinterpret_cast<const void *>(conv_umma_kernel<T, 1, true, false>);
     if constexpr (sizeof(T) == 4) {
-        if (u.k_split > 1) return reinterpret_cast<const void *>(conv_umma_kernel<T, 1, false, false, kActGeneric, false, true>);
+        if (u.k_split > 1) return u.stage_blocks == 2 ? reinterpret_cast<const void *>(conv_umma_kernel<T, 1, false, false, kActGeneric, false, true, false, 2>)
+                                                      : reinterpret_cast<const void *>(conv_umma_kernel<T, 1, false, false, kActGeneric, false, true>);
         if (u.k_shares > 1) {
             if (u.m_mult == 4) return reinterpret_cast<const void *>(conv_umma_kernel<T, 4, false, false, kActGeneric, false, false, true>);
             if (u.m_mult == 3) return reinterpret_cast<const void *>(conv_umma_kernel<T, 3, false, false, kActGeneric, false, false, true>);

@@ -472,8 +472,9 @@ int configure_conv_umma(MsnhB200Plan *pl, TileTuning &tt, Launch &L) {
     u.tmem_cols = cols;
     const int b_rows = u.pair ? u.bn / 2 : u.bn;                     // weight rows one CTA stages
     const size_t stage = static_cast<size_t>(kUmmaM * u.m_mult + b_rows) * u.bk_bytes;
-    u.num_stages = static_cast<int>(std::min<size_t>(kUmmaMaxStages, budget / stage));
-    L.smem = u.num_stages * stage + fixed;
+    u.stage_blocks = u.k_split > 1 && budget / (2 * stage) >= 3 ? 2 : 1;
+    u.num_stages = static_cast<int>(std::min<size_t>(kUmmaMaxStages / u.stage_blocks, budget / (u.stage_blocks * stage)));
+    L.smem = u.num_stages * u.stage_blocks * stage + fixed;
     L.grid = u.pair ? 2 * std::min(u.tiles_m * u.tiles_n, ctx->sm_count / 2) : u.k_split > 1 ? u.tiles_m * u.tiles_n * u.k_split : std::min(u.tiles_m * u.tiles_n, ctx->sm_count);
     u.out = L.out.ptr; u.ldc_out = L.out.ldc;
     u.sk_ws = nullptr; u.sk_flags = nullptr;
