@@ -86,17 +86,20 @@ __device__ __forceinline__ void tmem_ld_columns(uint32_t taddr, uint32_t (&r)[N]
 template <int kBn, int kThreads, int kBatch>
 struct SplitFinish {
     static constexpr int kQuads = kBn / 4, kRows = kThreads / kQuads;
-    int row, col, c;
+    int row, col, c, cout;
+    const TView &out;
     float4 sc, bi;
     bool live;
-    __device__ __forceinline__ SplitFinish(const ConvSplitParams &p, int n0, int t) : row(t / kQuads), col(4 * (t % kQuads)), c(n0 + col), live(t < kRows * kQuads && c < p.cout) {
+    __device__ __forceinline__ SplitFinish(const ConvSplitParams &p, const TView &out1, const TView &out2, int n0, int t)
+        : row(t / kQuads), col(4 * (t % kQuads)), c(n0 + col), cout(n0 < p.split_n ? p.split_n : p.cout), out(n0 < p.split_n ? out1 : out2), live(t < kRows * kQuads && c < cout) {
         if (live) { sc = __ldg(reinterpret_cast<const float4 *>(p.scale + c)); bi = __ldg(reinterpret_cast<const float4 *>(p.bias + c)); }   // (padded past the last channel tile)
     }
     template <typename Sum>
-    __device__ __forceinline__ void operator()(const ConvSplitParams &p, const TView &out, int m0, int row0, int step, Sum &&sum) const {
+    __device__ __forceinline__ void operator()(const ConvSplitParams &p, int m0, int row0, int step, Sum &&sum) const {
         if (!live) return;
         const int rows = min(kUmmaM, p.m_total - m0);
-        const bool whole = c + 4 <= p.cout;
+        const bool whole = c + 4 <= cout;
+        float *const dst0 = static_cast<float *>(out.ptr) + (c < p.split_n ? c : c - p.split_n);
         for (int j = row0 + row * step; j < rows; j += kBatch * kRows * step) {
             float y[4 * kBatch], rr[4 * kBatch];
 #pragma unroll
@@ -110,7 +113,7 @@ struct SplitFinish {
                         rr[4 * q] = t.x; rr[4 * q + 1] = t.y; rr[4 * q + 2] = t.z; rr[4 * q + 3] = t.w;
                     } else {
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) rr[4 * q + e] = c + e < p.cout ? rp[e] : 0.f;
+                        for (int e = 0; e < 4; ++e) rr[4 * q + e] = c + e < cout ? rp[e] : 0.f;
                     }
                 }
             }
@@ -126,11 +129,11 @@ struct SplitFinish {
             for (int q = 0; q < kBatch; ++q) {
                 const int r = j + q * kRows * step;
                 if (r >= rows) break;
-                float *dst = static_cast<float *>(out.ptr) + static_cast<size_t>(m0 + r) * out.ldc + c;
+                float *dst = dst0 + static_cast<size_t>(m0 + r) * out.ldc;
                 if (whole) *reinterpret_cast<float4 *>(dst) = make_float4(y[4 * q], y[4 * q + 1], y[4 * q + 2], y[4 * q + 3]);
                 else {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) if (c + e < p.cout) dst[e] = y[4 * q + e];
+                    for (int e = 0; e < 4; ++e) if (c + e < cout) dst[e] = y[4 * q + e];
                 }
             }
         }
@@ -152,7 +155,7 @@ struct SplitFinish {
 
 template <int kBn, bool kSplit>
 __global__ void __launch_bounds__(kSpThreads, 1)
-conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TView out, const ConvSplitParams p) {
+conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ TView out, const __grid_constant__ TView out2, const __grid_constant__ ConvSplitParams p) {
     constexpr int kCols = kBn / 4;                                   // channels of a pixel an adding thread holds
     constexpr int kPitch = kBn + 4;                                  // floats of a row of the tile of sums
     constexpr uint32_t kABytes = kUmmaM * 128, kBBytes = 2 * kBn * 128;
@@ -374,7 +377,7 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             for (int c = 0; c < kCols; ++c) asm volatile("" : "+r"(v[c]));      // (no use of them moves up past the wait)
         };
         for (int tile = first_tile; tile < num_tiles && ok; tile += tile_stride) {
-            const SplitFinish<kBn, 512, 4> finish(p, tile % p.tiles_n * kBn, t);
+            const SplitFinish<kBn, 512, 4> finish(p, out, out2, tile % p.tiles_n * kBn, t);
             for (int share = share_first; share < share_end && ok; ++share) {
                 const int k0 = num_k * share / p.shares, k1 = num_k * (share + 1) / p.shares;
                 float acc[kCols];
@@ -435,7 +438,7 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 ok = all_ok != 0;
                 if (!ok) break;
                 if (p.res) pdl_wait();                               // the residual is an earlier kernel's output
-                finish(p, out, tile / p.tiles_n * kUmmaM, 0, 1, [&](uint32_t at, float *y) {
+                finish(p, tile / p.tiles_n * kUmmaM, 0, 1, [&](uint32_t at, float *y) {
                     asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(y[0]), "=f"(y[1]), "=f"(y[2]), "=f"(y[3]) : "r"(sum_base + at) : "memory");
                 });
                 asm volatile("bar.sync 1, 512;" ::: "memory");        // the tile of sums is free for the next tile
@@ -446,11 +449,11 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     tcgen05_fence_before();
     __syncthreads();
     if constexpr (kSplit) {
-        const SplitFinish<kBn, kSpThreads, 1> finish(p, first_tile % p.tiles_n * kBn, static_cast<int>(threadIdx.x));
+        const SplitFinish<kBn, kSpThreads, 1> finish(p, out, out2, first_tile % p.tiles_n * kBn, static_cast<int>(threadIdx.x));
         cluster_sync_all();          // every share of the tile is in some CTA's shared memory
         if (*cta_abort == 0) {
             if (p.res) pdl_wait();
-            finish(p, out, first_tile / p.tiles_n * kUmmaM, rank, p.shares, [&](uint32_t at, float *y) {
+            finish(p, first_tile / p.tiles_n * kUmmaM, rank, p.shares, [&](uint32_t at, float *y) {
 #pragma unroll
                 for (int q = 0; q < kUmmaMaxKSplit; ++q)
                     if (q < p.shares) {

@@ -97,6 +97,7 @@ constexpr uint32_t kSpSlots = 3, kSpRing = 6;          // split activations in T
 static_assert(kSpAStages % 2 == 0 && kSpRing % 2 == 0, "a stage belongs to one group of splitting warps");
 struct ConvSplitParams {
     int m_total, cout, tiles_m, tiles_n;
+    int split_n;          // two 1x1 convs over the same input in one launch: channels from split_n on (a multiple of the tile) are the second one's
     int shares;           // the k of a tile is summed in this many shares, added in their order
     int a_mode;
     int taps, kw, chunks_per_tap, cin_pad, dil_h, dil_w;
@@ -109,6 +110,8 @@ struct ConvSplitParams {
     int act1; float act1_param; int act2; float act2_param;
     int *err_flag;
 };
+// channels of a tile: up to 64 (what TMEM holds beside three slots of split activations), evenly wide
+constexpr int split_tile_channels(int cout) { return ((cout + (cout + 63) / 64 - 1) / ((cout + 63) / 64) + 15) / 16 * 16; }
 constexpr size_t split_smem_bytes(int bn) {
     return 1024 + kSpAStages * kUmmaM * 128 + kSpBStages * 2 * bn * 128 + static_cast<size_t>(kUmmaM) * (bn + 4) * 4 + 512;
 }

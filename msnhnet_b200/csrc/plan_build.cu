@@ -689,7 +689,7 @@ int build_launches(MsnhB200Plan *pl) {
         const int slab_cols = 128 / es;
         auto off_of = [](const void *tagged) { return static_cast<size_t>(reinterpret_cast<uintptr_t>(tagged) & (kPackTag - 1)); };
         auto plain_1x1 = [&](const Pending &q) {
-            return q.L.kind == L_CONV_UMMA && q.L.op != patch_op && q.L.op >= 0 && pl->ops[q.L.op].d.kind == MSNH_OP_CONV && q.L.note.empty() && q.L.kh == 1 && q.L.kw == 1 &&
+            return (q.L.kind == L_CONV_UMMA || q.L.kind == L_CONV_SPLIT) && q.L.op != patch_op && q.L.op >= 0 && pl->ops[q.L.op].d.kind == MSNH_OP_CONV && q.L.note.empty() && q.L.kh == 1 && q.L.kw == 1 &&
                    q.L.sh == 1 && q.L.sw == 1 && q.L.ph == 0 && q.L.pw == 0 && q.L.groups == 1 && q.res_t < 0 && q.out2_t < 0 && q.c_sub < 0 && q.L.act2 == MSNH_ACT_NONE;
         };
         auto same_data = [&](int t0, int t1) {
@@ -700,20 +700,24 @@ int build_launches(MsnhB200Plan *pl) {
         for (size_t i = 0; i < pend.size(); ++i) {
             if (!plain_1x1(pend[i])) continue;
             const int ca = pl->tensors[pend[i].out_t].s.C;
-            if (ca % slab_cols) continue;                     // the second conv's channels start on a store slab
+            const bool split = pend[i].L.kind == L_CONV_SPLIT;
+            if (ca % (split ? split_tile_channels(ca) : slab_cols)) continue;      // the second conv's channels start on a store slab (split operands: on a tile)
             for (size_t j = i + 1; j < pend.size(); ++j) {
                 const Pending &b = pend[j];
                 Pending &a = pend[i];
-                if (!plain_1x1(b) || !same_data(a.in_t, b.in_t) || b.out_t == a.out_t || b.L.act1 != a.L.act1 || b.L.act1_p != a.L.act1_p ||
+                if (!plain_1x1(b) || b.L.kind != a.L.kind || !same_data(a.in_t, b.in_t) || b.out_t == a.out_t || b.L.act1 != a.L.act1 || b.L.act1_p != a.L.act1_p ||
                     b.L.cin_pad != a.L.cin_pad) continue;
                 const int cb = pl->tensors[b.out_t].s.C;
                 const size_t row_bytes = static_cast<size_t>(a.L.cin_pad) * es;
                 const size_t wa = off_of(a.L.weights), wb = off_of(b.L.weights), sa = off_of(a.L.scale), sb = off_of(b.L.scale), ba = off_of(a.L.bias), bb = off_of(b.L.bias);
-                PackSlot<uint8_t> ws = reserve_pack<uint8_t>(pl, (static_cast<size_t>(ca) + cb) * row_bytes);
-                if (ws.host) {       // (nullptr: the arena comes from a pack file, which holds the merged copy at this offset)
-                    std::memcpy(ws.host, pl->pack_host.data() + wa, ca * row_bytes);
-                    std::memcpy(ws.host + ca * row_bytes, pl->pack_host.data() + wb, cb * row_bytes);
-                }
+                const int parts = split ? 2 : 1;              // (split operands: two matrices, one behind the other)
+                PackSlot<uint8_t> ws = reserve_pack<uint8_t>(pl, parts * (static_cast<size_t>(ca) + cb) * row_bytes);
+                if (ws.host)         // (nullptr: the arena comes from a pack file, which holds the merged copy at this offset)
+                    for (int k = 0; k < parts; ++k) {
+                        uint8_t *to = ws.host + k * (static_cast<size_t>(ca) + cb) * row_bytes;
+                        std::memcpy(to, pl->pack_host.data() + wa + k * ca * row_bytes, ca * row_bytes);
+                        std::memcpy(to + ca * row_bytes, pl->pack_host.data() + wb + k * cb * row_bytes, cb * row_bytes);
+                    }
                 std::vector<float> sc(round_up(ca + cb, 256) + 64, 1.f), bi(round_up(ca + cb, 256) + 64, 0.f);
                 if (!pl->pack_loaded) {
                     const uint8_t *base = pl->pack_host.data();
@@ -902,7 +906,7 @@ int build_launches(MsnhB200Plan *pl) {
         }
         if (L.kind == L_CONV_UMMA) { const int rc = configure_conv_umma(pl, tt, L); if (rc) return rc; }
         if (L.kind == L_CONV_SPLIT) {
-            if (!aligned(L.in) || !aligned(L.out) || (L.res && (reinterpret_cast<uintptr_t>(L.res) % 16 || L.ldc_res % V)))
+            if (!aligned(L.in) || !aligned(L.out) || !aligned(L.out2) || (L.res && (reinterpret_cast<uintptr_t>(L.res) % 16 || L.ldc_res % V)))
                 return fail(ctx, MSNH_B200_ERR_STATE, "fp32 conv of op %d landed on an unaligned view", L.op);
             const int rc = configure_conv_split(pl, L);
             if (rc) return rc;

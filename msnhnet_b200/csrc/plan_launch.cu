@@ -226,7 +226,7 @@ void launch_typed(MsnhB200Ctx *ctx, const Launch &L, cudaStream_t st) {
             if (L.sp_split > 1) { attr[na].id = cudaLaunchAttributeClusterDimension; attr[na].val.clusterDim.x = L.sp_split; attr[na].val.clusterDim.y = 1; attr[na].val.clusterDim.z = 1; ++na; }
             if (ctx->pdl) { attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization; attr[na].val.programmaticStreamSerializationAllowed = 1; ++na; }
             cfg.attrs = attr; cfg.numAttrs = na;
-            void *args[4] = {const_cast<CUtensorMap *>(&L.map_a), const_cast<CUtensorMap *>(&L.map_b), const_cast<TView *>(&L.out), const_cast<ConvSplitParams *>(&L.sp)};
+            void *args[5] = {const_cast<CUtensorMap *>(&L.map_a), const_cast<CUtensorMap *>(&L.map_b), const_cast<TView *>(&L.out), const_cast<TView *>(&L.out2), const_cast<ConvSplitParams *>(&L.sp)};
             cudaLaunchKernelExC(&cfg, split_kernel(L.sp_bn, L.sp_split > 1), args);
             break;
         }

@@ -161,11 +161,10 @@ void configure_conv_fp32(MsnhB200Plan *pl, Launch &L) {
 int configure_conv_split(MsnhB200Plan *pl, Launch &L) {
     MsnhB200Ctx *ctx = pl->ctx;
     ConvSplitParams &u = L.sp;
-    const int cin = L.in.C, cout = L.out.C;
-    u.m_total = L.out.N * L.out.H * L.out.W; u.cout = cout;
-    // tiles of up to 64 channels (what TMEM holds beside four slots of split activations), evenly wide
-    u.tiles_n = (cout + 63) / 64;
-    L.sp_bn = round_up((cout + u.tiles_n - 1) / u.tiles_n, 16);
+    const int cin = L.in.C, cout = L.out.C + (L.out2.ptr ? L.out2.C : 0);   // (two merged convs: both channel ranges)
+    u.m_total = L.out.N * L.out.H * L.out.W; u.cout = cout; u.split_n = L.out2.ptr ? L.split_n : cout;
+    L.sp_bn = split_tile_channels(L.out.C);                                  // (merged convs: the first one's, which its channels are a multiple of)
+    u.tiles_n = (cout + L.sp_bn - 1) / L.sp_bn;
     u.tiles_m = (u.m_total + kUmmaM - 1) / kUmmaM;
     u.taps = L.kh * L.kw; u.kw = L.kw;
     // What an accumulator loses to truncation shows beside the FMA chain it replaces where k is very short (norm error against 64 bits,

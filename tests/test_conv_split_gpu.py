@@ -106,6 +106,34 @@ def test_values_that_are_not_finite_go_where_fp32_takes_them(shares, monkeypatch
     assert np.all(np.abs(got[fine] - want[fine]) <= 1e-5 * np.maximum(np.abs(want[fine]), 1))
 
 
+@pytest.mark.parametrize("ca,cb", [(48, 48), (96, 33), (64, 255), (192, 192)])
+def test_two_1x1_convs_over_one_input_in_one_launch(ca, cb, monkeypatch):
+    x, wa, bias = tensors(40, ca, 13, 17, 1, 3)
+    wb = tensors(40, cb, 1, 1, 1, 1, seed=9)[1]
+    out = {}
+    for merge in (True, False):
+        monkeypatch.setenv("MSNH_B200_CONV_SPLIT", "1")
+        if merge:
+            monkeypatch.delenv("MSNH_B200_NO_MERGE", raising=False)
+        else:
+            monkeypatch.setenv("MSNH_B200_NO_MERGE", "1")
+        ctx = ffi.Context(0)
+        plan = ffi.Plan(ctx, [ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=ca, act=ffi.ACT_LEAKY, act_param=0.1, is_output=1),
+                              ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=cb, act=ffi.ACT_LEAKY, act_param=0.1, is_output=1)], (40, 13, 17), 3, ffi.F32, ffi.PLAN_NO_TENSOR_CORE)
+        try:
+            plan.set_weights(0, ffi.W_WEIGHTS, wa)
+            plan.set_weights(1, ffi.W_WEIGHTS, wb)
+            plan.finalize()
+            assert ("with the 1x1 conv of op 1" in plan.describe()) == merge
+            plan.run(x)
+            out[merge] = [plan.read_output(i, 3) for i in (0, 1)]
+        finally:
+            plan.close()
+            ctx.close()
+    for a, b in zip(out[True], out[False]):
+        assert np.array_equal(a, b)
+
+
 def test_runs_of_many_layers_agree_bit_for_bit(monkeypatch):
     """A chain of convs of every tile width, run again and again: what one warp hands another must not depend on timing."""
     monkeypatch.setenv("MSNH_B200_CONV_SPLIT", "3")
