@@ -16,6 +16,10 @@ namespace msnh {
 // is accumulated over one k-block at a time (32 values of k, four tensor-core steps) and the k-blocks are added up in registers
 // with ordinary rounded additions; the two small products, 2^-11 of the large one, stay in an accumulator of their own
 // over the whole share of k.
+// What truncation takes from a k-block's sum is random but for its mean, which is towards zero: a gain a little below one, 3.7e-8 for one step, 8.9e-8
+// for four, the same whatever the layer. Layers upon layers would all lose it, so the sums of a share are multiplied by 1 + p.gain, which
+// leaves +-4e-9 (slope of the result over the sums in 64 bits). Without it the boxes of YOLOv5m-352 were 6e-5 from those of fp32 FMAs (median of
+// 72 images), with it 4.5e-6; two orders of the FMAs differ by 2.8e-6.
 // (inf and NaN: x1 of an infinite x is NaN, so where the large sum is not finite it is the result and the small one is dropped.)
 //
 // Roles of the 28 warps, connected by rings of mbarriers. A wait costs a single thread some 170 cycles even where it passes, so the
@@ -39,7 +43,7 @@ namespace msnh {
 // and sums a tile's shares one after the other.
 //
 // Measured against fp32 FMAs on the CUDA cores (conv_fp32_kernel), a forward in us: YOLOv3-tiny-416, one image 431 -> 207 and sixteen
-// 3965 -> 1490; YOLOv5m-352, three images 2889 -> 1407; YOLOv5m-640, two 4604 -> 1925. Norm error against 64 bits, FMAs / here: 64 values
+// 3965 -> 1490; YOLOv5m-352, three images 2889 -> 1209; YOLOv5m-640, two 4604 -> 1785. Norm error against 64 bits, FMAs / here: 64 values
 // of k 1.44e-7 / 1.28e-7, 288 1.54e-7 / 1.46e-7, 2304 3.8e-7 / 2.0e-7, 4608 4.3e-7 / 2.5e-7 (one share; less in several). A k-block takes 550-650 cycles: its 12
 // MMAs 300 (48 channels) to 400 (64), the rest is the way of a slot round the roles (split, MMA, commit, sums read, some 1800 cycles
 // for three k-blocks). With one MMA thread it took 780, with eight adding warps the end of a tile 2600 cycles (now half), with
@@ -119,7 +123,7 @@ struct SplitFinish {
             }
 #pragma unroll
             for (int q = 0; q < 4 * kBatch; q += 4) { y[q] = fmaf(y[q], sc.x, bi.x); y[q + 1] = fmaf(y[q + 1], sc.y, bi.y); y[q + 2] = fmaf(y[q + 2], sc.z, bi.z); y[q + 3] = fmaf(y[q + 3], sc.w, bi.w); }
-            activate_all(y, p.act1, p.act1_param);
+            activate_all(y, c < p.split_n ? p.act1 : p.act1_b, c < p.split_n ? p.act1_param : p.act1_b_param);
             if (p.res) {
 #pragma unroll
                 for (int q = 0; q < 4 * kBatch; ++q) y[q] = __fadd_rn(y[q], rr[q]);
@@ -413,7 +417,7 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 #pragma unroll
                 for (int c = 0; c < kCols; ++c) {
                     asm volatile("" : "+r"(w[c]));
-                    if ((__float_as_uint(acc[c]) & 0x7f800000u) != 0x7f800000u) acc[c] = __fadd_rn(acc[c], __fadd_rn(__uint_as_float(v[c]), __uint_as_float(w[c])));
+                    if ((__float_as_uint(acc[c]) & 0x7f800000u) != 0x7f800000u) acc[c] = __fadd_rn(acc[c], __fmaf_rn(acc[c], p.gain, __fadd_rn(__uint_as_float(v[c]), __uint_as_float(w[c]))));
                 }
                 tcgen05_fence_before();
                 __syncwarp();

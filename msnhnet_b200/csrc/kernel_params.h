@@ -104,10 +104,12 @@ struct ConvSplitParams {
     int chunk_elems, chunk_steps;   // channels of a k-block (32, fewer where the whole k is short) and the tensor-core steps they take (8 values of k each)
     int tail_steps;       // steps of a tap's last k-block
     int all_products;     // x1 w1 too
+    float gain;           // what the accumulators' truncation takes from the large products on average, relative
     int oh, ow, stride_h, stride_w, pad_h, pad_w;
     const void *res; int ldc_res;
     const float *scale, *bias;
     int act1; float act1_param; int act2; float act2_param;
+    int act1_b; float act1_b_param;   // activation of the second of two merged convs
     int *err_flag;
 };
 // channels of a tile: up to 64 (what TMEM holds beside three slots of split activations), evenly wide

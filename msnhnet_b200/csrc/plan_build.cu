@@ -705,7 +705,7 @@ int build_launches(MsnhB200Plan *pl) {
             for (size_t j = i + 1; j < pend.size(); ++j) {
                 const Pending &b = pend[j];
                 Pending &a = pend[i];
-                if (!plain_1x1(b) || b.L.kind != a.L.kind || !same_data(a.in_t, b.in_t) || b.out_t == a.out_t || b.L.act1 != a.L.act1 || b.L.act1_p != a.L.act1_p ||
+                if (!plain_1x1(b) || b.L.kind != a.L.kind || !same_data(a.in_t, b.in_t) || b.out_t == a.out_t || (!split && (b.L.act1 != a.L.act1 || b.L.act1_p != a.L.act1_p)) ||
                     b.L.cin_pad != a.L.cin_pad) continue;
                 const int cb = pl->tensors[b.out_t].s.C;
                 const size_t row_bytes = static_cast<size_t>(a.L.cin_pad) * es;
@@ -728,6 +728,7 @@ int build_launches(MsnhB200Plan *pl) {
                 a.L.scale = static_cast<const float *>(upload(pl, sc));
                 a.L.bias = static_cast<const float *>(upload(pl, bi));
                 a.out2_t = b.out_t; a.L.split_n = ca;
+                a.L.act_mid = b.L.act1; a.L.act_mid_p = b.L.act1_p;
                 const Shape is = pl->tensors[a.in_t].s;
                 a.L.flops += b.L.flops;
                 a.L.bytes += b.L.bytes - static_cast<double>(is.C) * is.H * is.W * pl->batch * es;

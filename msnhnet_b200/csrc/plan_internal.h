@@ -155,7 +155,7 @@ struct Launch {
     // umma
     CUtensorMap map_a, map_b, map_c, map_c2, map_res;
     TView out2{};              // second output of two 1x1 convs over the same input merged into this launch (ptr == nullptr: none)
-    int split_n = 0;           // its first channel in the merged channel range
+    int split_n = 0;           // its first channel in the merged channel range (split operands: act_mid is its activation)
     ConvUmmaParams up{};
     ConvSplitParams sp{}; int sp_bn = 0, sp_split = 1;   // L_CONV_SPLIT: channels of a tile; CTAs of a cluster its shares are spread over
     int grid = 0; size_t smem = 0;

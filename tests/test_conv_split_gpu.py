@@ -119,7 +119,7 @@ def test_two_1x1_convs_over_one_input_in_one_launch(ca, cb, monkeypatch):
             monkeypatch.setenv("MSNH_B200_NO_MERGE", "1")
         ctx = ffi.Context(0)
         plan = ffi.Plan(ctx, [ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=ca, act=ffi.ACT_LEAKY, act_param=0.1, is_output=1),
-                              ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=cb, act=ffi.ACT_LEAKY, act_param=0.1, is_output=1)], (40, 13, 17), 3, ffi.F32, ffi.PLAN_NO_TENSOR_CORE)
+                              ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=cb, act=ffi.ACT_HARD_SWISH, is_output=1)], (40, 13, 17), 3, ffi.F32, ffi.PLAN_NO_TENSOR_CORE)
         try:
             plan.set_weights(0, ffi.W_WEIGHTS, wa)
             plan.set_weights(1, ffi.W_WEIGHTS, wb)
