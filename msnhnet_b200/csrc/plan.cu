@@ -337,11 +337,17 @@ int msnh_b200_plan_set_weights(MsnhB200Plan *pl, int op, int slot, const float *
     return MSNH_B200_OK;
 } catch (...) { return caught(pl ? pl->ctx : nullptr); }
 
+// The debug switches as they stand now. MSNH_B200_CONV_SPLIT takes any fp32 plan that may use the tensor cores to the split-operand convs.
+static void read_debug_options(MsnhB200Plan *pl) {
+    pl->dbg = PlanDebugOptions::from_env();
+    if (pl->dbg.conv_split && pl->dtype == MSNH_B200_F32 && !(pl->flags & MSNH_PLAN_NO_TENSOR_CORE)) { pl->split_fp32 = true; pl->flags |= MSNH_PLAN_NO_TENSOR_CORE; }
+}
+
 int msnh_b200_plan_use_pack(MsnhB200Plan *pl, const char *path, uint64_t weights_tag, int *usable) try {
     if (!pl || !path || !*path) return MSNH_B200_ERR_ARG;
     if (pl->finalized) return fail(pl->ctx, MSNH_B200_ERR_STATE, "use_pack after finalize");
     pl->pack_path = path; pl->pack_tag = weights_tag;
-    pl->dbg = PlanDebugOptions::from_env();
+    read_debug_options(pl);
     if (usable) *usable = pack_probe(pl) ? 1 : 0;
     return MSNH_B200_OK;
 } catch (...) { return caught(pl ? pl->ctx : nullptr); }
@@ -375,7 +381,7 @@ int msnh_b200_plan_finalize(MsnhB200Plan *pl) try {
     if (pl->finalized) return fail(ctx, MSNH_B200_ERR_STATE, "finalize called twice");
     if (pl->finalize_failed) return fail(ctx, MSNH_B200_ERR_STATE, "an earlier finalize of this plan failed: destroy it and build a new one");
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
-    pl->dbg = PlanDebugOptions::from_env();
+    read_debug_options(pl);
     int rc = build_launches(pl);
     if (rc) {
         // weights that were merely missing can still be set; anything later leaves half-built state behind

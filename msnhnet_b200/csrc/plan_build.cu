@@ -228,7 +228,7 @@ int build_launches(MsnhB200Plan *pl) {
     // few channels that per-tap im2col loads would move 6 useful bytes per 32-byte row.
     int patch_op = -1, patch_k = 0;
     bool row_patches = false;
-    if (!no_fusion && (!(pl->flags & MSNH_PLAN_NO_TENSOR_CORE) || splits_fp32(pl))) {
+    if (!no_fusion && (!(pl->flags & MSNH_PLAN_NO_TENSOR_CORE) || pl->split_fp32)) {
         int users = 0, user = -1;
         for (int i = 0; i < n_ops; ++i) for (int k = 0; k < pl->ops[i].d.n_in; ++k) if (pl->ops[i].d.in[k] == MSNH_B200_INPUT) { ++users; user = i; }
         if (users == 1 && pl->ops[user].d.kind == MSNH_OP_CONV && pl->ops[user].d.groups == 1 && pl->ops[user].absorbed_into < 0 &&
@@ -241,7 +241,7 @@ int build_launches(MsnhB200Plan *pl) {
         // input row and output column, the kw pixels that the filter's rows cover there, and the conv runs as kh x 1 over those, one
         // k-block a filter row. Tap by tap the stem of ResNet-18 fp32 was 49 k-blocks of three useful values: a forward with 32
         // images 641 -> 524 us, with one 159 -> 153.
-        else if (users == 1 && pl->ops[user].d.kind == MSNH_OP_CONV && pl->ops[user].d.groups == 1 && pl->ops[user].absorbed_into < 0 && !splits_fp32(pl) &&
+        else if (users == 1 && pl->ops[user].d.kind == MSNH_OP_CONV && pl->ops[user].d.groups == 1 && pl->ops[user].absorbed_into < 0 && !pl->split_fp32 &&
                  pl->ops[user].d.k_w > 1 && pl->ops[user].d.dil_w == 1 && pl->in_c <= 4 && pl->in_c * pl->ops[user].d.k_w <= 64 &&
                  row_patch_smem(pl->in_c, pl->in_w, pl->ops[user].d.k_w, pl->ops[user].d.pad_w, pl->ops[user].d.stride_w, pl->ops[user].out.W) <= 48 * 1024) {
             patch_op = user; row_patches = true;
@@ -447,7 +447,7 @@ int build_launches(MsnhB200Plan *pl) {
                         p.L.weights = ps.dev;
                     } else {
                         // split operands: the matrix of the nearest tf32 values and, behind it, that of what they leave
-                        split = splits_fp32(pl) && tma_walks && aligned_view(in0) && aligned_view(o.tensor) && (p.res_t < 0 || aligned_view(p.res_t));
+                        split = pl->split_fp32 && tma_walks && aligned_view(in0) && aligned_view(o.tensor) && (p.res_t < 0 || aligned_view(p.res_t));
                         PackSlot<float> ps = reserve_pack<float>(pl, split ? 2 * n : n);
                         float *pk = ps.host;
                         const bool tc = groups == 1 && !(pl->flags & MSNH_PLAN_NO_TENSOR_CORE);

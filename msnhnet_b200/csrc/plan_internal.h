@@ -201,7 +201,8 @@ struct MsnhB200Plan {
     MsnhB200Ctx *ctx = nullptr;
     int in_c = 0, in_h = 0, in_w = 0, batch = 0, dtype = 0;
     uint32_t flags = 0;
-    bool split_fp32 = false;                        // convs in fp32 arithmetic on the tensor cores (conv_split.cuh) where they can
+    bool split_fp32 = false;                        // convs in fp32 arithmetic on the tensor cores (conv_split.cuh) where they can: the default of
+                                                    // fp32 detection nets. Never where the caller asked for MSNH_PLAN_NO_TENSOR_CORE
     msnh::PlanDebugOptions dbg;                     // the debug switches as they stood when plan_finalize began
     std::vector<msnh::OpState> ops;
     std::vector<msnh::Tensor> tensors;
@@ -265,8 +266,6 @@ struct MsnhB200Plan {
 
 namespace msnh {
 
-// fp32 convs on split operands (conv_split.cuh): the default of detection nets
-inline bool splits_fp32(const MsnhB200Plan *pl) { return pl->dtype == MSNH_B200_F32 && (pl->flags & MSNH_PLAN_NO_TENSOR_CORE) && (pl->split_fp32 || pl->dbg.conv_split != 0); }
 inline int esize(int dtype) { return dtype == MSNH_B200_F16 ? 2 : 4; }
 inline int vec_of(int dtype) { return dtype == MSNH_B200_F16 ? 8 : 4; }
 inline int round_up(int x, int m) { return (x + m - 1) / m * m; }

@@ -19,8 +19,7 @@ def test_results_are_no_smaller_than_the_sums(cin, k, shares, monkeypatch):
     x = rng.standard_normal((1, cin, size, size), dtype=np.float32)
     wt = (rng.standard_normal((cout, cin, k, k)) / np.sqrt(cin * k * k)).astype(np.float32)
     ctx = ffi.Context(0)
-    plan = ffi.Plan(ctx, [ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=cout, k_h=k, k_w=k, pad_h=k // 2, pad_w=k // 2, is_output=1)], (cin, size, size), 1, ffi.F32,
-                    ffi.PLAN_NO_TENSOR_CORE)
+    plan = ffi.Plan(ctx, [ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=cout, k_h=k, k_w=k, pad_h=k // 2, pad_w=k // 2, is_output=1)], (cin, size, size), 1, ffi.F32, 0)
     try:
         plan.set_weights(0, ffi.W_WEIGHTS, wt)
         plan.finalize()

@@ -28,7 +28,7 @@ def conv(x, wt, bias, stride, shares, monkeypatch, act=ffi.ACT_NONE, residual=No
     if residual is not None:
         ops.append(ffi.make_op(ffi.OP_ADD, [0, at], act=act, act_param=0.1, is_output=1))
     ctx = ffi.Context(0)
-    plan = ffi.Plan(ctx, ops, (cin, h, w), batch, ffi.F32, ffi.PLAN_NO_TENSOR_CORE)
+    plan = ffi.Plan(ctx, ops, (cin, h, w), batch, ffi.F32, ffi.PLAN_NO_TENSOR_CORE if shares is None else 0)
     try:
         plan.set_weights(at, ffi.W_WEIGHTS, wt)
         plan.set_weights(at, ffi.W_BIAS, bias)
@@ -119,7 +119,7 @@ def test_two_1x1_convs_over_one_input_in_one_launch(ca, cb, monkeypatch):
             monkeypatch.setenv("MSNH_B200_NO_MERGE", "1")
         ctx = ffi.Context(0)
         plan = ffi.Plan(ctx, [ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=ca, act=ffi.ACT_LEAKY, act_param=0.1, is_output=1),
-                              ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=cb, act=ffi.ACT_HARD_SWISH, is_output=1)], (40, 13, 17), 3, ffi.F32, ffi.PLAN_NO_TENSOR_CORE)
+                              ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=cb, act=ffi.ACT_HARD_SWISH, is_output=1)], (40, 13, 17), 3, ffi.F32, 0)
         try:
             plan.set_weights(0, ffi.W_WEIGHTS, wa)
             plan.set_weights(1, ffi.W_WEIGHTS, wb)
@@ -143,7 +143,7 @@ def test_runs_of_many_layers_agree_bit_for_bit(monkeypatch):
     for i, cout in enumerate(widths):
         ops.append(ffi.make_op(ffi.OP_CONV, [i - 1 if i else ffi.INPUT], filters=cout, k_h=3, k_w=3, pad_h=1, pad_w=1, act=ffi.ACT_LEAKY, act_param=0.1, is_output=1))
     ctx = ffi.Context(0)
-    plan = ffi.Plan(ctx, ops, (3, 52, 52), 2, ffi.F32, ffi.PLAN_NO_TENSOR_CORE)
+    plan = ffi.Plan(ctx, ops, (3, 52, 52), 2, ffi.F32, 0)
     try:
         for i, cout in enumerate(widths):
             plan.set_weights(i, ffi.W_WEIGHTS, (rng.standard_normal((cout, cin, 3, 3)) / np.sqrt(4.5 * cin)).astype(np.float32))
@@ -157,6 +157,20 @@ def test_runs_of_many_layers_agree_bit_for_bit(monkeypatch):
             want = want or got
             for i, (a, b) in enumerate(zip(got, want)):
                 assert np.array_equal(a, b), f"layer {i}"
+    finally:
+        plan.close()
+        ctx.close()
+
+
+def test_a_plan_without_tensor_cores_stays_without(monkeypatch):
+    monkeypatch.setenv("MSNH_B200_CONV_SPLIT", "2")
+    ctx = ffi.Context(0)
+    plan = ffi.Plan(ctx, [ffi.make_op(ffi.OP_CONV, [ffi.INPUT], filters=16, is_output=1)], (40, 5, 5), 1, ffi.F32, ffi.PLAN_NO_TENSOR_CORE)
+    try:
+        plan.set_weights(0, ffi.W_WEIGHTS, np.zeros((16, 40, 1, 1), np.float32))
+        plan.finalize()
+        launch = [line for line in plan.describe().splitlines() if " op=0 " in line][-1]
+        assert "conv_direct " in launch
     finally:
         plan.close()
         ctx.close()
