@@ -1,5 +1,5 @@
-// fp32 convolution on the tensor cores: every fp32 operand is split into two tf32 numbers whose sum it is to 2^-24, and a
-// product into three tensor-core products. What the fp32 plans of detection nets run (boxes decoded through exp() do not hold
+// fp32 convolution on the tensor cores: every fp32 operand is the sum of three bf16 numbers, and a product that of eight
+// tensor-core products. What the fp32 plans of detection nets run (boxes decoded through exp() do not hold
 // through tf32's 10 mantissa bits); the CUDA-core form of the same arithmetic is conv_fp32_kernel (conv_tiled.cuh). Replaces the
 // reference's im2col + cublasSgemm (src/layers/MsnhConvolutionalLayer.cpp:1026-1160).
 #pragma once
@@ -8,34 +8,32 @@
 namespace msnh {
 
 // ---------------------------------------------------------------------------------------------------------------------------
-// x = x0 + x1, w = w0 + w1, each part the nearest tf32 of what is left. x w = x0 w0 + (x0 w1 + x1 w0) + x1 w1, the last term below
-// 2^-24 and left out where k is long enough for it to drown in the rounding of the sums. Weights are split on the host, activations here.
+// x = x0 + x1 + x2 exactly: x0 the nearest number of 6 significant bits, x1 the nearest bf16 (8 bits) of what that leaves, x2 the rest, which
+// fits 8 bits; w the same. Weights are split on the host, activations here. Of the nine products x2 w2, below 2^-30 of x w, is left out:
+// a product keeps more than an fp32 one would.
 //
-// The sums. The tensor core adds into its fp32 accumulator without rounding to nearest, an error of up to an ulp of the sum for
-// every eight products and always towards zero, which over a few hundred k-steps is worse than a chain of fp32 FMAs. So x0 w0
-// is accumulated over one k-block at a time (32 values of k, four tensor-core steps) and the k-blocks are added up in registers
-// with ordinary rounded additions; the two small products, 2^-11 of the large one, stay in an accumulator of their own
-// over the whole share of k.
-// What truncation takes from a k-block's sum is random but for its mean, which is towards zero: a gain a little below one, 3.7e-8 for one step, 8.9e-8
-// for four, the same whatever the layer. Layers upon layers would all lose it, so the sums of a share are multiplied by 1 + p.gain, which
-// leaves +-4e-9 (slope of the result over the sums in 64 bits). Without it the boxes of YOLOv5m-352 were 6e-5 from those of fp32 FMAs (median of
-// 72 images), with it 4.5e-6; two orders of the FMAs differ by 2.8e-6.
-// (inf and NaN: x1 of an infinite x is NaN, so where the large sum is not finite it is the result and the small one is dropped.)
+// The sums. The tensor core adds into its fp32 accumulator without rounding to nearest: what does not fit 24 bits is cut off, always
+// towards zero, and layers upon layers would multiply such a loss. Products of two 6-bit numbers have 12 bits, so 32 of them hardly ever
+// need more than 24: x0 w0 is accumulated over one k-block at a time (32 values of k, two tensor-core steps), with a mean loss of
+// 1.5e-9 (activations behind a ReLU) to 5e-9 (all products positive; simulated), and the k-blocks are added up in registers with ordinary rounded
+// additions. With tf32 parts of 11 bits the same sums lost 8.5-10e-8, and a factor that made up for the mean of it was off by 1-5e-8 for other data
+// than it was measured on, exact sums among them. x0 w1 + x1 w0, below 2^-5 and some 2^-7 of the large product, and the other five, some
+// 2^-14, have an accumulator each over the whole share of k.
+// (inf and NaN stay whole in x0, with x1 = x2 = 0; where the large sum is not finite it is the result and the small ones, which hold inf * 0, are dropped.)
 //
 // Roles of the 28 warps, connected by rings of mbarriers. A wait costs a single thread some 170 cycles even where it passes, so the
 // MMA threads have one a k-block: ready(k-block) counts the four splitting warps, the weights' bytes and the sixteen adding warps
-// that have emptied the accumulator; the one commit, done(k-block), frees the slot and the weights and says that the sums are there.
+// that have emptied the accumulator; the two commits, done(k-block), free the slot and the weights and say that the sums are there.
 //   0      loads activations, fp32 as they are: 128 pixels x 32 values of k (one filter tap), im2col or 2-D TMA, 128-byte swizzle
-//   1      loads the weights' two parts: 2 x kBn channels x 32 values of k, one 3-D TMA
-//   4-11   split: shared memory -> registers -> TMEM, a pixel (TMEM lane) per thread, 32 columns of x0 and 32 of x1; two groups
-//          of four warps take k-blocks in turn. With both parts in TMEM the tensor core reads only the weights from shared memory and an
-//          MMA of N channels takes N / 2 cycles (17 at 32, 33 at 64); with A in shared memory it takes 41 and 49, bound by
-//          reading A.
-//   2, 3   issue the MMAs of k-blocks in turn (beside its 400 cycles of MMAs a k-block costs its thread some 300 of its own, which the
-//          other one's MMAs cover; each has an accumulator of small products): 12 of N = kBn for a k-block (four steps x three products), fewer where a tap's last channels end
+//   1      loads the weights' three parts: 3 x kBn channels x 32 values of k, one 3-D TMA, 64-byte swizzle
+//   4-11   split: shared memory -> registers -> TMEM, a pixel (TMEM lane) per thread, 16 columns (two values each) of every part; two groups
+//          of four warps take k-blocks in turn. With the parts in TMEM the tensor core reads only the weights from shared memory and an
+//          MMA of N channels takes N / 2 cycles; with A in shared memory it is bound by reading A.
+//   2, 3   issue the MMAs, 2 to x0 w0, x0 w1 and x1 w0 and 3 to the other five products: an accumulator has one issuer, so that the order of its
+//          sums is fixed. 16 of N = kBn for a k-block (two steps x eight products), half as many where a tap's last channels end
 //   12-27  add up: the k-block's sums, TMEM -> registers, kBn / 4 channels of a pixel per thread; at the end of a share of k
 //          to shared memory; then scale / bias, activation, residual and the store, in rows of 16-byte vectors
-// TMEM: columns 0-319 a ring of accumulators of x0 w0 and those of the small products, then three slots of x0 | x1 (320 + 64 s).
+// TMEM: columns 0-319 a ring of accumulators of x0 w0 and those of the small products, then four slots of x0 | x1 | x2 (320 + 48 s).
 //
 // The k of a tile is summed in p.shares shares that are added in their order. How many comes from the layer and one image
 // (configure_conv_split), so an image has the same bits in a plan of any batch size. kSplit: a cluster of that many CTAs sums one
@@ -54,19 +52,16 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
         ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
-// D (TMEM) += A (TMEM) x B (shared memory), tf32
-__device__ __forceinline__ void tcgen05_mma_ts_tf32(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// D (TMEM) += A (TMEM) x B (shared memory), bf16
+__device__ __forceinline__ void tcgen05_mma_ts_bf16(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t taddr, const uint32_t *r) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 "
-        "[%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-        ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
-          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr) : "memory");
+__device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                 ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_32x32b_x8(uint32_t taddr, uint32_t *r) {
@@ -81,6 +76,36 @@ __device__ __forceinline__ void tmem_ld_columns(uint32_t taddr, uint32_t (&r)[N]
 #pragma unroll
     for (int c = 0; c + 8 <= N; c += 8) tmem_ld_32x32b_x8(taddr + static_cast<uint32_t>(c), r + c);
     if constexpr (N % 8 != 0) tmem_ld_32x32b_x4(taddr + static_cast<uint32_t>(N - 4), r + N - 4);
+}
+
+// The three parts of sixteen values (as bits), two to a register. kCareful: for values that round to infinity, which are cut off
+// in place of it, and for inf and NaN, whose other parts are zero. Returns a NaN where the careful form is needed, else zero.
+template <bool kCareful>
+__device__ __forceinline__ float split_values(const uint32_t (&x)[16], uint32_t (&p0)[8], uint32_t (&p1)[8], uint32_t (&p2)[8]) {
+    float bad = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        uint32_t h[2];
+        float r[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const uint32_t u = x[2 * q + e];
+            h[e] = (u + (1u << (kSplitLeadCut - 1))) & ~((1u << kSplitLeadCut) - 1u);
+            if (kCareful) {
+                const uint32_t mag = u & 0x7fffffffu;
+                if (mag >= kSplitLeadMax) h[e] = mag > 0x7f800000u ? 0x7fc00000u : u & 0xffff0000u;
+                r[e] = mag >= 0x7f800000u ? 0.f : __fsub_rn(__uint_as_float(u), __uint_as_float(h[e]));
+            } else {
+                r[e] = __fsub_rn(__uint_as_float(u), __uint_as_float(h[e]));
+            }
+        }
+        p0[q] = __byte_perm(h[0], h[1], 0x7632);
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1[q]) : "f"(r[1]), "f"(r[0]));
+        const float s0 = __fsub_rn(r[0], __uint_as_float(p1[q] << 16)), s1 = __fsub_rn(r[1], __uint_as_float(p1[q] & 0xffff0000u));
+        p2[q] = __byte_perm(__float_as_uint(s0), __float_as_uint(s1), 0x7632);       // (what is left has eight bits)
+        bad = __fmaf_rn(s0, 0.f, bad); bad = __fmaf_rn(s1, 0.f, bad);
+    }
+    return bad;
 }
 
 // The end of a tile: scale / bias, activation, residual (+ second activation), store. Of kThreads threads each has four channels of
@@ -162,10 +187,10 @@ __global__ void __launch_bounds__(kSpThreads, 1)
 conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ TView out, const __grid_constant__ TView out2, const __grid_constant__ ConvSplitParams p) {
     constexpr int kCols = kBn / 4;                                   // channels of a pixel an adding thread holds
     constexpr int kPitch = kBn + 4;                                  // floats of a row of the tile of sums
-    constexpr uint32_t kABytes = kUmmaM * 128, kBBytes = 2 * kBn * 128;
+    constexpr uint32_t kABytes = kUmmaM * 128, kPartBytes = kBn * 64, kBBytes = 3 * kPartBytes;
     // TMEM columns 0-319: accumulators of x0 w0 (a ring) and of the small products (one per issuer, twice where there is room)
     constexpr uint32_t kMain = kBn >= 48 ? 3 : 4, kSmall = kBn >= 48 ? 1 : 2, kSmallCol = kMain * kBn, kSlotCol = 320;
-    static_assert((kMain + 2 * kSmall) * kBn <= kSlotCol && kSlotCol + 64 * kSpSlots <= 512, "TMEM columns");
+    static_assert((kMain + 2 * kSmall) * kBn <= kSlotCol && kSlotCol + 48 * kSpSlots <= 512, "TMEM columns");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t a_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t b_base = a_base + kSpAStages * kABytes;
@@ -191,7 +216,7 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     pdl_launch_dependents();
     if (threadIdx.x < 36) {             // a barrier per thread
         const uint32_t t = threadIdx.x;
-        mbar_init(bar_base + 8u * t, t < 8 ? 1u : t < 16 ? 4u : t < 24 ? 4 + 1 + 16u : t < 32 ? 1u : t < 34 ? 2u : 16u);      // full_a, empty_a, ready, done, s_full, s_empty
+        mbar_init(bar_base + 8u * t, t < 8 ? 1u : t < 16 ? 4u : t < 24 ? 4 + 1 + 16u : t < 34 ? 2u : 16u);      // full_a, empty_a, ready, done, s_full, s_empty
         if (t == 0) cta_abort_slot = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -227,8 +252,8 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     ok = mbar_wait(empty_a(stage), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_EMPTY);
                     if (!ok) break;
                     mbar_expect_tx(full_a(stage), kABytes);
-                    if (im2col) tma_load_im2col_4d(a_base + stage * kABytes, &map_a, full_a(stage), p.chunk_elems * chunk, cx, cy, img, static_cast<uint16_t>(off_w), static_cast<uint16_t>(off_h));
-                    else        tma_load_2d(a_base + stage * kABytes, &map_a, full_a(stage), p.chunk_elems * chunk, m0);
+                    if (im2col) tma_load_im2col_4d(a_base + stage * kABytes, &map_a, full_a(stage), 32 * chunk, cx, cy, img, static_cast<uint16_t>(off_w), static_cast<uint16_t>(off_h));
+                    else        tma_load_2d(a_base + stage * kABytes, &map_a, full_a(stage), 32 * chunk, m0);
                     if (++stage == kSpAStages) { stage = 0; phase ^= 1u; }
                     if (++chunk == p.chunks_per_tap) {
                         chunk = 0; off_w += p.dil_w;
@@ -255,7 +280,7 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         if (++freed == kSpRing) { freed = 0; phase ^= 1u; }
                     }
                     mbar_expect_tx(ready(at), kBBytes);
-                    tma_load_3d(b_base + stage * kBBytes, &map_b, ready(at), c_tap + p.chunk_elems * chunk, n0, 0);
+                    tma_load_3d(b_base + stage * kBBytes, &map_b, ready(at), c_tap + 32 * chunk, n0, 0);
                     if (++stage == kSpBStages) stage = 0;
                     if (++at == kSpRing) at = 0;
                     if (++chunk == p.chunks_per_tap) { chunk = 0; c_tap += p.cin_pad; }
@@ -263,12 +288,12 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             }
         }
     } else if (warp < 4) {
-        // ------------------------------ MMA issuers: k-blocks in turn ------------------------------
+        // ------------------------------ MMA issuers: the products of every k-block shared between them ------------------------------
         if (elect_one()) {
-            constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(kBn >> 3) << 17) | (static_cast<uint32_t>(kUmmaM >> 4) << 24);
-            const uint32_t turn = static_cast<uint32_t>(warp - 2);
-            const uint64_t desc_b0 = make_smem_desc(b_base, 128);
-            uint32_t at = 0, phase = 0, stage = 0, slot = 0, acc = 0;          // of the next k-block, whoever issues it
+            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(kBn >> 3) << 17) | (static_cast<uint32_t>(kUmmaM >> 4) << 24);
+            const uint32_t issuer = static_cast<uint32_t>(warp - 2);
+            const uint64_t desc_b0 = make_smem_desc(b_base, 64);
+            uint32_t at = 0, phase = 0, stage = 0, slot = 0, acc = 0;
             uint32_t small = 0, small_phase = 1;
             bool ok = true;
             for (int tile = first_tile; tile < num_tiles && ok; tile += tile_stride)
@@ -277,38 +302,33 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                     int chunk = k0 % p.chunks_per_tap;
                     ok = mbar_wait(s_empty(small), small_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_ACC_EMPTY);
                     if (!ok) break;
-                    const uint32_t d_small = tmem + kSmallCol + kBn * (2 * small + turn);
+                    const uint32_t d_small = tmem + kSmallCol + kBn * (2 * small + issuer);
                     uint32_t more = 0;                                          // the share's first MMA begins its small sums
                     for (int kt = k0; kt < k1; ++kt) {
                         const bool last = ++chunk == p.chunks_per_tap;
                         if (last) chunk = 0;
-                        if ((at & 1u) == turn) {
-                            ok = mbar_wait(ready(at), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
-                            if (!ok) break;
-                            tcgen05_fence_after();
-                            const uint64_t w0 = desc_b0 + static_cast<uint64_t>(stage) * (kBBytes >> 4), w1 = w0 + (kBn * 128 >> 4);
-                            const uint32_t x0 = tmem + kSlotCol + 64u * slot, x1 = x0 + 32u, d_main = tmem + kBn * acc;
-                            const uint32_t steps = static_cast<uint32_t>(last ? p.tail_steps : p.chunk_steps);
-                            if (steps == 4) {
-#pragma unroll
-                                for (uint32_t k = 0; k < 4; ++k) {
-                                    tcgen05_mma_ts_tf32(d_small, x0 + 8 * k, w1 + 2 * k, idesc, k ? 1u : more);
-                                    tcgen05_mma_ts_tf32(d_small, x1 + 8 * k, w0 + 2 * k, idesc, 1u);
-                                    tcgen05_mma_ts_tf32(d_main, x0 + 8 * k, w0 + 2 * k, idesc, k ? 1u : 0u);
-                                }
+                        ok = mbar_wait(ready(at), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
+                        if (!ok) break;
+                        tcgen05_fence_after();
+                        const uint64_t w0 = desc_b0 + static_cast<uint64_t>(stage) * (kBBytes >> 4), w1 = w0 + (kPartBytes >> 4), w2 = w1 + (kPartBytes >> 4);
+                        const uint32_t x0 = tmem + kSlotCol + 48u * slot, x1 = x0 + 16u, x2 = x1 + 16u, d_main = tmem + kBn * acc;
+                        auto step = [&](uint32_t k, uint32_t begin_main, uint32_t begin_small) {
+                            if (issuer == 0) {
+                                tcgen05_mma_ts_bf16(d_small, x0 + 8 * k, w1 + 2 * k, idesc, begin_small);
+                                tcgen05_mma_ts_bf16(d_small, x1 + 8 * k, w0 + 2 * k, idesc, 1u);
+                                tcgen05_mma_ts_bf16(d_main, x0 + 8 * k, w0 + 2 * k, idesc, begin_main);
                             } else {
-                                for (uint32_t k = 0; k < steps; ++k) {
-                                    tcgen05_mma_ts_tf32(d_small, x0 + 8 * k, w1 + 2 * k, idesc, k ? 1u : more);
-                                    tcgen05_mma_ts_tf32(d_small, x1 + 8 * k, w0 + 2 * k, idesc, 1u);
-                                    tcgen05_mma_ts_tf32(d_main, x0 + 8 * k, w0 + 2 * k, idesc, k ? 1u : 0u);
-                                }
+                                tcgen05_mma_ts_bf16(d_small, x1 + 8 * k, w1 + 2 * k, idesc, begin_small);
+                                tcgen05_mma_ts_bf16(d_small, x0 + 8 * k, w2 + 2 * k, idesc, 1u);
+                                tcgen05_mma_ts_bf16(d_small, x2 + 8 * k, w0 + 2 * k, idesc, 1u);
+                                tcgen05_mma_ts_bf16(d_small, x1 + 8 * k, w2 + 2 * k, idesc, 1u);
+                                tcgen05_mma_ts_bf16(d_small, x2 + 8 * k, w1 + 2 * k, idesc, 1u);
                             }
-                            if (p.all_products) {
-                                for (uint32_t k = 0; k < steps; ++k) tcgen05_mma_ts_tf32(d_small, x1 + 8 * k, w1 + 2 * k, idesc, 1u);
-                            }
-                            more = 1;
-                            tcgen05_commit(done(at));
-                        }
+                        };
+                        step(0u, 0u, more);
+                        if (!last || p.tail_steps == 2) step(1u, 1u, 1u);
+                        more = 1;
+                        tcgen05_commit(done(at));
                         if (++at == kSpRing) { at = 0; phase ^= 1u; }
                         if (++stage == kSpBStages) stage = 0;
                         if (++slot == kSpSlots) slot = 0;
@@ -320,7 +340,7 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 }
         }
     } else if (warp >= 4 && warp < 12) {
-        // ------------------------------ split: fp32 in shared memory -> two tf32 parts in TMEM ------------------------------
+        // ------------------------------ split: fp32 in shared memory -> three bf16 parts in TMEM ------------------------------
         const int group = (warp - 4) >> 2;
         const uint32_t row = static_cast<uint32_t>((warp & 3) * 32 + lane), swz = row & 7u;
         const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
@@ -331,27 +351,28 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         for (long long q = group; q < total; q += 2) {
             bool ok = mbar_wait(full_a(stage), a_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
             if (!__all_sync(0xffffffffu, ok)) break;
-            const uint32_t src = a_base + stage * kABytes + row * 128u, dst = tmem + lanes + kSlotCol + 64u * slot;
-            uint32_t x[32];
+            const uint32_t src = a_base + stage * kABytes + row * 128u, dst = tmem + lanes + kSlotCol + 48u * slot;
+            uint32_t x[16];
+            auto fetch = [&](uint32_t h) {          // half a row
 #pragma unroll
-            for (uint32_t j = 0; j < 8; ++j)
-                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[4 * j]), "=r"(x[4 * j + 1]), "=r"(x[4 * j + 2]), "=r"(x[4 * j + 3]) : "r"(src + ((j ^ swz) << 4)) : "memory");
+                for (uint32_t j = 0; j < 4; ++j)
+                    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x[4 * j]), "=r"(x[4 * j + 1]), "=r"(x[4 * j + 2]), "=r"(x[4 * j + 3]) : "r"(src + (((j + 4u * h) ^ swz) << 4)) : "memory");
+            };
+            fetch(0);
             if (q >= kSpSlots) {                    // the slot's k-block before this one
                 ok = mbar_wait(done(freed), s_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_EMPTY);
                 if (!__all_sync(0xffffffffu, ok)) break;
             }
             tcgen05_fence_after();
 #pragma unroll
-            for (int h = 0; h < 32; h += 16) {
-                uint32_t x1[16];
-#pragma unroll
-                for (int e = 0; e < 16; ++e) {
-                    const float v = __uint_as_float(x[h + e]);
-                    x[h + e] = (x[h + e] + 0x1000u) & 0xffffe000u;
-                    x1[e] = __float_as_uint(__fsub_rn(v, __uint_as_float(x[h + e])));
-                }
-                tmem_st_32x32b_x16(dst + static_cast<uint32_t>(h), x + h);
-                tmem_st_32x32b_x16(dst + 32u + static_cast<uint32_t>(h), x1);
+            for (uint32_t h = 0; h < 2; ++h) {
+                uint32_t p0[8], p1[8], p2[8];
+                const float bad = split_values<false>(x, p0, p1, p2);
+                if (__any_sync(0xffffffffu, bad != 0.f)) split_values<true>(x, p0, p1, p2);
+                if (h == 0) fetch(1);
+                tmem_st_32x32b_x8(dst + 8u * h, p0);
+                tmem_st_32x32b_x8(dst + 16u + 8u * h, p1);
+                tmem_st_32x32b_x8(dst + 32u + 8u * h, p2);
             }
             tmem_st_wait();
             tcgen05_fence_before();
@@ -407,17 +428,13 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tcgen05_fence_after();
-                // the small sums of both issuers (of the only one, where the share is a single k-block)
-                const uint32_t first = (at + kSpRing - 1u) & 1u;                  // issuer of the share's last k-block
                 uint32_t v[kCols], w[kCols];
-#pragma unroll
-                for (int c = 0; c < kCols; ++c) w[c] = 0u;
-                if (k1 - k0 > 1) tmem_ld_columns(from + kSmallCol + kBn * (2 * small + 1u - first), w);
-                load(from + kSmallCol + kBn * (2 * small + first), v);
+                tmem_ld_columns(from + kSmallCol + kBn * (2 * small + 1u), w);
+                load(from + kSmallCol + kBn * (2 * small), v);
 #pragma unroll
                 for (int c = 0; c < kCols; ++c) {
                     asm volatile("" : "+r"(w[c]));
-                    if ((__float_as_uint(acc[c]) & 0x7f800000u) != 0x7f800000u) acc[c] = __fadd_rn(acc[c], __fmaf_rn(acc[c], p.gain, __fadd_rn(__uint_as_float(v[c]), __uint_as_float(w[c]))));
+                    if ((__float_as_uint(acc[c]) & 0x7f800000u) != 0x7f800000u) acc[c] = __fadd_rn(acc[c], __fadd_rn(__uint_as_float(v[c]), __uint_as_float(w[c])));
                 }
                 tcgen05_fence_before();
                 __syncwarp();

@@ -93,18 +93,18 @@ constexpr int kSpThreads = 896;      // warp 0: activations, 1: weights, 2 and 3
 // (an even ring of activations: the two groups of splitting warps take k-blocks in turn, and a stage has to be the same group's every
 // time, or a group could be a whole round of its barrier behind and take an old phase for the one it waits for)
 constexpr uint32_t kSpAStages = 6, kSpBStages = 5;     // rings of activations and weights in shared memory
-constexpr uint32_t kSpSlots = 3, kSpRing = 6;          // split activations in TMEM; barriers of the k-blocks under way
-static_assert(kSpAStages % 2 == 0 && kSpRing % 2 == 0, "a stage belongs to one group of splitting warps");
+constexpr uint32_t kSpSlots = 4, kSpRing = 6;          // split activations in TMEM; barriers of the k-blocks under way
+static_assert(kSpAStages % 2 == 0 && kSpRing % 2 == 0 && kSpSlots % 2 == 0, "a stage and a slot belong to one group of splitting warps");
+// x0 of a split value: six significant bits, the magnitude from which rounding to them gives infinity
+constexpr int kSplitLeadCut = 18;
+constexpr uint32_t kSplitLeadMax = 0x7f800000u - (1u << (kSplitLeadCut - 1));
 struct ConvSplitParams {
     int m_total, cout, tiles_m, tiles_n;
     int split_n;          // two 1x1 convs over the same input in one launch: channels from split_n on (a multiple of the tile) are the second one's
     int shares;           // the k of a tile is summed in this many shares, added in their order
     int a_mode;
     int taps, kw, chunks_per_tap, cin_pad, dil_h, dil_w;
-    int chunk_elems, chunk_steps;   // channels of a k-block (32, fewer where the whole k is short) and the tensor-core steps they take (8 values of k each)
-    int tail_steps;       // steps of a tap's last k-block
-    int all_products;     // x1 w1 too
-    float gain;           // what the accumulators' truncation takes from the large products on average, relative
+    int tail_steps;       // tensor-core steps (16 values of k each) of a tap's last k-block, the others have two
     int oh, ow, stride_h, stride_w, pad_h, pad_w;
     const void *res; int ldc_res;
     const float *scale, *bias;
@@ -115,7 +115,7 @@ struct ConvSplitParams {
 // channels of a tile: up to 64 (what TMEM holds beside three slots of split activations), evenly wide
 constexpr int split_tile_channels(int cout) { return ((cout + (cout + 63) / 64 - 1) / ((cout + 63) / 64) + 15) / 16 * 16; }
 constexpr size_t split_smem_bytes(int bn) {
-    return 1024 + kSpAStages * kUmmaM * 128 + kSpBStages * 2 * bn * 128 + static_cast<size_t>(kUmmaM) * (bn + 4) * 4 + 512;
+    return 1024 + kSpAStages * kUmmaM * 128 + kSpBStages * 3 * bn * 64 + static_cast<size_t>(kUmmaM) * (bn + 4) * 4 + 512;
 }
 constexpr int kSbMaxChannels = 1024;   // capacity of the staged scale / bias tables
 // Activation handled by a dedicated epilogue instantiation (no switch inside the loops); every other activation takes

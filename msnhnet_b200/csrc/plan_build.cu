@@ -81,6 +81,26 @@ float host_round_tf32(float x) {
     return x;
 }
 
+// the three parts of a value, as split_values (conv_split.cuh) takes them
+void host_split_bf16(float x, uint16_t &p0, uint16_t &p1, uint16_t &p2) {
+    uint32_t u;
+    std::memcpy(&u, &x, 4);
+    const uint32_t mag = u & 0x7fffffffu;
+    uint32_t lead = (u + (1u << (kSplitLeadCut - 1))) & ~((1u << kSplitLeadCut) - 1u);
+    if (mag >= kSplitLeadMax) lead = mag > 0x7f800000u ? 0x7fc00000u : u & 0xffff0000u;
+    p0 = static_cast<uint16_t>(lead >> 16); p1 = p2 = 0;
+    if (mag >= 0x7f800000u) return;
+    float l, m;
+    std::memcpy(&l, &lead, 4);
+    const float rest = x - l;
+    std::memcpy(&u, &rest, 4);
+    u = (u + 0x7fffu + (u >> 16 & 1u)) & 0xffff0000u;
+    std::memcpy(&m, &u, 4);
+    p1 = static_cast<uint16_t>(u >> 16);
+    const float last = rest - m;
+    std::memcpy(&u, &last, 4);
+    p2 = static_cast<uint16_t>(u >> 16);
+}
 
 // the same algebra as the reference's convBn kernel (src/layers/cuda/MsnhConvolutionalLayerGPU.cu:6-35).
 void fold_bn(const OpState &o, int channels, std::vector<float> &scale, std::vector<float> &bias) {
@@ -425,17 +445,18 @@ int build_launches(MsnhB200Plan *pl) {
                         p.L.weights = ps.dev;
                     }
                 } else {
+                    // what an im2col tensor map can walk
+                    const bool tma_walks = groups == 1 && p.L.sh <= 8 && p.L.sw <= 8 && p.L.ph < 128 && p.L.pw < 128 && kh * p.L.dh < 256 && kw * p.L.dw < 256;
                     // [Cout][Cin/g][kh][kw] -> [Cout][tap][cin_pad], zero in the pad channels
                     // (patch mode: one "tap" of patch_k values ordered tap-major, like the patch matrix)
                     // (row patches: one "tap" per filter row, of kw x cin values)
-                    const int cin_pad = patched ? patch_k : round_up(rows ? kw * cin_g : cin_g, V);
+                    // (split operands: whole tensor-core steps of 16 values, so that a step never reads the next tap's weights)
+                    const bool split = pl->split_fp32 && tma_walks && aligned_view(in0) && aligned_view(o.tensor) && (p.res_t < 0 || aligned_view(p.res_t));
+                    const int cin_pad = patched ? patch_k : round_up(rows ? kw * cin_g : cin_g, split ? 16 : V);
                     const size_t row_len = patched ? static_cast<size_t>(patch_k) : static_cast<size_t>(rows ? kh : taps) * cin_pad;
                     auto tap_at = [&](int t) { return static_cast<size_t>(patched ? t * cin_g : rows ? t / kw * cin_pad + t % kw * cin_g : t * cin_pad); };   // where a tap starts inside a row
                     p.L.cin_pad = cin_pad;
                     const size_t n = static_cast<size_t>(cout) * row_len;
-                    // what an im2col tensor map can walk
-                    const bool tma_walks = groups == 1 && p.L.sh <= 8 && p.L.sw <= 8 && p.L.ph < 128 && p.L.pw < 128 && kh * p.L.dh < 256 && kw * p.L.dw < 256;
-                    bool split = false;
                     // packed straight into the arena's staging bytes (zero-filled, so the pad channels stay zero)
                     if (pl->dtype == MSNH_B200_F16) {
                         PackSlot<__half> ps = reserve_pack<__half>(pl, n);
@@ -445,18 +466,25 @@ int build_launches(MsnhB200Plan *pl) {
                                 pk[static_cast<size_t>(co) * row_len + tap_at(t) + ci] = __float2half_rn(w[(static_cast<size_t>(co) * cin_g + ci) * taps + t]);
                         });
                         p.L.weights = ps.dev;
+                    } else if (split) {
+                        // three matrices, one behind the other
+                        PackSlot<uint16_t> ps = reserve_pack<uint16_t>(pl, 3 * n);
+                        uint16_t *pk = ps.host;
+                        if (pk) parallel_rows(cout, static_cast<size_t>(cin_g) * taps, [&](int co) {
+                            for (int ci = 0; ci < cin_g; ++ci) for (int t = 0; t < taps; ++t) {
+                                const size_t at = static_cast<size_t>(co) * row_len + tap_at(t) + ci;
+                                host_split_bf16(w[(static_cast<size_t>(co) * cin_g + ci) * taps + t], pk[at], pk[n + at], pk[2 * n + at]);
+                            }
+                        });
+                        p.L.weights = ps.dev;
                     } else {
-                        // split operands: the matrix of the nearest tf32 values and, behind it, that of what they leave
-                        split = pl->split_fp32 && tma_walks && aligned_view(in0) && aligned_view(o.tensor) && (p.res_t < 0 || aligned_view(p.res_t));
-                        PackSlot<float> ps = reserve_pack<float>(pl, split ? 2 * n : n);
+                        PackSlot<float> ps = reserve_pack<float>(pl, n);
                         float *pk = ps.host;
                         const bool tc = groups == 1 && !(pl->flags & MSNH_PLAN_NO_TENSOR_CORE);
                         if (pk) parallel_rows(cout, static_cast<size_t>(cin_g) * taps, [&](int co) {
                             for (int ci = 0; ci < cin_g; ++ci) for (int t = 0; t < taps; ++t) {
                                 const float v = w[(static_cast<size_t>(co) * cin_g + ci) * taps + t];
-                                const size_t at = static_cast<size_t>(co) * row_len + tap_at(t) + ci;
-                                pk[at] = tc || split ? host_round_tf32(v) : v;
-                                if (split) pk[n + at] = host_round_tf32(v - pk[at]);
+                                pk[static_cast<size_t>(co) * row_len + tap_at(t) + ci] = tc ? host_round_tf32(v) : v;
                             }
                         });
                         p.L.weights = ps.dev;
@@ -708,9 +736,9 @@ int build_launches(MsnhB200Plan *pl) {
                 if (!plain_1x1(b) || b.L.kind != a.L.kind || !same_data(a.in_t, b.in_t) || b.out_t == a.out_t || (!split && (b.L.act1 != a.L.act1 || b.L.act1_p != a.L.act1_p)) ||
                     b.L.cin_pad != a.L.cin_pad) continue;
                 const int cb = pl->tensors[b.out_t].s.C;
-                const size_t row_bytes = static_cast<size_t>(a.L.cin_pad) * es;
+                const size_t row_bytes = static_cast<size_t>(a.L.cin_pad) * (split ? 2 : es);
                 const size_t wa = off_of(a.L.weights), wb = off_of(b.L.weights), sa = off_of(a.L.scale), sb = off_of(b.L.scale), ba = off_of(a.L.bias), bb = off_of(b.L.bias);
-                const int parts = split ? 2 : 1;              // (split operands: two matrices, one behind the other)
+                const int parts = split ? 3 : 1;              // (split operands: three matrices, one behind the other)
                 PackSlot<uint8_t> ws = reserve_pack<uint8_t>(pl, parts * (static_cast<size_t>(ca) + cb) * row_bytes);
                 if (ws.host)         // (nullptr: the arena comes from a pack file, which holds the merged copy at this offset)
                     for (int k = 0; k < parts; ++k) {

@@ -167,20 +167,8 @@ int configure_conv_split(MsnhB200Plan *pl, Launch &L) {
     u.tiles_n = (cout + L.sp_bn - 1) / L.sp_bn;
     u.tiles_m = (u.m_total + kUmmaM - 1) / kUmmaM;
     u.taps = L.kh * L.kw; u.kw = L.kw;
-    // What an accumulator loses to truncation shows beside the FMA chain it replaces where k is very short (norm error against 64 bits,
-    // 27 values of k: FMAs 9.6e-8, k-blocks of 32 / 16 / 8 values 1.35e-7 / 1.00e-7 / 9.2e-8; 48 values: 1.27e-7 and 1.20e-7 in blocks of 32), and so
-    // does the smallest product (64 values: 1.46e-7, without it 1.33e-7, with it 1.28e-7).
-    u.chunk_elems = u.taps * cin < 48 ? 8 : 32; u.chunk_steps = u.chunk_elems / 8;
-    u.all_products = u.taps * cin <= 128;
-    u.chunks_per_tap = (cin + u.chunk_elems - 1) / u.chunk_elems; u.cin_pad = L.cin_pad;
-    u.tail_steps = (cin - u.chunk_elems * (u.chunks_per_tap - 1) + 7) / 8;
-    // Mean loss of a k-block of n steps, measured as the slope of the results over sums in 64 bits (27 to 2304 values of k, four layers of n = 4):
-    // 3.2-3.8e-8 for one step, 5.4e-8 for two, 7.1e-8 for three, 8.5-9.0e-8 for four; k-blocks of a tap count by their channels.
-    {
-        auto loss = [](int steps) { return 1.9e-8 + 1.74e-8 * steps; };
-        const int last = cin - u.chunk_elems * (u.chunks_per_tap - 1);
-        u.gain = static_cast<float>((loss(u.chunk_steps) * (cin - last) + loss(u.tail_steps) * last) / cin);
-    }
+    u.chunks_per_tap = (cin + 31) / 32; u.cin_pad = L.cin_pad;
+    u.tail_steps = (cin - 32 * (u.chunks_per_tap - 1) + 15) / 16;
     u.dil_h = L.dh; u.dil_w = L.dw;
     u.oh = L.out.H; u.ow = L.out.W; u.stride_h = L.sh; u.stride_w = L.sw; u.pad_h = L.ph; u.pad_w = L.pw;
     u.res = L.res; u.ldc_res = L.ldc_res; u.scale = L.scale; u.bias = L.bias;
@@ -224,10 +212,10 @@ int configure_conv_split(MsnhB200Plan *pl, Launch &L) {
     else        rc = make_map_im2col(ctx, &L.map_a, MSNH_B200_F32, L.in, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, L.dh, L.dw, 32, 128, kUmmaM);
     if (rc) return rc;
     const cuuint64_t ktot = static_cast<cuuint64_t>(u.taps) * u.cin_pad;
-    cuuint64_t dims[3] = {ktot, static_cast<cuuint64_t>(cout), 2}, strides[2] = {ktot * 4, ktot * 4 * cout};
-    cuuint32_t box[3] = {32, static_cast<cuuint32_t>(L.sp_bn), 2}, estr[3] = {1, 1, 1};
-    const CUresult r = ctx->encode_tiled(&L.map_b, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(L.weights), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    cuuint64_t dims[3] = {ktot, static_cast<cuuint64_t>(cout), 3}, strides[2] = {ktot * 2, ktot * 2 * cout};
+    cuuint32_t box[3] = {32, static_cast<cuuint32_t>(L.sp_bn), 3}, estr[3] = {1, 1, 1};
+    const CUresult r = ctx->encode_tiled(&L.map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(L.weights), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                         CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ctx, MSNH_B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d): split weights %llu x %d", (int)r, (unsigned long long)ktot, cout);
     prepare_conv_split_launch();
     char note[128];
