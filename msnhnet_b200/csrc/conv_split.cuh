@@ -1,4 +1,4 @@
-// fp32 convolution on the tensor cores: every fp32 operand is the sum of three bf16 numbers, and a product that of eight
+// fp32 convolution on the tensor cores: every fp32 operand is the sum of four bf16 numbers, and a product that of ten
 // tensor-core products. What the fp32 plans of detection nets run (boxes decoded through exp() do not hold
 // through tf32's 10 mantissa bits); the CUDA-core form of the same arithmetic is conv_fp32_kernel (conv_tiled.cuh). Replaces the
 // reference's im2col + cublasSgemm (src/layers/MsnhConvolutionalLayer.cpp:1026-1160).
@@ -8,44 +8,49 @@
 namespace msnh {
 
 // ---------------------------------------------------------------------------------------------------------------------------
-// x = x0 + x1 + x2 exactly: x0 the nearest number of 6 significant bits, x1 the nearest bf16 (8 bits) of what that leaves, x2 the rest, which
-// fits 8 bits; w the same. Weights are split on the host, activations here. Of the nine products x2 w2, below 2^-30 of x w, is left out:
-// a product keeps more than an fp32 one would.
+// x = x0 + x1 + x2 + x3 exactly: x0 the nearest number of 4 significant bits, x1 and x2 the nearest bf16 (8 bits) of what is left, x3 the rest;
+// w the same. Weights are split on the host, activations here. Of the sixteen products ten are taken; the largest of the others, x2 w2, x1 w3
+// and x3 w1, are below 2^-26 of x w and some 2^-29: a product keeps more than an fp32 one would.
 //
 // The sums. The tensor core adds into its fp32 accumulator without rounding to nearest: what does not fit 24 bits is cut off, always
-// towards zero, and layers upon layers would multiply such a loss. Products of two 6-bit numbers have 12 bits, so 32 of them hardly ever
-// need more than 24: x0 w0 is accumulated over one k-block at a time (32 values of k, two tensor-core steps), with a mean loss of
-// 1.5e-9 (activations behind a ReLU) to 5e-9 (all products positive; simulated), and the k-blocks are added up in registers with ordinary rounded
-// additions. With tf32 parts of 11 bits the same sums lost 8.5-10e-8, and a factor that made up for the mean of it was off by 1-5e-8 for other data
-// than it was measured on, exact sums among them. x0 w1 + x1 w0, below 2^-5 and some 2^-7 of the large product, and the other five, some
-// 2^-14, have an accumulator each over the whole share of k.
-// (inf and NaN stay whole in x0, with x1 = x2 = 0; where the large sum is not finite it is the result and the small ones, which hold inf * 0, are dropped.)
+// towards zero, and layers upon layers would multiply such a loss. Products of two 4-bit numbers have 8 bits, so a sum of 32 hardly ever
+// needs more than 24: x0 w0 is accumulated over one k-block at a time (32 values of k, two tensor-core steps), and so is x0 w1 + x1 w0, some 2^-5
+// of it; both are added up over the k-blocks in registers with ordinary rounded additions. The other seven products, some 2^-10, stay in an accumulator of
+// their own over the whole share of k. What a sum of 32 products loses on average, relative (a simulation that fits the tensor core's results):
+//     bits of x0, w0                       4         5         6         8        11 (tf32)
+//     normal                            3e-10     1e-9      3.4e-9    2.5e-8    1.0e-7
+//     normal, behind a LeakyReLU        1.2e-9    3.4e-9    1.0e-8
+//     positive activations and weights  5e-10     1.6e-9    5e-9      3.3e-8
+// YOLOv5m, whose 94 convs multiply it most, needs 2e-9: with 6 bits its heads (352, 640 pixels) were 1.6 and 2.3 times as far from the net in 64 bits as
+// with fp32 FMAs, with tf32 parts, four products and a factor that made up for the mean loss on normal data 1.9 and 3.3 times.
+// (inf and NaN stay whole in x0, with the other parts zero; where the large sum is not finite it is the result and the small ones, which hold inf * 0, are dropped.)
 //
 // Roles of the 28 warps, connected by rings of mbarriers. A wait costs a single thread some 170 cycles even where it passes, so the
 // MMA threads have one a k-block: ready(k-block) counts the four splitting warps, the weights' bytes and the sixteen adding warps
 // that have emptied the accumulator; the two commits, done(k-block), free the slot and the weights and say that the sums are there.
 //   0      loads activations, fp32 as they are: 128 pixels x 32 values of k (one filter tap), im2col or 2-D TMA, 128-byte swizzle
-//   1      loads the weights' three parts: 3 x kBn channels x 32 values of k, one 3-D TMA, 64-byte swizzle
+//   1      loads the weights' four parts: 4 x kBn channels x 32 values of k, one 3-D TMA, 64-byte swizzle
 //   4-11   split: shared memory -> registers -> TMEM, a pixel (TMEM lane) per thread, 16 columns (two values each) of every part; two groups
 //          of four warps take k-blocks in turn. With the parts in TMEM the tensor core reads only the weights from shared memory and an
-//          MMA of N channels takes N / 2 cycles; with A in shared memory it is bound by reading A.
-//   2, 3   issue the MMAs, 2 to x0 w0, x0 w1 and x1 w0 and 3 to the other five products: an accumulator has one issuer, so that the order of its
-//          sums is fixed. 16 of N = kBn for a k-block (two steps x eight products), half as many where a tap's last channels end
-//   12-27  add up: the k-block's sums, TMEM -> registers, kBn / 4 channels of a pixel per thread; at the end of a share of k
-//          to shared memory; then scale / bias, activation, residual and the store, in rows of 16-byte vectors
-// TMEM: columns 0-319 a ring of accumulators of x0 w0 and those of the small products, then four slots of x0 | x1 | x2 (320 + 48 s).
+//          MMA of N channels takes N / 2 cycles.
+//   2, 3   issue the MMAs, 2 those of x0 w0, x0 w1 and x1 w0, 3 those of the other seven products: an accumulator has one issuer, so that the order of
+//          its sums is fixed. 20 of N = kBn for a k-block (two steps x ten products), half as many where a tap's last channels end
+//   12-27  add up: the k-block's sums, TMEM -> registers, kBn / 4 channels of a pixel per thread; at the end of a share of k to shared memory, and
+//          where a tile's k is one share after every kSpFlush k-blocks (a chain of rounded additions over all of them would lose more than the shares
+//          of conv_fp32_kernel); then scale / bias, activation, residual and the store, in rows of 16-byte vectors
+// TMEM: columns 0-319 a ring of accumulators of x0 w0 | x0 w1 + x1 w0 and those of the other products, then three slots of x0 | x1 | x2 | x3
+// (320 + 64 s).
 //
 // The k of a tile is summed in p.shares shares that are added in their order. How many comes from the layer and one image
 // (configure_conv_split), so an image has the same bits in a plan of any batch size. kSplit: a cluster of that many CTAs sums one
 // each, one tile per cluster, and every CTA finishes every shares-th row through distributed shared memory. Else a CTA walks tiles
 // and sums a tile's shares one after the other.
 //
-// Measured against fp32 FMAs on the CUDA cores (conv_fp32_kernel), a forward in us: YOLOv3-tiny-416, one image 431 -> 207 and sixteen
-// 3965 -> 1490; YOLOv5m-352, three images 2889 -> 1209; YOLOv5m-640, two 4604 -> 1785. Norm error against 64 bits, FMAs / here: 64 values
-// of k 1.44e-7 / 1.28e-7, 288 1.54e-7 / 1.46e-7, 2304 3.8e-7 / 2.0e-7, 4608 4.3e-7 / 2.5e-7 (one share; less in several). A k-block takes 550-650 cycles: its 12
-// MMAs 300 (48 channels) to 400 (64), the rest is the way of a slot round the roles (split, MMA, commit, sums read, some 1800 cycles
-// for three k-blocks). With one MMA thread it took 780, with eight adding warps the end of a tile 2600 cycles (now half), with
-// cvt.rna.tf32 in place of integer rounding (a quarter of the rate) 1000.
+// Measured against fp32 FMAs on the CUDA cores (conv_fp32_kernel), a forward in us: YOLOv3-tiny-416, one image 441 -> 243 and sixteen
+// 3984 -> 1726; YOLOv5m-352, three images 2973 -> 1520; YOLOv5m-640, two 4717 -> 2381; YOLOv4-416, one 3520 -> 1835. (Two tf32 parts and four products:
+// 219, 1532, 1308, 1942 and 1548.) Norm error against 64 bits, FMAs / here in one share: 27 values of k 9.4e-8 / 2.6e-8, 64 1.44e-7 / 2.6e-8,
+// 576 1.6e-7 / 3.6e-8, 2304 3.1e-7 / 5.3e-8, 4608 4.3e-7 / 7.4e-8 (normal data; tests/test_conv_split_precision_gpu.py has other kinds). Heads of whole nets against the
+// net in 64 bits: YOLOv3-tiny-416 7e-7 / 1.5e-7, YOLOv5m-640 2.1-2.9e-6 / 0.8-1.1e-6, YOLOv4-416 1.0-1.2e-6 / 2.2-2.7e-7.
 // ---------------------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int c0, int c1, int c2) {
     asm volatile(
@@ -78,34 +83,39 @@ __device__ __forceinline__ void tmem_ld_columns(uint32_t taddr, uint32_t (&r)[N]
     if constexpr (N % 8 != 0) tmem_ld_32x32b_x4(taddr + static_cast<uint32_t>(N - 4), r + N - 4);
 }
 
-// The three parts of sixteen values (as bits), two to a register. kCareful: for values that round to infinity, which are cut off
-// in place of it, and for inf and NaN, whose other parts are zero. Returns a NaN where the careful form is needed, else zero.
+// Sixteen values (as bits) to their leading parts, two to a register, and what those leave. kCareful: for values that round to infinity,
+// which are cut off in place of it, and for inf and NaN, which leave nothing. Returns a NaN where the careful form is needed, else zero.
 template <bool kCareful>
-__device__ __forceinline__ float split_values(const uint32_t (&x)[16], uint32_t (&p0)[8], uint32_t (&p1)[8], uint32_t (&p2)[8]) {
+__device__ __forceinline__ float split_lead(uint32_t (&x)[16], uint32_t (&part)[8]) {
     float bad = 0.f;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    for (int q = 0; q < 16; q += 2) {
         uint32_t h[2];
-        float r[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-            const uint32_t u = x[2 * q + e];
+            const uint32_t u = x[q + e];
             h[e] = (u + (1u << (kSplitLeadCut - 1))) & ~((1u << kSplitLeadCut) - 1u);
             if (kCareful) {
                 const uint32_t mag = u & 0x7fffffffu;
                 if (mag >= kSplitLeadMax) h[e] = mag > 0x7f800000u ? 0x7fc00000u : u & 0xffff0000u;
-                r[e] = mag >= 0x7f800000u ? 0.f : __fsub_rn(__uint_as_float(u), __uint_as_float(h[e]));
+                x[q + e] = mag >= 0x7f800000u ? 0u : __float_as_uint(__fsub_rn(__uint_as_float(u), __uint_as_float(h[e])));
             } else {
-                r[e] = __fsub_rn(__uint_as_float(u), __uint_as_float(h[e]));
+                x[q + e] = __float_as_uint(__fsub_rn(__uint_as_float(u), __uint_as_float(h[e])));
+                bad = __fmaf_rn(__uint_as_float(x[q + e]), 0.f, bad);
             }
         }
-        p0[q] = __byte_perm(h[0], h[1], 0x7632);
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p1[q]) : "f"(r[1]), "f"(r[0]));
-        const float s0 = __fsub_rn(r[0], __uint_as_float(p1[q] << 16)), s1 = __fsub_rn(r[1], __uint_as_float(p1[q] & 0xffff0000u));
-        p2[q] = __byte_perm(__float_as_uint(s0), __float_as_uint(s1), 0x7632);       // (what is left has eight bits)
-        bad = __fmaf_rn(s0, 0.f, bad); bad = __fmaf_rn(s1, 0.f, bad);
+        part[q / 2] = __byte_perm(h[0], h[1], 0x7632);
     }
     return bad;
+}
+// their next parts, the nearest bf16, and what those leave
+__device__ __forceinline__ void split_next(uint32_t (&x)[16], uint32_t (&part)[8]) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(part[q]) : "f"(__uint_as_float(x[2 * q + 1])), "f"(__uint_as_float(x[2 * q])));
+        x[2 * q] = __float_as_uint(__fsub_rn(__uint_as_float(x[2 * q]), __uint_as_float(part[q] << 16)));
+        x[2 * q + 1] = __float_as_uint(__fsub_rn(__uint_as_float(x[2 * q + 1]), __uint_as_float(part[q] & 0xffff0000u)));
+    }
 }
 
 // The end of a tile: scale / bias, activation, residual (+ second activation), store. Of kThreads threads each has four channels of
@@ -187,10 +197,10 @@ __global__ void __launch_bounds__(kSpThreads, 1)
 conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ TView out, const __grid_constant__ TView out2, const __grid_constant__ ConvSplitParams p) {
     constexpr int kCols = kBn / 4;                                   // channels of a pixel an adding thread holds
     constexpr int kPitch = kBn + 4;                                  // floats of a row of the tile of sums
-    constexpr uint32_t kABytes = kUmmaM * 128, kPartBytes = kBn * 64, kBBytes = 3 * kPartBytes;
-    // TMEM columns 0-319: accumulators of x0 w0 (a ring) and of the small products (one per issuer, twice where there is room)
-    constexpr uint32_t kMain = kBn >= 48 ? 3 : 4, kSmall = kBn >= 48 ? 1 : 2, kSmallCol = kMain * kBn, kSlotCol = 320;
-    static_assert((kMain + 2 * kSmall) * kBn <= kSlotCol && kSlotCol + 48 * kSpSlots <= 512, "TMEM columns");
+    constexpr uint32_t kABytes = kUmmaM * 128, kPartBytes = kBn * 64, kBBytes = 4 * kPartBytes;
+    // TMEM columns 0-319: accumulators of x0 w0 and of x0 w1 + x1 w0 side by side (a ring) and of the other products (twice where there is room)
+    constexpr uint32_t kMain = kBn >= 48 ? 2 : 4, kSmall = kBn == 64 ? 1 : 2, kSmallCol = 2 * kMain * kBn, kSlotCol = 320;
+    static_assert((2 * kMain + kSmall) * kBn <= kSlotCol && kSlotCol + 64 * kSpSlots <= 512, "TMEM columns");
     extern __shared__ uint8_t smem_raw[];
     const uint32_t a_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t b_base = a_base + kSpAStages * kABytes;
@@ -216,7 +226,7 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     pdl_launch_dependents();
     if (threadIdx.x < 36) {             // a barrier per thread
         const uint32_t t = threadIdx.x;
-        mbar_init(bar_base + 8u * t, t < 8 ? 1u : t < 16 ? 4u : t < 24 ? 4 + 1 + 16u : t < 34 ? 2u : 16u);      // full_a, empty_a, ready, done, s_full, s_empty
+        mbar_init(bar_base + 8u * t, t < 8 ? 1u : t < 16 ? 4u : t < 24 ? 4 + 1 + 16u : t < 32 ? 2u : t < 34 ? 1u : 16u);      // full_a, empty_a, ready, done, s_full, s_empty
         if (t == 0) cta_abort_slot = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -300,9 +310,11 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                 for (int share = share_first; share < share_end && ok; ++share) {
                     const int k0 = num_k * share / p.shares, k1 = num_k * (share + 1) / p.shares;
                     int chunk = k0 % p.chunks_per_tap;
-                    ok = mbar_wait(s_empty(small), small_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_ACC_EMPTY);
-                    if (!ok) break;
-                    const uint32_t d_small = tmem + kSmallCol + kBn * (2 * small + issuer);
+                    if (issuer == 1) {
+                        ok = mbar_wait(s_empty(small), small_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_ACC_EMPTY);
+                        if (!ok) break;
+                    }
+                    const uint32_t d_small = tmem + kSmallCol + kBn * small;
                     uint32_t more = 0;                                          // the share's first MMA begins its small sums
                     for (int kt = k0; kt < k1; ++kt) {
                         const bool last = ++chunk == p.chunks_per_tap;
@@ -310,19 +322,21 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         ok = mbar_wait(ready(at), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
                         if (!ok) break;
                         tcgen05_fence_after();
-                        const uint64_t w0 = desc_b0 + static_cast<uint64_t>(stage) * (kBBytes >> 4), w1 = w0 + (kPartBytes >> 4), w2 = w1 + (kPartBytes >> 4);
-                        const uint32_t x0 = tmem + kSlotCol + 48u * slot, x1 = x0 + 16u, x2 = x1 + 16u, d_main = tmem + kBn * acc;
-                        auto step = [&](uint32_t k, uint32_t begin_main, uint32_t begin_small) {
+                        const uint64_t w0 = desc_b0 + static_cast<uint64_t>(stage) * (kBBytes >> 4), w1 = w0 + (kPartBytes >> 4), w2 = w1 + (kPartBytes >> 4), w3 = w2 + (kPartBytes >> 4);
+                        const uint32_t x0 = tmem + kSlotCol + 64u * slot, x1 = x0 + 16u, x2 = x1 + 16u, x3 = x2 + 16u, d_main = tmem + 2 * kBn * acc, d_mid = d_main + kBn;
+                        auto step = [&](uint32_t k, uint32_t more_main, uint32_t more_small) {
                             if (issuer == 0) {
-                                tcgen05_mma_ts_bf16(d_small, x0 + 8 * k, w1 + 2 * k, idesc, begin_small);
-                                tcgen05_mma_ts_bf16(d_small, x1 + 8 * k, w0 + 2 * k, idesc, 1u);
-                                tcgen05_mma_ts_bf16(d_main, x0 + 8 * k, w0 + 2 * k, idesc, begin_main);
+                                tcgen05_mma_ts_bf16(d_mid, x0 + 8 * k, w1 + 2 * k, idesc, more_main);
+                                tcgen05_mma_ts_bf16(d_main, x0 + 8 * k, w0 + 2 * k, idesc, more_main);
+                                tcgen05_mma_ts_bf16(d_mid, x1 + 8 * k, w0 + 2 * k, idesc, 1u);
                             } else {
-                                tcgen05_mma_ts_bf16(d_small, x1 + 8 * k, w1 + 2 * k, idesc, begin_small);
+                                tcgen05_mma_ts_bf16(d_small, x1 + 8 * k, w1 + 2 * k, idesc, more_small);
                                 tcgen05_mma_ts_bf16(d_small, x0 + 8 * k, w2 + 2 * k, idesc, 1u);
                                 tcgen05_mma_ts_bf16(d_small, x2 + 8 * k, w0 + 2 * k, idesc, 1u);
                                 tcgen05_mma_ts_bf16(d_small, x1 + 8 * k, w2 + 2 * k, idesc, 1u);
                                 tcgen05_mma_ts_bf16(d_small, x2 + 8 * k, w1 + 2 * k, idesc, 1u);
+                                tcgen05_mma_ts_bf16(d_small, x0 + 8 * k, w3 + 2 * k, idesc, 1u);
+                                tcgen05_mma_ts_bf16(d_small, x3 + 8 * k, w0 + 2 * k, idesc, 1u);
                             }
                         };
                         step(0u, 0u, more);
@@ -335,12 +349,12 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
                         if (++acc == kMain) acc = 0;
                     }
                     if (!ok) break;
-                    tcgen05_commit(s_full(small));
+                    if (issuer == 1) tcgen05_commit(s_full(small));
                     if (++small == kSmall) { small = 0; small_phase ^= 1u; }
                 }
         }
     } else if (warp >= 4 && warp < 12) {
-        // ------------------------------ split: fp32 in shared memory -> three bf16 parts in TMEM ------------------------------
+        // ------------------------------ split: fp32 in shared memory -> four bf16 parts in TMEM ------------------------------
         const int group = (warp - 4) >> 2;
         const uint32_t row = static_cast<uint32_t>((warp & 3) * 32 + lane), swz = row & 7u;
         const uint32_t lanes = static_cast<uint32_t>((warp & 3) * 32) << 16;
@@ -351,7 +365,7 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         for (long long q = group; q < total; q += 2) {
             bool ok = mbar_wait(full_a(stage), a_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_FULL);
             if (!__all_sync(0xffffffffu, ok)) break;
-            const uint32_t src = a_base + stage * kABytes + row * 128u, dst = tmem + lanes + kSlotCol + 48u * slot;
+            const uint32_t src = a_base + stage * kABytes + row * 128u, dst = tmem + lanes + kSlotCol + 64u * slot;
             uint32_t x[16];
             auto fetch = [&](uint32_t h) {          // half a row
 #pragma unroll
@@ -366,13 +380,18 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
             tcgen05_fence_after();
 #pragma unroll
             for (uint32_t h = 0; h < 2; ++h) {
-                uint32_t p0[8], p1[8], p2[8];
-                const float bad = split_values<false>(x, p0, p1, p2);
-                if (__any_sync(0xffffffffu, bad != 0.f)) split_values<true>(x, p0, p1, p2);
-                if (h == 0) fetch(1);
-                tmem_st_32x32b_x8(dst + 8u * h, p0);
-                tmem_st_32x32b_x8(dst + 16u + 8u * h, p1);
-                tmem_st_32x32b_x8(dst + 32u + 8u * h, p2);
+                uint32_t part[8];
+                if (h == 1) fetch(1);
+                const float bad = split_lead<false>(x, part);
+                if (__any_sync(0xffffffffu, bad != 0.f)) { fetch(h); split_lead<true>(x, part); }
+                tmem_st_32x32b_x8(dst + 8u * h, part);
+                split_next(x, part);
+                tmem_st_32x32b_x8(dst + 16u + 8u * h, part);
+                split_next(x, part);
+                tmem_st_32x32b_x8(dst + 32u + 8u * h, part);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) part[q] = __byte_perm(x[2 * q], x[2 * q + 1], 0x7632);      // (what is left has two bits)
+                tmem_st_32x32b_x8(dst + 48u + 8u * h, part);
             }
             tmem_st_wait();
             tcgen05_fence_before();
@@ -403,53 +422,65 @@ conv_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         };
         for (int tile = first_tile; tile < num_tiles && ok; tile += tile_stride) {
             const SplitFinish<kBn, 512, 4> finish(p, out, out2, tile % p.tiles_n * kBn, t);
+            bool begun = false;                       // sums of this tile are in shared memory
             for (int share = share_first; share < share_end && ok; ++share) {
                 const int k0 = num_k * share / p.shares, k1 = num_k * (share + 1) / p.shares;
-                float acc[kCols];
+                float acc[kCols], mid[kCols];
 #pragma unroll
-                for (int c = 0; c < kCols; ++c) acc[c] = 0.f;
+                for (int c = 0; c < kCols; ++c) acc[c] = mid[c] = 0.f;
+                // the sums so far to shared memory, behind those that are there: earlier k-blocks and shares, in their order
+                auto flush = [&]() {
+#pragma unroll
+                    for (int c = 0; c < kCols; c += 4) {
+                        const uint32_t to = mine + 4u * static_cast<uint32_t>(c);
+                        if (begun) {
+                            float4 s;
+                            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(s.x), "=f"(s.y), "=f"(s.z), "=f"(s.w) : "r"(to) : "memory");
+                            acc[c] = __fadd_rn(s.x, acc[c]); acc[c + 1] = __fadd_rn(s.y, acc[c + 1]); acc[c + 2] = __fadd_rn(s.z, acc[c + 2]); acc[c + 3] = __fadd_rn(s.w, acc[c + 3]);
+                        }
+                        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(acc[c]), "f"(acc[c + 1]), "f"(acc[c + 2]), "f"(acc[c + 3]) : "memory");
+                        acc[c] = acc[c + 1] = acc[c + 2] = acc[c + 3] = 0.f;
+                    }
+                    begun = true;
+                };
                 for (int kt = k0; kt < k1; ++kt) {
                     ok = mbar_wait(done(at), phase, cta_abort, p.err_flag, DEV_ERR_WAIT_ACC_FULL);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tcgen05_fence_after();
                     uint32_t v[kCols];
-                    load(from + kBn * from_acc, v);
+                    load(from + 2 * kBn * from_acc, v);
+#pragma unroll
+                    for (int c = 0; c < kCols; ++c) acc[c] = __fadd_rn(acc[c], __uint_as_float(v[c]));
+                    load(from + 2 * kBn * from_acc + kBn, v);
                     tcgen05_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(ready((at + kMain) % kSpRing));      // the accumulator is the k-block's that comes kMain later
+                    if (lane == 0) mbar_arrive(ready((at + kMain) % kSpRing));      // the accumulators are the k-block's that comes kMain later
                     if (++at == kSpRing) { at = 0; phase ^= 1u; }
                     if (++from_acc == kMain) from_acc = 0;
 #pragma unroll
-                    for (int c = 0; c < kCols; ++c) acc[c] = __fadd_rn(acc[c], __uint_as_float(v[c]));
+                    for (int c = 0; c < kCols; ++c) mid[c] = __fadd_rn(mid[c], __uint_as_float(v[c]));
+                    if (!kSplit && p.shares == 1 && kt % kSpFlush == kSpFlush - 1 && kt + 1 < k1) flush();
                 }
                 if (!ok) break;
                 ok = mbar_wait(s_full(small), small_phase, cta_abort, p.err_flag, DEV_ERR_WAIT_ACC_FULL);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tcgen05_fence_after();
-                uint32_t v[kCols], w[kCols];
-                tmem_ld_columns(from + kSmallCol + kBn * (2 * small + 1u), w);
-                load(from + kSmallCol + kBn * (2 * small), v);
+                {
+                    uint32_t v[kCols];
+                    load(from + kSmallCol + kBn * small, v);
 #pragma unroll
-                for (int c = 0; c < kCols; ++c) {
-                    asm volatile("" : "+r"(w[c]));
-                    if ((__float_as_uint(acc[c]) & 0x7f800000u) != 0x7f800000u) acc[c] = __fadd_rn(acc[c], __fadd_rn(__uint_as_float(v[c]), __uint_as_float(w[c])));
+                    for (int c = 0; c < kCols; ++c) mid[c] = __fadd_rn(mid[c], __uint_as_float(v[c]));
                 }
                 tcgen05_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(s_empty(small));
                 if (++small == kSmall) { small = 0; small_phase ^= 1u; }
+                // (a large sum that is not finite may have gone to shared memory: the small sums are asked, which are then not finite either)
 #pragma unroll
-                for (int c = 0; c < kCols; c += 4) {
-                    const uint32_t to = mine + 4u * static_cast<uint32_t>(c);
-                    if (!kSplit && share > 0) {      // the shares before this one, in their order
-                        float4 s;
-                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(s.x), "=f"(s.y), "=f"(s.z), "=f"(s.w) : "r"(to) : "memory");
-                        acc[c] = __fadd_rn(s.x, acc[c]); acc[c + 1] = __fadd_rn(s.y, acc[c + 1]); acc[c + 2] = __fadd_rn(s.z, acc[c + 2]); acc[c + 3] = __fadd_rn(s.w, acc[c + 3]);
-                    }
-                    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(to), "f"(acc[c]), "f"(acc[c + 1]), "f"(acc[c + 2]), "f"(acc[c + 3]) : "memory");
-                }
+                for (int c = 0; c < kCols; ++c) if ((__float_as_uint(mid[c]) & 0x7f800000u) != 0x7f800000u) acc[c] = __fadd_rn(acc[c], mid[c]);
+                flush();
             }
             if constexpr (!kSplit) {
                 // the sixteen warps decide together: they meet at the tile of sums

@@ -93,10 +93,11 @@ constexpr int kSpThreads = 896;      // warp 0: activations, 1: weights, 2 and 3
 // (an even ring of activations: the two groups of splitting warps take k-blocks in turn, and a stage has to be the same group's every
 // time, or a group could be a whole round of its barrier behind and take an old phase for the one it waits for)
 constexpr uint32_t kSpAStages = 6, kSpBStages = 5;     // rings of activations and weights in shared memory
-constexpr uint32_t kSpSlots = 4, kSpRing = 6;          // split activations in TMEM; barriers of the k-blocks under way
-static_assert(kSpAStages % 2 == 0 && kSpRing % 2 == 0 && kSpSlots % 2 == 0, "a stage and a slot belong to one group of splitting warps");
-// x0 of a split value: six significant bits, the magnitude from which rounding to them gives infinity
-constexpr int kSplitLeadCut = 18;
+constexpr uint32_t kSpSlots = 3, kSpRing = 6;          // split activations in TMEM; barriers of the k-blocks under way
+static_assert(kSpAStages % 2 == 0 && kSpRing % 2 == 0, "a stage belongs to one group of splitting warps");
+constexpr int kSpFlush = 8;          // k-blocks that are added up in registers
+// x0 of a split value: four significant bits, the magnitude from which rounding to them gives infinity
+constexpr int kSplitLeadCut = 20;
 constexpr uint32_t kSplitLeadMax = 0x7f800000u - (1u << (kSplitLeadCut - 1));
 struct ConvSplitParams {
     int m_total, cout, tiles_m, tiles_n;
@@ -115,7 +116,7 @@ struct ConvSplitParams {
 // channels of a tile: up to 64 (what TMEM holds beside three slots of split activations), evenly wide
 constexpr int split_tile_channels(int cout) { return ((cout + (cout + 63) / 64 - 1) / ((cout + 63) / 64) + 15) / 16 * 16; }
 constexpr size_t split_smem_bytes(int bn) {
-    return 1024 + kSpAStages * kUmmaM * 128 + kSpBStages * 3 * bn * 64 + static_cast<size_t>(kUmmaM) * (bn + 4) * 4 + 512;
+    return 1024 + kSpAStages * kUmmaM * 128 + kSpBStages * 4 * bn * 64 + static_cast<size_t>(kUmmaM) * (bn + 4) * 4 + 512;
 }
 constexpr int kSbMaxChannels = 1024;   // capacity of the staged scale / bias tables
 // Activation handled by a dedicated epilogue instantiation (no switch inside the loops); every other activation takes

@@ -81,25 +81,25 @@ float host_round_tf32(float x) {
     return x;
 }
 
-// the three parts of a value, as split_values (conv_split.cuh) takes them
-void host_split_bf16(float x, uint16_t &p0, uint16_t &p1, uint16_t &p2) {
+// the four parts of a value, as split_lead and split_next (conv_split.cuh) take them
+std::array<uint16_t, 4> host_split_bf16(float x) {
     uint32_t u;
     std::memcpy(&u, &x, 4);
     const uint32_t mag = u & 0x7fffffffu;
     uint32_t lead = (u + (1u << (kSplitLeadCut - 1))) & ~((1u << kSplitLeadCut) - 1u);
     if (mag >= kSplitLeadMax) lead = mag > 0x7f800000u ? 0x7fc00000u : u & 0xffff0000u;
-    p0 = static_cast<uint16_t>(lead >> 16); p1 = p2 = 0;
-    if (mag >= 0x7f800000u) return;
-    float l, m;
-    std::memcpy(&l, &lead, 4);
-    const float rest = x - l;
-    std::memcpy(&u, &rest, 4);
-    u = (u + 0x7fffu + (u >> 16 & 1u)) & 0xffff0000u;
-    std::memcpy(&m, &u, 4);
-    p1 = static_cast<uint16_t>(u >> 16);
-    const float last = rest - m;
-    std::memcpy(&u, &last, 4);
-    p2 = static_cast<uint16_t>(u >> 16);
+    std::array<uint16_t, 4> part{static_cast<uint16_t>(lead >> 16), 0, 0, 0};
+    if (mag >= 0x7f800000u) return part;
+    float taken;
+    std::memcpy(&taken, &lead, 4);
+    for (int k = 1; k < 4; ++k) {
+        x -= taken;
+        std::memcpy(&u, &x, 4);
+        u = (u + 0x7fffu + (u >> 16 & 1u)) & 0xffff0000u;
+        std::memcpy(&taken, &u, 4);
+        part[k] = static_cast<uint16_t>(u >> 16);
+    }
+    return part;
 }
 
 // the same algebra as the reference's convBn kernel (src/layers/cuda/MsnhConvolutionalLayerGPU.cu:6-35).
@@ -467,13 +467,14 @@ int build_launches(MsnhB200Plan *pl) {
                         });
                         p.L.weights = ps.dev;
                     } else if (split) {
-                        // three matrices, one behind the other
-                        PackSlot<uint16_t> ps = reserve_pack<uint16_t>(pl, 3 * n);
+                        // four matrices, one behind the other
+                        PackSlot<uint16_t> ps = reserve_pack<uint16_t>(pl, 4 * n);
                         uint16_t *pk = ps.host;
                         if (pk) parallel_rows(cout, static_cast<size_t>(cin_g) * taps, [&](int co) {
                             for (int ci = 0; ci < cin_g; ++ci) for (int t = 0; t < taps; ++t) {
                                 const size_t at = static_cast<size_t>(co) * row_len + tap_at(t) + ci;
-                                host_split_bf16(w[(static_cast<size_t>(co) * cin_g + ci) * taps + t], pk[at], pk[n + at], pk[2 * n + at]);
+                                const std::array<uint16_t, 4> part = host_split_bf16(w[(static_cast<size_t>(co) * cin_g + ci) * taps + t]);
+                                for (int k = 0; k < 4; ++k) pk[k * n + at] = part[k];
                             }
                         });
                         p.L.weights = ps.dev;
@@ -738,7 +739,7 @@ int build_launches(MsnhB200Plan *pl) {
                 const int cb = pl->tensors[b.out_t].s.C;
                 const size_t row_bytes = static_cast<size_t>(a.L.cin_pad) * (split ? 2 : es);
                 const size_t wa = off_of(a.L.weights), wb = off_of(b.L.weights), sa = off_of(a.L.scale), sb = off_of(b.L.scale), ba = off_of(a.L.bias), bb = off_of(b.L.bias);
-                const int parts = split ? 3 : 1;              // (split operands: three matrices, one behind the other)
+                const int parts = split ? 4 : 1;              // (split operands: four matrices, one behind the other)
                 PackSlot<uint8_t> ws = reserve_pack<uint8_t>(pl, parts * (static_cast<size_t>(ca) + cb) * row_bytes);
                 if (ws.host)         // (nullptr: the arena comes from a pack file, which holds the merged copy at this offset)
                     for (int k = 0; k < parts; ++k) {

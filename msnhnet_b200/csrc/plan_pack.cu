@@ -52,7 +52,7 @@ uint64_t checksum64(const uint8_t *p, size_t n, uint64_t seed) {
 uint64_t pack_key(const MsnhB200Plan *pl) {
     uint64_t h = 1469598103934665603ull;
     for (const OpState &o : pl->ops) h = fnv1a(h, &o.d, sizeof(o.d));
-    const int32_t v[10] = {pl->in_c, pl->in_h, pl->in_w, pl->batch, pl->dtype, static_cast<int32_t>(pl->flags & (MSNH_PLAN_NO_FUSION | MSNH_PLAN_NO_TENSOR_CORE | MSNH_PLAN_KEEP_ALL)), 11 /* layout version */,
+    const int32_t v[10] = {pl->in_c, pl->in_h, pl->in_w, pl->batch, pl->dtype, static_cast<int32_t>(pl->flags & (MSNH_PLAN_NO_FUSION | MSNH_PLAN_NO_TENSOR_CORE | MSNH_PLAN_KEEP_ALL)), 12 /* layout version */,
                           pl->ctx->sm_count /* the stored tile shapes were timed on this many SMs */, pl->dbg.no_merge ? 1 : 0, pl->split_fp32 ? 1 : 0};
     return fnv1a(h, v, sizeof(v));
 }

@@ -212,8 +212,8 @@ int configure_conv_split(MsnhB200Plan *pl, Launch &L) {
     else        rc = make_map_im2col(ctx, &L.map_a, MSNH_B200_F32, L.in, L.kh, L.kw, L.sh, L.sw, L.ph, L.pw, L.dh, L.dw, 32, 128, kUmmaM);
     if (rc) return rc;
     const cuuint64_t ktot = static_cast<cuuint64_t>(u.taps) * u.cin_pad;
-    cuuint64_t dims[3] = {ktot, static_cast<cuuint64_t>(cout), 3}, strides[2] = {ktot * 2, ktot * 2 * cout};
-    cuuint32_t box[3] = {32, static_cast<cuuint32_t>(L.sp_bn), 3}, estr[3] = {1, 1, 1};
+    cuuint64_t dims[3] = {ktot, static_cast<cuuint64_t>(cout), 4}, strides[2] = {ktot * 2, ktot * 2 * cout};
+    cuuint32_t box[3] = {32, static_cast<cuuint32_t>(L.sp_bn), 4}, estr[3] = {1, 1, 1};
     const CUresult r = ctx->encode_tiled(&L.map_b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(L.weights), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                          CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(ctx, MSNH_B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d): split weights %llu x %d", (int)r, (unsigned long long)ktot, cout);

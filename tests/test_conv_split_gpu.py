@@ -1,4 +1,4 @@
-"""The fp32 convolution on split operands (two tf32 parts of every fp32 value, three tensor-core products, k-blocks added up in fp32):
+"""The fp32 convolution on split operands (four bf16 parts of every fp32 value, ten tensor-core products, k-blocks added up in fp32):
 edges of its tiles and k-blocks, several tiles a CTA, shares of k on a cluster and in one CTA, values that are not finite."""
 import numpy as np
 import pytest
@@ -71,10 +71,12 @@ def test_split_conv_is_an_fp32_conv(shares, cin, cout, h, w, k, stride, batch, m
     got, desc = conv(x, wt, bias, stride, shares, monkeypatch)
     assert "conv_direct_tf32x3" in desc
     want, size = reference(x, wt, bias, stride, k // 2)
-    # the split leaves 2^-24 of each operand (and of the product left out), a k-block's four accumulations an ulp each, every addition of
-    # k-blocks, shares and bias half an ulp: all of them of sums no larger than `size`
-    blocks = k * k * ((cin + 7) // 8)
-    assert np.all(np.abs(got - want) <= size * 2.0 ** -24 * (3 + 8 + blocks + abs(shares) + 1))
+    # In units of 2^-24, all of sums no larger than `size`: 1 for the products left out; an ulp (2) for each of a k-block's two accumulations of the large
+    # products and a quarter of that for its four of the middle ones, 2^-3 of them (5, the k-blocks' sums being parts of `size`); half an ulp for every addition
+    # of k-blocks (1 each, the middle ones' 1/8), of what goes to shared memory (every eighth), of shares and bias; an ulp for each of the fourteen accumulations
+    # of a k-block's other products, 2^-7 of the sum (1/4 each)
+    blocks = k * k * ((cin + 31) // 32)
+    assert np.all(np.abs(got - want) <= size * 2.0 ** -24 * (1 + 5 + 1.5 * blocks + abs(shares) + 2))
 
 
 @pytest.mark.parametrize("act", ACTS)
@@ -103,6 +105,24 @@ def test_values_that_are_not_finite_go_where_fp32_takes_them(shares, monkeypatch
     assert np.isinf(want).any() and np.isnan(want).any()
     assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
     fine = np.isfinite(want)
+    assert np.all(np.abs(got[fine] - want[fine]) <= 1e-5 * np.maximum(np.abs(want[fine]), 1))
+
+
+@pytest.mark.parametrize("shares", [1, 2])
+def test_nan_beside_an_infinity_and_the_largest_numbers(shares, monkeypatch):
+    """The NaN of all ones, which CUDA's own operations give, in the window of an infinity; values that six, four or eight bits round up to infinity."""
+    x, wt, bias = tensors(40, 48, 12, 12, 3, 1)
+    x[0, 3, 2, 2] = np.inf
+    x[0, 7, 3, 3] = np.array([0x7fffffff], np.uint32).view(np.float32)[0]
+    x[0, 8, 9, 3] = np.array([0xff800001], np.uint32).view(np.float32)[0]           # (a NaN whose low bits alone tell it from an infinity)
+    x[0, 5, 9, 9] = np.finfo(np.float32).max
+    wt[:, 5] *= 1e-2                                                             # (products of the largest number that fp32 holds, alone in their sums)
+    wt[3, 7, 1, 1] = np.inf
+    want, _ = conv(x, wt, bias, 1, None, monkeypatch)
+    got, _ = conv(x, wt, bias, 1, shares, monkeypatch)
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want)) and np.array_equal(np.isneginf(got), np.isneginf(want))
+    fine = np.isfinite(want)
+    assert np.abs(want[fine]).max() > 1e35
     assert np.all(np.abs(got[fine] - want[fine]) <= 1e-5 * np.maximum(np.abs(want[fine]), 1))
 
 

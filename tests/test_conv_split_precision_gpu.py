@@ -72,7 +72,12 @@ def test_no_further_from_the_sums_than_fp32_fmas(kind, cin, k, monkeypatch):
     for shares in (1, 3):
         got = np.linalg.norm(conv(x, wt, shares, monkeypatch) - want)
         # 65536 results: the norms of two errors of the same distribution differ by well under 2 %
-        assert got <= plain * 1.02, f"{shares} shares: {got / np.linalg.norm(want):.2e}, FMAs {plain / np.linalg.norm(want):.2e}"
+        bound = plain * 1.02
+        if kind == "wide":
+            # Where one of a few products outweighs the rest fp32 FMAs round once or twice. A tensor core cuts off once (a remainder of up to an ulp) and
+            # the k-blocks' sum is rounded (half an ulp): sqrt(1/3 + 1/12) ulp, 2^-23 * 0.72 of a value on average over its binade
+            bound = max(bound, np.sqrt(5 / 12) * 0.72 * 2.0 ** -23 * np.linalg.norm(want))
+        assert got <= bound, f"{shares} shares: {got / np.linalg.norm(want):.2e}, FMAs {plain / np.linalg.norm(want):.2e}"
 
 
 @pytest.mark.parametrize("cin,k", LAYERS)
