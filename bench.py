@@ -321,9 +321,9 @@ def layer_table(desc, per, pk, title):
         if t <= 0 or (fl == 0 and by == 0):
             continue
         ai = fl / by if by else 0.0
-        if f[1] == "conv_direct_tf32x3":       # three tf32 products a product, tf32 at half the 16-bit rate
-            ach, roof = fl / (t * 1e-3) / 1e12, "tensor, 3 x tf32"
-            frac, ach_s = ach / (pk["tflops"] / 6), f"{ach:.1f} TFLOP/s"
+        if f[1] == "conv_split":       # ten bf16 products a product
+            ach, roof = fl / (t * 1e-3) / 1e12, "tensor, 10 x bf16"
+            frac, ach_s = ach / (pk["tflops"] / 10), f"{ach:.1f} TFLOP/s"
         elif "fp32 arithmetic" in line and ai >= FP32_FMA_TFLOPS * 1e3 / pk["hbm_gbs"]:
             ach = fl / (t * 1e-3) / 1e12
             roof, frac, ach_s = "fp32 FMA", ach / FP32_FMA_TFLOPS, f"{ach:.1f} TFLOP/s"

@@ -148,7 +148,7 @@ enum { MSNH_PLAN_NO_GRAPH   = 1u,   /* launch kernels directly instead of replay
        MSNH_PLAN_NO_TENSOR_CORE = 8u,/* run convs on the CUDA-core kernel (device cross-check)     */
        MSNH_PLAN_TRACE      = 16u,  /* tensor-core convs record per-CTA clock stamps (read_trace)  */
        /* fp32 plans of detection nets (plans with a MSNH_OP_YOLO op) run their convs in fp32 arithmetic by default - on the
-        * tensor cores, every operand the sum of four bf16 parts (sums beyond 0.9 of the largest fp32 number may come out
+        * tensor cores, every operand the sum of four bf16 parts (sums beyond 0.88 of the largest fp32 number may come out
         * infinite); with MSNH_PLAN_NO_TENSOR_CORE on the CUDA cores: the
         * reference's GPU path is fp32 Sgemm (src/layers/MsnhConvolutionalLayer.cpp:1026-1160) and exp()-decoded box sizes
         * do not hold 1e-3 through tf32's 10-bit mantissa. This flag asks for plain tf32 tensor-core convs all the same

@@ -20,7 +20,7 @@ namespace msnh {
 const char *const kLaunchNames[] = {"input_nchw_to_nhwc", "conv_umma", "conv_direct", "dwconv", "scale_bias_act",
                                     "add_n", "binary", "maxpool", "avgpool", "upsample", "slice", "pad", "softmax",
                                     "yolo_decode", "collect_zero", "yolo_collect", "input_nchw_to_patches",
-                                    "yolo_decode_collect", "focus_slices", "bilinear", "deconv_col2im", "clip", "remap", "reduce", "prelu", "maxpool_depth", "conv_direct_tf32x3", "input_nchw_to_row_patches"};
+                                    "yolo_decode_collect", "focus_slices", "bilinear", "deconv_col2im", "clip", "remap", "reduce", "prelu", "maxpool_depth", "conv_split", "input_nchw_to_row_patches"};
 
 int fail(MsnhB200Ctx *ctx, int code, const char *fmt, ...) {
     char buf[1024];

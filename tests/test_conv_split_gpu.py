@@ -69,7 +69,7 @@ def reference(x, wt, bias, stride, pad):
 def test_split_conv_is_an_fp32_conv(shares, cin, cout, h, w, k, stride, batch, monkeypatch):
     x, wt, bias = tensors(cin, cout, h, w, k, batch)
     got, desc = conv(x, wt, bias, stride, shares, monkeypatch)
-    assert "conv_direct_tf32x3" in desc
+    assert "conv_split " in desc
     want, size = reference(x, wt, bias, stride, k // 2)
     # In units of 2^-24, all of sums no larger than `size`: 1 for the products left out; an ulp (2) for each of a k-block's two accumulations of the large
     # products and a quarter of that for its four of the middle ones, 2^-3 of them (5, the k-blocks' sums being parts of `size`); half an ulp for every addition

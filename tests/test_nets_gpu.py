@@ -18,7 +18,7 @@ SMALL = [("resnet18", 224), ("yolov3_tiny", 416), ("mobilenetv2", 224), ("yolov4
 # fp32 storage with tf32 tensor-core products keeps 10 mantissa bits per operand, like fp16; its
 # error on inner layers and on exp()-decoded box sizes is therefore of fp16's order, not 1e-3.
 # The 1e-3 bar is held on classifier logits with tf32 and everywhere with the exact fp32 path.
-TOL_LAYER = {("f32", "exact"): 2e-5, ("f32", "tc"): 8e-3, ("f16", "tc"): H.TOL_F16}
+TOL_LAYER = {("f32", "exact"): 2e-5, ("f32", "split"): 2e-5, ("f32", "tc"): 8e-3, ("f16", "tc"): H.TOL_F16}
 # (fp32 plans of detection nets run fp32 arithmetic unless MSNH_PLAN_TF32_DETECT asks for tf32: the "tc" mode sets it)
 
 
@@ -32,15 +32,47 @@ def oracle_run(name, size, batch):
     return text, blob, imgs, net, [net.forward(imgs[i]) for i in range(batch)]
 
 
+def convs_of(description):
+    """The kernels that a plan runs its dense convs on."""
+    return {line.split()[1] for line in description.splitlines() if line.split()[1:2] and line.split()[1].startswith("conv_")}
+
+
 @pytest.mark.parametrize("name,size", SMALL)
 @pytest.mark.parametrize("mode", [("f32", "exact"), ("f32", "tc"), ("f16", "tc")])
 def test_every_layer_matches_the_oracle(name, size, mode):
+    check_every_layer(name, size, mode)
+
+
+@pytest.mark.parametrize("name,size", [(n, s) for n, s in SMALL if n.startswith("yolo")])
+def test_every_layer_of_a_default_fp32_detector_matches_the_oracle(name, size):
+    """fp32 detection nets without a flag that picks the arithmetic: split operands on the tensor cores, held to what the CUDA-core form is held to."""
+    check_every_layer(name, size, ("f32", "split"))
+
+
+@pytest.mark.parametrize("name,size", [("yolov4", 160), ("yolov5m", 160), ("yolov5m_silu", 160), ("yolov5m", 256)])
+def test_default_fp32_detection_plans_match_the_oracle(name, size):
+    """The plan a user gets - fused residuals, merged 1x1 convs, concat slices, SPP, focus, CUDA graph - end to end."""
     batch = 2
     text, blob, imgs, onet, ores = oracle_run(name, size, batch)
-    flags = _ffi.PLAN_KEEP_ALL | (_ffi.PLAN_NO_TENSOR_CORE if mode[1] == "exact" else _ffi.PLAN_TF32_DETECT)
+    g = H.GpuNet(text, blob, fp16=False, batch=batch, flags=0)
+    try:
+        result = g.yolo(imgs)
+        assert convs_of(g.plan_describe()) == {"conv_split"} and "with the 1x1 conv of op" in g.plan_describe()
+        for i in range(batch):
+            check_detections(g, i, batch, ores[i], result[i], exact=True)
+    finally:
+        g.close()
+
+
+def check_every_layer(name, size, mode):
+    batch = 2
+    text, blob, imgs, onet, ores = oracle_run(name, size, batch)
+    flags = _ffi.PLAN_KEEP_ALL | {"exact": _ffi.PLAN_NO_TENSOR_CORE, "tc": _ffi.PLAN_TF32_DETECT, "split": 0}[mode[1]]
     g = H.GpuNet(text, blob, fp16=mode[0] == "f16", batch=batch, flags=flags)
     try:
         result = g.yolo(imgs) if g.is_yolo else g.classify(imgs)
+        if mode[1] != "tc" and g.is_yolo:
+            assert convs_of(g.plan_describe()) == {"conv_direct" if mode[1] == "exact" else "conv_split"}
         tol = TOL_LAYER[mode]
         for li in range(g.n_layers):
             if ores[0]["layers"][li] is None:
@@ -51,7 +83,7 @@ def test_every_layer_matches_the_oracle(name, size, mode):
             assert H.rel_err(got, ref) < tol, f"layer {li} ({onet.layers[li]['kind']})"
         if g.is_yolo:
             for i in range(batch):
-                check_detections(g, i, batch, ores[i], result[i], exact=mode[1] == "exact")
+                check_detections(g, i, batch, ores[i], result[i], exact=mode[1] != "tc")
         else:
             ref = np.stack([ores[i]["out"] for i in range(batch)])
             # layer_zoo and fcns are no classifiers: layer_zoo's ten outputs sit behind 14 tf32 contractions, a clip and
@@ -104,7 +136,7 @@ def test_fp32_detection_net_meets_1e_3_with_the_default_plan(batch):
     try:
         boxes = g.yolo(imgs)
         cand = g.candidates(batch, 60000)
-        assert "conv_direct" in g.plan_describe() and "conv_umma" not in g.plan_describe()
+        assert convs_of(g.plan_describe()) == {"conv_split"}
         for i in range(batch):
             ocand, oboxes = ores[i]["candidates"], ores[i]["boxes"]
             assert np.array_equal(cand[i][:, 7], ocand[:, 7])                      # the same cells
