@@ -445,8 +445,10 @@ int build_launches(MsnhB200Plan *pl) {
                         p.L.weights = ps.dev;
                     }
                 } else {
-                    // what an im2col tensor map can walk
-                    const bool tma_walks = groups == 1 && p.L.sh <= 8 && p.L.sw <= 8 && p.L.ph < 128 && p.L.pw < 128 && kh * p.L.dh < 256 && kw * p.L.dw < 256;
+                    // what an im2col tensor map can walk: the offsets of the taps, and the corners of its box, which lie -pad from the first pixel
+                    // and pad - dilation * (k - 1) from the last, in [-128, 127]
+                    const bool tma_walks = groups == 1 && p.L.sh <= 8 && p.L.sw <= 8 && p.L.ph < 128 && p.L.pw < 128 && kh * p.L.dh < 256 && kw * p.L.dw < 256 &&
+                                           p.L.ph - p.L.dh * (kh - 1) >= -128 && p.L.pw - p.L.dw * (kw - 1) >= -128;
                     // [Cout][Cin/g][kh][kw] -> [Cout][tap][cin_pad], zero in the pad channels
                     // (patch mode: one "tap" of patch_k values ordered tap-major, like the patch matrix)
                     // (row patches: one "tap" per filter row, of kw x cin values)

@@ -194,3 +194,32 @@ def test_a_plan_without_tensor_cores_stays_without(monkeypatch):
     finally:
         plan.close()
         ctx.close()
+
+
+# a dilated filter, and a fully connected layer, that just fits the box of an im2col tensor map and that just does not
+@pytest.mark.parametrize("k,dil,h,w,fits", [(3, 64, 131, 130, True), (3, 65, 133, 134, False), (3, 80, 170, 163, False), (0, 1, 129, 3, True), (0, 1, 130, 3, False), (0, 1, 2, 200, False)])
+@pytest.mark.parametrize("flags", [0, ffi.PLAN_NO_TENSOR_CORE])
+def test_layers_that_an_im2col_map_cannot_walk_run_on_the_cuda_cores(flags, k, dil, h, w, fits, monkeypatch):
+    if not flags:
+        monkeypatch.setenv("MSNH_B200_CONV_SPLIT", "1")
+    rng = np.random.default_rng(4)
+    x = rng.standard_normal((2, 8, h, w), dtype=np.float32)
+    conv_op = dict(filters=20, k_h=k, k_w=k, dil_h=dil, dil_w=dil) if k else dict(filters=20)
+    wt = (rng.standard_normal((20, 8, k or h, k or w)) / 50).astype(np.float32)
+    ctx = ffi.Context(0)
+    plan = ffi.Plan(ctx, [ffi.make_op(ffi.OP_CONV if k else ffi.OP_CONNECTED, [ffi.INPUT], is_output=1, **conv_op)], (8, h, w), 2, ffi.F32, flags)
+    try:
+        plan.set_weights(0, ffi.W_WEIGHTS, wt)
+        plan.finalize()
+        launch = [line for line in plan.describe().splitlines() if " op=0 " in line][-1]
+        assert ("conv_split " in launch) == (fits and not flags)
+        plan.run(x)
+        got = plan.read_output(0, 2)
+    finally:
+        plan.close()
+        ctx.close()
+    X, W = torch.from_numpy(x).double(), torch.from_numpy(wt).double()
+    want = torch.nn.functional.conv2d(X, W, dilation=dil).numpy()
+    size = torch.nn.functional.conv2d(X.abs(), W.abs(), dilation=dil).numpy()
+    terms = 8 * wt.shape[2] * wt.shape[3]
+    assert np.all(np.abs(got - want) <= size * 2.0 ** -24 * (terms + 8))         # (a chain of as many roundings of sums no larger than `size`)
