@@ -138,7 +138,7 @@ int build_launches(MsnhB200Plan *pl) {
     const bool fresh = !pl->pack_loaded;
     if (fresh) {
         size_t guess = 0;
-        for (const OpState &o : pl->ops) guess += o.wcount[MSNH_W_WEIGHTS] * static_cast<size_t>(esize(pl->dtype));
+        for (const OpState &o : pl->ops) guess += o.wcount[MSNH_W_WEIGHTS] * static_cast<size_t>(pl->split_fp32 ? 8 : esize(pl->dtype));      // (four parts of 16 bits)
         pl->pack_host.reserve(guess + guess / 4 + (1u << 20));
     }
     for (int i = 0; i < n_ops; ++i) {
