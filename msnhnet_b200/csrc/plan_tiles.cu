@@ -185,7 +185,8 @@ int configure_conv_split(MsnhB200Plan *pl, Launch &L) {
     // The number of shares decides the order of a layer's sums, so it comes from the layer alone, by the least product of the costs of
     // one (twice), four and sixteen images; who sums them does not. A forward in us with one image counted once / twice / alone:
     // YOLOv5m-352, one image 834 / 795 / 741, three 1174 / 1209 / 1419; YOLOv4-416, one 1590 / 1511 / 1469; YOLOv3-tiny-416, one 212 / 205 / 203,
-    // four 474 / 490 / 510, sixteen 1470 / 1488 / 1502.
+    // four 474 / 490 / 510, sixteen 1470 / 1488 / 1502. (Those and the model's costs are of an earlier form of the kernel whose k-blocks took 0.3 us in a
+    // forward; four bf16 parts take 1.4 times that, and a share about the same.)
     const long long m_image = static_cast<long long>(L.out.H) * L.out.W;
     u.shares = 1;
     double best = 0;
